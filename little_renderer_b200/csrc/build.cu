@@ -377,12 +377,26 @@ __global__ void __launch_bounds__(256) lbvh_kernel(const K *__restrict__ codes, 
 }
 
 // ---- PLOC -------------------------------------------------------------------------------------
+// A round is one pass over tiles of the cluster list: every cluster's nearest within +-16, mutual
+// pairs, the tiles' keep / merge counts summed over the tiles before, merges and compaction.
+// The tile's clusters sit in shared memory by component (their lows, highs and ids in arrays of
+// their own), so that a thread reads 4 neighbours' components with one 16-byte load and its 4
+// clusters are tested against them from registers: 32 distances a cluster, no bounds in the loop.
+// The counts of the tiles before come from a look-back by the whole block, 512 statuses at once (one
+// thread reading them one by one took a round most of its time: 871k surface triangles, the whole build: 2.93 ms
+// against 0.67 ms). PER: clusters a thread. 4 while the list fills the grid; with fewer clusters 1, so
+// that a round keeps more SMs busy and each thread's chain is a quarter as long; the last 256
+// clusters are merged by one block without leaving shared memory.
 constexpr int PL_THREADS = 256;
-constexpr int PL_PER = 4;                          // clusters per thread
-constexpr int PL_TILE = PL_THREADS * PL_PER;       // 1024 clusters per tile
 constexpr int PL_R = 16;                           // the search radius (trace_ploc.wgsl R)
-constexpr int PL_WIN = PL_TILE + 4 * PL_R;         // the tile's clusters with their neighbours' neighbours
-constexpr int PL_NN = PL_TILE + 2 * PL_R;          // the clusters whose nearest the tile needs
+template <int PER> struct PlTile {
+    static constexpr int NN = PL_THREADS * PER;    // the clusters whose nearest the tile needs
+    static constexpr int TILE = NN - 2 * PL_R;     // the clusters it keeps or merges
+    static constexpr int WIN = TILE + 4 * PL_R;    // the clusters it reads: with their neighbours' neighbours
+};
+constexpr int PL_TILE = PlTile<4>::TILE, PL_TILE1 = PlTile<1>::TILE;
+constexpr int PL_MAX_GRID = 2048;                  // (statuses kept for the rounds of PL_TILE1 tiles)
+constexpr int PL_LAST = PL_THREADS;                // the last clusters: one block, in shared memory
 
 // a cluster: its box and id (internal k 0..n-2, leaf j at n - 1 + j), laid out as a Node
 struct __align__(16) Cl {
@@ -400,18 +414,28 @@ struct PlocState {
 };
 
 struct PlocShared {
-    Cl win[PL_WIN];
-    uint32_t nn[PL_NN];
+    float c[6][PlTile<4>::WIN];      // lo.xyz, hi.xyz of the window's clusters
+    uint32_t id[PlTile<4>::WIN];
+    uint32_t nn[PlTile<4>::NN];      // the nearest's position in the list
     uint32_t scan[PL_THREADS / 32];
-    uint64_t prefix;         // (keep, merge) of the tiles before this one
+    unsigned long long sums[PL_THREADS / 32];
+    int found[PL_THREADS / 32];
     uint32_t keep_total;
 };
 
-// area (trace_ploc.wgsl:18) of the two clusters' joined box, the reference's order of operations
-__device__ __forceinline__ float joined_area(const Cl &a, const Cl &b) {
-    float ex = fsub(wmax(a.hi[0], b.hi[0]), wmin(a.lo[0], b.lo[0]));
-    float ey = fsub(wmax(a.hi[1], b.hi[1]), wmin(a.lo[1], b.lo[1]));
-    float ez = fsub(wmax(a.hi[2], b.hi[2]), wmin(a.lo[2], b.lo[2]));
+// area (trace_ploc.wgsl:18) of the two boxes' joined box, the reference's order of operations
+__device__ __forceinline__ float joined_area(const float *a, const float *b) {
+    float ex = fsub(wmax(a[3], b[3]), wmin(a[0], b[0]));
+    float ey = fsub(wmax(a[4], b[4]), wmin(a[1], b[1]));
+    float ez = fsub(wmax(a[5], b[5]), wmin(a[2], b[2]));
+    return fadd(fadd(fmul(ex, ey), fmul(ey, ez)), fmul(ez, ex));
+}
+// the same for boxes without a NaN, where the hardware's minimum and maximum give what wmin / wmax
+// give up to the sign of a zero, which no comparison of areas sees
+__device__ __forceinline__ float joined_area_fin(const float *a, const float *b) {
+    float ex = fsub(fmaxf(a[3], b[3]), fminf(a[0], b[0]));
+    float ey = fsub(fmaxf(a[4], b[4]), fminf(a[1], b[1]));
+    float ez = fsub(fmaxf(a[5], b[5]), fminf(a[2], b[2]));
     return fadd(fadd(fmul(ex, ey), fmul(ey, ez)), fmul(ez, ex));
 }
 // nearer (trace_ploc.wgsl:60-66)
@@ -422,11 +446,11 @@ __device__ __forceinline__ bool nearer(float d, uint32_t i, uint32_t j, float bd
     return mn < bmn || (mn == bmn && max(i, j) < max(i, bj));
 }
 
-__device__ __forceinline__ void final_node(const Cl &c, uint32_t n, uint32_t node0, uint32_t ref0, Node *out) {
-    uint32_t x = c.id, a, b;
+__device__ __forceinline__ void final_node(const float *c, uint32_t x, uint32_t n, uint32_t node0, uint32_t ref0, Node *out) {
+    uint32_t a, b;
     if (x < n - 1) { a = node0 + 1 + 2 * x; b = node0 + 2 + 2 * x; }
     else { a = ref0 + x - (n - 1); b = LEAF_BIT | 1u; }
-    store_node(out, c.lo[0], c.lo[1], c.lo[2], a, c.hi[0], c.hi[1], c.hi[2], b);
+    store_node(out, c[0], c[1], c[2], a, c[3], c[4], c[5], b);
 }
 
 __device__ __forceinline__ uint64_t ld_volatile64(const uint64_t *p) { return *(const volatile uint64_t *)p; }
@@ -435,15 +459,16 @@ __device__ __forceinline__ void st_volatile64(uint64_t *p, uint64_t v) { *(volat
 constexpr uint64_t PF_AGG = 1ull << 62, PF_PRE = 2ull << 62, PF_MASK = 3ull << 62;
 __device__ __forceinline__ uint64_t pack_km(uint64_t keep, uint64_t merge) { return (keep << 31) | merge; }
 
-// A grid barrier for a cooperative launch (all blocks resident), bounded: after SPIN_LIMIT polls it
-// flags ST_TIMEOUT_BARRIER and lets the block go on (the result is then wrong, and said to be).
-__device__ void grid_barrier(PlocState *st, uint32_t *err) {
+// A grid barrier for a cooperative launch (all blocks resident) over its first `blocks` blocks,
+// bounded: after SPIN_LIMIT polls it flags ST_TIMEOUT_BARRIER and lets the block go on (the result is
+// then wrong, and said to be).
+__device__ void grid_barrier(PlocState *st, uint32_t blocks, uint32_t *err) {
     __syncthreads();
     if (threadIdx.x == 0) {
         volatile uint32_t *gen = &st->bar_gen;
         uint32_t g = *gen;
         __threadfence();
-        if (atomicAdd(&st->bar_count, 1u) == gridDim.x - 1) {
+        if (atomicAdd(&st->bar_count, 1u) == blocks - 1) {
             atomicExch(&st->bar_count, 0u);
             __threadfence();
             atomicAdd(&st->bar_gen, 1u);
@@ -451,7 +476,7 @@ __device__ void grid_barrier(PlocState *st, uint32_t *err) {
             uint32_t spins = 0;
             while (*gen == g) {
                 if (++spins > SPIN_LIMIT) { atomicOr(err, ST_TIMEOUT_BARRIER); break; }
-                __nanosleep(64);
+                __nanosleep(32);
             }
         }
         __threadfence();
@@ -459,51 +484,176 @@ __device__ void grid_barrier(PlocState *st, uint32_t *err) {
     __syncthreads();
 }
 
-// One tile of one round: nearest, keep/merge, prefix (look-back when lookback), merges, compaction.
-// Returns (to thread 0's caller through S.keep_total) the clusters the tile keeps.
-__device__ void ploc_tile(PlocShared &S, const Cl *__restrict__ Lp, Cl *__restrict__ Lq, uint32_t nc, uint32_t tile,
-                          uint32_t ntiles, uint32_t n, uint32_t node0, uint32_t ref0, Node *nodes, uint64_t *stat,
-                          bool lookback, PlocState *st, uint32_t *err) {
-    const int tid = threadIdx.x;
-    const int64_t base = (int64_t)tile * PL_TILE;
-    const int64_t w0 = base - 2 * PL_R;                          // the window's first position
-    // the window: clusters w0 .. w0 + PL_WIN - 1 that exist
-    for (int i = tid; i < PL_WIN; i += PL_THREADS) {
-        int64_t g = w0 + i;
-        if (g >= 0 && g < (int64_t)nc) {
-            const float4 *src = reinterpret_cast<const float4 *>(&Lp[g]);
-            float4 *dst = reinterpret_cast<float4 *>(&S.win[i]);
-            dst[0] = __ldcg(src);
-            dst[1] = __ldcg(src + 1);
-        }
+// window slot i: the cluster at list position p, or far away where there is none (farther than any
+// cluster the fast search takes: below, PL_FAR)
+constexpr float PL_FAR = 1e18f;
+__device__ __forceinline__ bool ploc_load(PlocShared &S, int i, const Cl *__restrict__ L, int64_t p, uint32_t nc) {
+    float4 a = make_float4(1e19f, 1e19f, 1e19f, 0.0f), b = a;
+    bool plain = true;
+    if (p >= 0 && p < (int64_t)nc) {
+        const float4 *src = reinterpret_cast<const float4 *>(&L[p]);
+        a = __ldcg(src);
+        b = __ldcg(src + 1);
+        // (a NaN fails the comparison)
+        plain = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z)) <= PL_FAR &&
+                fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fabsf(b.z)) <= PL_FAR && a.x == a.x && a.y == a.y && a.z == a.z &&
+                b.x == b.x && b.y == b.y && b.z == b.z;
     }
-    __syncthreads();
-    // nearest of the clusters base - R .. base + TILE + R
-    for (int i = tid; i < PL_NN; i += PL_THREADS) {
-        int64_t p = base - PL_R + i;
+    S.c[0][i] = a.x; S.c[1][i] = a.y; S.c[2][i] = a.z;
+    S.c[3][i] = b.x; S.c[4][i] = b.y; S.c[5][i] = b.z;
+    S.id[i] = __float_as_uint(a.w);
+    return plain;
+}
+__device__ __forceinline__ void ploc_get(const PlocShared &S, int i, float *c) {
+#pragma unroll
+    for (int q = 0; q < 6; q++) c[q] = S.c[q][i];
+}
+
+// nearest of window slots PL_R + tid * PER + k (list positions p0 + tid * PER + k) into S.nn. The slots
+// are tested in ascending order, so that the first of equal distances wins, as nearer's rule has
+// it (the lower pair: of two neighbours of i the one before).
+template <int PER>
+__device__ __forceinline__ void ploc_nearest(PlocShared &S, int64_t p0, uint32_t nc, bool plain) {
+    const int at = threadIdx.x * PER;                // (the first neighbour's slot)
+    if (plain) {
+        float c[PER][6], bd[PER];
+        int bj[PER];
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            ploc_get(S, PL_R + at + k, c[k]);
+            bd[k] = __int_as_float(0x7f800000);
+            bj[k] = 0;
+        }
+        if constexpr (PER == 4) {
+#pragma unroll
+            for (int m = 0; m < 9; m++) {
+                float4 v[6];
+#pragma unroll
+                for (int q = 0; q < 6; q++) v[q] = *reinterpret_cast<const float4 *>(&S.c[q][at + 4 * m]);
+#pragma unroll
+                for (int jj = 0; jj < 4; jj++) {
+                    float o[6];
+#pragma unroll
+                    for (int q = 0; q < 6; q++) o[q] = jj == 0 ? v[q].x : jj == 1 ? v[q].y : jj == 2 ? v[q].z : v[q].w;
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const int off = 4 * m + jj - (PL_R + k);
+                        if (off == 0 || off < -PL_R || off > PL_R) continue;
+                        const float d = joined_area_fin(c[k], o);
+                        if (d < bd[k]) { bd[k] = d; bj[k] = 4 * m + jj; }
+                    }
+                }
+            }
+        } else {
+#pragma unroll 8
+            for (int m = 0; m <= 2 * PL_R; m++) {
+                if (m == PL_R) continue;
+                float o[6];
+                ploc_get(S, at + m, o);
+                const float d = joined_area_fin(c[0], o);
+                if (d < bd[0]) { bd[0] = d; bj[0] = m; }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < PER; k++) S.nn[at + k] = (uint32_t)(p0 - PL_R + at + bj[k]);
+        return;
+    }
+    // (boxes with a NaN, an infinity or beyond 1e18: the reference's rule as it is written)
+    for (int k = 0; k < PER; k++) {
+        const int64_t p = p0 + at + k;
         if (p < 0 || p >= (int64_t)nc) continue;
         const uint32_t pi = (uint32_t)p;
-        const uint32_t j0 = pi > PL_R ? pi - PL_R : 0u;
-        const uint32_t j1 = min(pi + PL_R, nc - 1);
-        const Cl &c = S.win[p - w0];
-        float bd = 0.0f;
+        const uint32_t j0 = pi > PL_R ? pi - PL_R : 0u, j1 = min(pi + PL_R, nc - 1);
+        float c[6], o[6], bd = 0.0f;
+        ploc_get(S, PL_R + at + k, c);
         uint32_t bj = 0xffffffffu;
         for (uint32_t j = j0; j <= j1; j++) {
             if (j == pi) continue;
-            float d = joined_area(c, S.win[(int64_t)j - w0]);
+            ploc_get(S, (int)((int64_t)j - (p0 - PL_R)), o);
+            const float d = joined_area(c, o);
             if (nearer(d, pi, j, bd, bj)) { bd = d; bj = j; }
         }
-        S.nn[i] = bj;
+        S.nn[at + k] = bj;
     }
+}
+
+// the clusters kept and merged by the tiles before `tile` (pack_km), from their statuses: 512 at once,
+// nearest first, up to the first inclusive prefix. Called by the whole block; every thread gets it.
+__device__ __forceinline__ uint64_t ploc_lookback(PlocShared &S, const uint64_t *stat, uint32_t tile, uint32_t *err) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    uint64_t total = 0;
+    for (int64_t t = (int64_t)tile - 1; t >= 0; t -= 2 * PL_THREADS) {
+        uint64_t s[2];
+        int pre = 2 * PL_THREADS;                    // the nearest prefix's place among the 512
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int64_t i = t - 2 * tid - h;
+            s[h] = 0;
+            if (i < 0) continue;
+            s[h] = ld_volatile64(&stat[i]);
+            uint32_t spins = 0;
+            while ((s[h] & PF_MASK) == 0) {
+                if (++spins > SPIN_LIMIT) { atomicOr(err, ST_TIMEOUT_PLOC); break; }
+                __nanosleep(32);
+                s[h] = ld_volatile64(&stat[i]);
+            }
+            if ((s[h] & PF_MASK) != PF_AGG) pre = min(pre, 2 * tid + h);
+        }
+        pre = __reduce_min_sync(0xffffffffu, pre);
+        if (lane == 0) S.found[w] = pre;
+        __syncthreads();
+        for (int ww = 0; ww < PL_THREADS / 32; ww++) pre = min(pre, S.found[ww]);
+        uint64_t v = 0;
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            if (2 * tid + h <= pre) v += s[h] & ~PF_MASK;
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) S.sums[w] = v;
+        __syncthreads();
+        for (int ww = 0; ww < PL_THREADS / 32; ww++) total += S.sums[ww];
+        __syncthreads();                             // (found and sums are written again)
+        if (pre < 2 * PL_THREADS) break;
+    }
+    return total;
+}
+
+// merge number m (of nc clusters): its node's id, and its two clusters' nodes written
+__device__ __forceinline__ uint32_t ploc_merge(const PlocShared &S, int i, int j, uint32_t nc, uint32_t m, uint32_t n,
+                                               uint32_t node0, uint32_t ref0, Node *nodes, float *out) {
+    const uint32_t kid = nc - 2 - m;                 // (n - 2) - (merges before it)
+    float c[6], d[6];
+    ploc_get(S, i, c);
+    ploc_get(S, j, d);
+#pragma unroll
+    for (int q = 0; q < 3; q++) { out[q] = wmin(c[q], d[q]); out[3 + q] = wmax(c[3 + q], d[3 + q]); }
+    final_node(c, S.id[i], n, node0, ref0, &nodes[1 + 2 * (size_t)kid]);
+    final_node(d, S.id[j], n, node0, ref0, &nodes[2 + 2 * (size_t)kid]);
+    if (kid == 0) store_node(&nodes[0], out[0], out[1], out[2], node0 + 1, out[3], out[4], out[5], node0 + 2);
+    return kid;
+}
+
+// One tile of one round: nearest, keep/merge, the tiles before it, merges, compaction.
+template <int PER>
+__device__ void ploc_tile(PlocShared &S, const Cl *__restrict__ Lp, Cl *__restrict__ Lq, uint32_t nc, uint32_t tile,
+                          uint32_t ntiles, uint32_t n, uint32_t node0, uint32_t ref0, Node *nodes, uint64_t *stat,
+                          PlocState *st, uint32_t *err) {
+    using T = PlTile<PER>;
+    const int tid = threadIdx.x;
+    const int64_t base = (int64_t)tile * T::TILE;
+    const int64_t w0 = base - 2 * PL_R;                          // the window's first position
+    bool plain = true;
+    for (int i = tid; i < T::WIN; i += PL_THREADS) plain = ploc_load(S, i, Lp, w0 + i, nc) && plain;
+    plain = __syncthreads_and(plain);
+    ploc_nearest<PER>(S, base - PL_R, nc, plain);
     __syncthreads();
     // keep / merge of this thread's clusters base + tid * PER + k
     uint32_t keepm = 0, mergem = 0;
 #pragma unroll
-    for (int k = 0; k < PL_PER; k++) {
-        int64_t i = base + tid * PL_PER + k;
-        if (i >= (int64_t)nc) continue;
-        uint32_t j = S.nn[i - (base - PL_R)];
-        bool mu = j < nc && S.nn[(int64_t)j - (base - PL_R)] == (uint32_t)i;
+    for (int k = 0; k < PER; k++) {
+        const int64_t i = base + tid * PER + k;
+        if (tid * PER + k >= T::TILE || i >= (int64_t)nc) continue;
+        const uint32_t j = S.nn[i - (base - PL_R)];
+        const bool mu = j < nc && S.nn[(int64_t)j - (base - PL_R)] == (uint32_t)i;
         if (!(mu && (uint32_t)i > j)) keepm |= 1u << k;
         if (mu && (uint32_t)i < j) mergem |= 1u << k;
     }
@@ -511,65 +661,109 @@ __device__ void ploc_tile(PlocShared &S, const Cl *__restrict__ Lp, Cl *__restri
     const uint32_t packed = __popc(keepm) | (__popc(mergem) << 16);
     const uint32_t excl = block_excl_scan<PL_THREADS>(packed, S.scan, tot);
     const uint32_t tile_keep = tot & 0xffffu, tile_merge = tot >> 16;
+    if (tid == 0) st_volatile64(&stat[tile], (tile ? PF_AGG : PF_PRE) | pack_km(tile_keep, tile_merge));
+    const uint64_t pre = ploc_lookback(S, stat, tile, err);
+    const uint32_t keep0 = (uint32_t)((pre >> 31) & 0x7fffffffull), merge0 = (uint32_t)(pre & 0x7fffffffull);
     if (tid == 0) {
-        uint64_t pre = 0;
-        if (lookback) {
-            if (tile == 0) st_volatile64(&stat[0], PF_PRE | pack_km(tile_keep, tile_merge));
-            else {
-                st_volatile64(&stat[tile], PF_AGG | pack_km(tile_keep, tile_merge));
-                int64_t t = (int64_t)tile - 1;
-                uint64_t kk = 0, mm = 0;
-                while (t >= 0) {
-                    uint64_t s = ld_volatile64(&stat[t]);
-                    uint32_t spins = 0;
-                    while ((s & PF_MASK) == 0) {
-                        if (++spins > SPIN_LIMIT) { atomicOr(err, ST_TIMEOUT_PLOC); break; }
-                        __nanosleep(32);
-                        s = ld_volatile64(&stat[t]);
-                    }
-                    kk += (s >> 31) & 0x7fffffffull;
-                    mm += s & 0x7fffffffull;
-                    if ((s & PF_MASK) != PF_AGG) break;
-                    t--;
-                }
-                pre = pack_km(kk, mm);
-                st_volatile64(&stat[tile], PF_PRE | pack_km(kk + tile_keep, mm + tile_merge));
-            }
-            if (tile == ntiles - 1) st->nc_next = (uint32_t)((pre >> 31) & 0x7fffffffull) + tile_keep;
-        }
-        S.prefix = pre;
-        S.keep_total = tile_keep;
+        if (tile) st_volatile64(&stat[tile], PF_PRE | pack_km(keep0 + tile_keep, merge0 + tile_merge));
+        if (tile == ntiles - 1) st->nc_next = keep0 + tile_keep;
     }
-    __syncthreads();
-    uint32_t dest = (uint32_t)((S.prefix >> 31) & 0x7fffffffull) + (excl & 0xffffu);
-    uint32_t m = (uint32_t)(S.prefix & 0x7fffffffull) + (excl >> 16);
+    uint32_t dest = keep0 + (excl & 0xffffu);
+    uint32_t m = merge0 + (excl >> 16);
 #pragma unroll
-    for (int k = 0; k < PL_PER; k++) {
+    for (int k = 0; k < PER; k++) {
         if (!((keepm >> k) & 1u)) continue;
-        int64_t i = base + tid * PL_PER + k;
-        const Cl &c = S.win[i - w0];
-        Cl out = c;
+        const int64_t i = base + tid * PER + k;
         if (dest >= nc || m + 1 >= nc) {                         // only after a look-back that ran out
             atomicOr(err, ST_TIMEOUT_PLOC);
             break;
         }
+        const int wi = (int)(i - w0);
+        float out[6];
+        uint32_t id = S.id[wi];
         if ((mergem >> k) & 1u) {
-            uint32_t j = S.nn[i - (base - PL_R)];
-            const Cl &dd = S.win[(int64_t)j - w0];
-            uint32_t kid = nc - 2 - m;                           // (n - 2) - (merges before it)
+            id = ploc_merge(S, wi, (int)((int64_t)S.nn[i - (base - PL_R)] - w0), nc, m, n, node0, ref0, nodes, out);
             m++;
-#pragma unroll
-            for (int q = 0; q < 3; q++) { out.lo[q] = wmin(c.lo[q], dd.lo[q]); out.hi[q] = wmax(c.hi[q], dd.hi[q]); }
-            out.id = kid;
-            final_node(c, n, node0, ref0, &nodes[1 + 2 * kid]);
-            final_node(dd, n, node0, ref0, &nodes[2 + 2 * kid]);
-            if (kid == 0)
-                store_node(&nodes[0], out.lo[0], out.lo[1], out.lo[2], node0 + 1, out.hi[0], out.hi[1], out.hi[2], node0 + 2);
+        } else {
+            ploc_get(S, wi, out);
         }
         float4 *dst = reinterpret_cast<float4 *>(&Lq[dest]);
-        dst[0] = make_float4(out.lo[0], out.lo[1], out.lo[2], __uint_as_float(out.id));
-        dst[1] = make_float4(out.hi[0], out.hi[1], out.hi[2], 0.0f);
+        dst[0] = make_float4(out[0], out[1], out[2], __uint_as_float(id));
+        dst[1] = make_float4(out[3], out[4], out[5], 0.0f);
         dest++;
+    }
+}
+
+// The last nc <= PL_LAST clusters, by one block: the list stays in shared memory from round to round
+// (slots 2 R .. 2 R + nc, nothing around them).
+__device__ void ploc_last(PlocShared &S, const Cl *__restrict__ L, uint32_t nc, uint32_t n, uint32_t node0, uint32_t ref0,
+                          Node *nodes, uint32_t *err) {
+    const int tid = threadIdx.x;
+    constexpr int AT = 2 * PL_R, WIN = PL_LAST + 4 * PL_R;
+    bool plain = true;
+    for (int i = tid; i < WIN; i += PL_THREADS) plain = ploc_load(S, i, L, (int64_t)i - AT, nc) && plain;
+    plain = __syncthreads_and(plain);                            // (merged boxes are as plain as their clusters)
+    while (nc > 1) {
+        // (S.nn[t]: list position t - R; thread t's nearest is position t's, R slots on)
+        uint32_t near;
+        {
+            PlocShared &Q = S;
+            float c[6], o[6], bd = __int_as_float(0x7f800000);
+            ploc_get(Q, AT + tid, c);
+            near = 0xffffffffu;
+            if (plain) {
+#pragma unroll 8
+                for (int m = 0; m <= 2 * PL_R; m++) {
+                    if (m == PL_R) continue;
+                    ploc_get(Q, AT - PL_R + tid + m, o);
+                    const float d = joined_area_fin(c, o);
+                    if (d < bd) { bd = d; near = (uint32_t)(tid + m - PL_R); }
+                }
+            } else if ((uint32_t)tid < nc) {
+                const uint32_t j0 = tid > PL_R ? (uint32_t)tid - PL_R : 0u, j1 = min((uint32_t)tid + PL_R, nc - 1);
+                bd = 0.0f;
+                for (uint32_t j = j0; j <= j1; j++) {
+                    if (j == (uint32_t)tid) continue;
+                    ploc_get(Q, AT + (int)j, o);
+                    const float d = joined_area(c, o);
+                    if (nearer(d, (uint32_t)tid, j, bd, near)) { bd = d; near = j; }
+                }
+            }
+        }
+        S.nn[tid] = near;
+        __syncthreads();
+        bool keep = false, merge = false;
+        if ((uint32_t)tid < nc) {
+            const bool mu = near < nc && S.nn[near] == (uint32_t)tid;
+            keep = !(mu && (uint32_t)tid > near);
+            merge = mu && (uint32_t)tid < near;
+        }
+        uint32_t tot;
+        const uint32_t excl = block_excl_scan<PL_THREADS>((keep ? 1u : 0u) | (merge ? 1u << 16 : 0u), S.scan, tot);
+        const uint32_t next = tot & 0xffffu;
+        if (next >= nc) {                                        // every round merges at least one pair
+            if (tid == 0) atomicOr(err, ST_TIMEOUT_PLOC);
+            return;
+        }
+        float out[6];
+        uint32_t id = 0;
+        if (keep) {
+            id = S.id[AT + tid];
+            if (merge) id = ploc_merge(S, AT + tid, AT + (int)near, nc, excl >> 16, n, node0, ref0, nodes, out);
+            else ploc_get(S, AT + tid, out);
+        }
+        __syncthreads();                                         // (the list is written in its place)
+        if (keep) {
+            const int i = AT + (int)(excl & 0xffffu);
+#pragma unroll
+            for (int q = 0; q < 6; q++) S.c[q][i] = out[q];
+            S.id[i] = id;
+        }
+        if ((uint32_t)tid >= next && (uint32_t)tid < nc)
+#pragma unroll
+            for (int q = 0; q < 6; q++) S.c[q][AT + tid] = 1e19f;
+        nc = next;
+        __syncthreads();
     }
 }
 
@@ -580,33 +774,23 @@ __global__ void __launch_bounds__(PL_THREADS) ploc_kernel(Cl *listA, Cl *listB, 
     PlocShared &S = *reinterpret_cast<PlocShared *>(pl_smem);
     uint32_t nc = n, r = 0;
     Cl *Lp = listA, *Lq = listB;
-    while (nc > 1) {
-        const uint32_t ntiles = (nc + PL_TILE - 1) / PL_TILE;
-        if (ntiles == 1) {                                       // the rest in one block
-            if (blockIdx.x != 0) return;
-            while (nc > 1) {
-                ploc_tile(S, Lp, Lq, nc, 0, 1, n, node0, ref0, nodes, nullptr, false, st, err);
-                __syncthreads();
-                const uint32_t next = S.keep_total;
-                if (next >= nc) {                                // every round merges at least one pair
-                    if (threadIdx.x == 0) atomicOr(err, ST_TIMEOUT_PLOC);
-                    return;
-                }
-                nc = next;
-                Cl *t = Lp; Lp = Lq; Lq = t;
-                __threadfence_block();
-                __syncthreads();
-            }
-            return;
-        }
+    while (nc > PL_LAST) {
+        // the blocks this round and the later ones need: the others are done
+        const uint32_t tiles1 = (nc + PL_TILE1 - 1) / PL_TILE1, blocks = min(gridDim.x, tiles1);
+        if (blockIdx.x >= blocks) return;
         uint64_t *stat = (r & 1) ? stat1 : stat0, *other = (r & 1) ? stat0 : stat1;
-        for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-            ploc_tile(S, Lp, Lq, nc, tile, ntiles, n, node0, ref0, nodes, stat, true, st, err);
+        const bool one = tiles1 <= gridDim.x;                    // (the list no longer fills the grid)
+        const uint32_t ntiles = one ? tiles1 : (nc + PL_TILE - 1) / PL_TILE;
+        for (uint32_t tile = blockIdx.x; tile < ntiles; tile += blocks) {
+            if (one) ploc_tile<1>(S, Lp, Lq, nc, tile, ntiles, n, node0, ref0, nodes, stat, st, err);
+            else ploc_tile<4>(S, Lp, Lq, nc, tile, ntiles, n, node0, ref0, nodes, stat, st, err);
             __syncthreads();
         }
-        for (uint32_t i = blockIdx.x * PL_THREADS + threadIdx.x; i < ntiles; i += gridDim.x * PL_THREADS) other[i] = 0;
+        // the next round's statuses (as many tiles as this round's, or a grid of the smaller ones)
+        for (uint32_t i = blockIdx.x * PL_THREADS + threadIdx.x; i < max(ntiles, gridDim.x); i += blocks * PL_THREADS)
+            other[i] = 0;
         __threadfence();
-        grid_barrier(st, err);
+        grid_barrier(st, blocks, err);
         const uint32_t next = ld_volatile(&st->nc_next);
         if (next >= nc || (ld_volatile(err) & (ST_TIMEOUT_PLOC | ST_TIMEOUT_BARRIER))) {
             if (threadIdx.x == 0) atomicOr(err, ST_TIMEOUT_PLOC);
@@ -616,6 +800,7 @@ __global__ void __launch_bounds__(PL_THREADS) ploc_kernel(Cl *listA, Cl *listB, 
         Cl *t = Lp; Lp = Lq; Lq = t;
         r++;
     }
+    if (blockIdx.x == 0 && nc > 1) ploc_last(S, Lp, nc, n, node0, ref0, nodes, err);
 }
 
 // the first clusters: the leaves in sorted order, and aux (the reference's `leaves` in PLOC mode;
@@ -791,7 +976,7 @@ static BuildLayout layout_for(uint32_t n, int key_bits, int builder) {
     L.status = put((size_t)passes * L.tiles * 256 * 4);
     L.counters = put((size_t)passes * 4);
     if (builder == 1) {
-        const size_t pt = (nn + PL_TILE - 1) / PL_TILE;
+        const size_t pt = (nn + PL_TILE - 1) / PL_TILE + PL_MAX_GRID;
         L.list_a = put(nn * sizeof(Cl));
         L.list_b = put(nn * sizeof(Cl));
         L.stat0 = put(pt * 8);
@@ -858,8 +1043,8 @@ static cudaError_t build_typed(const lrc_build_params &p, const float *d_boxes, 
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ploc_kernel, PL_THREADS, psmem);
         if (per_sm < 1) per_sm = 1;
     }
-    const uint32_t want = (n + PL_TILE - 1) / PL_TILE;
-    uint32_t grid = std::min<uint32_t>((uint32_t)(per_sm * num_sms), std::max<uint32_t>(want, 1));
+    const uint32_t want = (n + PL_TILE1 - 1) / PL_TILE1;
+    uint32_t grid = std::min<uint32_t>((uint32_t)std::min(per_sm * num_sms, PL_MAX_GRID), std::max<uint32_t>(want, 1));
     uint32_t node0 = p.node0, ref0 = p.ref0, nn_ = n;
     void *args[] = {&la, &lb, &nn_, &node0, &ref0, &d_nodes, &s0, &s1, &ps, &d_status};
     e = cudaLaunchCooperativeKernel((void *)ploc_kernel, dim3(grid), dim3(PL_THREADS), args, psmem, st);
