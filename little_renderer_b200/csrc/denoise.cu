@@ -108,14 +108,49 @@ __device__ __forceinline__ V3 irradiance(const float4 *__restrict__ px, size_t N
 }
 
 // prep: the packed guide, and each pixel's irradiance with the variance of its mean (its own
-// moments from 4 samples on, else the spread of its 7 x 7 neighbours on the same surface)
-__global__ void __launch_bounds__(256) prep_kernel(const float4 *__restrict__ px, int W, int H, uint2 *__restrict__ dst,
-                                                   float4 *__restrict__ gd) {
-    const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
-    if (x >= W || y >= H) return;
+// moments from 4 samples on, else the spread of its 7 x 7 neighbours on the same surface).
+// The neighbours are the cost (49 of them, each a mean over an albedo): a block whose pixels need
+// them makes each pixel's luminance once, into shared memory with its normal and kind (a 32 x 16
+// tile with its border of 3: 1.6 pixels made a pixel, 49 before), and the spread is summed from there
+// in the same order.
+constexpr int PREP_W = 32, PREP_H = 16, PREP_R = 3;
+constexpr int PREP_TW = PREP_W + 2 * PREP_R, PREP_TH = PREP_H + 2 * PREP_R;
+__global__ void __launch_bounds__(PREP_W *PREP_H) prep_kernel(const float4 *__restrict__ px, int W, int H,
+                                                               uint2 *__restrict__ dst, float4 *__restrict__ gd) {
+    __shared__ float4 s_nl[PREP_TH][PREP_TW];        // the normal, the luminance of the irradiance
+    __shared__ float s_kind[PREP_TH][PREP_TW];       // the kind; -1: no samples, or outside the image
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int x0 = blockIdx.x * PREP_W, y0 = blockIdx.y * PREP_H;
+    const int x = x0 + tx, y = y0 + ty;
+    const bool in = x < W && y < H;
     const size_t N = (size_t)W * H, k = (size_t)y * W + x;
-    const float4 a = px[k], g = px[3 * N + k], n = px[2 * N + k];
+    float4 a = make_float4(0, 0, 0, 0), g = a, n = a;
+    if (in) {
+        a = px[k];
+        g = px[3 * N + k];
+        n = px[2 * N + k];
+    }
     const float gk = gkind(g.w);
+    const bool spread = in && a.w != 0.0f && gk != 1.0f && !(a.w >= 4.0f);
+    if (__syncthreads_or(spread)) {
+        for (int i = threadIdx.x; i < PREP_TW * PREP_TH; i += PREP_W * PREP_H) {
+            const int r = i / PREP_TW, c = i - r * PREP_TW;
+            const int qx = x0 + c - PREP_R, qy = y0 + r - PREP_R;
+            float kind = -1.0f;
+            if (qx >= 0 && qy >= 0 && qx < W && qy < H) {
+                const size_t q = (size_t)qy * W + qx;
+                if (px[q].w != 0.0f) {
+                    kind = gkind(px[3 * N + q].w);
+                    const float4 nq = px[2 * N + q];
+                    const V3 iq = irradiance(px, N, q);
+                    s_nl[r][c] = make_float4(nq.x, nq.y, nq.z, luma(iq.x, iq.y, iq.z));
+                }
+            }
+            s_kind[r][c] = kind;
+        }
+        __syncthreads();
+    }
+    if (!in) return;
     const float e = gk == 0.0f ? n.w : (gk == 1.0f ? -2e38f : -(n.w + 1.0f));
     const V3 nd = unoct(unsnorm16x2(oct(n.x, n.y, n.z)));
     gd[k] = make_float4(nd.x, nd.y, nd.z, e);
@@ -129,26 +164,20 @@ __global__ void __launch_bounds__(256) prep_kernel(const float4 *__restrict__ px
         return;
     }
     float v;
-    if (a.w >= 4.0f) {
+    if (!spread) {
         const float4 m = px[N + k];
         const float el = m.x / a.w;
         v = fmaxf(m.y / a.w - el * el, 0.0f) / a.w;
     } else {
         float s1 = 0.0f, s2 = 0.0f, c = 0.0f;
-        for (int dy = -3; dy <= 3; dy++)
-            for (int dx = -3; dx <= 3; dx++) {
-                const int qx = x + dx, qy = y + dy;
-                if (qx < 0 || qy < 0 || qx >= W || qy >= H) continue;
-                const size_t q = (size_t)qy * W + qx;
-                if (px[q].w == 0.0f || gkind(px[3 * N + q].w) != gk) continue;
-                if (gk == 0.0f) {
-                    const float4 nq = px[2 * N + q];
-                    if (nq.x * n.x + nq.y * n.y + nq.z * n.z < 0.9f) continue;
-                }
-                const V3 iq = irradiance(px, N, q);
-                const float l = luma(iq.x, iq.y, iq.z);
-                s1 += l;
-                s2 += l * l;
+        for (int dy = 0; dy <= 2 * PREP_R; dy++)
+#pragma unroll
+            for (int dx = 0; dx <= 2 * PREP_R; dx++) {
+                if (s_kind[ty + dy][tx + dx] != gk) continue;
+                const float4 q = s_nl[ty + dy][tx + dx];
+                if (gk == 0.0f && q.x * n.x + q.y * n.y + q.z * n.z < 0.9f) continue;
+                s1 += q.w;
+                s2 += q.w * q.w;
                 c += 1.0f;
             }
         const float el = s1 / c;
@@ -160,10 +189,30 @@ __global__ void __launch_bounds__(256) prep_kernel(const float4 *__restrict__ px
 // the B3 spline's weights 1/16, 1/4, 3/8, 1/4, 1/16
 __device__ __forceinline__ float b3(int i) { return i == 2 ? 0.375f : (i == 1 || i == 3 ? 0.25f : 0.0625f); }
 
+// 2^x and the square root of the special function unit (2 ulp and 1 ulp of a float: their results go
+// into weights whose sums are kept as halves)
+__device__ __forceinline__ float ex2(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float sqrt_sfu(float x) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // One a-trous pass: a 5 x 5 B3 spline with holes `step` apart, each tap jittered within its hole
 // (but the centre), weighted by luminance (against the noise of the noisier of the two), normal
 // (cos^128) and distance (against how fast it changes here); the variance filtered with the
 // squared weights. The last pass writes the image (times the albedo on surfaces).
+//
+// Bound by instructions (84 % of the issue slots, the taps hit L1 / L2), so a tap is kept short: the
+// centre (the only tap that can fall on the pixel itself: a jitter is at most half a hole) is no
+// longer told apart at run time, a surface's taps read the distance and the kind as one sign test,
+// the luminance's and the distance's exponentials are one 2^x, and JIT = false (step 1) has no
+// random numbers.
+template <bool JIT>
 __global__ void __launch_bounds__(256) atrous_kernel(const float4 *__restrict__ px, int W, int H, int step, int last,
                                                      float sigma_l, float sigma_z, const uint2 *__restrict__ src,
                                                      uint2 *__restrict__ dst, const float4 *__restrict__ gd,
@@ -180,13 +229,15 @@ __global__ void __launch_bounds__(256) atrous_kernel(const float4 *__restrict__ 
     }
     // the variance blurred 3 x 3
     float v = 0.0f, vw = 0.0f;
+#pragma unroll
     for (int dy = -1; dy <= 1; dy++)
+#pragma unroll
         for (int dx = -1; dx <= 1; dx++) {
             const int qx = min(max(x + dx, 0), W - 1), qy = min(max(y + dy, 0), H - 1);
-            const float4 s = get_iv(src[(uint32_t)qy * W + qx]);
-            if (s.w < 0.0f) continue;
+            const float sw = __half2float(__ushort_as_half((unsigned short)(src[(uint32_t)qy * W + qx].y >> 16)));
+            if (sw < 0.0f) continue;
             const float w = (dx != 0 ? 0.25f : 0.5f) * (dy != 0 ? 0.25f : 0.5f);
-            v += w * s.w;
+            v += w * sw;
             vw += w;
         }
     v /= fmaxf(vw, 1e-6f);
@@ -200,45 +251,60 @@ __global__ void __launch_bounds__(256) atrous_kernel(const float4 *__restrict__ 
         gx = fminf(fabsf(gp.z - l), fabsf(gp.z - r));
         gy = fminf(fabsf(gp.z - d), fabsf(gp.z - u));
     }
-    uint32_t seed = hash32((k * 0x9e3779b9u) ^ ((uint32_t)step * 0x85ebca6bu));
+    const float zb = 1e-3f * gp.z + 1e-6f;
+    gx *= sigma_z;
+    gy *= sigma_z;
+    constexpr float L2E = 1.4426950408889634f;       // (exp(x) = 2^(x log2 e))
+    uint32_t seed = JIT ? hash32((k * 0x9e3779b9u) ^ ((uint32_t)step * 0x85ebca6bu)) : 0u;
     const int jit = step / 2;
     const uint32_t jn = (uint32_t)(2 * jit + 1);
     float sr = 0.0f, sg = 0.0f, sb = 0.0f, vsum = 0.0f, wsum = 0.0f;
-#pragma unroll 1
-    for (int j = 0; j < 5; j++) {
+    auto add_tap = [&](float w, const float4 s) {
+        sr += w * s.x;
+        sg += w * s.y;
+        sb += w * s.z;
+        vsum += w * w * s.w;
+        wsum += w;
+    };
+    auto row = [&](int j, float bj) {
 #pragma unroll
         for (int i = 0; i < 5; i++) {
+            if (i == 2 && j == 2) {
+                add_tap(b3(2) * b3(2), c);
+                continue;
+            }
             int ox = (i - 2) * step, oy = (j - 2) * step;
-            if (jit > 0 && (i != 2 || j != 2)) {
+            if (JIT) {
                 seed = hash32(seed);
                 ox += (int)(((seed & 0xffffu) * jn) >> 16) - jit;
                 oy += (int)(((seed >> 16) * jn) >> 16) - jit;
             }
             const int qx = x + ox, qy = y + oy;
-            if (qx < 0 || qy < 0 || qx >= W || qy >= H) continue;
+            if ((uint32_t)qx >= (uint32_t)W || (uint32_t)qy >= (uint32_t)H) continue;
             const uint32_t q = (uint32_t)qy * W + qx;
+            const float4 gq = gd[q];
             const float4 s = get_iv(src[q]);
-            float w = b3(i) * b3(j);
-            if (q != k) {
-                const G gq = get_g(gd[q]);
-                if (s.w < 0.0f || gq.kind != gp.kind) continue;
-                w *= __expf(__fdividef(-fabsf(lp - luma(s.x, s.y, s.z)), sigma_l * sqrtf(fmaxf(v, s.w)) + 1e-6f));
-                if (surface) {
-                    float wn = fmaxf(gp.n.x * gq.n.x + gp.n.y * gq.n.y + gp.n.z * gq.n.z, 0.0f);
+            if (s.w < 0.0f) continue;
+            float ex = __fdividef(fabsf(lp - luma(s.x, s.y, s.z)), sigma_l * sqrt_sfu(fmaxf(v, s.w)) + 1e-6f);
+            float w = b3(i) * bj;
+            if (surface) {
+                if (!(gq.w >= 0.0f)) continue;       // (not a surface)
+                float wn = fmaxf(gp.n.x * gq.x + gp.n.y * gq.y + gp.n.z * gq.z, 0.0f);
 #pragma unroll
-                    for (int e = 0; e < 7; e++) wn *= wn;   // cos^128
-                    w *= wn;
-                    const float expect = gx * fabsf((float)ox) + gy * fabsf((float)oy);
-                    w *= __expf(__fdividef(-fabsf(gp.z - gq.z), sigma_z * expect + 1e-3f * gp.z + 1e-6f));
-                }
+                for (int e = 0; e < 7; e++) wn *= wn;   // cos^128
+                w *= wn;
+                ex += __fdividef(fabsf(gp.z - gq.w), gx * fabsf((float)ox) + gy * fabsf((float)oy) + zb);
+            } else if (gq.w >= 0.0f || gq.w < -1e37f) {
+                continue;                            // (not a medium)
             }
-            sr += w * s.x;
-            sg += w * s.y;
-            sb += w * s.z;
-            vsum += w * w * s.w;
-            wsum += w;
+            add_tap(w * ex2(-L2E * ex), s);
         }
-    }
+    };
+    row(0, b3(0));
+    row(1, b3(1));
+    row(2, b3(2));
+    row(3, b3(3));
+    row(4, b3(4));
     const float o0 = sr / wsum, o1 = sg / wsum, o2 = sb / wsum;
     if (last) {
         const float4 al = px[3 * (size_t)N + k];
@@ -522,12 +588,14 @@ cudaError_t dn_denoise(const float4 *d_planes, int W, int H, int passes, float4 
     uint2 *a = static_cast<uint2 *>(scratch), *b = a + N;
     float4 *gd = reinterpret_cast<float4 *>(b + N);
     const dim3 grid((unsigned)((W + 31) / 32), (unsigned)((H + 7) / 8));
-    dn::prep_kernel<<<grid, 256, 0, st>>>(d_planes, W, H, a, gd);
+    const dim3 pgrid((unsigned)((W + dn::PREP_W - 1) / dn::PREP_W), (unsigned)((H + dn::PREP_H - 1) / dn::PREP_H));
+    dn::prep_kernel<<<pgrid, dn::PREP_W * dn::PREP_H, 0, st>>>(d_planes, W, H, a, gd);
     // a -> b, b -> a, ...; the last pass into out
     for (int i = 1; i <= passes; i++) {
         const uint2 *in = i % 2 ? a : b;
         uint2 *to = i % 2 ? b : a;
-        dn::atrous_kernel<<<grid, 256, 0, st>>>(d_planes, W, H, 1 << (i - 1), i == passes, 4.0f, 1.0f, in, to, gd, d_out);
+        (i == 1 ? dn::atrous_kernel<false> : dn::atrous_kernel<true>)<<<grid, 256, 0, st>>>(
+            d_planes, W, H, 1 << (i - 1), i == passes, 4.0f, 1.0f, in, to, gd, d_out);
     }
     return cudaGetLastError();
 }
