@@ -57,6 +57,22 @@ template <typename K> struct KeyTraits;
 template <> struct KeyTraits<uint32_t> { static constexpr int PASSES = 4; };
 template <> struct KeyTraits<uint64_t> { static constexpr int PASSES = 8; };
 
+// the Morton code of an item's box (30 or 63 bits)
+template <typename K>
+__device__ __forceinline__ K morton_code(float4 lo, float4 hi, float3 plo, float3 pext) {
+    if constexpr (sizeof(K) == 4) {
+        uint32_t qx = quantise(lo.x, hi.x, plo.x, pext.x, 1024.0f);
+        uint32_t qy = quantise(lo.y, hi.y, plo.y, pext.y, 1024.0f);
+        uint32_t qz = quantise(lo.z, hi.z, plo.z, pext.z, 1024.0f);
+        return (spread10(qx) << 2) | (spread10(qy) << 1) | spread10(qz);
+    } else {
+        uint32_t qx = quantise(lo.x, hi.x, plo.x, pext.x, 2097152.0f);
+        uint32_t qy = quantise(lo.y, hi.y, plo.y, pext.y, 2097152.0f);
+        uint32_t qz = quantise(lo.z, hi.z, plo.z, pext.z, 2097152.0f);
+        return (spread21(qx) << 2) | (spread21(qy) << 1) | spread21(qz);
+    }
+}
+
 constexpr int MH_THREADS = 256;
 
 // codes of n items, and the 256-bin histogram of every radix pass's digit into hist[pass][256]
@@ -74,18 +90,7 @@ __global__ void __launch_bounds__(MH_THREADS) morton_hist_kernel(const float4 *_
     __syncthreads();
     for (uint32_t i = blockIdx.x * MH_THREADS + threadIdx.x; i < n; i += gridDim.x * MH_THREADS) {
         float4 lo = __ldg(&boxes[2 * (size_t)i]), hi = __ldg(&boxes[2 * (size_t)i + 1]);
-        K code;
-        if constexpr (sizeof(K) == 4) {
-            uint32_t qx = quantise(lo.x, hi.x, plo.x, pext.x, 1024.0f);
-            uint32_t qy = quantise(lo.y, hi.y, plo.y, pext.y, 1024.0f);
-            uint32_t qz = quantise(lo.z, hi.z, plo.z, pext.z, 1024.0f);
-            code = (spread10(qx) << 2) | (spread10(qy) << 1) | spread10(qz);
-        } else {
-            uint32_t qx = quantise(lo.x, hi.x, plo.x, pext.x, 2097152.0f);
-            uint32_t qy = quantise(lo.y, hi.y, plo.y, pext.y, 2097152.0f);
-            uint32_t qz = quantise(lo.z, hi.z, plo.z, pext.z, 2097152.0f);
-            code = (spread21(qx) << 2) | (spread21(qy) << 1) | spread21(qz);
-        }
+        const K code = morton_code<K>(lo, hi, plo, pext);
         codes[i] = code;
 #pragma unroll
         for (int p = 0; p < P; p++) atomicAdd(&sh[p * 256 + (uint32_t)((code >> (8 * p)) & 255u)], 1u);
@@ -296,6 +301,123 @@ __global__ void __launch_bounds__(OS_THREADS, OS_MINB) onesweep_kernel(const K *
     }
 }
 
+// ---- codes and sort of a tile's items at most, in one block ---------------------------------------
+// A tree over at most SS_ITEMS items (a frame's top level) spends its time in launches and in passes of
+// one tile each, so the codes and every pass run in one launch: 1024 threads, the keys and items in
+// registers between passes and in shared memory across one (the onesweep pass's ranking, without
+// its histograms and its look-back). The line is the block's capacity; a whole build of 4988 items,
+// 30-bit keys, with the block-wise climb below: 94 -> 58 us.
+constexpr int SS_THREADS = 1024, SS_WARPS = SS_THREADS / 32, SS_PER = 8;
+constexpr int SS_ITEMS = SS_THREADS * SS_PER;
+template <typename K>
+struct SsShared {
+    uint16_t warp_hist[SS_WARPS][256];
+    uint32_t start[256];
+    uint32_t scan[SS_WARPS];
+    K key[SS_ITEMS];
+    uint32_t val[SS_ITEMS];
+};
+
+// (PER: items a thread; the block's items are in order by warp, then item of the thread, then lane)
+template <typename K, int PER>
+__device__ __forceinline__ void small_sort_passes(SsShared<K> &S, K (&key)[PER], uint32_t (&val)[PER], uint32_t n) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const uint32_t lt = (1u << lane) - 1u, i0 = w * (32 * PER) + lane;
+    constexpr int P = KeyTraits<K>::PASSES;
+    for (int pass = 0; pass < P; pass++) {
+        for (uint32_t i = tid; i < SS_WARPS * 256 / 2; i += SS_THREADS) reinterpret_cast<uint32_t *>(S.warp_hist)[i] = 0;
+        __syncthreads();
+        uint32_t rank[PER];
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            const bool on_list = i0 + 32 * k < n;
+            const uint32_t d = on_list ? (uint32_t)((key[k] >> (8 * pass)) & 255u) : 0x100u;
+            uint32_t peers = 0xffffffffu;
+#pragma unroll
+            for (int bit = 0; bit < 9; bit++) {
+                const bool on = (d >> bit) & 1u;
+                const uint32_t bal = __ballot_sync(0xffffffffu, on);
+                peers &= on ? bal : ~bal;
+            }
+            // (the warp's own counters: the leader reads and adds, nobody else does meanwhile)
+            const int leader = __ffs(peers) - 1;
+            uint32_t base = 0;
+            if (on_list && (int)lane == leader) {
+                base = S.warp_hist[w][d];
+                S.warp_hist[w][d] = (uint16_t)(base + __popc(peers));
+            }
+            rank[k] = __shfl_sync(0xffffffffu, base, leader) + __popc(peers & lt);
+            __syncwarp();
+        }
+        __syncthreads();
+        uint32_t count = 0, tot;
+        if (tid < 256) {
+#pragma unroll 8
+            for (int ww = 0; ww < SS_WARPS; ww++) {
+                const uint32_t c = S.warp_hist[ww][tid];
+                S.warp_hist[ww][tid] = (uint16_t)count;
+                count += c;
+            }
+        }
+        const uint32_t start = block_excl_scan<SS_THREADS>(count, S.scan, tot);
+        if (tid < 256) S.start[tid] = start;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < PER; k++)
+            if (i0 + 32 * k < n) {
+                const uint32_t d = (uint32_t)((key[k] >> (8 * pass)) & 255u);
+                const uint32_t at = S.start[d] + S.warp_hist[w][d] + rank[k];
+                S.key[at] = key[k];
+                S.val[at] = val[k];
+            }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < PER; k++)
+            if (i0 + 32 * k < n) {
+                key[k] = S.key[i0 + 32 * k];
+                val[k] = S.val[i0 + 32 * k];
+            }
+    }
+}
+
+template <typename K, int PER>
+__device__ __forceinline__ void small_sort(SsShared<K> &S, const float4 *__restrict__ boxes, uint32_t n, float3 plo,
+                                           float3 pext, K *__restrict__ codes, uint32_t *__restrict__ items) {
+    const uint32_t i0 = (threadIdx.x >> 5) * (32 * PER) + (threadIdx.x & 31);
+    K key[PER];
+    uint32_t val[PER];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const uint32_t i = i0 + 32 * k;
+        key[k] = 0;
+        val[k] = i;
+        if (i < n) key[k] = morton_code<K>(__ldg(&boxes[2 * (size_t)i]), __ldg(&boxes[2 * (size_t)i + 1]), plo, pext);
+    }
+    small_sort_passes<K, PER>(S, key, val, n);
+#pragma unroll
+    for (int k = 0; k < PER; k++)
+        if (i0 + 32 * k < n) {
+            codes[i0 + 32 * k] = key[k];
+            items[i0 + 32 * k] = val[k];
+        }
+}
+
+// codes: the sorted codes; items: their items
+template <typename K>
+__global__ void __launch_bounds__(SS_THREADS) small_sort_kernel(const float4 *__restrict__ boxes, uint32_t n, float3 plo,
+                                                                float3 pext, const float *__restrict__ dlo_ext,
+                                                                K *__restrict__ codes, uint32_t *__restrict__ items) {
+    extern __shared__ __align__(16) unsigned char ss_smem[];
+    SsShared<K> &S = *reinterpret_cast<SsShared<K> *>(ss_smem);
+    if (dlo_ext) {
+        plo = make_float3(dlo_ext[0], dlo_ext[1], dlo_ext[2]);
+        pext = make_float3(dlo_ext[3], dlo_ext[4], dlo_ext[5]);
+    }
+    if (n <= 2 * SS_THREADS) small_sort<K, 2>(S, boxes, n, plo, pext, codes, items);
+    else if (n <= 5 * SS_THREADS) small_sort<K, 5>(S, boxes, n, plo, pext, codes, items);
+    else small_sort<K, SS_PER>(S, boxes, n, plo, pext, codes, items);
+}
+
 // ---- LBVH: Karras's tree, made bottom-up in one pass -----------------------------------------
 template <typename K>
 __device__ __forceinline__ int delta_at(const K *__restrict__ codes, uint32_t i, uint32_t j) {
@@ -321,6 +443,74 @@ __device__ __forceinline__ void store_node(Node *p, float lx, float ly, float lz
     q[1] = make_float4(hx, hy, hz, __uint_as_float(b));
 }
 
+// A subtree's way up: the node cur over the leaves [l, r], its box, and whether it is its parent's left child.
+struct Climb {
+    uint32_t l, r, cur;
+    bool left;
+    float bl[3], bh[3];
+};
+// the parent of c (a left child's or a right child's subtree) and its sibling `got` leaves away: node
+// numbers as Karras gives them, the box the left child's with the right's joined (min / max), stored;
+// c becomes the parent. True: it was the root.
+template <typename K>
+__device__ __forceinline__ bool lbvh_parent(Climb &c, uint32_t got, const float *sl, const float *sh, bool left_next, uint32_t n,
+                                            uint32_t node0, Node *nodes) {
+    const uint32_t split = c.left ? c.r : c.l - 1;
+    uint32_t L, R, lc, rc;
+    if (c.left) { L = c.l; R = got; lc = c.cur; rc = got == split + 1 ? n + split : split + 1; }
+    else { L = got; R = c.r; rc = c.cur; lc = got == split ? n - 1 + split : split; }
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        c.bl[k] = c.left ? wmin(c.bl[k], sl[k]) : wmin(sl[k], c.bl[k]);
+        c.bh[k] = c.left ? wmax(c.bh[k], sh[k]) : wmax(sh[k], c.bh[k]);
+    }
+    const bool root = L == 0 && R == n - 1;
+    const uint32_t pidx = root ? 0u : left_next ? R : L;
+    store_node(&nodes[pidx], c.bl[0], c.bl[1], c.bl[2], node0 + lc, c.bh[0], c.bh[1], c.bh[2], node0 + rc);
+    c.l = L;
+    c.r = R;
+    c.cur = pidx;
+    c.left = left_next;
+    return root;
+}
+
+// the climb of c (its sibling elsewhere) through memory: up to where the sibling is not there yet
+template <typename K>
+__device__ __forceinline__ void lbvh_climb(Climb &c, const K *__restrict__ codes, uint32_t n, uint32_t node0, Node *nodes,
+                                           uint32_t *other) {
+    while (true) {
+        const uint32_t split = c.left ? c.r : c.l - 1;
+        __threadfence();                             // our node before the exchange
+        const uint32_t got = atomicExch(&other[split], c.left ? c.l : c.r);
+        if (got == 0xffffffffu) return;              // the sibling makes the parent
+        __threadfence();
+        const uint32_t sib = c.left ? (got == split + 1 ? n + split : split + 1) : (got == split ? n - 1 + split : split);
+        const float4 *sp = reinterpret_cast<const float4 *>(&nodes[sib]);
+        const float4 s0 = __ldcg(sp), s1 = __ldcg(sp + 1);
+        const float sl[3] = {s0.x, s0.y, s0.z}, sh[3] = {s1.x, s1.y, s1.z};
+        const uint32_t L = c.left ? c.l : got, R = c.left ? got : c.r;
+        const bool root = L == 0 && R == n - 1;
+        if (lbvh_parent<K>(c, got, sl, sh, !root && is_left_child(codes, L, R, n), n, node0, nodes)) return;
+    }
+}
+// leaf j's node and its aux word; c: its subtree (its side is the caller's to say)
+__device__ __forceinline__ void lbvh_leaf(Climb &c, uint32_t j, const uint32_t *__restrict__ items,
+                                          const float4 *__restrict__ boxes, uint32_t n, uint32_t ref0, uint32_t ref_add,
+                                          Node *nodes, uint32_t *__restrict__ aux, uint32_t *err) {
+    uint32_t item = __ldg(&items[j]);
+    if (item >= n) {                                 // (a sort that went wrong: said, not followed)
+        atomicOr(err, ST_TIMEOUT_SORT);
+        item = 0;
+    }
+    const float4 lo = __ldg(&boxes[2 * (size_t)item]), hi = __ldg(&boxes[2 * (size_t)item + 1]);
+    c.bl[0] = lo.x; c.bl[1] = lo.y; c.bl[2] = lo.z;
+    c.bh[0] = hi.x; c.bh[1] = hi.y; c.bh[2] = hi.z;
+    c.cur = n - 1 + j;                               // relative to node0
+    c.l = c.r = j;
+    store_node(&nodes[c.cur], lo.x, lo.y, lo.z, ref0 + j, hi.x, hi.y, hi.z, LEAF_BIT | 1u);
+    aux[j] = item + ref_add;
+}
+
 template <typename K>
 __global__ void __launch_bounds__(256) lbvh_kernel(const K *__restrict__ codes, const uint32_t *__restrict__ items,
                                                    const float4 *__restrict__ boxes, uint32_t n, uint32_t node0,
@@ -328,51 +518,88 @@ __global__ void __launch_bounds__(256) lbvh_kernel(const K *__restrict__ codes, 
                                                    uint32_t *other, uint32_t *err) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    uint32_t item = __ldg(&items[j]);
-    if (item >= n) {                                            // (a sort that went wrong: said, not followed)
-        atomicOr(err, ST_TIMEOUT_SORT);
-        item = 0;
-    }
-    float4 lo = __ldg(&boxes[2 * (size_t)item]), hi = __ldg(&boxes[2 * (size_t)item + 1]);
-    float bl[3] = {lo.x, lo.y, lo.z}, bh[3] = {hi.x, hi.y, hi.z};
-    uint32_t cur = n - 1 + j;                                   // relative to node0
-    store_node(&nodes[cur], bl[0], bl[1], bl[2], ref0 + j, bh[0], bh[1], bh[2], LEAF_BIT | 1u);
-    aux[j] = item + ref_add;
+    Climb c;
+    lbvh_leaf(c, j, items, boxes, n, ref0, ref_add, nodes, aux, err);
     if (n == 1) return;
-    uint32_t l = j, r = j;
-    bool left = is_left_child(codes, l, r, n);
-    while (true) {
-        const uint32_t split = left ? r : l - 1;
-        __threadfence();                                        // our node before the exchange
-        const uint32_t got = atomicExch(&other[split], left ? l : r);
-        if (got == 0xffffffffu) return;                         // the sibling makes the parent
-        __threadfence();
-        uint32_t L, R, lc, rc;
-        if (left) { L = l; R = got; lc = cur; rc = got == split + 1 ? n + split : split + 1; }
-        else { L = got; R = r; rc = cur; lc = got == split ? n - 1 + split : split; }
-        const uint32_t sib = left ? rc : lc;
-        const float4 *sp = reinterpret_cast<const float4 *>(&nodes[sib]);
-        float4 s0 = __ldcg(sp), s1 = __ldcg(sp + 1);
-        float al[3], ah[3], cl[3], ch[3];                        // left child's box, right child's
-        if (left) {
-            al[0] = bl[0]; al[1] = bl[1]; al[2] = bl[2]; ah[0] = bh[0]; ah[1] = bh[1]; ah[2] = bh[2];
-            cl[0] = s0.x; cl[1] = s0.y; cl[2] = s0.z; ch[0] = s1.x; ch[1] = s1.y; ch[2] = s1.z;
-        } else {
-            al[0] = s0.x; al[1] = s0.y; al[2] = s0.z; ah[0] = s1.x; ah[1] = s1.y; ah[2] = s1.z;
-            cl[0] = bl[0]; cl[1] = bl[1]; cl[2] = bl[2]; ch[0] = bh[0]; ch[1] = bh[1]; ch[2] = bh[2];
+    c.left = is_left_child(codes, j, j, n);
+    lbvh_climb(c, codes, n, node0, nodes, other);
+}
+
+// The climb is a chain of exchanges, a level after a level, each a trip through memory. A short list
+// is one such chain long whatever its length, so there a block first joins what meets among its own 512
+// leaves, with the exchange, the boxes and the codes in shared memory; what is left over - a subtree
+// whose sibling reaches out of the block - goes on through memory, from where it was left. A long
+// list has the blocks to cover the trips, and the barrier costs it more than they do: LB_SHARED_TO is
+// the line (whole builds, 30-bit keys, through memory against in blocks: 65k items 118 and 116 us, 202k
+// 137 and 139, 871k 226 and 231, 4M 684 and 702).
+constexpr int LB_THREADS = 512;
+constexpr uint32_t LB_SHARED_TO = 1u << 16;
+
+template <typename K>
+__global__ void __launch_bounds__(LB_THREADS) lbvh_block_kernel(const K *__restrict__ codes, const uint32_t *__restrict__ items,
+                                                                const float4 *__restrict__ boxes, uint32_t n, uint32_t node0,
+                                                                uint32_t ref0, uint32_t ref_add, Node *nodes,
+                                                                uint32_t *__restrict__ aux, uint32_t *other, uint32_t *err) {
+    __shared__ K s_code[LB_THREADS + 2];             // codes of leaves b0 - 1 .. b0 + LB_THREADS
+    __shared__ uint32_t s_met[LB_THREADS];           // split b0 + i: 0 nobody yet, 1 its left child, 2 its right one, 3 both
+    __shared__ float s_box[2][LB_THREADS][6];        // the child waiting there: its box, its far end and node
+    __shared__ uint32_t s_end[2][LB_THREADS], s_cur[2][LB_THREADS];
+    const uint32_t t = threadIdx.x, b0 = blockIdx.x * LB_THREADS, j = b0 + t;
+    s_met[t] = 0;
+    for (uint32_t i = t; i < LB_THREADS + 2; i += LB_THREADS) {
+        const uint32_t q = b0 + i - 1u;              // (wraps below 0: past n)
+        s_code[i] = q < n ? codes[q] : K(0);
+    }
+    __syncthreads();
+    // (delta_at over the codes here, for leaves of this block and the one before and after)
+    auto delta = [&](uint32_t i, uint32_t k) {
+        const K a = s_code[i - b0 + 1u], b = s_code[k - b0 + 1u];
+        if constexpr (sizeof(K) == 4) return a == b ? 32 + __clz(i ^ k) : __clz(a ^ b);
+        else return a == b ? 64 + __clz(i ^ k) : __clzll((long long)(a ^ b));
+    };
+    auto left_child = [&](uint32_t l, uint32_t r) { return l == 0 || (r != n - 1 && delta(r, r + 1) > delta(l - 1, l)); };
+    Climb c;
+    bool going = j < n, out = false;                 // out: to be gone on with through memory
+    if (going) {
+        lbvh_leaf(c, j, items, boxes, n, ref0, ref_add, nodes, aux, err);
+        if (n == 1) going = false;
+        else c.left = left_child(j, j);
+    }
+    while (going) {
+        const uint32_t split = c.left ? c.r : c.l - 1, i = split - b0;
+        if (i >= LB_THREADS - 1) {                   // (the sibling is another block's)
+            out = true;
+            break;
         }
+        const int side = c.left ? 0 : 1;
 #pragma unroll
-        for (int k = 0; k < 3; k++) { bl[k] = wmin(al[k], cl[k]); bh[k] = wmax(ah[k], ch[k]); }
+        for (int k = 0; k < 3; k++) { s_box[side][i][k] = c.bl[k]; s_box[side][i][3 + k] = c.bh[k]; }
+        s_end[side][i] = c.left ? c.l : c.r;
+        s_cur[side][i] = c.cur;
+        __threadfence_block();                       // our child before the word that shows it
+        if (atomicExch(&s_met[i], 1u + side) == 0u) break;   // the sibling makes the parent
+        __threadfence_block();
+        s_met[i] = 3u;
+        const volatile float *sb = s_box[1 - side][i];
+        const float sl[3] = {sb[0], sb[1], sb[2]}, sh[3] = {sb[3], sb[4], sb[5]};
+        const uint32_t got = *(volatile uint32_t *)&s_end[1 - side][i];
+        const uint32_t L = c.left ? c.l : got, R = c.left ? got : c.r;
         const bool root = L == 0 && R == n - 1;
-        bool pleft = false;
-        uint32_t pidx = 0;
-        if (!root) {
-            pleft = is_left_child(codes, L, R, n);
-            pidx = pleft ? R : L;
-        }
-        store_node(&nodes[pidx], bl[0], bl[1], bl[2], node0 + lc, bh[0], bh[1], bh[2], node0 + rc);
-        if (root) return;
-        cur = pidx; l = L; r = R; left = pleft;
+        if (lbvh_parent<K>(c, got, sl, sh, !root && left_child(L, R), n, node0, nodes)) break;
+    }
+    __syncthreads();
+    // through memory: this thread's own subtree, then the one left waiting at split b0 + t
+    if (out) lbvh_climb(c, codes, n, node0, nodes, other);
+    const uint32_t met = s_met[t];
+    if (met == 1u || met == 2u) {
+        const int side = (int)met - 1;
+        c.left = side == 0;
+        c.l = c.left ? s_end[0][t] : b0 + t + 1u;
+        c.r = c.left ? b0 + t : s_end[1][t];
+        c.cur = s_cur[side][t];
+#pragma unroll
+        for (int k = 0; k < 3; k++) { c.bl[k] = s_box[side][t][k]; c.bh[k] = s_box[side][t][3 + k]; }
+        lbvh_climb(c, codes, n, node0, nodes, other);
     }
 }
 
@@ -886,7 +1113,7 @@ static size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 // kernel attributes set once per device (a context is used from one host thread at a time, as the
 // reference's Gpu is: engine/gpu/gpu.h:32-42)
 struct DevCache {
-    bool os_attr[2];
+    bool os_attr[2], ss_attr[2];
     int ploc_per_sm;
 };
 static DevCache g_dev_cache[64];
@@ -1006,18 +1233,28 @@ static cudaError_t build_typed(const lrc_build_params &p, const float *d_boxes, 
     uint32_t *status = reinterpret_cast<uint32_t *>(scratch + L.status);
     uint32_t *counters = reinterpret_cast<uint32_t *>(scratch + L.counters);
     if (tm) tm->begin(LRC_TS_MORTON, st);
-    cudaError_t e = cudaMemsetAsync(scratch + L.hist, 0, L.counters + (size_t)P * 4 - L.hist, st);
-    if (e) return e;
+    cudaError_t e = cudaSuccess;
     const float4 *boxes = reinterpret_cast<const float4 *>(d_boxes);
-    {
-        int grid = (int)std::min<uint64_t>(((uint64_t)n + MH_THREADS - 1) / MH_THREADS, (uint64_t)num_sms * 8);
-        morton_hist_kernel<K><<<std::max(grid, 1), MH_THREADS, 0, st>>>(
-            boxes, n, make_float3(p.lo[0], p.lo[1], p.lo[2]), make_float3(p.ext[0], p.ext[1], p.ext[2]), dlo_ext, ca, hist);
-    }
-    if (tm) tm->begin(LRC_TS_SORT, st);
+    const float3 plo = make_float3(p.lo[0], p.lo[1], p.lo[2]), pext = make_float3(p.ext[0], p.ext[1], p.ext[2]);
     K *kin = ca, *kout = cb;
     uint32_t *vin = va, *vout = vb;
-    onesweep_passes<K>(kin, kout, vin, vout, n, hist, status, counters, L.tiles, d_status, st);
+    if (n <= (uint32_t)SS_ITEMS) {
+        // (one block has them all)
+        if (tm) tm->begin(LRC_TS_SORT, st);
+        bool &attr = dev_cache().ss_attr[sizeof(K) == 8];
+        if (!attr) {
+            cudaFuncSetAttribute(small_sort_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SsShared<K>));
+            attr = true;
+        }
+        small_sort_kernel<K><<<1, SS_THREADS, sizeof(SsShared<K>), st>>>(boxes, n, plo, pext, dlo_ext, kin, vin);
+    } else {
+        e = cudaMemsetAsync(scratch + L.hist, 0, L.counters + (size_t)P * 4 - L.hist, st);
+        if (e) return e;
+        int grid = (int)std::min<uint64_t>(((uint64_t)n + MH_THREADS - 1) / MH_THREADS, (uint64_t)num_sms * 8);
+        morton_hist_kernel<K><<<std::max(grid, 1), MH_THREADS, 0, st>>>(boxes, n, plo, pext, dlo_ext, ca, hist);
+        if (tm) tm->begin(LRC_TS_SORT, st);
+        onesweep_passes<K>(kin, kout, vin, vout, n, hist, status, counters, L.tiles, d_status, st);
+    }
     // sorted: codes in kin, items in vin
     if (d_sorted_codes_out)
         cudaMemcpyAsync(d_sorted_codes_out, kin, (size_t)n * sizeof(K), cudaMemcpyDeviceToDevice, st);
@@ -1026,7 +1263,10 @@ static cudaError_t build_typed(const lrc_build_params &p, const float *d_boxes, 
     if (!ploc) {
         uint32_t *other = reinterpret_cast<uint32_t *>(scratch + L.other);
         if (n > 1) cudaMemsetAsync(other, 0xff, (size_t)(n - 1) * 4, st);
-        lbvh_kernel<K><<<blocks, 256, 0, st>>>(kin, vin, boxes, n, p.node0, p.ref0, p.ref_add, d_nodes, d_aux, other, d_status);
+        if (n <= LB_SHARED_TO)
+            lbvh_block_kernel<K><<<(n + LB_THREADS - 1) / LB_THREADS, LB_THREADS, 0, st>>>(kin, vin, boxes, n, p.node0, p.ref0, p.ref_add, d_nodes, d_aux, other, d_status);
+        else
+            lbvh_kernel<K><<<blocks, 256, 0, st>>>(kin, vin, boxes, n, p.node0, p.ref0, p.ref_add, d_nodes, d_aux, other, d_status);
         if (tm) tm->end(st);
         return cudaGetLastError();
     }
