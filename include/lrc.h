@@ -157,15 +157,16 @@ int lrc_scene_tree_device(lrc_scene *s, const uint32_t **nodes, const uint32_t *
  * change of its shapes, replaces it. lrc_scene_tree then copies out nnodes and naux entries. */
 int lrc_scene_set_tree(lrc_scene *s, const uint32_t *nodes, uint32_t nnodes, const uint32_t *aux, uint32_t naux,
                        unsigned flags);
-/* The walk's tree of a scene of triangles alone (no primitives). mode 1 (the default): after each
- * lrc_scene_build or lrc_scene_set_tree, the ray queries below (closest hit, any hit, walk
- * statistics) follow a copy of the tree - the same nodes and leaves - whose boxes are the
- * triangles' own bounds widened by 2^-17 of the root box's largest coordinate (at most the 1e-3
- * of triangle_bounds, scene.c:65-74), inner boxes their unions: the same hits as the padded tree,
- * fewer box tests where the padding is large beside the triangles. mode 2: that tree collapsed
- * into 8-wide nodes with their children's boxes quantised to bytes (80 bytes a node; a tree whose
- * leaves hold more triangles than a node's slots keeps mode 1). mode 0: the tree as built.
- * lrc_scene_tree always gives the tree as built (the reference's); the path tracer walks that. */
+/* The walk's tree of a scene of triangles alone (no primitives). Modes 1 (the default) and 2: after
+ * each lrc_scene_build or lrc_scene_set_tree, the ray queries below (closest hit, any hit) follow a
+ * copy of the tree whose boxes are the triangles' own bounds widened by 2^-17 of the root box's
+ * largest coordinate (at most the 1e-3 of triangle_bounds, scene.c:65-74), inner boxes their unions,
+ * collapsed into 8-wide nodes with their children's boxes quantised to bytes (80 bytes a node; a given
+ * tree whose leaves hold more than 8 shapes, or that names a node twice, is walked as it is): the same
+ * hits as the tree as built, two shapes hit at the same t among them (the binary walk decides those).
+ * The modes differ in what lrc_scene_trace_stats counts: 1 the binary walk of that copy, 2 the wide
+ * one. mode 0: the tree as built. lrc_scene_tree always gives the tree as built (the reference's); the
+ * path tracer walks that tree's own 8-wide nodes, made when it first traces it. */
 int lrc_scene_set_walk(lrc_scene *s, int mode);
 
 /* Closest hits of nrays rays (origins, directions: 3 floats each) in (tmin, tmax) through the
@@ -178,7 +179,7 @@ int lrc_scene_intersect(lrc_scene *s, const float *orig, const float *dir, uint6
 int lrc_scene_occluded(lrc_scene *s, const float *orig, const float *dir, const float *tmax, uint64_t nrays,
                        float tmin, uint8_t *out, unsigned flags);
 /* The closest-hit walk of lrc_scene_intersect, counting instead of answering: stats[0] = box tests
- * (32-byte node records read; with the 8-wide walk, each 80-byte node read counts 2.5), stats[1] =
+ * (32-byte node records read; in walk mode 2, each 80-byte node read counts 2.5), stats[1] =
  * triangle tests (48-byte triangles read), over all rays.
  * The traversal's algorithmic bytes (as the reference's tree statistics, LR_GPU_BVH_CHECK's cost
  * and depth, trace_gpu.c:768-805, describe a tree). stats: host. */
@@ -327,7 +328,7 @@ int lrc_trace(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows,
 #define LRC_TRACE_GUIDED 64u  /* flag: accum is the denoiser's 4 planes (below); each sample's luminance
                                  over the guide's albedo is added to plane 1's (sum l, sum l^2) */
 #define LRC_TRACE_MEGAKERNEL 256u  /* flag: the one-kernel path tracer whatever the size */
-#define LRC_TRACE_WAVEFRONT_PATHS (1u << 20)
+#define LRC_TRACE_WAVEFRONT_PATHS (3u << 15)   /* 98304: where the two take the same time (256 x 256 is below) */
 
 /* ---- the denoiser: replaces gpu_denoise_create / gpu_denoise_encode (engine/gpu/denoise_gpu.c;
  * denoise.wgsl `prep`, `atrous`) and the guide pass `gbuf` (trace.wgsl:1045-1104, 1319-1337) ----
@@ -457,7 +458,7 @@ int lrc_batch_rays(lrc_batch *b, uint64_t *per_job, uint64_t *total);
 int lrc_batch_passes(lrc_batch *b, uint32_t *passes, uint64_t *kernels);
 /* The last LRC_BATCH_STEPPED run of the wavefront (each optional): its closest-hit kernel's device
  * time (CUDA events around each launch) and the rays it traced; with LRC_BATCH_COUNT its walks' box
- * tests (32-byte node records read) and triangle tests (48-byte triangles read), counted by a
+ * tests (32-byte node records read; an 80-byte wide node counts 2.5) and triangle tests (48-byte triangles read), counted by a
  * counting build of that kernel (for the launch shapes of 128 threads, registers capped for 4 or 8
  * blocks an SM, the default's among them; with other shapes the counts are 0; it tests what the
  * plain one does: the same hits, the images the same to the bit); and the kernels the run

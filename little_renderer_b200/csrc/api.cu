@@ -32,6 +32,8 @@ int scene_build_on(lrc_scene *s, int builder, int key_bits, void **scratch, size
     s->tree_nnodes = s->tree_naux = 0;
     s->walk_ok = false;
     s->wide_ok = false;
+    s->pwide_ok = false;
+    s->most_leaf = 1;
     if (!n) return LRC_OK;
     const size_t need_scratch = lrc::build_scratch_bytes(n, key_bits, builder);
     if (no_alloc) {
@@ -70,6 +72,27 @@ int scene_build_on(lrc_scene *s, int builder, int key_bits, void **scratch, size
                                       c->num_sms, st, nullptr, timer);
     if (e) return cuda_status(c, e, "lrc_scene_build");
     s->built_n = n;
+    return LRC_OK;
+}
+
+int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc) {
+    if (s->pwide_ok || !s->built_n || !s->most_leaf || s->most_leaf > kMostLeaf) return LRC_OK;
+    lrc_ctx *c = s->ctx;
+    const bool single = !s->tree_nnodes;
+    const uint32_t nn = single ? 2 * s->built_n - 1 : s->tree_nnodes, na = single ? s->built_n : s->tree_naux;
+    const size_t bytes = lrc::wide_bytes(na, single);
+    if (s->pwide_cap < bytes) {
+        if (no_alloc) return fail(c, LRC_E_INVALID, "a build to capture needs its buffers sized by an earlier run");
+        if (s->d_pwide) cudaStreamSynchronize(c->st);   // (work that walks the old ones)
+        if (reserve(&s->d_pwide, &s->pwide_cap, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return LRC_OK;
+        }
+    }
+    cudaError_t e = lrc::wide_build(s->d_nodes, nn, s->d_aux, na, s->nprims, reinterpret_cast<const float *>(s->d_tris), s->ntris,
+                                    s->d_pwide, single, c->d_status, c->num_sms, st);
+    if (e) return cuda_status(c, e, "the path tracer's wide nodes");
+    s->pwide_ok = true;
     return LRC_OK;
 }
 
@@ -114,41 +137,60 @@ int make_walk(lrc_scene *s) {
     c->timer.end(c->st);
     if (e) return cuda_status(c, e, "the walk's tree");
     s->walk_ok = true;
-    if (s->walk_mode != 2) return LRC_OK;
-    // the 8-wide nodes from it (a tree whose leaves do not fit a node's slots keeps the binary walk)
-    const size_t wcap = lrc::wide_node_cap((uint32_t)na);
-    if (s->wide_cap < wcap) {
-        cudaFree(s->d_wide);
-        s->d_wide = nullptr;
-        s->wide_cap = 0;
-        e = cudaMalloc(&s->d_wide, wcap * 80);
-        if (!e) s->wide_cap = wcap;
-    }
-    if (!e && s->wrefs_cap < wcap) {
-        cudaFree(s->d_wrefs);
-        s->d_wrefs = nullptr;
-        s->wrefs_cap = 0;
-        e = cudaMalloc(&s->d_wrefs, wcap * 4);
-        if (!e) s->wrefs_cap = wcap;
-    }
-    if (!e) e = reserve(&c->scratch, &c->scratch_cap, lrc::wide_scratch_bytes((uint32_t)na));
-    c->timer.begin(LRC_TS_HIERARCHY, c->st);
-    uint32_t nwide = 0;
-    if (!e) e = lrc::wide_build(s->d_wnodes, (uint32_t)nn, s->d_aux, (uint32_t)na, reinterpret_cast<const float *>(s->d_tris),
-                                s->ntris, s->d_wide, (uint32_t)s->wide_cap, s->d_wrefs, (uint32_t)s->wrefs_cap, c->scratch,
-                                c->scratch_cap, c->d_status, c->st, &nwide);
-    c->timer.end(c->st);
-    if (e) return cuda_status(c, e, "the walk's wide tree");
-    uint32_t status = 0;
-    e = cudaMemcpy(&status, c->d_status, 4, cudaMemcpyDeviceToHost);
-    if (e) return cuda_status(c, e, "the walk's wide tree");
-    if (status & lrc::ST_BAD_TREE) {                   // (leaves too large: the binary walk stays)
-        cudaMemset(c->d_status, 0, 4);
+    // the wide nodes from it (a tree with larger leaves than a node has slots, or no memory: the binary walk)
+    const bool single = !s->tree_nnodes;
+    if (!s->most_leaf || s->most_leaf > kMostLeaf) return LRC_OK;
+    if (reserve(&s->d_wide, &s->wide_cap, lrc::wide_bytes((uint32_t)na, single)) != cudaSuccess) {
+        cudaGetLastError();
         return LRC_OK;
     }
-    s->nwide = nwide;
-    s->wide_ok = nwide > 0;
+    c->timer.begin(LRC_TS_HIERARCHY, c->st);
+    e = lrc::wide_build(s->d_wnodes, (uint32_t)nn, s->d_aux, (uint32_t)na, 0, reinterpret_cast<const float *>(s->d_tris),
+                        s->ntris, s->d_wide, single, c->d_status, c->num_sms, c->st);
+    c->timer.end(c->st);
+    if (e) return cuda_status(c, e, "the walk's wide nodes");
+    s->wide_ok = true;
     return LRC_OK;
+}
+
+// A large image runs as a one-job batch on the wavefront engine: its kernels keep their own registers
+// (the one-kernel path sits at its cap with every bounce's code in one loop), and its image is the
+// call's to the bit (a batch task traces a pixel's samples as the one-kernel path's lanes do and the
+// resolve pass adds them in that path's order). The line (LRC_TRACE_WAVEFRONT_PATHS): a pass of the
+// wavefront waits for its longest walk whatever its size, which the one-kernel path does not; scenes of 4k
+// / 20k / 200k triangles at 256 x 256 pixels, 1 spp: the one-kernel path 0.83 / 1.13 / 1.36 ms, the
+// wavefront 1.08 / 1.46 / 1.67; at 360 x 360 1.45 / 1.77 / 2.26 and 1.23 / 1.65 / 1.90.
+bool wavefront_call(const lrc_scene *s, const lrc_trace_params *p, int32_t rows, uint32_t spp) {
+    const uint64_t paths = (uint64_t)p->width * (uint64_t)rows * spp;
+    return !s->nvol && rows > 0 && spp > 0 && paths >= LRC_TRACE_WAVEFRONT_PATHS;
+}
+
+int trace_wavefront(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows, uint32_t spp0, uint32_t spp,
+                    float *d_acc, bool guided) {
+    lrc_ctx *c = s->ctx;
+    int rc = LRC_OK;
+    if (!c->single) {
+        rc = lrc_batch_create(c, &c->single);
+        if (rc) return rc;
+    }
+    // The paths in flight: all of them up to 2^22, in three sizes (a size's graph is captured when it is
+    // first used, and two are kept): a pass costs most in its longest walks, so there should be few.
+    // 640 x 640 pixels at 8 spp of 20k triangles: 2^20 12.4 ms, 2^21 11.9, 2^22 11.2. Up to 2^21 paths the
+    // walks run 6 blocks an SM (their registers unspilled: 410k paths 2.65 -> 2.50 ms), with more paths
+    // the default's 8 (3.3M paths: 11.55 against 11.19 ms).
+    const uint64_t tasks = (uint64_t)p->width * (uint64_t)rows * (p->exact ? 1u : std::min<uint32_t>(spp, 16u));
+    uint32_t slots = 1u << 18;
+    while (slots < tasks && slots < (1u << 22)) slots <<= 2;
+    const int32_t shape = tasks <= (1u << 21) ? lrc::LRC_WAVEFRONT_SMALL_VARIANT : LRC_WAVEFRONT_DEFAULT_VARIANT;
+    for (;; slots = 1u << 20) {
+        rc = lrc_batch_set_wavefront(c->single, slots, shape);
+        if (!rc) rc = lrc_batch_clear(c->single);
+        if (!rc) rc = guided ? lrc_batch_add_guided(c->single, s, p, y0, rows, spp0, spp, d_acc, -1, 30)
+                             : lrc_batch_add(c->single, s, p, y0, rows, spp0, spp, d_acc, -1, 30);
+        if (!rc) rc = lrc_batch_run(c->single, 0);
+        if (rc != LRC_RETRY || slots <= (1u << 20)) break;   // (no memory for so many: fewer)
+    }
+    return rc;
 }
 
 }  // namespace lrcapi
@@ -339,7 +381,7 @@ void lrc_scene_destroy(lrc_scene *s) {
     cudaFree(s->d_nodes);
     cudaFree(s->d_wnodes);
     cudaFree(s->d_wide);
-    cudaFree(s->d_wrefs);
+    cudaFree(s->d_pwide);
     cudaFree(s->d_aux);
     cudaFree(s->d_boxes);
     cudaFree(s->d_small);
@@ -377,6 +419,7 @@ int lrc_scene_set_triangles(lrc_scene *s, const uint32_t *tris, uint32_t n, unsi
     s->tree_nnodes = s->tree_naux = 0;
     s->walk_ok = false;
     s->wide_ok = false;
+    s->pwide_ok = false;
     if (!(flags & LRC_DEVICE)) return check_status(c);   // (the host array may be freed on return)
     return LRC_OK;
 }
@@ -415,23 +458,40 @@ int lrc_scene_set_tree(lrc_scene *s, const uint32_t *nodes, uint32_t nnodes, con
     lrc_ctx *c = s->ctx;
     const uint64_t shapes = (uint64_t)s->nprims + s->ntris;
     if (!shapes) return fail(c, LRC_E_INVALID, "the scene has no shapes (primitives or triangles) for a tree");
+    uint32_t most = 0;                                   // (device arrays are not looked into)
     if (!(flags & LRC_DEVICE)) {
+        std::vector<bool> named(nnodes, false);          // (a node named twice, entries in two leaves, an empty
+        uint64_t entries = 0;                            //  leaf: walked as given, not collapsed)
+        bool plain = true;
+        auto child = [&](uint32_t k) {
+            plain = plain && !named[k];
+            named[k] = true;
+        };
         // a tree the walks can follow: children and leaf ranges inside the arrays, shapes that exist
         for (uint32_t i = 0; i < nnodes; i++) {
             const uint32_t a = nodes[8 * (size_t)i + 3], b = nodes[8 * (size_t)i + 7];
             if (b & lrc::LEAF_BIT) {
                 const uint32_t cnt = b & ~lrc::LEAF_BIT;
                 if (a >= naux || cnt > naux - a) return fail(c, LRC_E_INVALID, "a leaf's entries lie outside aux");
+                most = std::max(most, cnt);
+                entries += cnt;
+                plain = plain && cnt;
             } else if (a >= nnodes || b >= nnodes) {
                 return fail(c, LRC_E_INVALID, "a node's child lies outside the nodes");
+            } else {
+                child(a);
+                child(b);
             }
         }
+        if (!plain || named[0] || entries > naux) most = 0;
         for (uint32_t i = 0; i < naux; i++)
             if (aux[i] >= shapes) return fail(c, LRC_E_INVALID, "an aux entry names no shape of the scene");
     }
     DeviceGuard g(c->device);
     s->walk_ok = false;
     s->wide_ok = false;
+    s->pwide_ok = false;
+    s->most_leaf = most;
     const size_t cap = std::max<size_t>(naux, ((size_t)nnodes + 1) / 2);   // (2 cap - 1 nodes, cap aux)
     cudaError_t e = cudaSuccess;
     if (s->tree_cap < cap) {
@@ -520,6 +580,10 @@ int lrc_scene_intersect(lrc_scene *s, const float *orig, const float *dir, uint6
     if (!s->built_n) return fail(c, LRC_E_INVALID, "the scene has no built BVH (lrc_scene_build)");
     DeviceGuard g(c->device);
     lrc::TraceTables tt = tables(s);
+    if (s->nprims) {
+        int rc = scene_wide(s, c->st, false);
+        if (rc) return rc;
+    }
     // LRC_SORT_RAYS: the reordering's scratch (large batches); without it the rays go in their order
     void *sort_scratch = nullptr;
     if ((flags & LRC_SORT_RAYS) && lrc::intersect_scratch_bytes(nrays)) {
@@ -529,7 +593,8 @@ int lrc_scene_intersect(lrc_scene *s, const float *orig, const float *dir, uint6
     // a world with primitives walks shape ids (primitives, then triangles); a mesh, triangles alone
     auto run = [&](const float *o, const float *d, int32_t *p, float *tt_out) {
         if (s->nprims) return lrc::pt_intersect(pt_scene(s), o, d, nrays, tmin, tmax, p, nullptr, tt_out, c->d_status, c->st);
-        if (s->wide_ok) return lrc::wide_intersect(wide_tables(s), o, d, nrays, tmin, tmax, p, tt_out, c->d_status, c->st);
+        if (s->wide_ok && !sort_scratch)
+            return lrc::wide_intersect(wide_tables(s), tt, o, d, nrays, tmin, tmax, p, tt_out, c->d_status, c->st);
         return lrc::intersect_device(tt, o, d, nrays, tmin, tmax, p, tt_out, c->d_status, c->st, c->num_sms, sort_scratch,
                                      c->scratch_cap);
     };
@@ -577,12 +642,14 @@ int lrc_scene_trace_stats(lrc_scene *s, const float *orig, const float *dir, uin
         d_o = o;
         d_d = d;
     }
-    if (!e) e = s->wide_ok ? lrc::wide_count(wide_tables(s), d_o, d_d, nrays, tmin, tmax, d_stats, c->d_status, c->st)
-                           : lrc::count_device(tt, d_o, d_d, nrays, tmin, tmax, d_stats, c->d_status, c->st);
+    // (mode 2 counts the wide walk, mode 1 the binary one over the tree the wide nodes are made from)
+    const bool wide = s->wide_ok && s->walk_mode == 2;
+    if (!e) e = wide ? lrc::wide_count(wide_tables(s), tt, d_o, d_d, nrays, tmin, tmax, d_stats, c->d_status, c->st)
+                     : lrc::count_device(tt, d_o, d_d, nrays, tmin, tmax, d_stats, c->d_status, c->st);
     if (!e) e = cudaMemcpyAsync(stats, d_stats, 16, cudaMemcpyDeviceToHost, c->st);
     if (e) return cuda_status(c, e, "lrc_scene_trace_stats");
     const int rc = check_status(c);
-    if (!rc && s->wide_ok) stats[0] = (stats[0] * 5 + 1) / 2;   // (an 80-byte wide node: 2.5 records of 32 bytes)
+    if (!rc && wide) stats[0] = (stats[0] * 5 + 1) / 2;   // (an 80-byte wide node: 2.5 records of 32 bytes)
     return rc;
 }
 
@@ -594,7 +661,7 @@ int lrc_scene_occluded(lrc_scene *s, const float *orig, const float *dir, const 
     DeviceGuard g(c->device);
     lrc::TraceTables tt = tables(s);
     if (flags & LRC_DEVICE) {
-        cudaError_t e = s->wide_ok ? lrc::wide_occluded(wide_tables(s), orig, dir, tmax, nrays, tmin, out, c->d_status, c->st)
+        cudaError_t e = s->wide_ok ? lrc::wide_occluded(wide_tables(s), tt, orig, dir, tmax, nrays, tmin, out, c->d_status, c->st)
                                    : lrc::occluded_device(tt, orig, dir, tmax, nrays, tmin, out, c->d_status, c->st);
         return cuda_status(c, e, "lrc_scene_occluded");
     }
@@ -608,7 +675,7 @@ int lrc_scene_occluded(lrc_scene *s, const float *orig, const float *dir, const 
     e = cudaMemcpyAsync(d_o, orig, nrays * 12, cudaMemcpyHostToDevice, c->st);
     if (!e) e = cudaMemcpyAsync(d_d, dir, nrays * 12, cudaMemcpyHostToDevice, c->st);
     if (!e) e = cudaMemcpyAsync(d_tm, tmax, nrays * 4, cudaMemcpyHostToDevice, c->st);
-    if (!e) e = s->wide_ok ? lrc::wide_occluded(wide_tables(s), d_o, d_d, d_tm, nrays, tmin, d_out, c->d_status, c->st)
+    if (!e) e = s->wide_ok ? lrc::wide_occluded(wide_tables(s), tt, d_o, d_d, d_tm, nrays, tmin, d_out, c->d_status, c->st)
                            : lrc::occluded_device(tt, d_o, d_d, d_tm, nrays, tmin, d_out, c->d_status, c->st);
     if (!e) e = cudaMemcpyAsync(out, d_out, nrays, cudaMemcpyDeviceToHost, c->st);
     if (e) return cuda_status(c, e, "lrc_scene_occluded");
@@ -630,6 +697,7 @@ int lrc_scene_set_prims(lrc_scene *s, const float *prims, uint32_t n, unsigned f
     s->tree_nnodes = s->tree_naux = 0;
     s->walk_ok = false;
     s->wide_ok = false;
+    s->pwide_ok = false;
     return (flags & LRC_DEVICE) ? LRC_OK : check_status(c);
 }
 
@@ -931,6 +999,10 @@ int lrc_scene_intersect_ex(lrc_scene *s, const float *orig, const float *dir, ui
     lrc_ctx *c = s->ctx;
     if (!s->built_n && !(s->meshes_built && s->tlas_n)) return fail(c, LRC_E_INVALID, "the scene has nothing built");
     DeviceGuard g(c->device);
+    {
+        int rc = scene_wide(s, c->st, false);
+        if (rc) return rc;
+    }
     if (flags & LRC_DEVICE) {
         cudaError_t e = lrc::pt_intersect(pt_scene(s), orig, dir, nrays, tmin, tmax, prim, inst, t, c->d_status, c->st);
         return cuda_status(c, e, "lrc_scene_intersect_ex");
@@ -967,6 +1039,10 @@ int lrc_trace(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows,
         int rc = lrc_scene_set_tables(s, nullptr, nullptr);
         if (rc) return rc;
     }
+    {
+        int rc = scene_wide(s, c->st, false);
+        if (rc) return rc;
+    }
     cudaError_t e = cudaSuccess;
     if (!s->d_rays) e = cudaMalloc(&s->d_rays, 256);
     if (!e) e = cudaMemsetAsync(s->d_rays, 0, 8, c->st);
@@ -1000,24 +1076,9 @@ int lrc_trace(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows,
         P.moments = reinterpret_cast<float4 *>(d_acc) + N;
         P.guide = reinterpret_cast<const float4 *>(d_acc) + 3 * N;
     }
-    // a large image runs as a one-job batch on the wavefront engine: its kernels keep their own
-    // registers (the one-kernel path sits at its cap with every bounce's code in one loop), and its
-    // image is this call's to the bit (a batch task traces a pixel's samples as the one-kernel
-    // path's lanes do and the resolve pass adds them in that path's order)
-    const uint64_t paths = (uint64_t)p->width * (uint64_t)rows * spp;
-    if (!e && !(flags & LRC_TRACE_MEGAKERNEL) && !s->nvol && rows > 0 && spp > 0 && paths >= LRC_TRACE_WAVEFRONT_PATHS) {
-        int rc = LRC_OK;
-        if (!c->single) {
-            rc = lrc_batch_create(c, &c->single);
-            if (rc) return rc;
-        }
-        rc = lrc_batch_set_wavefront(c->single, paths >= (8u << 20) ? 1u << 22 : 1u << 20,
-                                     LRC_WAVEFRONT_DEFAULT_VARIANT);
-        if (!rc) rc = lrc_batch_clear(c->single);
-        if (!rc) rc = guided ? lrc_batch_add_guided(c->single, s, p, y0, rows, spp0, spp, d_acc, -1, 30)
-                             : lrc_batch_add(c->single, s, p, y0, rows, spp0, spp, d_acc, -1, 30);
+    if (!e && !(flags & LRC_TRACE_MEGAKERNEL) && wavefront_call(s, p, rows, spp)) {
         c->timer.begin(LRC_TS_SHADE, c->st);
-        if (!rc) rc = lrc_batch_run(c->single, 0);
+        int rc = trace_wavefront(s, p, y0, rows, spp0, spp, d_acc, guided);
         c->timer.end(c->st);
         if (rc) return rc;
         if (!(flags & LRC_DEVICE)) {

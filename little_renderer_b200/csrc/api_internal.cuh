@@ -40,12 +40,13 @@ struct lrc_scene {
     size_t wnodes_cap = 0;        // (nodes)
     bool walk_ok = false;         // d_wnodes is the current tree's
     int walk_mode = 1;            // 0 the tree as built, 1 tight boxes, 2 tight 8-wide nodes
-    float4 *d_wide = nullptr;     // the walk's 8-wide nodes (walk_mode 2) and their triangle entries
+    void *d_wide = nullptr;       // the ray queries' wide nodes, made from d_wnodes (walk_mode 1, 2)
     size_t wide_cap = 0;
-    uint32_t *d_wrefs = nullptr;
-    size_t wrefs_cap = 0;
-    uint32_t nwide = 0;
     bool wide_ok = false;
+    void *d_pwide = nullptr;      // the path tracer's wide nodes, made from d_nodes when first traced
+    size_t pwide_cap = 0;
+    bool pwide_ok = false;
+    uint32_t most_leaf = 1;       // the largest leaf of the tree (0: not known)
     float *d_boxes = nullptr;
     size_t boxes_cap = 0;
     uint32_t *d_small = nullptr;  // 6 bound keys, 6 bounds, 6 lo/ext
@@ -178,6 +179,7 @@ inline lrc::PtScene pt_scene(const lrc_scene *s) {
     S.root = 0;
     S.nnodes = s->tree_nnodes ? s->tree_nnodes : (s->built_n ? 2 * s->built_n - 1 : 0);
     S.naux = s->tree_nnodes ? s->tree_naux : s->built_n;
+    if (s->pwide_ok) S.wide = lrc::wide_view(s->d_pwide, S.naux, !s->tree_nnodes);
     S.prims = reinterpret_cast<const float4 *>(s->d_prims);
     S.nprims = s->nprims;
     S.tris = reinterpret_cast<const float4 *>(s->d_tris);
@@ -249,17 +251,26 @@ inline lrc::TraceTables tables(const lrc_scene *s) {
     return tt;
 }
 
-// the wide walk's view of a scene (walk_mode 2, made)
-inline lrc::WideTables wide_tables(const lrc_scene *s) {
-    lrc::WideTables wt{};
-    wt.nodes = s->d_wide;
-    wt.refs = s->d_wrefs;
-    wt.tris = reinterpret_cast<const float4 *>(s->d_tris);
-    wt.nnodes = s->nwide;
-    wt.nrefs = (uint32_t)std::min<size_t>(s->wrefs_cap, 0xffffffffu);
-    wt.ntris = s->ntris;
-    return wt;
+// the wide walk's view of a scene of triangles (made)
+inline lrc::WideScene wide_tables(const lrc_scene *s) {
+    return lrc::wide_view(s->d_wide, s->tree_nnodes ? s->tree_naux : s->built_n, !s->tree_nnodes);
 }
+
+// leaves of more entries than a wide node has slots are walked in the binary tree
+constexpr uint32_t kMostLeaf = 8;
+
+// the path tracer's wide nodes of the scene's world tree, on stream st, unless they are there: every
+// caller that traces paths asks first, so that a tree is collapsed once, by the first call that traces
+// it, and a build that is only queried or refitted does not pay for it. A tree that cannot be (no memory,
+// leaves too large) is walked as it is.
+// no_alloc: within a graph's capture (a buffer too small is then an error).
+int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc);
+
+// lrc_trace's way of a large image: whether a call goes the wavefront engine's way, and the call (device
+// image, or planes when guided)
+bool wavefront_call(const lrc_scene *s, const lrc_trace_params *p, int32_t rows, uint32_t spp);
+int trace_wavefront(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows, uint32_t spp0, uint32_t spp,
+                    float *d_acc, bool guided);
 
 // builds the scene's world tree (triangles and primitives) on stream st with the given scratch
 // arena; with no_alloc set, a buffer too small is an error instead of a cudaMalloc (the batch's

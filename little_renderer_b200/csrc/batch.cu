@@ -154,6 +154,8 @@ lrc::PtScene view_of(const lrc_batch::Job &J, bool building) {
         const uint32_t n = J.s->ntris + J.s->nprims;
         S.nnodes = n ? 2 * n - 1 : 0;
         S.naux = n;
+        // (its wide nodes are made behind the build, in the buffer an earlier run sized)
+        S.wide = n && J.s->pwide_cap >= lrc::wide_bytes(n, true) ? lrc::wide_view(J.s->d_pwide, n, true) : lrc::WideScene{};
     }
     return S;
 }
@@ -215,6 +217,7 @@ int build_job(lrc_batch *b, const lrc_batch::Job *J, cudaStream_t st, bool captu
     const int first = J->builder == 2 ? 0 : J->builder;
     int rc = scene_build_on(J->s, first, J->key_bits, &b->scratch, &b->scratch_cap, st, nullptr, capturing);
     if (!rc && J->builder == 2) rc = scene_build_on(J->s, 1, J->key_bits, &b->scratch, &b->scratch_cap, st, nullptr, capturing);
+    if (!rc) rc = scene_wide(J->s, st, capturing);
     return rc;
 }
 
@@ -226,6 +229,11 @@ uint32_t max_passes(const lrc_batch *b, unsigned long long limit);
 int prepare(lrc_batch *b, bool building) {
     lrc_ctx *c = b->ctx;
     const size_t nj = b->jobs.size();
+    for (const lrc_batch::Job &J : b->jobs) {
+        if (building && J.builder >= 0) continue;
+        int rc = scene_wide(J.s, c->st, false);
+        if (rc) return rc;
+    }
     b->order.resize(nj);
     std::iota(b->order.begin(), b->order.end(), 0u);
     // longest-processing-time order: samples per task, then pixels, most first
@@ -508,7 +516,11 @@ int tune_wavefront(lrc_batch *b, unsigned long long n, int32_t *variant, int32_t
 }
 
 void note_built(lrc_batch *b) {   // (what captured builds' host side records)
-    for (const lrc_batch::Job *J : builds_of(b)) J->s->built_n = J->s->ntris + J->s->nprims;
+    for (const lrc_batch::Job *J : builds_of(b)) {
+        J->s->built_n = J->s->ntris + J->s->nprims;
+        J->s->most_leaf = 1;
+        J->s->pwide_ok = J->s->built_n && J->s->pwide_cap >= lrc::wide_bytes(J->s->built_n, true);
+    }
 }
 
 }  // namespace

@@ -98,7 +98,7 @@ __device__ __forceinline__ unsigned long long fetch_stream(unsigned long long *n
 // per, photons)). INST = false: the world alone (no two-level walk compiled in). MINB: the
 // register cap's blocks per SM.
 template <bool INST, int MINB>
-__global__ void __launch_bounds__(128, MINB) caustics_kernel(PtScene S, PtParams P, unsigned long long photons,
+__global__ void __launch_bounds__(128, MINB) caustics_kernel(const __grid_constant__ PtScene S, const __grid_constant__ PtParams P, unsigned long long photons,
                                                              unsigned long long per, uint64_t seed, double scale,
                                                              unsigned long long *__restrict__ sums,
                                                              unsigned long long *next, unsigned long long *ray_count,
@@ -322,8 +322,12 @@ int lt_check(lrc_scene *s, const lrc_trace_params *p, uint64_t photons, bool *sk
     if (!s->d_mats || !s->nmats) return fail(c, LRC_E_INVALID, "the scene has no materials (lrc_scene_set_materials)");
     if (s->light >= (int32_t)s->nprims) return fail(c, LRC_E_INVALID, "the light is not one of the primitives");
     *skip = photons == 0 || s->light < 0 || !s->specular;
-    if (!*skip && !s->tables) return lrc_scene_set_tables(s, nullptr, nullptr);
-    return LRC_OK;
+    if (*skip) return LRC_OK;
+    if (!s->tables) {
+        int rc = lrc_scene_set_tables(s, nullptr, nullptr);
+        if (rc) return rc;
+    }
+    return scene_wide(s, c->st, false);
 }
 
 int lt_run(lrc_scene *s, const lrc_trace_params *p, uint64_t photons, uint64_t seed, unsigned long long *d_sums,

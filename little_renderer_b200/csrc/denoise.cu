@@ -316,12 +316,12 @@ __global__ void __launch_bounds__(256) atrous_kernel(const float4 *__restrict__ 
 
 // ---- the guide: the ray through the pixel's centre to the first rough surface, through mirrors
 // and glass (refracting unless the glass reflects all), with the albedo of the whole way ------
-__global__ void __launch_bounds__(128) guide_kernel(PtScene S, PtParams P, float4 *__restrict__ planes,
-                                                    uint32_t *err) {
+__global__ void __launch_bounds__(128) guide_kernel(const __grid_constant__ PtScene S, const __grid_constant__ PtParams P,
+                                                    float4 *__restrict__ planes, uint32_t *err) {
     using namespace pt;
     const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
     const size_t N = (size_t)P.W * P.H;
-    if (idx >= N) return;
+    const bool in = idx < N;
     const uint32_t x = idx % P.W, y = idx / P.W;
     const V3 pc = vsub(vadd(P.upper_left, vscale(P.horizontal, (x + 0.5f) / (float)P.W)),
                        vscale(P.vertical, (y + 0.5f) / (float)P.H));
@@ -329,9 +329,11 @@ __global__ void __launch_bounds__(128) guide_kernel(PtScene S, PtParams P, float
     V3 gn = v3(0, 0, 0), ga = v3(1, 1, 1), a = v3(1, 1, 1);
     float gz = 1e30f, dist = 0.0f, kind = 1.0f;
     int ginst = -1;
-    for (int i = 0; i < 6; i++) {
+    bool go = in;                                    // (the warp's lanes walk together: warp_intersect)
+    for (int i = 0; i < 6 && __any_sync(0xffffffffu, go); i++) {
         Hit h;
-        if (!scene_intersect(S, ro, rd, RT_EPS, 1e30f, h, err)) break;
+        go = warp_intersect(S, go, ro, rd, RT_EPS, 1e30f, h, err);
+        if (!go) continue;
         Mat m = load_mat(S.mats, hit_material(S, h) & 63);
         if (textured(m)) m = hit_shading(S, h, ro, rd, vneg(rd), m);   // (shade_tex)
         // a lamp, or a surface glowing at least as bright as white paper under a light of 1
@@ -339,7 +341,8 @@ __global__ void __launch_bounds__(128) guide_kernel(PtScene S, PtParams P, float
             gn = h.n;
             gz = dist + h.t;
             ginst = h.inst;
-            break;
+            go = false;
+            continue;
         }
         Bsdf b = bsdf_make(m, h.front, S.tab);
         if (bsdf_rough_part(b)) {                    // a surface the light scatters on
@@ -348,7 +351,8 @@ __global__ void __launch_bounds__(128) guide_kernel(PtScene S, PtParams P, float
             ga = v3(a.x * m.albedo.x, a.y * m.albedo.y, a.z * m.albedo.z);
             kind = 0.0f;
             ginst = h.inst;
-            break;
+            go = false;
+            continue;
         }
         a = v3(a.x * m.albedo.x, a.y * m.albedo.y, a.z * m.albedo.z);
         dist += h.t;
@@ -360,6 +364,7 @@ __global__ void __launch_bounds__(128) guide_kernel(PtScene S, PtParams P, float
         ro = h.p;
         rd = vnorm(nxt);
     }
+    if (!in) return;
     const float w = kind + 4.0f * (float)(ginst >= 0 ? ((uint32_t)ginst & 0x3fffffu) + 1u : 0u);
     planes[2 * N + idx] = make_float4(gn.x, gn.y, gn.z, gz);
     planes[3 * N + idx] = make_float4(ga.x, ga.y, ga.z, w);
@@ -626,8 +631,11 @@ int scene_traceable(lrc_scene *s) {
     if (s->ninst && s->tlas_n != s->ninst) return fail(c, LRC_E_INVALID, "instances changed: lrc_scene_build_instances");
     if (!s->d_mats || !s->nmats) return fail(c, LRC_E_INVALID, "the scene has no materials (lrc_scene_set_materials)");
     if (s->light >= (int32_t)s->nprims) return fail(c, LRC_E_INVALID, "the light is not one of the primitives");
-    if (!s->tables) return lrc_scene_set_tables(s, nullptr, nullptr);
-    return LRC_OK;
+    if (!s->tables) {
+        int rc = lrc_scene_set_tables(s, nullptr, nullptr);
+        if (rc) return rc;
+    }
+    return scene_wide(s, c->st, false);
 }
 
 lrc::PtParams trace_params_of(const lrc_trace_params *p) {
@@ -684,6 +692,10 @@ int lrc_guide(lrc_scene *s, const lrc_trace_params *p, float *planes, unsigned f
     DeviceGuard g(c->device);
     if (!s->tables) {
         int rc = lrc_scene_set_tables(s, nullptr, nullptr);
+        if (rc) return rc;
+    }
+    {
+        int rc = scene_wide(s, c->st, false);
         if (rc) return rc;
     }
     const size_t N = (size_t)p->width * p->height;
@@ -848,8 +860,12 @@ int lrc_trace_frame(lrc_scene *s, const lrc_trace_params *old_p, const lrc_trace
     } else if (!e) {
         e = cudaMemsetAsync(d_new, 0, N * 32, c->st);   // (the first frame: no history)
     }
-    if (!e) e = lrc::pt_trace(pt_scene(s), P, reinterpret_cast<float *>(d_new), s->d_rays, c->d_status, c->st);
+    if (!e && wavefront_call(s, new_p, H, spp))
+        rc = trace_wavefront(s, new_p, 0, H, spp0, spp, reinterpret_cast<float *>(d_new), true);
+    else if (!e)
+        e = lrc::pt_trace(pt_scene(s), P, reinterpret_cast<float *>(d_new), s->d_rays, c->d_status, c->st);
     c->timer.end(c->st);
+    if (rc) return rc;
     if (!e && !(flags & LRC_DEVICE)) e = cudaMemcpyAsync(new_planes, d_new, N * 64, cudaMemcpyDeviceToHost, c->st);
     if (e) return cuda_status(c, e, "lrc_trace_frame");
     return (flags & LRC_DEVICE) ? LRC_OK : check_status(c);

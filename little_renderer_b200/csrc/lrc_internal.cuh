@@ -137,29 +137,31 @@ cudaError_t refit_device(Node *d_nodes, const uint32_t *d_aux, uint32_t n, uint3
                          uint32_t stride4, uint32_t lo_at, void *scratch, size_t scratch_bytes, uint32_t *d_status,
                          cudaStream_t st);
 cudaError_t tree_cost_device(const Node *d_nodes, uint32_t n, double *d_out, cudaStream_t st);
-// the ray queries' walk over 8-wide nodes (wide.cu): 80-byte nodes (5 float4), triangle entries
-struct WideTables {
-    const float4 *nodes;
-    const uint32_t *refs;
-    const float4 *tris;      // 3 float4 per triangle
-    uint32_t nnodes, nrefs, ntris;
+// the walk over 8-wide nodes (wide.cuh, wide.cu): 80-byte nodes (5 float4), 48-byte leaf entries
+struct WideScene {
+    const float4 *nodes;     // (null: none)
+    const float4 *leaves;
+    uint32_t nnodes, nleaves;   // their capacities: an index out of them is reported (ST_BAD_TREE)
 };
-// capacity of wide nodes and triangle entries for a binary tree with naux leaf entries
-size_t wide_node_cap(uint32_t naux);
-size_t wide_scratch_bytes(uint32_t naux);
-// the wide tree of the binary tree d_bin (nn nodes, root 0, leaves' aux = triangle ids) into
-// d_wnodes (wcap nodes) and d_wrefs (rcap entries); *nwide: the wide nodes made. Waits for the stream
-// (one launch a level). A leaf that does not fit a node's slots: ST_BAD_TREE.
-cudaError_t wide_build(const Node *d_bin, uint32_t nn, const uint32_t *d_aux, uint32_t naux, const float *d_tris,
-                       uint32_t ntris, float4 *d_wnodes, uint32_t wcap, uint32_t *d_wrefs, uint32_t rcap, void *scratch,
-                       size_t scratch_bytes, uint32_t *d_status, cudaStream_t st, uint32_t *nwide);
-cudaError_t wide_intersect(const WideTables &wt, const float *d_orig, const float *d_dir, uint64_t nrays, float tmin,
-                           float tmax, int32_t *d_prim, float *d_t, uint32_t *d_status, cudaStream_t st);
-cudaError_t wide_occluded(const WideTables &wt, const float *d_orig, const float *d_dir, const float *d_tmax, uint64_t nrays,
-                          float tmin, uint8_t *d_out, uint32_t *d_status, cudaStream_t st);
+struct TraceTables;
+// the bytes of a wide tree over a binary one with naux leaf entries (single: one a leaf, as the
+// builders make them), and its view in such a buffer (256-byte aligned)
+size_t wide_bytes(uint32_t naux, bool single);
+WideScene wide_view(void *buf, uint32_t naux, bool single);
+// the wide tree of the binary tree d_bin (nn nodes, root 0, leaves of at most 8 entries, aux = shape ids:
+// nprims primitives, then triangles) into buf; enqueued, no waiting, no other memory
+cudaError_t wide_build(const Node *d_bin, uint32_t nn, const uint32_t *d_aux, uint32_t naux, uint32_t nprims,
+                       const float *d_tris, uint32_t ntris, void *buf, bool single, uint32_t *d_status, int num_sms,
+                       cudaStream_t st);
+// queries of a scene of triangles alone; tt: the binary tree the wide one was made from
+cudaError_t wide_intersect(const WideScene &W, const TraceTables &tt, const float *d_orig, const float *d_dir, uint64_t nrays,
+                           float tmin, float tmax, int32_t *d_prim, float *d_t, uint32_t *d_status, cudaStream_t st);
+cudaError_t wide_occluded(const WideScene &W, const TraceTables &tt, const float *d_orig, const float *d_dir,
+                          const float *d_tmax, uint64_t nrays, float tmin, uint8_t *d_out, uint32_t *d_status,
+                          cudaStream_t st);
 // totals: [0] wide nodes fetched (80 bytes each), [1] triangle tests
-cudaError_t wide_count(const WideTables &wt, const float *d_orig, const float *d_dir, uint64_t nrays, float tmin, float tmax,
-                       unsigned long long *d_stats, uint32_t *d_status, cudaStream_t st);
+cudaError_t wide_count(const WideScene &W, const TraceTables &tt, const float *d_orig, const float *d_dir, uint64_t nrays,
+                       float tmin, float tmax, unsigned long long *d_stats, uint32_t *d_status, cudaStream_t st);
 // the walk's tree of a triangle tree (nn nodes, root at 0, leaves' aux = triangle ids): the same
 // nodes with each leaf's box the bounds of its triangles' corners widened by 2^-17 of the largest
 // coordinate of the source root box (at most the 1e-3 the builders pad with), inner boxes the unions
@@ -205,6 +207,7 @@ struct PtScene {
     const float4 *nodes;        // the world's BVH (shape ids in aux: primitives, then triangles)
     const uint32_t *aux;
     uint32_t root, nnodes, naux;
+    WideScene wide;             // the same tree's 8-wide nodes (nodes null: none, the binary ones are walked)
     const float4 *prims;        // 6 float4 per primitive (upload_world's layout)
     uint32_t nprims;
     const float4 *tris;         // 3 float4 per triangle
@@ -363,6 +366,7 @@ WfState wf_carve(void *base, uint32_t M);
 // the wavefront's trace shapes (closest-hit and shadow kernels: threads per block, register-cap
 // blocks per SM, blocks per SM that fit): how many; -1 for none
 int wf_variants();
+constexpr int LRC_WAVEFRONT_SMALL_VARIANT = 11;   // (128 threads, 6 blocks an SM; shading 4): one image's calls
 int wf_variant_shape(int variant, int *block, int *minb);
 // Captures the wavefront's loop into the graph stream st is capturing: the slots cleared and the
 // task queue set to the run block's tasks (W.run[0]), then a while node whose body (captured on

@@ -5,6 +5,7 @@
 #include "lrc_internal.cuh"
 #include "bsdf.cuh"
 #include "media.cuh"
+#include "wide.cuh"
 
 namespace lrc {
 namespace pt {
@@ -173,6 +174,52 @@ __device__ int32_t walk(const PtScene &S, const float4 *nodes, uint32_t root, ui
         }
         return false;
     }, cnt);
+    return hit;
+}
+
+// The same walk compiled once (not inlined), for what the wide walk leaves to it: two shapes hit at the
+// same t (this walk's order decides) and scenes without wide nodes.
+template <bool ANY>
+static __device__ __noinline__ int32_t walk_binary(const PtScene &S, V3 o, V3 d, float tmin, float &best, uint32_t *err) {
+    return walk<ANY>(S, S.nodes, S.root, S.nnodes, S.aux, S.naux, o, d, tmin, best, err);
+}
+// a leaf entry's shape: a primitive's record, or the entry's own triangle; t in (tmin, tmax]
+struct WorldLeaf {
+    const PtScene &S;
+    __device__ __forceinline__ bool operator()(uint32_t id, float4 q, const float4 *lp, const WideRay &r, float tmin, float tmax,
+                                               float &t) const {
+        if (id >= S.nprims) return wide_tri(q, __ldg(lp + 1), __ldg(lp + 2), r.o, r.d, tmin, tmax, t);
+        const float4 *pr = S.prims + 6 * (size_t)id;
+        const float4 c = ld4(pr);
+        const float end = __uint_as_float(__float_as_uint(tmax) + 1u);   // (the float after tmax: their ends are open)
+        return (ld4(pr + 1).w == 0.0f ? hit_sphere_t(v3(c.x, c.y, c.z), c.w, r.o, r.d, tmin, end, t)
+                                      : hit_quad_t(pr, r.o, r.d, tmin, end, t)) && t <= tmax;
+    }
+};
+__device__ __forceinline__ bool world_wide(const PtScene &S) { return S.wide.nodes && wide_walked(S.wide); }
+// Lane `on`'s ray through the world's wide nodes, the whole warp calling (every lane, `on` or not): the
+// steps of its lanes stay in step. The closest (ANY = false) or any shape in (tmin, best), or -1.
+// Without wide nodes, and where two shapes are hit at the same t, the binary walk.
+template <bool ANY>
+__device__ __forceinline__ int32_t warp_walk(const PtScene &S, bool on, V3 o, V3 d, float tmin, float &best, uint32_t *err) {
+    int32_t hit = -1;
+    bool binary = on && S.nnodes;
+    if (world_wide(S)) {
+        const WideRay r = wide_ray(o, d);
+        uint2 stack[WD_STACK];
+        WideWalk w;
+        wide_begin(w, best);
+        bool going = on;
+        while (true) {
+            const uint32_t m = __ballot_sync(0xffffffffu, going);
+            if (!m) break;
+            if (going && wide_step<ANY, false>(S.wide, r, w, stack, tmin, __popc(m), err, WorldLeaf{S})) going = false;
+        }
+        binary = on && !ANY && w.tie;
+        hit = w.hit;
+        if (on && !binary) best = w.best;
+    }
+    if (binary) hit = walk_binary<ANY>(S, o, d, tmin, best, err);
     return hit;
 }
 
@@ -923,6 +970,52 @@ __device__ __forceinline__ V3 trace_path(const PtScene &S, const PtParams &P, V3
     return ps.radiance;
 }
 
+// scene_intersect with the whole warp calling (lanes not `on` have no ray)
+__device__ __forceinline__ bool warp_intersect(const PtScene &S, bool on, V3 o, V3 d, float tmin, float tmax, Hit &h, uint32_t *err) {
+    float t = tmax;
+    const int32_t id = warp_walk<false>(S, on, o, d, tmin, t, err);
+    int inst = -1, tri = -1;
+    if (on && S.ninst) walk_instances<false>(S, o, d, tmin, t, inst, tri, err);
+    return on && make_hit(S, o, d, t, id, inst, tri, h);
+}
+// scene_occluded likewise
+__device__ __forceinline__ bool warp_occluded(const PtScene &S, bool on, V3 o, V3 d, float tmin, float tmax, uint32_t *err) {
+    int inst, tri;
+    float t = tmax;
+    const bool by_inst = on && S.ninst && walk_instances<true>(S, o, d, tmin, t, inst, tri, err);
+    t = tmax;
+    return warp_walk<true>(S, on && !by_inst, o, d, tmin, t, err) >= 0 || by_inst;
+}
+
+// path_bounce with the whole warp calling (scenes without media): the walks are the warp's, so that its
+// lanes, parted by the shading before, walk together again; the shading leaves its shadow rays to
+// them and their contributions are added in its order (as the wavefront's kernels do). Returns false
+// on a lane whose path has ended, and on lanes without one (on false).
+__device__ __forceinline__ bool warp_bounce(const PtScene &S, int max_depth, int mis, PathState &ps, bool on, Sampler &sm,
+                                            uint32_t *err, uint32_t &rays) {
+    Hit h;
+    const bool found = warp_intersect(S, on, ps.ro, ps.rd, RT_EPS, 1e30f, h, err);
+    Nee nee;
+    nee.flags = 0;
+    bool cont = false;
+    if (on) {
+        rays++;
+        cont = path_shade<true>(S, max_depth, mis, ps, found, h, sm, err, rays, nee);
+    }
+#pragma unroll 1
+    for (int e = 0; e < 2; e++) {                    // the lamp's ray, then the sky's
+        const bool has = (nee.flags & (e ? NEE_E : NEE_L)) != 0, ray = (nee.flags & (e ? NEE_RE : NEE_RL)) != 0;
+        bool dark = true;
+        if (__any_sync(0xffffffffu, ray))
+            dark = warp_occluded(S, ray, nee.p, e ? nee.we : nee.wl, RT_EPS, e ? 1e30f : nee.tl, err);
+        if (has) {
+            const V3 v = vmul(nee.thr, ray && !dark ? (e ? nee.ve : nee.vl) : v3(0, 0, 0));
+            ps.radiance = vadd(ps.radiance, indirect_cap(v, (nee.flags & NEE_ROUGH) != 0, ps.icap));
+        }
+    }
+    return cont;
+}
+
 // camera_ray (camera.h:38-42)
 __device__ __forceinline__ void camera_ray(const PtParams &P, float s, float t, V3 &o, V3 &d) {
     V3 target = vsub(vadd(P.upper_left, vscale(P.horizontal, s)), vscale(P.vertical, t));
@@ -936,6 +1029,12 @@ __device__ __forceinline__ float sample_luma(V3 c, float4 ga) {
     const float kind = ga.w - 4.0f * floorf(ga.w * 0.25f);
     if (kind == 0.0f) c = v3(c.x / fmaxf(ga.x, 1e-3f), c.y / fmaxf(ga.y, 1e-3f), c.z / fmaxf(ga.z, 1e-3f));
     return 0.2126f * c.x + 0.7152f * c.y + 0.0722f * c.z;
+}
+
+// plane 1's w after a guided call: its last sample's number (low 24 bits) + 1, as trace.wgsl keeps
+// it for the temporal gradients (trace.wgsl:1306-1310)
+__device__ __forceinline__ float last_sample_tag(const PtParams &P) {
+    return (float)((((uint32_t)(P.spp0 + P.spp - 1)) & 0xffffffu) + 1u);
 }
 
 __device__ __forceinline__ bool is_number(V3 c) { return c.x == c.x && c.y == c.y && c.z == c.z; }

@@ -172,6 +172,11 @@ int admit(lrc_server *sv, lrc_server::Job *J) {
         e = cudaMallocAsync(reinterpret_cast<void **>(&J->d_planes), N * 64, c->st);
         if (!e) e = cudaMemsetAsync(J->d_planes, 0, N * 32, c->st);
         if (!e) {
+            int rc = scene_wide(J->s, c->st, false);
+            if (rc) {
+                free_job(sv, J);
+                return rc;
+            }
             lrc::PtParams P{};
             P.W = J->p.width; P.H = J->p.height; P.rows = J->p.height;
             P.origin = {J->p.origin[0], J->p.origin[1], J->p.origin[2]};

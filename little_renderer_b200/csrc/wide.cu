@@ -1,396 +1,478 @@
-// wide.cu - the ray queries' walk over 8-wide nodes with quantised child boxes, made on the device
-// from a binary tree (the walk's tree: the reference's topology with tight boxes). The node is the
-// compressed wide node of Ylitie, Karras and Laine ("Efficient incoherent ray traversal on GPUs
-// through compressed wide BVHs", HPG 2017) in a layout of our own: 80 bytes for up to 8 children
-// (a binary walk reads 64 bytes for 2), so a ray's walk fetches fewer bytes and makes fewer
-// dependent loads.
+// wide.cu - the 8-wide nodes (wide.cuh) made on the device from a binary tree, and the ray queries
+// over them: closest hit (scene_intersect, engine/rt/accel.c:252) and any hit (scene_occluded, :280)
+// of a scene of triangles.
 //
-// Node (5 x 16 bytes): the grid origin p (the node box's lo) and the three axes' scale exponents
-// (scale = a power of two, its float exponent field), the first inner child, the first triangle
-// entry, one byte per slot (0 empty, 1 + k the k-th inner child, 0x80 | k the k-th triangle
-// entry), then the slots' boxes as bytes: lo = p + q_lo scale rounded down, hi = p + q_hi scale
-// rounded up, so a decoded box holds the box it was made from.
-//
-// Collapse (top down, one level of wide nodes per launch): a wide node takes its binary node's two
-// children and opens the inner one with the largest surface area while fewer than 8 slots are
-// used; a leaf of several triangles opens into one slot per triangle (each slot the triangle's own
-// box, widened as the walk's tree widens leaves). No kernel waits on another; a leaf too large for
-// the slots left is reported (ST_BAD_TREE) and the caller keeps the binary walk.
-#include "lrc_internal.cuh"
+// Collapse: one launch, 8 lanes a wide node. A wide node takes its binary node's two children and
+// opens the one with the largest surface area while fewer than 8 slots are used; a leaf of several
+// entries opens into one slot per entry (or, where they do not fit, gets a node of its own). The nodes
+// are numbered as they are found, and node i's binary node is posted at items[i]: groups of lanes
+// take numbers in order and wait for theirs to be posted, so a tree's levels follow one another
+// without a launch or the host between them (the wait is bounded, and a group whose number is never
+// posted leaves when every node posted has been made). Bound by the chain of node reads a level (an
+// opened child's record, 7 times) times the levels: 71 us for 4k triangles, 88 for 20k, 148 for 200k
+// and 812 for 2M.
+#include "pt_device.cuh"
+#include <algorithm>
 
 namespace lrc {
 
 namespace {
 
+using namespace pt;
+
 constexpr int WD_THREADS = 128;
-constexpr int WD_SSTACK = 8;                // stack entries per thread in shared memory
-constexpr int WD_LSTACK = 120;              // then in local memory
+enum { CT_HEAD = 0, CT_MADE = 2, CT_STOP = 3, CT_ALLOC = 4 };   // words of the counters (CT_ALLOC: 64 bits)
 
-__device__ __forceinline__ float area(const float lo[3], const float hi[3]) {
-    const float dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
-    return dx * dy + dy * dz + dz * dx;
-}
+struct Collapse {
+    const Node *bin;
+    uint32_t nn;
+    const uint32_t *aux;
+    uint32_t naux;
+    const float4 *tris;
+    uint32_t nprims, ntris;
+    float4 *nodes;
+    uint32_t ncap;
+    float4 *leaves;
+    uint32_t *items;
+    uint32_t *ctr;
+    uint32_t *err;
+};
 
-// the scale exponent field for an axis of extent ext: the smallest power of two s with ext / s <= 255
-__device__ __forceinline__ uint32_t scale_bits(float ext) {
-    const float x = __fdiv_ru(fmaxf(ext, 0x1p-120f), 255.0f);
-    const uint32_t e = (__float_as_uint(x) >> 23) & 0xffu;  // x < 2^(e - 126)
-    return min(e + 1u, 254u);
-}
+__device__ __forceinline__ uint32_t ld_now(const uint32_t *p) { return *(const volatile uint32_t *)p; }
 
-struct Slot {
+enum { K_NONE = 0, K_INNER = 1, K_GROUP = 2, K_ENTRY = 3 };   // nothing, an inner node, a leaf of several, one entry
+
+struct Child {
+    int kind;
+    uint32_t ref;                                // K_INNER, K_GROUP: the binary node; K_ENTRY: its place in aux
+    uint32_t a, b;                               // K_INNER, K_GROUP: the binary node's words
     float lo[3], hi[3];
-    uint32_t ref;                            // inner: binary node index; triangle: triangle id
-    bool inner;
+    bool shut;                                   // (a leaf of several that does not fit)
 };
 
-// one wide node per item of this level: items[i] = (binary node, wide node); the next level's items
-// appended at next[]; counts: [0] wide nodes made, [1] triangle entries, [2] next level's items
-__global__ void __launch_bounds__(128) collapse_kernel(const Node *__restrict__ bin, uint32_t nn, const uint32_t *__restrict__ aux,
-                                                       uint32_t naux, const float4 *__restrict__ tris, uint32_t ntris, float pad,
-                                                       const uint2 *__restrict__ items, const uint32_t *__restrict__ nitems,
-                                                       uint2 *__restrict__ next, uint32_t *counts, float4 *wnodes,
-                                                       uint32_t wcap, uint32_t *wrefs, uint32_t rcap, uint32_t *err) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= *nitems) return;
-    const uint2 it = items[i];
-    Slot s[8];
-    int n = 0;
-    bool bad = false;
-    auto triangle_slot = [&](uint32_t id, Slot &o) {
-        if (id >= ntris) { bad = true; return; }
-        const float4 q = __ldg(&tris[3 * (size_t)id]), u = __ldg(&tris[3 * (size_t)id + 1]), v = __ldg(&tris[3 * (size_t)id + 2]);
-        const float cx[3] = {q.x, q.x + u.x, q.x + v.x}, cy[3] = {q.y, q.y + u.y, q.y + v.y},
-                    cz[3] = {q.z, q.z + u.z, q.z + v.z};
-        o.lo[0] = fminf(fminf(cx[0], cx[1]), cx[2]) - pad; o.hi[0] = fmaxf(fmaxf(cx[0], cx[1]), cx[2]) + pad;
-        o.lo[1] = fminf(fminf(cy[0], cy[1]), cy[2]) - pad; o.hi[1] = fmaxf(fmaxf(cy[0], cy[1]), cy[2]) + pad;
-        o.lo[2] = fminf(fminf(cz[0], cz[1]), cz[2]) - pad; o.hi[2] = fmaxf(fmaxf(cz[0], cz[1]), cz[2]) + pad;
-        o.ref = id;
-        o.inner = false;
-    };
-    // a binary child into slots: inner -> one slot; a leaf -> one slot per triangle (room permitting)
-    auto add = [&](uint32_t c) {
-        if (c >= nn) { bad = true; return; }
-        const Node &m = bin[c];
-        if (m.b & LEAF_BIT) {
-            const uint32_t cnt = m.b & ~LEAF_BIT;
-            if (m.a >= naux || cnt > naux - m.a || n + (int)cnt > 8) { bad = true; return; }
-            for (uint32_t k = 0; k < cnt && !bad; k++) triangle_slot(__ldg(&aux[m.a + k]), s[n++]);
-        } else {
-            if (n >= 8) { bad = true; return; }
-            Slot &o = s[n++];
-            for (int a = 0; a < 3; a++) { o.lo[a] = m.lo[a]; o.hi[a] = m.hi[a]; }
-            o.ref = c;
-            o.inner = true;
-        }
-    };
-    if (it.x >= nn) {
-        atomicOr(err, ST_BAD_TREE);
+__device__ __forceinline__ void take_node(const Collapse &C, uint32_t c, Child &o) {
+    o.kind = K_NONE;
+    o.shut = false;
+    if (c >= C.nn) {
+        atomicOr(C.err, ST_BAD_TREE);
         return;
     }
-    const Node &r = bin[it.x];
-    if (r.b & LEAF_BIT) {                                      // (a root that is a leaf)
-        const uint32_t cnt = r.b & ~LEAF_BIT;
-        if (r.a >= naux || cnt > naux - r.a || cnt > 8) bad = true;
-        for (uint32_t k = 0; k < cnt && !bad; k++) triangle_slot(__ldg(&aux[r.a + k]), s[n++]);
-    } else {
-        add(r.a);
-        if (!bad) add(r.b);
-    }
-    // open the largest inner slot while there is room (a bounded number of times: a slot is opened
-    // at most once, and at most 8 can be)
-    for (int opened = 0; !bad && n < 8 && opened < 16; opened++) {
-        int best = -1;
-        float ba = -1.0f;
-        for (int k = 0; k < n; k++)
-            if (s[k].inner) {
-                const float a = area(s[k].lo, s[k].hi);
-                if (a > ba) { ba = a; best = k; }
-            }
-        if (best < 0) break;
-        const Node &m = bin[s[best].ref];
-        const uint32_t ca = m.a, cb = m.b;
-        // the slots the two children take; a child that does not fit leaves the slot unopened
-        uint32_t need = 0;
-        for (uint32_t c : {ca, cb}) {
-            if (c >= nn) { need = 99u; break; }
-            const Node &x = bin[c];
-            need += (x.b & LEAF_BIT) ? (x.b & ~LEAF_BIT) : 1u;
-        }
-        if (need > 8u || n - 1 + (int)need > 8) break;
-        s[best] = s[n - 1];                                   // (the opened slot's place: the last slot)
-        n--;
-        add(ca);
-        if (!bad) add(cb);
-    }
-    if (bad || n == 0) {
-        atomicOr(err, ST_BAD_TREE);
+    const float4 *p = reinterpret_cast<const float4 *>(&C.bin[c]);
+    const float4 l = __ldg(p), h = __ldg(p + 1);
+    o.lo[0] = l.x; o.lo[1] = l.y; o.lo[2] = l.z;
+    o.hi[0] = h.x; o.hi[1] = h.y; o.hi[2] = h.z;
+    o.a = __float_as_uint(l.w);
+    o.b = __float_as_uint(h.w);
+    o.ref = c;
+    if (!(o.b & LEAF_BIT)) {
+        o.kind = K_INNER;
         return;
     }
-    // the node's box, the grid, the slots' bytes
-    float lo[3] = {s[0].lo[0], s[0].lo[1], s[0].lo[2]}, hi[3] = {s[0].hi[0], s[0].hi[1], s[0].hi[2]};
-    int ninner = 0, ntri = 0;
-    for (int k = 0; k < n; k++) {
-        for (int a = 0; a < 3; a++) { lo[a] = fminf(lo[a], s[k].lo[a]); hi[a] = fmaxf(hi[a], s[k].hi[a]); }
-        if (s[k].inner) ninner++;
-        else ntri++;
+    const uint32_t n = o.b & ~LEAF_BIT;
+    if (o.a > C.naux || n > C.naux - o.a) {
+        atomicOr(C.err, ST_BAD_TREE);
+    } else if (n == 1) {
+        o.kind = K_ENTRY;
+        o.ref = o.a;
+    } else if (n) {
+        o.kind = K_GROUP;
     }
-    uint32_t eb[3];
-    float scale[3];
-    for (int a = 0; a < 3; a++) {
-        eb[a] = scale_bits(__fsub_ru(hi[a], lo[a]));
-        scale[a] = __uint_as_float(eb[a] << 23);
-    }
-    const uint32_t child0 = ninner ? atomicAdd(&counts[0], (uint32_t)ninner) : 0u;
-    const uint32_t tri0 = ntri ? atomicAdd(&counts[1], (uint32_t)ntri) : 0u;
-    if (child0 + ninner > wcap || tri0 + ntri > rcap) {
-        atomicOr(err, ST_BAD_TREE);
-        return;
-    }
-    const uint32_t next0 = ninner ? atomicAdd(&counts[2], (uint32_t)ninner) : 0u;
-    uint8_t meta[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    uint8_t q[6][8];
-    for (int k = 0; k < 8; k++)
-        for (int a = 0; a < 6; a++) q[a][k] = 0;
-    int ki = 0, kt = 0;
-    for (int k = 0; k < n; k++) {
-        for (int a = 0; a < 3; a++) {
-            const float l = floorf(__fdiv_rd(__fsub_rd(s[k].lo[a], lo[a]), scale[a]));
-            const float h = ceilf(__fdiv_ru(__fsub_ru(s[k].hi[a], lo[a]), scale[a]));
-            q[a][k] = (uint8_t)fminf(fmaxf(l, 0.0f), 255.0f);
-            q[3 + a][k] = (uint8_t)fminf(fmaxf(h, 0.0f), 255.0f);
+}
+
+// the scale's exponent field for an axis from lo to hi: 253 steps hold it, and a step is no smaller
+// than the floats there, so that the grid's origin one step below lo costs at most half a step
+__device__ __forceinline__ uint32_t scale_field(float lo, float hi) {
+    const uint32_t e = (__float_as_uint(__fdiv_ru(__fsub_ru(hi, lo), 253.0f)) >> 23) + 1u;
+    const uint32_t u = __float_as_uint(fmaxf(fabsf(lo), fabsf(hi))) >> 23;
+    return min(max(max(e, u > 23u ? u - 23u : 0u), 1u), 253u);
+}
+
+__global__ void __launch_bounds__(WD_THREADS) collapse_kernel(const __grid_constant__ Collapse C) {
+    const uint32_t all = 0xffffffffu, lane = threadIdx.x & 31u, s = lane & 7u;
+    uint32_t idx = 0, spins = 0, made = 0;       // made: the nodes this warp made, not yet counted in CT_MADE
+    bool claimed = false;
+    for (;;) {
+        // the groups without a number take the next ones
+        const uint32_t want = __ballot_sync(all, !claimed && s == 0u);
+        if (want) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(&C.ctr[CT_HEAD], (uint32_t)__popc(want));
+            base = __shfl_sync(all, base, 0);
+            if (!claimed) idx = base + __popc(want & ((1u << (lane & 24u)) - 1u));
+            claimed = true;
         }
-        if (s[k].inner) {
-            meta[k] = (uint8_t)(1 + ki);
-            next[next0 + ki] = make_uint2(s[k].ref, child0 + ki);
-            ki++;
-        } else {
-            meta[k] = (uint8_t)(0x80 | kt);
-            wrefs[tri0 + kt] = s[k].ref;
-            kt++;
-        }
-    }
-    auto pack4 = [](const uint8_t *b) { return (uint32_t)b[0] | (uint32_t)b[1] << 8 | (uint32_t)b[2] << 16 | (uint32_t)b[3] << 24; };
-    float4 *o = wnodes + 5 * (size_t)it.y;
-    o[0] = make_float4(lo[0], lo[1], lo[2], __uint_as_float(eb[0] | eb[1] << 8 | eb[2] << 16 | (uint32_t)n << 24));
-    o[1] = make_float4(__uint_as_float(child0), __uint_as_float(tri0), __uint_as_float(pack4(meta)), __uint_as_float(pack4(meta + 4)));
-    o[2] = make_float4(__uint_as_float(pack4(q[0])), __uint_as_float(pack4(q[0] + 4)), __uint_as_float(pack4(q[1])),
-                       __uint_as_float(pack4(q[1] + 4)));
-    o[3] = make_float4(__uint_as_float(pack4(q[2])), __uint_as_float(pack4(q[2] + 4)), __uint_as_float(pack4(q[3])),
-                       __uint_as_float(pack4(q[3] + 4)));
-    o[4] = make_float4(__uint_as_float(pack4(q[4])), __uint_as_float(pack4(q[4] + 4)), __uint_as_float(pack4(q[5])),
-                       __uint_as_float(pack4(q[5] + 4)));
-}
-
-__global__ void root_item_kernel(uint2 *items, uint32_t *nitems, uint32_t *counts) {
-    items[0] = make_uint2(0u, 0u);
-    *nitems = 1;
-    counts[0] = 1;                                      // (the root is wide node 0)
-    counts[1] = 0;
-    counts[2] = 0;
-}
-
-__global__ void next_level_kernel(uint32_t *nitems, uint32_t *counts) {
-    *nitems = counts[2];
-    counts[2] = 0;
-}
-
-// ---- the walk ---------------------------------------------------------------------------------
-struct WRay {
-    float ox, oy, oz, dx, dy, dz, ix, iy, iz, ax, ay, az;
-};
-__device__ __forceinline__ float inv_safe(float d) {
-    const float eps = 1e-20f;
-    return 1.0f / (fabsf(d) < eps ? copysignf(eps, d) : d);
-}
-__device__ __forceinline__ WRay wray(const float *o, const float *d) {
-    WRay r;
-    r.ox = o[0]; r.oy = o[1]; r.oz = o[2];
-    r.dx = d[0]; r.dy = d[1]; r.dz = d[2];
-    r.ix = inv_safe(r.dx); r.iy = inv_safe(r.dy); r.iz = inv_safe(r.dz);
-    r.ax = r.ox * r.ix; r.ay = r.oy * r.iy; r.az = r.oz * r.iz;
-    return r;
-}
-
-// Moller-Trumbore rounded as the reference rounds it (intersect.h:96-112), as the binary walk's
-__device__ __forceinline__ bool tri_hit(const WRay &r, float4 q, float4 u, float4 v, float tmin, float tmax, float &tout) {
-    float px = fsub(fmul(r.dy, v.z), fmul(r.dz, v.y));
-    float py = fsub(fmul(r.dz, v.x), fmul(r.dx, v.z));
-    float pz = fsub(fmul(r.dx, v.y), fmul(r.dy, v.x));
-    float det = fadd(fadd(fmul(u.x, px), fmul(u.y, py)), fmul(u.z, pz));
-    if (fabsf(det) < 1e-12f) return false;
-    float inv = __fdiv_rn(1.0f, det);
-    float tx = fsub(r.ox, q.x), ty = fsub(r.oy, q.y), tz = fsub(r.oz, q.z);
-    float b1 = fmul(fadd(fadd(fmul(tx, px), fmul(ty, py)), fmul(tz, pz)), inv);
-    if (b1 < 0.0f || b1 > 1.0f) return false;
-    float qx = fsub(fmul(ty, u.z), fmul(tz, u.y));
-    float qy = fsub(fmul(tz, u.x), fmul(tx, u.z));
-    float qz = fsub(fmul(tx, u.y), fmul(ty, u.x));
-    float b2 = fmul(fadd(fadd(fmul(r.dx, qx), fmul(r.dy, qy)), fmul(r.dz, qz)), inv);
-    if (b2 < 0.0f || fadd(b1, b2) > 1.0f) return false;
-    float t = fmul(fadd(fadd(fmul(v.x, qx), fmul(v.y, qy)), fmul(v.z, qz)), inv);
-    if (t <= tmin || t >= tmax) return false;
-    tout = t;
-    return true;
-}
-
-__device__ __forceinline__ uint32_t byte_of(uint32_t lo4, uint32_t hi4, int k) {
-    return ((k < 4 ? lo4 : hi4) >> (8 * (k & 3))) & 0xffu;
-}
-__device__ __forceinline__ void cswap(float &ta, uint32_t &ca, float &tb, uint32_t &cb) {
-    if (tb < ta) {
-        float t = ta; ta = tb; tb = t;
-        uint32_t c = ca; ca = cb; cb = c;
-    }
-}
-
-struct WStack {
-    uint32_t (*sh)[WD_THREADS];
-    uint32_t loc[WD_LSTACK];
-    int sp;
-    __device__ __forceinline__ bool push(uint32_t e) {
-        if (sp < WD_SSTACK) sh[sp][threadIdx.x] = e;
-        else if (sp < WD_SSTACK + WD_LSTACK) loc[sp - WD_SSTACK] = e;
-        else return false;
-        sp++;
-        return true;
-    }
-    __device__ __forceinline__ uint32_t pop() {
-        sp--;
-        return sp < WD_SSTACK ? sh[sp][threadIdx.x] : loc[sp - WD_SSTACK];
-    }
-};
-
-// closest (ANY = false) or any hit of one ray over the wide tree; the triangle id or -1, best its t.
-// A node's children are all tested at once: its triangles at their slots, its inner children hit
-// visited nearest first (the others wait on the stack). Every child index is higher than its
-// node's (the collapse hands indices out level by level), so the walk ends. COUNT: cnt[0] += the
-// nodes fetched (80 bytes each), cnt[1] += the triangle tests
-template <bool ANY, bool COUNT = false>
-__device__ __forceinline__ int32_t wide_walk(const WideTables &wt, const WRay &r, float tmin, float &best, WStack &stk,
-                                             uint32_t *err, uint32_t *cnt = nullptr) {
-    stk.sp = 0;
-    int32_t hit = -1;
-    uint32_t node = 0;
-    while (true) {
-        if (node >= wt.nnodes) { atomicOr(err, ST_BAD_TREE); return -1; }
-        const float4 *np = wt.nodes + 5 * (size_t)node;
-        const float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3), n4 = __ldg(np + 4);
-        if constexpr (COUNT) cnt[0]++;
-        const uint32_t ex = __float_as_uint(n0.w);
-        const float sx = __uint_as_float((ex & 0xffu) << 23), sy = __uint_as_float(((ex >> 8) & 0xffu) << 23),
-                    sz = __uint_as_float(((ex >> 16) & 0xffu) << 23);
-        const uint32_t child0 = __float_as_uint(n1.x), tri0 = __float_as_uint(n1.y);
-        const uint32_t m0 = __float_as_uint(n1.z), m1 = __float_as_uint(n1.w);
-        const uint32_t qlx0 = __float_as_uint(n2.x), qlx1 = __float_as_uint(n2.y), qly0 = __float_as_uint(n2.z),
-                       qly1 = __float_as_uint(n2.w), qlz0 = __float_as_uint(n3.x), qlz1 = __float_as_uint(n3.y),
-                       qhx0 = __float_as_uint(n3.z), qhx1 = __float_as_uint(n3.w), qhy0 = __float_as_uint(n4.x),
-                       qhy1 = __float_as_uint(n4.y), qhz0 = __float_as_uint(n4.z), qhz1 = __float_as_uint(n4.w);
-        float tk[8];
-        uint32_t ck[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            tk[k] = __int_as_float(0x7f800000);
-            ck[k] = 0;
-            const uint32_t m = byte_of(m0, m1, k);
-            if (!m) continue;
-            const float lx = __fmaf_rd((float)byte_of(qlx0, qlx1, k), sx, n0.x);
-            const float ly = __fmaf_rd((float)byte_of(qly0, qly1, k), sy, n0.y);
-            const float lz = __fmaf_rd((float)byte_of(qlz0, qlz1, k), sz, n0.z);
-            const float hx = __fmaf_ru((float)byte_of(qhx0, qhx1, k), sx, n0.x);
-            const float hy = __fmaf_ru((float)byte_of(qhy0, qhy1, k), sy, n0.y);
-            const float hz = __fmaf_ru((float)byte_of(qhz0, qhz1, k), sz, n0.z);
-            const float x0 = fmaf(lx, r.ix, -r.ax), x1 = fmaf(hx, r.ix, -r.ax);
-            const float y0 = fmaf(ly, r.iy, -r.ay), y1 = fmaf(hy, r.iy, -r.ay);
-            const float z0 = fmaf(lz, r.iz, -r.az), z1 = fmaf(hz, r.iz, -r.az);
-            const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), tmin));
-            const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), best));
-            if (!(tn <= tf)) continue;
-            if (m & 0x80u) {                                   // a triangle: tested at once
-                const uint32_t e = tri0 + (m & 7u);
-                if (e >= wt.nrefs) { atomicOr(err, ST_BAD_TREE); return -1; }
-                const uint32_t id = __ldg(&wt.refs[e]);
-                if (id >= wt.ntris) { atomicOr(err, ST_BAD_TREE); return -1; }
-                const float4 *tp = wt.tris + 3 * (size_t)id;
-                if constexpr (COUNT) cnt[1]++;
-                float t;
-                if (tri_hit(r, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), tmin, best, t)) {
-                    best = t;
-                    hit = (int32_t)id;
-                    if (ANY) return hit;
+        uint32_t item = 0;
+        if (s == 0u && idx < C.ncap) item = idx ? ld_now(&C.items[idx]) : 1u;
+        item = __shfl_sync(all, item, 0, 8);
+        const bool ready = item != 0u;
+        if (!__any_sync(all, ready)) {
+            uint32_t done = 0;
+            if (lane == 0) {
+                if (made) {
+                    __threadfence();
+                    atomicAdd(&C.ctr[CT_MADE], made);
+                    made = 0;
                 }
-            } else {
-                tk[k] = tn;
-                ck[k] = child0 + m - 1u;
+                // (made first: a node counted there had its children's numbers taken before)
+                const uint32_t m = ld_now(&C.ctr[CT_MADE]);
+                __threadfence();
+                const uint32_t n = ld_now(&C.ctr[CT_ALLOC]) + 1u;   // (the root has no number taken)
+                done = m == n || ld_now(&C.ctr[CT_STOP]) ? 1u : 0u;
+                if (!done && ++spins > SPIN_LIMIT) {
+                    atomicOr(C.err, ST_TIMEOUT_BARRIER);
+                    done = 1u;
+                }
             }
-        }
-        // the inner children hit, nearest first: sorted by entry distance (Batcher's network of 19)
-        cswap(tk[0], ck[0], tk[1], ck[1]); cswap(tk[2], ck[2], tk[3], ck[3]);
-        cswap(tk[4], ck[4], tk[5], ck[5]); cswap(tk[6], ck[6], tk[7], ck[7]);
-        cswap(tk[0], ck[0], tk[2], ck[2]); cswap(tk[1], ck[1], tk[3], ck[3]);
-        cswap(tk[4], ck[4], tk[6], ck[6]); cswap(tk[5], ck[5], tk[7], ck[7]);
-        cswap(tk[1], ck[1], tk[2], ck[2]); cswap(tk[5], ck[5], tk[6], ck[6]);
-        cswap(tk[0], ck[0], tk[4], ck[4]); cswap(tk[3], ck[3], tk[7], ck[7]);
-        cswap(tk[1], ck[1], tk[5], ck[5]); cswap(tk[2], ck[2], tk[6], ck[6]);
-        cswap(tk[1], ck[1], tk[4], ck[4]); cswap(tk[3], ck[3], tk[6], ck[6]);
-        cswap(tk[2], ck[2], tk[4], ck[4]); cswap(tk[3], ck[3], tk[5], ck[5]);
-        cswap(tk[3], ck[3], tk[4], ck[4]);
-        // (an entry farther than the best hit found meanwhile is still walked: as the binary walk)
-#pragma unroll
-        for (int k = 7; k >= 1; k--)
-            if (tk[k] <= best && !stk.push(ck[k])) { atomicOr(err, ST_STACK_OVERFLOW); return -1; }
-        if (tk[0] <= best) {
-            node = ck[0];
+            if (__shfl_sync(all, done, 0)) return;
+            __nanosleep(40);
             continue;
         }
-        if (stk.sp == 0) break;
-        node = stk.pop();
+        spins = 0;
+        // the node's two children (or a leaf's entries), one a lane
+        Child c;
+        c.kind = K_NONE;
+        c.shut = false;
+        uint32_t n = 0;
+        if (ready) {
+            const Node &x = C.bin[item - 1u];
+            const uint32_t xa = x.a, xb = x.b;
+            if (xb & LEAF_BIT) {
+                n = min(xb & ~LEAF_BIT, 8u);
+                if (s < n) {
+                    take_node(C, item - 1u, c);
+                    if (c.kind != K_NONE) {
+                        c.kind = K_ENTRY;
+                        c.ref = xa + s;
+                    }
+                }
+            } else {
+                n = 2;
+                if (s < 2u) take_node(C, s ? xb : xa, c);
+            }
+        }
+        // the largest one opened while there is room
+        for (int round = 0; round < 16; round++) {
+            float area = -1.0f;
+            if (n < 8u && (c.kind == K_INNER || (c.kind == K_GROUP && !c.shut))) {
+                const float dx = c.hi[0] - c.lo[0], dy = c.hi[1] - c.lo[1], dz = c.hi[2] - c.lo[2];
+                area = fmaxf(dx * dy + dy * dz + dz * dx, 0.0f);
+            }
+            uint32_t who = s;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                const float oa = __shfl_xor_sync(all, area, o, 8);
+                const uint32_t ow = __shfl_xor_sync(all, who, o, 8);
+                if (oa > area || (oa == area && ow < who)) { area = oa; who = ow; }
+            }
+            const bool open = area >= 0.0f;
+            if (!__any_sync(all, open)) break;
+            const uint32_t wa = __shfl_sync(all, c.a, who, 8), wb = __shfl_sync(all, c.b, who, 8),
+                           wr = __shfl_sync(all, c.ref, who, 8);
+            if (!open) continue;
+            if (!(wb & LEAF_BIT)) {
+                if (s == who) take_node(C, wa, c);
+                else if (s == n) take_node(C, wb, c);
+                n++;
+            } else {
+                const uint32_t cnt = wb & ~LEAF_BIT;
+                if (n - 1u + cnt <= 8u) {
+                    if (s == who || (s >= n && s < n - 1u + cnt)) {
+                        take_node(C, wr, c);
+                        c.kind = K_ENTRY;
+                        c.ref = wa + (s == who ? 0u : s - n + 1u);
+                    }
+                    n += cnt - 1u;
+                } else if (s == who) {
+                    c.shut = true;
+                }
+            }
+        }
+        // the node's box
+        const bool have = c.kind != K_NONE;
+        const float inf = __int_as_float(0x7f800000);
+        float lo[3], hi[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            lo[a] = have ? c.lo[a] : inf;
+            hi[a] = have ? c.hi[a] : -inf;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                lo[a] = fminf(lo[a], __shfl_xor_sync(all, lo[a], o, 8));
+                hi[a] = fmaxf(hi[a], __shfl_xor_sync(all, hi[a], o, 8));
+            }
+        }
+        // boxes the grid cannot hold (a NaN, an infinity, coordinates beyond 1e18): the tree is not
+        // walked (the root's last word says so; the callers walk the binary one)
+        bool plain = true;
+#pragma unroll
+        for (int a = 0; a < 3; a++) plain = plain && (!have || (fabsf(c.lo[a]) <= 1e18f && fabsf(c.hi[a]) <= 1e18f));
+        if (!plain) atomicOr(reinterpret_cast<uint32_t *>(C.nodes) + 7, 1u);
+        // a slot for each child: of the pairs left the one that lies best (its middle farthest to the
+        // slot's corner), again and again
+        float e[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++) e[a] = have ? (c.lo[a] + c.hi[a]) - (lo[a] + hi[a]) : 0.0f;
+        uint32_t taken = 0, slot = 0;
+        bool placed = !have;
+        for (int round = 0; round < 8; round++) {
+            float best = -inf;
+            uint32_t at = 0;
+            if (!placed) {
+#pragma unroll
+                for (uint32_t k = 0; k < 8; k++) {
+                    const float v = (k & 1u ? e[0] : -e[0]) + (k & 2u ? e[1] : -e[1]) + (k & 4u ? e[2] : -e[2]);
+                    if (!(taken >> k & 1u) && (v > best || best == -inf)) { best = v; at = k; }
+                }
+            }
+            float v = placed ? -inf : fmaxf(best, -3e38f);
+            uint32_t who = s;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                const float ov = __shfl_xor_sync(all, v, o, 8);
+                const uint32_t ow = __shfl_xor_sync(all, who, o, 8);
+                if (ov > v || (ov == v && ow < who)) { v = ov; who = ow; }
+            }
+            const uint32_t got = __shfl_sync(all, at, who, 8);
+            if (v > -inf) {
+                taken |= 1u << got;
+                if (s == who) { slot = got; placed = true; }
+            }
+        }
+        // lanes without a child: the slots left, in order
+        const uint32_t idle = (__ballot_sync(all, !have) >> (lane & 24u)) & 0xffu;
+        if (!have) {
+            uint32_t left = ~taken & 0xffu;
+            for (uint32_t k = __popc(idle & ((1u << s) - 1u)); k; k--) left &= left - 1u;
+            slot = __ffs(left) - 1;
+        }
+        uint32_t inner = 0, leaf = 0;
+        if (c.kind == K_INNER || c.kind == K_GROUP) inner = 1u << slot;
+        if (c.kind == K_ENTRY) leaf = 1u << slot;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            inner |= __shfl_xor_sync(all, inner, o, 8);
+            leaf |= __shfl_xor_sync(all, leaf, o, 8);
+        }
+        // numbers for the warp's children and leaf entries, one addition for its 4 nodes
+        uint32_t sum = ready ? (uint32_t)__popc(inner) | (uint32_t)__popc(leaf) << 16 : 0u, before = 0;
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+            const uint32_t v = __shfl_sync(all, sum, 8 * g);
+            if (8u * g < (lane & 24u)) before += v;
+        }
+        const uint32_t total = __shfl_sync(all, before + sum, 31);
+        unsigned long long base = 0;
+        if (lane == 0)
+            base = atomicAdd(reinterpret_cast<unsigned long long *>(&C.ctr[CT_ALLOC]),
+                             (unsigned long long)(total & 0xffffu) | (unsigned long long)(total >> 16) << 32);
+        base = __shfl_sync(all, base, 0);
+        const uint32_t child0 = 1u + (uint32_t)base + (before & 0xffffu), leaf0 = (uint32_t)(base >> 32) + (before >> 16);
+        const bool fits = child0 + __popc(inner) <= C.ncap && leaf0 + __popc(leaf) <= C.naux;
+        if (ready && !fits) {                    // (more nodes than a tree of this size has)
+            atomicOr(C.err, ST_BAD_TREE);
+            C.ctr[CT_STOP] = 1u;
+        }
+        if (ready && fits) {
+            // the grid and the slot's bytes
+            uint8_t *out = reinterpret_cast<uint8_t *>(C.nodes + 5 * (size_t)idx);
+            uint32_t field[3];
+            float p[3];
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                field[a] = scale_field(lo[a], hi[a]);
+                const float step = __uint_as_float(field[a] << 23);
+                p[a] = __fsub_rd(lo[a], step);
+                const double per = (double)__uint_as_float((254u - field[a]) << 23);   // 1 / step
+                const double l = ((double)c.lo[a] - (double)p[a]) * per - 0x1p-6, h = ((double)c.hi[a] - (double)p[a]) * per + 0x1p-6;
+                out[32 + 8 * a + slot] = have ? (uint8_t)fmin(fmax(floor(l), 0.0), 255.0) : (uint8_t)255;
+                out[56 + 8 * a + slot] = have ? (uint8_t)fmin(fmax(ceil(h), 0.0), 255.0) : (uint8_t)0;
+            }
+            if (s == 0u) {
+                C.nodes[5 * (size_t)idx] =
+                    make_float4(p[0], p[1], p[2], __uint_as_float(field[0] | field[1] << 8 | field[2] << 16 | inner << 24));
+                uint32_t *w = reinterpret_cast<uint32_t *>(out) + 4;
+                w[0] = child0;
+                w[1] = leaf0;
+                w[2] = leaf;                     // (the last word is the root's alone: above)
+            }
+            if (c.kind == K_ENTRY) {
+                const uint32_t at = leaf0 + __popc(leaf & ((1u << slot) - 1u)), id = __ldg(&C.aux[c.ref]);
+                float4 q = make_float4(0, 0, 0, 0), u = q, v = q;
+                if (id >= C.nprims && id - C.nprims < C.ntris) {
+                    const float4 *t = C.tris + 3 * (size_t)(id - C.nprims);
+                    q = __ldg(t);
+                    u = __ldg(t + 1);
+                    v = __ldg(t + 2);
+                } else if (id >= C.nprims) {
+                    atomicOr(C.err, ST_BAD_TREE);
+                }
+                q.w = __uint_as_float(id);
+                C.leaves[3 * (size_t)at] = q;
+                C.leaves[3 * (size_t)at + 1] = u;
+                C.leaves[3 * (size_t)at + 2] = v;
+            } else if (have) {
+                *(volatile uint32_t *)&C.items[child0 + __popc(inner & ((1u << slot) - 1u))] = c.ref + 1u;
+            }
+        }
+        made += __popc(__ballot_sync(all, ready && s == 0u));
+        if (ready) claimed = false;
     }
-    return hit;
 }
 
-__global__ void __launch_bounds__(WD_THREADS) wide_closest_kernel(WideTables wt, const float *__restrict__ orig,
-                                                                  const float *__restrict__ dir, uint64_t nrays, float tmin,
-                                                                  float tmax, int32_t *__restrict__ prim,
-                                                                  float *__restrict__ tout, uint32_t *err) {
-    __shared__ uint32_t sstack[WD_SSTACK][WD_THREADS];
-    const uint64_t i = (uint64_t)blockIdx.x * WD_THREADS + threadIdx.x;
-    if (i >= nrays) return;
-    const WRay r = wray(orig + 3 * i, dir + 3 * i);
-    WStack stk;
-    stk.sh = sstack;
-    float best = tmax;
-    const int32_t h = wide_walk<false>(wt, r, tmin, best, stk, err);
-    prim[i] = h;
-    tout[i] = h >= 0 ? best : -1.0f;
+// ---- the queries ---------------------------------------------------------------------------------
+// A block takes `chunk` rays; its lanes whose ray is done take the block's next ones once fewer than
+// WD_REFILL of a warp's lanes are at work (the walks of a warp's rays differ in length several times
+// over).
+constexpr int WD_REFILL = 20;
+constexpr uint32_t WD_CHUNK = 2048;
+// Up to this many rays 8 lanes walk a ray: with fewer rays than the chip holds lanes the walks' length
+// decides, not their number (closest hits over 4M triangles, 8 lanes a ray and one: 20480 rays 330 and
+// 294 us, 32768 417 and 340; over 20k triangles 57 and 55, 71 and 57).
+constexpr uint64_t WD_EIGHT_LANES_TO = 1u << 14;
+
+struct Query {
+    WideScene W;
+    TraceTables tt;                              // the binary tree
+    const float *orig, *dir, *tmaxs;             // (tmaxs: any hit)
+    uint64_t n;
+    float tmin, tmax;
+    int32_t *prim;
+    float *t;
+    uint8_t *blocked;
+    uint32_t chunk;
+    uint32_t *err;
+};
+
+// a triangle's leaf entry (the scenes of the queries hold nothing else)
+struct TriLeaf {
+    __device__ __forceinline__ bool operator()(uint32_t, float4 q, const float4 *lp, const WideRay &r, float tmin, float tmax,
+                                               float &t) const {
+        return wide_tri(q, __ldg(lp + 1), __ldg(lp + 2), r.o, r.d, tmin, tmax, t);
+    }
+};
+
+__device__ __forceinline__ V3 query_v3(const float *p, uint64_t i) { return v3(p[3 * i], p[3 * i + 1], p[3 * i + 2]); }
+__device__ __forceinline__ WideRay query_ray(const Query &Q, uint64_t i) { return wide_ray(query_v3(Q.orig, i), query_v3(Q.dir, i)); }
+
+// ray i through the binary tree: where two triangles are hit at the same t (the binary walk's order
+// decides), and where the tree is not walked wide
+template <bool ANY>
+__device__ __noinline__ void query_binary(const Query &Q, uint64_t i) {
+    float best = ANY ? Q.tmaxs[i] : Q.tmax;
+    int32_t hit = -1;
+    const V3 o = query_v3(Q.orig, i), d = query_v3(Q.dir, i);
+    bvh_walk<false>(reinterpret_cast<const float4 *>(Q.tt.nodes), Q.tt.root, Q.tt.nnodes, Q.tt.aux, Q.tt.naux, o, d, Q.tmin,
+                    best, Q.err, [&](uint32_t id) {
+        if (id >= Q.tt.ntris) { atomicOr(Q.err, ST_BAD_TREE); return true; }
+        float t;
+        if (!hit_tri_t(Q.tt.tris + 3 * (size_t)id, o, d, Q.tmin, best, t)) return false;
+        best = t;
+        hit = (int32_t)id;
+        return ANY;
+    });
+    if (ANY) {
+        Q.blocked[i] = hit >= 0 ? 1 : 0;
+    } else {
+        Q.prim[i] = hit;
+        Q.t[i] = hit >= 0 ? best : -1.0f;
+    }
 }
 
-__global__ void __launch_bounds__(WD_THREADS) wide_any_kernel(WideTables wt, const float *__restrict__ orig,
-                                                              const float *__restrict__ dir, const float *__restrict__ tmaxs,
-                                                              uint64_t nrays, float tmin, uint8_t *__restrict__ out,
-                                                              uint32_t *err) {
-    __shared__ uint32_t sstack[WD_SSTACK][WD_THREADS];
-    const uint64_t i = (uint64_t)blockIdx.x * WD_THREADS + threadIdx.x;
-    if (i >= nrays) return;
-    const WRay r = wray(orig + 3 * i, dir + 3 * i);
-    WStack stk;
-    stk.sh = sstack;
-    float best = tmaxs[i];
-    out[i] = wide_walk<true>(wt, r, tmin, best, stk, err) >= 0 ? 1 : 0;
+template <bool ANY>
+__device__ __forceinline__ void query_done(const Query &Q, uint64_t i, int32_t hit, float best, bool tie) {
+    if (ANY) {
+        Q.blocked[i] = hit >= 0 ? 1 : 0;
+    } else if (tie) {
+        query_binary<false>(Q, i);
+    } else {
+        Q.prim[i] = hit;
+        Q.t[i] = hit >= 0 ? best : -1.0f;
+    }
 }
 
-__global__ void __launch_bounds__(WD_THREADS) wide_count_kernel(WideTables wt, const float *__restrict__ orig,
-                                                                const float *__restrict__ dir, uint64_t nrays, float tmin,
-                                                                float tmax, unsigned long long *stats, uint32_t *err) {
-    __shared__ uint32_t sstack[WD_SSTACK][WD_THREADS];
+template <bool ANY>
+__global__ void __launch_bounds__(WD_THREADS, 8) wide_query_kernel(const __grid_constant__ Query Q) {
+    constexpr int32_t TIE = (int32_t)0x80000000;
+    __shared__ uint32_t s_next, s_tie;
+    const uint32_t all = 0xffffffffu, lane = threadIdx.x & 31u;
+    const uint64_t first = (uint64_t)blockIdx.x * Q.chunk;
+    const uint32_t n = (uint32_t)(Q.n - first < Q.chunk ? Q.n - first : Q.chunk);
+    if (!wide_walked(Q.W)) {
+        for (uint32_t k = threadIdx.x; k < n; k += WD_THREADS) query_binary<ANY>(Q, first + k);
+        return;
+    }
+    if (threadIdx.x == 0) s_next = s_tie = 0;
+    __syncthreads();
+    uint2 stack[WD_STACK];
+    WideRay r = wide_ray(v3(0, 0, 0), v3(0, 0, 0));
+    WideWalk w;
+    wide_begin(w, 0.0f);
+    uint64_t i = 0;
+    bool at = false, more = true;
+    bool over = false;
+    while (!over) {
+        uint32_t m = __ballot_sync(all, at);
+        if (more && __popc(m) < WD_REFILL) {
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(&s_next, (uint32_t)__popc(~m));
+            base = __shfl_sync(all, base, 0);
+            more = base + __popc(~m) < n;
+            if (!at) {
+                const uint32_t k = base + __popc(~m & ((1u << lane) - 1u));
+                if (k < n) {
+                    at = true;
+                    i = first + k;
+                    r = query_ray(Q, i);
+                    wide_begin(w, ANY ? Q.tmaxs[i] : Q.tmax);
+                }
+            }
+            m = __ballot_sync(all, at);
+        }
+        over = !m;
+        if (at && wide_step<ANY, false>(Q.W, r, w, stack, Q.tmin, __popc(m), Q.err, TriLeaf{})) {
+            at = false;
+            if (ANY || !w.tie) {
+                query_done<ANY>(Q, i, w.hit, w.best, false);
+            } else {
+                Q.prim[i] = TIE;
+                s_tie = 1;
+            }
+        }
+    }
+    // (the binary walk's code and registers stay out of the loop above)
+    if (!ANY) {
+        __syncthreads();
+        if (s_tie)
+            for (uint32_t k = threadIdx.x; k < n; k += WD_THREADS)
+                if (Q.prim[first + k] == TIE) query_binary<false>(Q, first + k);
+    }
+}
+
+template <bool ANY>
+__global__ void __launch_bounds__(WD_THREADS, 8) wide_query8_kernel(const __grid_constant__ Query Q) {
+    const uint64_t i = ((uint64_t)blockIdx.x * WD_THREADS + threadIdx.x) >> 3;
+    if (i >= Q.n) return;
+    const bool one = (threadIdx.x & 7u) == 0u;
+    if (!wide_walked(Q.W)) {
+        if (one) query_binary<ANY>(Q, i);
+        return;
+    }
+    const WideRay r = query_ray(Q, i);
+    float best = ANY ? Q.tmaxs[i] : Q.tmax;
+    bool tie;
+    const int32_t hit = wide_walk8<ANY>(Q.W, r, Q.tmin, best, tie, Q.err, TriLeaf{});
+    if (one) query_done<ANY>(Q, i, hit, best, tie);
+}
+
+// the closest-hit walk's nodes and triangle tests: [0] and [1]
+__global__ void __launch_bounds__(WD_THREADS) wide_count_kernel(const __grid_constant__ Query Q, unsigned long long *stats) {
     const uint64_t i = (uint64_t)blockIdx.x * WD_THREADS + threadIdx.x;
     uint32_t cnt[2] = {0, 0};
-    if (i < nrays) {
-        const WRay r = wray(orig + 3 * i, dir + 3 * i);
-        WStack stk;
-        stk.sh = sstack;
-        float best = tmax;
-        wide_walk<false, true>(wt, r, tmin, best, stk, err, cnt);
+    if (i < Q.n && wide_walked(Q.W)) {
+        const WideRay r = query_ray(Q, i);
+        WideWalk w;
+        wide_begin(w, Q.tmax);
+        wide_run<false, true>(Q.W, r, w, Q.tmin, Q.err, TriLeaf{}, cnt);
     }
     unsigned long long a = cnt[0], b = cnt[1];
     for (int o = 16; o > 0; o >>= 1) {
@@ -403,71 +485,118 @@ __global__ void __launch_bounds__(WD_THREADS) wide_count_kernel(WideTables wt, c
     }
 }
 
+size_t up256(size_t x) { return (x + 255) / 256 * 256; }
+
+// Wide nodes of a tree with naux leaf entries: with one entry a leaf a node has 8 children, or all of
+// its subtree's entries (2 to 7): at most 4 / 7 of the entries; else fewer than the entries.
+uint32_t node_cap(uint32_t naux, bool single) { return single ? (uint32_t)((uint64_t)naux * 4 / 7 + 2) : naux + 1; }
+
+template <bool ANY>
+cudaError_t query(Query &Q, cudaStream_t st) {
+    if (!Q.n) return cudaSuccess;
+    if (Q.n <= WD_EIGHT_LANES_TO) {
+        wide_query8_kernel<ANY><<<(unsigned)((Q.n * 8 + WD_THREADS - 1) / WD_THREADS), WD_THREADS, 0, st>>>(Q);
+        return cudaGetLastError();
+    }
+    // A block's rays: enough to refill from, few enough that the last blocks end together (1M rays on 20k
+    // triangles: 256 a block 0.57 ms, 864 0.63).
+    Q.chunk = (uint32_t)std::min<uint64_t>(WD_CHUNK, std::max<uint64_t>(WD_THREADS, Q.n / 4096 / 32 * 32));
+    wide_query_kernel<ANY><<<(unsigned)((Q.n + Q.chunk - 1) / Q.chunk), WD_THREADS, 0, st>>>(Q);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
-size_t wide_node_cap(uint32_t naux) { return naux ? naux : 1; }   // (no more wide nodes than binary leaves)
+size_t wide_bytes(uint32_t naux, bool single) {
+    const size_t cap = node_cap(naux, single);
+    return up256(cap * 80) + up256((size_t)naux * 48) + up256(cap * 4) + 256;
+}
 
-size_t wide_scratch_bytes(uint32_t naux) { return 2 * wide_node_cap(naux) * 8 + 256; }
+WideScene wide_view(void *buf, uint32_t naux, bool single) {
+    WideScene W{};
+    W.nnodes = node_cap(naux, single);
+    W.nleaves = naux;
+    W.nodes = static_cast<const float4 *>(buf);
+    W.leaves = reinterpret_cast<const float4 *>(static_cast<char *>(buf) + up256((size_t)W.nnodes * 80));
+    return W;
+}
 
-cudaError_t wide_build(const Node *d_bin, uint32_t nn, const uint32_t *d_aux, uint32_t naux, const float *d_tris,
-                       uint32_t ntris, float4 *d_wnodes, uint32_t wcap, uint32_t *d_wrefs, uint32_t rcap, void *scratch,
-                       size_t scratch_bytes, uint32_t *d_status, cudaStream_t st, uint32_t *nwide) {
-    if (!nn) return cudaErrorInvalidValue;
-    if (scratch_bytes < wide_scratch_bytes(naux)) return cudaErrorInvalidValue;
-    const size_t cap = wide_node_cap(naux);
-    char *s = static_cast<char *>(scratch);
-    uint2 *items = reinterpret_cast<uint2 *>(s), *next = items + cap;
-    uint32_t *small = reinterpret_cast<uint32_t *>(next + cap);   // [0..2] counts, [3] items this level
-    // the widening of the triangle slots (the walk's tree's rule): from the root box
-    Node root;
-    cudaError_t e = cudaMemcpyAsync(&root, d_bin, sizeof(Node), cudaMemcpyDeviceToHost, st);
-    if (!e) e = cudaStreamSynchronize(st);
+cudaError_t wide_build(const Node *d_bin, uint32_t nn, const uint32_t *d_aux, uint32_t naux, uint32_t nprims,
+                       const float *d_tris, uint32_t ntris, void *buf, bool single, uint32_t *d_status, int num_sms,
+                       cudaStream_t st) {
+    if (!nn || !naux) return cudaErrorInvalidValue;
+    const WideScene W = wide_view(buf, naux, single);
+    Collapse C{};
+    C.bin = d_bin;
+    C.nn = nn;
+    C.aux = d_aux;
+    C.naux = naux;
+    C.tris = reinterpret_cast<const float4 *>(d_tris);
+    C.nprims = nprims;
+    C.ntris = ntris;
+    C.nodes = const_cast<float4 *>(W.nodes);
+    C.ncap = W.nnodes;
+    C.leaves = const_cast<float4 *>(W.leaves);
+    char *items = static_cast<char *>(buf) + up256((size_t)C.ncap * 80) + up256((size_t)naux * 48);
+    const size_t item_bytes = up256((size_t)C.ncap * 4);
+    C.items = reinterpret_cast<uint32_t *>(items);
+    C.ctr = reinterpret_cast<uint32_t *>(items + item_bytes);
+    C.err = d_status;
+    cudaError_t e = cudaMemsetAsync(items, 0, item_bytes + 256, st);
+    if (!e) e = cudaMemsetAsync(buf, 0, 80, st);
     if (e) return e;
-    const float m = fmaxf(fmaxf(fmaxf(fabsf(root.lo[0]), fabsf(root.lo[1])), fmaxf(fabsf(root.lo[2]), fabsf(root.hi[0]))),
-                          fmaxf(fabsf(root.hi[1]), fabsf(root.hi[2])));
-    const float pad = fminf(1e-3f, m * 0x1p-17f);
-    root_item_kernel<<<1, 1, 0, st>>>(items, small + 3, small);
-    // level by level: each launch makes the wide nodes of one level and lists the next
-    uint32_t level_items = 1;
-    for (uint32_t level = 0; level < 256 && level_items; level++) {
-        const uint32_t blocks = (level_items + 127) / 128;
-        collapse_kernel<<<blocks, 128, 0, st>>>(d_bin, nn, d_aux, naux, reinterpret_cast<const float4 *>(d_tris), ntris, pad,
-                                                items, small + 3, next, small, d_wnodes, wcap, d_wrefs, rcap, d_status);
-        next_level_kernel<<<1, 1, 0, st>>>(small + 3, small);
-        std::swap(items, next);
-        e = cudaMemcpyAsync(&level_items, small + 3, 4, cudaMemcpyDeviceToHost, st);
-        if (!e) e = cudaStreamSynchronize(st);
-        if (e) return e;
-    }
-    uint32_t counts[2] = {0, 0};
-    e = cudaMemcpyAsync(counts, small, 8, cudaMemcpyDeviceToHost, st);
-    if (!e) e = cudaStreamSynchronize(st);
-    if (nwide) *nwide = counts[0];
-    return e ? e : cudaGetLastError();
-}
-
-cudaError_t wide_intersect(const WideTables &wt, const float *d_orig, const float *d_dir, uint64_t nrays, float tmin,
-                           float tmax, int32_t *d_prim, float *d_t, uint32_t *d_status, cudaStream_t st) {
-    if (!nrays) return cudaSuccess;
-    const uint64_t blocks = (nrays + WD_THREADS - 1) / WD_THREADS;
-    wide_closest_kernel<<<(unsigned)blocks, WD_THREADS, 0, st>>>(wt, d_orig, d_dir, nrays, tmin, tmax, d_prim, d_t, d_status);
+    // 16 nodes a block at once; no more blocks than are resident together (they wait for one another's nodes)
+    const uint32_t blocks = std::min<uint32_t>((uint32_t)num_sms * 4u, std::max<uint32_t>(naux / 64u, 1u));
+    collapse_kernel<<<blocks, WD_THREADS, 0, st>>>(C);
     return cudaGetLastError();
 }
 
-cudaError_t wide_occluded(const WideTables &wt, const float *d_orig, const float *d_dir, const float *d_tmax, uint64_t nrays,
-                          float tmin, uint8_t *d_out, uint32_t *d_status, cudaStream_t st) {
-    if (!nrays) return cudaSuccess;
-    const uint64_t blocks = (nrays + WD_THREADS - 1) / WD_THREADS;
-    wide_any_kernel<<<(unsigned)blocks, WD_THREADS, 0, st>>>(wt, d_orig, d_dir, d_tmax, nrays, tmin, d_out, d_status);
-    return cudaGetLastError();
+cudaError_t wide_intersect(const WideScene &W, const TraceTables &tt, const float *d_orig, const float *d_dir, uint64_t nrays,
+                           float tmin, float tmax, int32_t *d_prim, float *d_t, uint32_t *d_status, cudaStream_t st) {
+    Query Q{};
+    Q.W = W;
+    Q.tt = tt;
+    Q.orig = d_orig;
+    Q.dir = d_dir;
+    Q.n = nrays;
+    Q.tmin = tmin;
+    Q.tmax = tmax;
+    Q.prim = d_prim;
+    Q.t = d_t;
+    Q.err = d_status;
+    return query<false>(Q, st);
 }
 
-cudaError_t wide_count(const WideTables &wt, const float *d_orig, const float *d_dir, uint64_t nrays, float tmin, float tmax,
-                       unsigned long long *d_stats, uint32_t *d_status, cudaStream_t st) {
+cudaError_t wide_occluded(const WideScene &W, const TraceTables &tt, const float *d_orig, const float *d_dir,
+                          const float *d_tmax, uint64_t nrays, float tmin, uint8_t *d_out, uint32_t *d_status,
+                          cudaStream_t st) {
+    Query Q{};
+    Q.W = W;
+    Q.tt = tt;
+    Q.orig = d_orig;
+    Q.dir = d_dir;
+    Q.tmaxs = d_tmax;
+    Q.n = nrays;
+    Q.tmin = tmin;
+    Q.blocked = d_out;
+    Q.err = d_status;
+    return query<true>(Q, st);
+}
+
+cudaError_t wide_count(const WideScene &W, const TraceTables &tt, const float *d_orig, const float *d_dir, uint64_t nrays,
+                       float tmin, float tmax, unsigned long long *d_stats, uint32_t *d_status, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(d_stats, 0, 16, st);
     if (e || !nrays) return e;
-    const uint64_t blocks = (nrays + WD_THREADS - 1) / WD_THREADS;
-    wide_count_kernel<<<(unsigned)blocks, WD_THREADS, 0, st>>>(wt, d_orig, d_dir, nrays, tmin, tmax, d_stats, d_status);
+    Query Q{};
+    Q.W = W;
+    Q.tt = tt;
+    Q.orig = d_orig;
+    Q.dir = d_dir;
+    Q.n = nrays;
+    Q.tmin = tmin;
+    Q.tmax = tmax;
+    Q.err = d_status;
+    wide_count_kernel<<<(unsigned)((nrays + WD_THREADS - 1) / WD_THREADS), WD_THREADS, 0, st>>>(Q, d_stats);
     return cudaGetLastError();
 }
 
