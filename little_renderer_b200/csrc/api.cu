@@ -75,7 +75,87 @@ int scene_build_on(lrc_scene *s, int builder, int key_bits, void **scratch, size
     return LRC_OK;
 }
 
+static bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus now = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &now) != cudaSuccess || now != cudaStreamCaptureStatusNone;
+}
+// Wide nodes are made on a first use, on the stream of that use. The scene's later uses may be on other
+// streams (lrc_set_stream), which the caller has no reason to order after it: each waits for the event.
+static int wide_noted(lrc_scene *s, cudaStream_t st) {
+    cudaError_t e = s->wide_made ? cudaSuccess : cudaEventCreateWithFlags(&s->wide_made, cudaEventDisableTiming);
+    if (!e) e = cudaEventRecord(s->wide_made, st);
+    s->wide_done = false;
+    return e ? cuda_status(s->ctx, e, "the wide nodes' event") : LRC_OK;
+}
+static int wide_ordered(lrc_scene *s, cudaStream_t st) {
+    if (s->wide_done) return LRC_OK;
+    const bool in_graph = capturing(st);
+    if (!in_graph && cudaEventQuery(s->wide_made) == cudaSuccess) {
+        s->wide_done = true;
+        return LRC_OK;
+    }
+    if (!in_graph) cudaGetLastError();               // (not ready)
+    cudaError_t e = cudaStreamWaitEvent(st, s->wide_made, in_graph ? cudaEventWaitExternal : 0);
+    return e ? cuda_status(s->ctx, e, "the wide nodes' event") : LRC_OK;
+}
+
+// both levels' wide nodes of a scene with instances, as scene_wide's (no memory: the binary ones are walked);
+// for the wavefront, which alone walks them
+int instances_wide(lrc_scene *s, cudaStream_t st) {
+    lrc_ctx *c = s->ctx;
+    if (!s->meshes_built || !s->ninst || s->tlas_n != s->ninst) return LRC_OK;
+    int rc = wide_ordered(s, st);
+    if (rc || (s->twide_ok && s->mwide_ok) || capturing(st)) return rc;
+    const size_t nm = s->mesh_counts.size();
+    cudaError_t e = cudaSuccess;
+    if (!s->mwide_ok) {
+        std::vector<lrc::WideScene> views(nm);
+        size_t off = al(nm * sizeof(lrc::WideScene)), nodes = 0;
+        for (uint32_t n : s->mesh_counts) {
+            off += n ? lrc::wide_bytes(n, true) : 0;
+            nodes += n ? 2 * (size_t)n - 1 : 0;
+        }
+        if (reserve(&s->d_mwide, &s->mwide_cap, off) != cudaSuccess) {
+            cudaGetLastError();
+            return LRC_OK;
+        }
+        char *b = static_cast<char *>(s->d_mwide);
+        off = al(nm * sizeof(lrc::WideScene));
+        uint32_t node0 = 0;
+        for (size_t m = 0; m < nm && !e; m++) {
+            const uint32_t n = s->mesh_counts[m];
+            if (!n) continue;
+            views[m] = lrc::wide_view(b + off, n, true);
+            e = lrc::wide_build_part(s->d_mnodes, node0, (uint32_t)nodes, s->d_maux, s->nmtris, n, 0,
+                                     reinterpret_cast<const float *>(s->d_mtris), s->nmtris, lrc::WD_WIDEN, b + off, true, c->d_status,
+                                     c->num_sms, st);
+            off += lrc::wide_bytes(n, true);
+            node0 += 2 * n - 1;
+        }
+        // (pageable memory: read before the call returns)
+        if (!e) e = cudaMemcpyAsync(b, views.data(), nm * sizeof(lrc::WideScene), cudaMemcpyHostToDevice, st);
+        if (e) return cuda_status(c, e, "the meshes' wide nodes");
+        s->mwide_ok = true;
+        rc = wide_noted(s, st);
+        if (rc) return rc;
+    }
+    if (reserve(&s->d_twide, &s->twide_cap, lrc::wide_bytes(s->ninst, true)) != cudaSuccess) {
+        cudaGetLastError();
+        return LRC_OK;
+    }
+    // (the entries are instances: nothing but their numbers)
+    e = lrc::wide_build(s->d_tlas_nodes, 2 * s->ninst - 1, s->d_tlas_aux, s->ninst, s->ninst, nullptr, 0, lrc::WD_WIDEN, s->d_twide, true,
+                        c->d_status, c->num_sms, st);
+    if (e) return cuda_status(c, e, "the top level's wide nodes");
+    s->twide_ok = true;
+    return wide_noted(s, st);
+}
+
 int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc) {
+    if (!no_alloc) {                                 // (no_alloc: a batch's capture, in its own order)
+        int rc = wide_ordered(s, st);
+        if (rc || capturing(st)) return rc;          // (what is made by now is walked, else the binary nodes)
+    }
     if (s->pwide_ok || !s->built_n || !s->most_leaf || s->most_leaf > kMostLeaf) return LRC_OK;
     lrc_ctx *c = s->ctx;
     const bool single = !s->tree_nnodes;
@@ -90,10 +170,30 @@ int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc) {
         }
     }
     cudaError_t e = lrc::wide_build(s->d_nodes, nn, s->d_aux, na, s->nprims, reinterpret_cast<const float *>(s->d_tris), s->ntris,
-                                    s->d_pwide, single, c->d_status, c->num_sms, st);
+                                    lrc::WD_WIDEN, s->d_pwide, single, c->d_status, c->num_sms, st);
     if (e) return cuda_status(c, e, "the path tracer's wide nodes");
     s->pwide_ok = true;
-    return LRC_OK;
+    return no_alloc ? LRC_OK : wide_noted(s, st);
+}
+
+// The queries' wide nodes, from the walk's tree (a tree with larger leaves than a node has slots, no memory,
+// a first query inside a capture: the binary walk). Made by the first query after a build: a scene that
+// is built each frame and only path traced would pay for nodes it never walks (scene builds of 200k / 4M
+// triangles 0.25 / 1.5 ms, with them 0.37 / 3.0).
+static int query_wide(lrc_scene *s) {
+    lrc_ctx *c = s->ctx;
+    int rc = wide_ordered(s, c->st);
+    if (rc || s->wide_ok || !s->walk_ok || !s->most_leaf || s->most_leaf > kMostLeaf || capturing(c->st)) return rc;
+    const bool single = !s->tree_nnodes;
+    const uint32_t nn = single ? 2 * s->built_n - 1 : s->tree_nnodes, na = single ? s->built_n : s->tree_naux;
+    if (s->wide_cap < lrc::wide_bytes(na, single)) return LRC_OK;
+    c->timer.begin(LRC_TS_HIERARCHY, c->st);
+    cudaError_t e = lrc::wide_build(s->d_wnodes, nn, s->d_aux, na, 0, reinterpret_cast<const float *>(s->d_tris), s->ntris,
+                                    lrc::WD_WIDEN_TIGHT, s->d_wide, single, c->d_status, c->num_sms, c->st);
+    c->timer.end(c->st);
+    if (e) return cuda_status(c, e, "the walk's wide nodes");
+    s->wide_ok = true;
+    return wide_noted(s, c->st);
 }
 
 // the top level over n instances (records at d_inst): LBVH over their world boxes, 30-bit keys,
@@ -137,19 +237,10 @@ int make_walk(lrc_scene *s) {
     c->timer.end(c->st);
     if (e) return cuda_status(c, e, "the walk's tree");
     s->walk_ok = true;
-    // the wide nodes from it (a tree with larger leaves than a node has slots, or no memory: the binary walk)
-    const bool single = !s->tree_nnodes;
-    if (!s->most_leaf || s->most_leaf > kMostLeaf) return LRC_OK;
-    if (reserve(&s->d_wide, &s->wide_cap, lrc::wide_bytes((uint32_t)na, single)) != cudaSuccess) {
+    // (room for the wide nodes that the first query makes; none: the binary walk)
+    if (s->most_leaf && s->most_leaf <= kMostLeaf &&
+        reserve(&s->d_wide, &s->wide_cap, lrc::wide_bytes((uint32_t)na, !s->tree_nnodes)) != cudaSuccess)
         cudaGetLastError();
-        return LRC_OK;
-    }
-    c->timer.begin(LRC_TS_HIERARCHY, c->st);
-    e = lrc::wide_build(s->d_wnodes, (uint32_t)nn, s->d_aux, (uint32_t)na, 0, reinterpret_cast<const float *>(s->d_tris),
-                        s->ntris, s->d_wide, single, c->d_status, c->num_sms, c->st);
-    c->timer.end(c->st);
-    if (e) return cuda_status(c, e, "the walk's wide nodes");
-    s->wide_ok = true;
     return LRC_OK;
 }
 
@@ -382,6 +473,9 @@ void lrc_scene_destroy(lrc_scene *s) {
     cudaFree(s->d_wnodes);
     cudaFree(s->d_wide);
     cudaFree(s->d_pwide);
+    if (s->wide_made) cudaEventDestroy(s->wide_made);
+    cudaFree(s->d_mwide);
+    cudaFree(s->d_twide);
     cudaFree(s->d_aux);
     cudaFree(s->d_boxes);
     cudaFree(s->d_small);
@@ -580,10 +674,7 @@ int lrc_scene_intersect(lrc_scene *s, const float *orig, const float *dir, uint6
     if (!s->built_n) return fail(c, LRC_E_INVALID, "the scene has no built BVH (lrc_scene_build)");
     DeviceGuard g(c->device);
     lrc::TraceTables tt = tables(s);
-    if (s->nprims) {
-        int rc = scene_wide(s, c->st, false);
-        if (rc) return rc;
-    }
+    if (int rc = s->nprims ? scene_wide(s, c->st, false) : query_wide(s)) return rc;
     // LRC_SORT_RAYS: the reordering's scratch (large batches); without it the rays go in their order
     void *sort_scratch = nullptr;
     if ((flags & LRC_SORT_RAYS) && lrc::intersect_scratch_bytes(nrays)) {
@@ -629,6 +720,8 @@ int lrc_scene_trace_stats(lrc_scene *s, const float *orig, const float *dir, uin
     if (!s->built_n) return fail(c, LRC_E_INVALID, "the scene has no built BVH (lrc_scene_build)");
     DeviceGuard g(c->device);
     lrc::TraceTables tt = tables(s);
+    if (s->walk_mode == 2)
+        if (int rc = query_wide(s)) return rc;
     const size_t b_ray = al(nrays * 12);
     cudaError_t e = reserve(&c->stage, &c->stage_cap, 2 * b_ray + 256);
     if (e) return cuda_status(c, e, "ray staging");
@@ -660,6 +753,7 @@ int lrc_scene_occluded(lrc_scene *s, const float *orig, const float *dir, const 
     if (!s->built_n) return fail(c, LRC_E_INVALID, "the scene has no built BVH (lrc_scene_build)");
     DeviceGuard g(c->device);
     lrc::TraceTables tt = tables(s);
+    if (int rc = query_wide(s)) return rc;
     if (flags & LRC_DEVICE) {
         cudaError_t e = s->wide_ok ? lrc::wide_occluded(wide_tables(s), tt, orig, dir, tmax, nrays, tmin, out, c->d_status, c->st)
                                    : lrc::occluded_device(tt, orig, dir, tmax, nrays, tmin, out, c->d_status, c->st);
@@ -784,6 +878,7 @@ int lrc_scene_set_meshes(lrc_scene *s, const uint32_t *tris, const uint32_t *tri
     cudaFree(s->d_mesh_info);
     s->d_mtris = nullptr; s->d_mnodes = nullptr; s->d_maux = nullptr; s->d_mesh_info = nullptr;
     s->meshes_built = false;
+    s->mwide_ok = false;
     s->mesh_counts.assign(tri_counts, tri_counts + nmeshes);
     s->nmtris = (uint32_t)total;
     size_t nodes = 0;
@@ -811,6 +906,7 @@ int lrc_scene_set_instances(lrc_scene *s, const float *records, uint32_t n, unsi
     if (e) return cuda_status(c, e, "instances");
     s->ninst = n;
     s->tlas_n = 0;
+    s->twide_ok = false;
     return (flags & LRC_DEVICE) ? LRC_OK : check_status(c);
 }
 
@@ -823,6 +919,7 @@ int lrc_scene_build_instances(lrc_scene *s, int mesh_builder, int key_bits) {
     uint32_t *keys = s->d_small;
     float *bounds = reinterpret_cast<float *>(s->d_small + 8), *lo_ext = reinterpret_cast<float *>(s->d_small + 16);
     if (!s->meshes_built) {
+        s->mwide_ok = false;
         // each mesh's tree as a dynamic mesh's (upload_instances, trace_gpu.c:1497-1512): its triangles'
         // boxes, its corners' box as the bounds; leaves' aux: the triangles' global indices
         std::vector<uint4> info(s->mesh_counts.size());
@@ -853,6 +950,7 @@ int lrc_scene_build_instances(lrc_scene *s, int mesh_builder, int key_bits) {
         s->meshes_built = true;
     }
     s->tlas_n = 0;
+    s->twide_ok = false;
     const uint32_t n = s->ninst;
     if (!n) return LRC_OK;
     if (s->tlas_cap < n) {
@@ -881,6 +979,7 @@ int lrc_scene_move_instances(lrc_scene *s, const float *records, uint32_t n, int
     if (mode < LRC_TLAS_REFIT || mode > LRC_TLAS_AUTO) return fail(c, LRC_E_INVALID, "mode: refit, rebuild or auto");
     if (!s->tlas_n || n != s->ninst) return fail(c, LRC_E_INVALID, "moves the built instances only (same count)");
     DeviceGuard g(c->device);
+    s->twide_ok = false;
     cudaError_t e = cudaMemcpyAsync(s->d_inst, records, (size_t)n * 128,
                                     (flags & LRC_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->st);
     if (e) return cuda_status(c, e, "instances");

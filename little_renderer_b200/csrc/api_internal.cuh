@@ -43,9 +43,17 @@ struct lrc_scene {
     void *d_wide = nullptr;       // the ray queries' wide nodes, made from d_wnodes (walk_mode 1, 2)
     size_t wide_cap = 0;
     bool wide_ok = false;
+    cudaEvent_t wide_made = nullptr;   // after the last wide nodes made on a first use (scene_wide, query_wide)
+    bool wide_done = true;        // it is known to have passed
     void *d_pwide = nullptr;      // the path tracer's wide nodes, made from d_nodes when first traced
     size_t pwide_cap = 0;
     bool pwide_ok = false;
+    void *d_mwide = nullptr;      // the meshes' wide trees (a table of their views, then the trees)
+    size_t mwide_cap = 0;
+    bool mwide_ok = false;
+    void *d_twide = nullptr;      // the top level's
+    size_t twide_cap = 0;
+    bool twide_ok = false;
     uint32_t most_leaf = 1;       // the largest leaf of the tree (0: not known)
     float *d_boxes = nullptr;
     size_t boxes_cap = 0;
@@ -206,6 +214,10 @@ inline lrc::PtScene pt_scene(const lrc_scene *s) {
         S.mnaux = s->nmtris;
         S.mesh_info = s->d_mesh_info;
         S.nmeshes = (uint32_t)s->mesh_counts.size();
+        if (s->twide_ok && s->mwide_ok) {
+            S.tlas_wide = lrc::wide_view(s->d_twide, s->ninst, true);
+            S.mesh_wide = static_cast<const lrc::WideScene *>(s->d_mwide);
+        }
     }
     if (s->nvol) {
         S.vols = static_cast<const lrc::VolDev *>(s->d_vols);
@@ -264,6 +276,7 @@ constexpr uint32_t kMostLeaf = 8;
 // it, and a build that is only queried or refitted does not pay for it. A tree that cannot be (no memory,
 // leaves too large) is walked as it is.
 // no_alloc: within a graph's capture (a buffer too small is then an error).
+int instances_wide(lrc_scene *s, cudaStream_t st);
 int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc);
 
 // lrc_trace's way of a large image: whether a call goes the wavefront engine's way, and the call (device

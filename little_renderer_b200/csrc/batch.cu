@@ -149,6 +149,7 @@ lrc::PtScene view_of(const lrc_batch::Job &J, bool building) {
         S.inst = reinterpret_cast<const float4 *>(J.view.inst);
         S.tlas_nodes = reinterpret_cast<const float4 *>(J.view.tlas_nodes);
         S.tlas_aux = J.view.tlas_aux;
+        S.tlas_wide = lrc::WideScene{};                  // (its own top level has no wide nodes)
     }
     if (building && J.builder >= 0) {
         const uint32_t n = J.s->ntris + J.s->nprims;
@@ -232,6 +233,7 @@ int prepare(lrc_batch *b, bool building) {
     for (const lrc_batch::Job &J : b->jobs) {
         if (building && J.builder >= 0) continue;
         int rc = scene_wide(J.s, c->st, false);
+        if (!rc && b->engine == 1) rc = instances_wide(J.s, c->st);
         if (rc) return rc;
     }
     b->order.resize(nj);

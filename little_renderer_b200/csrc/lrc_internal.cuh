@@ -149,10 +149,19 @@ struct TraceTables;
 size_t wide_bytes(uint32_t naux, bool single);
 WideScene wide_view(void *buf, uint32_t naux, bool single);
 // the wide tree of the binary tree d_bin (nn nodes, root 0, leaves of at most 8 entries, aux = shape ids:
-// nprims primitives, then triangles) into buf; enqueued, no waiting, no other memory
+// nprims primitives, then triangles) into buf; enqueued, no waiting, no other memory. Its boxes are wider
+// by `widen` of the root box's largest coordinate: the wide walk's slab test rounds about twice as often as
+// the binary one's, so a ray from far away needs that much more room for the same hits (WD_WIDEN: boxes
+// that have the reference's 1e-3; WD_WIDEN_TIGHT: the walk's tree, for origins within 60 times its size)
+constexpr float WD_WIDEN = 0x1p-20f, WD_WIDEN_TIGHT = 0x1p-16f;
 cudaError_t wide_build(const Node *d_bin, uint32_t nn, const uint32_t *d_aux, uint32_t naux, uint32_t nprims,
-                       const float *d_tris, uint32_t ntris, void *buf, bool single, uint32_t *d_status, int num_sms,
+                       const float *d_tris, uint32_t ntris, float widen, void *buf, bool single, uint32_t *d_status, int num_sms,
                        cudaStream_t st);
+// the same of one tree among several in d_bin and d_aux: its root, its leaf entries' number (entries of the
+// view in buf); nn and naux bound the arrays
+cudaError_t wide_build_part(const Node *d_bin, uint32_t root, uint32_t nn, const uint32_t *d_aux, uint32_t naux,
+                            uint32_t entries, uint32_t nprims, const float *d_tris, uint32_t ntris, float widen, void *buf,
+                            bool single, uint32_t *d_status, int num_sms, cudaStream_t st);
 // queries of a scene of triangles alone; tt: the binary tree the wide one was made from
 cudaError_t wide_intersect(const WideScene &W, const TraceTables &tt, const float *d_orig, const float *d_dir, uint64_t nrays,
                            float tmin, float tmax, int32_t *d_prim, float *d_t, uint32_t *d_status, cudaStream_t st);
@@ -233,6 +242,9 @@ struct PtScene {
     uint32_t mnnodes, mnaux;
     const uint4 *mesh_info;
     uint32_t nmeshes;
+    // both levels' wide nodes (none: null): the top level's (leaf entries: instances), each mesh's
+    WideScene tlas_wide;
+    const WideScene *mesh_wide;
     // the sky: radiance + pixel probability (w x h), each row's distribution, the rows'
     const float4 *env_rgbp;
     const float *env_cond, *env_marg;

@@ -371,6 +371,124 @@ __device__ bool walk_instances(const PtScene &S, V3 o, V3 d, float tmin, float &
     }
 }
 
+// ---- the world and the instances over wide nodes, in one walk ---------------------------------
+// A lane's walk of the world, then of the top level, into each instance's mesh and back: every level's
+// nodes take the same step (wide_step's), so the lanes of a warp run together whatever level they are
+// in. A top-level leaf entry is an instance: what is left of its group and of its node waits on the
+// stack, and the ray goes on in the mesh's space until the stack is back where it was. The same hits as
+// scene_find's: an instance's hit counts only before the world's, and where two triangles of instances
+// are hit at the same t, tie says so (scene_find then decides).
+// A field of instances of some 2000 triangles each, 640 x 640 pixels, through the binary nodes of both levels
+// 32 rays at a time and through this with the lanes refilled: 5.12 -> 4.17 ms at 1 spp, 20.1 -> 16.5 at 8.
+struct DeepWalk {
+    WideScene at;                                    // the tree walked
+    uint2 ng;
+    int sp, base;                                    // base: where the stack stood when the mesh was entered
+    int level;                                       // 0 the world, 1 the top level, 2 a mesh
+    int32_t id, inst, cur;                           // the hit's shape (instances: global triangle), its instance; the one walked
+    float best;
+    bool tie;
+};
+__device__ __forceinline__ bool deep_wide(const PtScene &S) {
+    return (!S.nnodes || world_wide(S)) && (!S.ninst || (S.tlas_wide.nodes && wide_walked(S.tlas_wide)));
+}
+__device__ __forceinline__ void deep_begin(const PtScene &S, DeepWalk &w, float tmax) {
+    w.level = S.nnodes ? 0 : 1;
+    w.at = w.level ? S.tlas_wide : S.wide;
+    w.ng = make_uint2(0u, S.nnodes || S.ninst ? 0x80000000u : 0u);
+    w.sp = w.base = 0;
+    w.id = w.inst = w.cur = -1;
+    w.best = tmax;
+    w.tie = false;
+}
+// world(o, d): the ray as it was given
+template <bool ANY, typename World>
+__device__ __forceinline__ bool deep_step(const PtScene &S, WideRay &r, DeepWalk &w, uint2 *stack, float tmin, int with,
+                                          uint32_t *err, World &&world) {
+    uint2 tg = make_uint2(0u, 0u);
+    if (w.ng.y & WD_INNER) {
+        const uint32_t bit = 31 - __clz(w.ng.y);
+        w.ng.y &= ~(1u << bit);
+        const uint32_t slot = (bit - 24u) ^ r.up;
+        const uint32_t ni = w.ng.x + __popc(w.ng.y & 0xffu & ((1u << slot) - 1u));
+        if (w.ng.y & WD_INNER) {
+            if (w.sp >= WD_STACK) { atomicOr(err, ST_STACK_OVERFLOW); return true; }
+            stack[w.sp++] = w.ng;
+        }
+        if (ni >= w.at.nnodes) { atomicOr(err, ST_BAD_TREE); return true; }
+        wide_node(w.at.nodes, ni, r, tmin, w.best, w.ng, tg);
+    } else {
+        tg = w.ng;
+        w.ng.y = 0u;
+    }
+    while (tg.y & 0xffu) {
+        if (!ANY && w.level == 2 && 4 * __popc(__activemask()) < with && (w.ng.y & WD_INNER) && w.sp < WD_PUT_OFF_BELOW) {
+            stack[w.sp++] = make_uint2(tg.x, tg.y & 0xffffu);
+            break;
+        }
+        const uint32_t slot = 31 - __clz(tg.y & 0xffu);
+        tg.y &= ~(1u << slot);
+        const uint32_t e = tg.x + __popc((tg.y >> 8) & ((1u << slot) - 1u));
+        if (e >= w.at.nleaves) { atomicOr(err, ST_BAD_TREE); return true; }
+        const float4 *lp = w.at.leaves + 3 * (size_t)e;
+        const float4 q = __ldg(lp);
+        const uint32_t id = __float_as_uint(q.w);
+        if (w.level == 1) {
+            if (id >= S.ninst) { atomicOr(err, ST_BAD_TREE); return true; }
+            const float4 *rec = S.inst + 8 * (size_t)id;
+            const uint32_t mesh = __float_as_uint(ld4(rec + 6).w);
+            if (mesh >= S.nmeshes) continue;         // (shapes: not in these scenes)
+            const WideScene m = S.mesh_wide[mesh];
+            if (!m.nodes) continue;                  // (a mesh of no triangles)
+            if (w.sp + 2 > WD_STACK) { atomicOr(err, ST_STACK_OVERFLOW); return true; }
+            if (w.ng.y & WD_INNER) stack[w.sp++] = w.ng;
+            if (tg.y & 0xffu) stack[w.sp++] = make_uint2(tg.x, tg.y & 0xffffu);
+            V3 o, d;
+            world(o, d);
+            r = wide_ray(xpoint(rec + 3, o), xdir(rec + 3, d));
+            w.at = m;
+            w.cur = (int32_t)id;
+            w.level = 2;
+            w.base = w.sp;
+            w.ng = make_uint2(0u, 0x80000000u);
+            break;
+        }
+        float t;
+        if (w.level == 0 ? !WorldLeaf{S}(id, q, lp, r, tmin, w.best, t)
+                         : !wide_tri(q, __ldg(lp + 1), __ldg(lp + 2), r.o, r.d, tmin, w.best, t)) continue;
+        const int32_t inst = w.level == 2 ? w.cur : -1;
+        if (t < w.best) {
+            w.best = t;
+            w.id = (int32_t)id;
+            w.inst = inst;
+            w.tie = false;
+            if (ANY) return true;
+        } else if (!ANY && w.id >= 0 && (w.inst >= 0) == (inst >= 0) && (w.id != (int32_t)id || w.inst != inst)) {
+            w.tie = true;
+        }
+    }
+    if (w.ng.y & WD_INNER) return false;
+    if (w.level == 2 && w.sp == w.base) {            // the mesh is done: back in the top level
+        V3 o, d;
+        world(o, d);
+        r = wide_ray(o, d);
+        w.at = S.tlas_wide;
+        w.level = 1;
+        w.base = 0;
+    }
+    if (w.sp > w.base) {
+        w.ng = stack[--w.sp];
+        return false;
+    }
+    if (w.level == 0 && S.ninst) {                   // the world is done: the top level
+        w.at = S.tlas_wide;
+        w.level = 1;
+        w.ng = make_uint2(0u, 0x80000000u);
+        return false;
+    }
+    return true;
+}
+
 }  // namespace pt
 }  // namespace lrc
 #include "textures.cuh"
@@ -777,6 +895,11 @@ __device__ __forceinline__ void scene_find(const PtScene &S, V3 o, V3 d, float t
         }
     }
     t = best;
+}
+// the same compiled once, for the ties of the wide walks
+static __device__ __noinline__ void find_binary(const PtScene &S, V3 o, V3 d, float tmin, float &t, int &id, int &inst, int &tri,
+                                                uint32_t *err) {
+    scene_find<true>(S, o, d, tmin, 1e30f, t, id, inst, tri, err);
 }
 __device__ __forceinline__ bool make_hit(const PtScene &S, V3 o, V3 d, float t, int id, int inst, int tri, Hit &h) {
     if (inst >= 0) instance_hit(S, inst, tri, o, d, t, h);

@@ -136,6 +136,7 @@ lrc::PtScene job_view(const lrc_server::Job *J) {
         S.inst = reinterpret_cast<const float4 *>(J->d_inst);
         S.tlas_nodes = reinterpret_cast<const float4 *>(J->d_tlas);
         S.tlas_aux = J->d_tlas_aux;
+        S.tlas_wide = lrc::WideScene{};
     }
     return S;
 }

@@ -262,10 +262,10 @@ __device__ __forceinline__ void wf_each(uint32_t *next, uint32_t count, Each &&e
         if (lane < share && base + lane < count) each(base + lane);
     }
 }
-// whether some job's world has no wide nodes to walk (then the binary ones are, for every job)
+// whether some job's scene has no wide nodes to walk (then the binary ones are, for every job)
 __device__ __forceinline__ bool wf_any_binary(const BatchJob *__restrict__ jobs, uint32_t njobs) {
     bool b = false;
-    for (uint32_t j = threadIdx.x; j < njobs; j += blockDim.x) b = b || (jobs[j].S.nnodes && !world_wide(jobs[j].S));
+    for (uint32_t j = threadIdx.x; j < njobs; j += blockDim.x) b = b || !deep_wide(jobs[j].S);
     return __syncthreads_or(b);
 }
 // a closest hit left to the shading kernel, which asks the binary walk: another shape was hit at its t
@@ -275,8 +275,12 @@ constexpr int WF_TIE = (int)0x80000000;
 // the closest hit of every queued ray; sets the loop's condition (another pass while rays are queued)
 // (COUNT: also the walks' box and triangle tests into W.next[2], W.next[3]; only the stepped runs
 // that measure the engine's algorithmic bytes launch it)
+// (the walk of two levels holds more: at most 768 threads an SM, 80 registers; at 1024 and 64 it spills: 640 x
+// 640 pixels of instances at 8 spp 21.0 ms against 16.5)
+constexpr int wf_min_blocks(int block, int minb, bool inst) { return inst && block * minb > 768 ? 768 / block : minb; }
+
 template <int BLOCK, int MINB, bool INST, bool COUNT = false>
-__global__ void __launch_bounds__(BLOCK, MINB) wf_intersect_kernel(const BatchJob *__restrict__ jobs,
+__global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_intersect_kernel(const BatchJob *__restrict__ jobs,
                                                                    const __grid_constant__ WfState W, uint32_t *err,
                                                                    cudaGraphConditionalHandle cond, int use_cond) {
     const uint32_t max_passes = (uint32_t)W.run[2];
@@ -295,7 +299,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) wf_intersect_kernel(const BatchJo
     auto answer = [&](uint32_t s, float t, int id, int inst, int tri) {
         W.hit[s] = make_float4(t, __int_as_float(id), __int_as_float(inst), __int_as_float(tri));
     };
-    if (INST || wf_any_binary(jobs, (uint32_t)W.run[1])) {
+    if ((INST && COUNT) || wf_any_binary(jobs, (uint32_t)W.run[1])) {
         wf_each(&W.ctl[2], count, [&](uint32_t k) {
             const uint32_t s = W.rq[k];
             const BatchJob &J = jobs[W.job[s]];
@@ -306,6 +310,29 @@ __global__ void __launch_bounds__(BLOCK, MINB) wf_intersect_kernel(const BatchJo
             else if (J.S.nnodes) id = walk_binary<false>(J.S, o, d, RT_EPS, t, err);
             answer(s, t, id, inst, tri);
         });
+    } else if constexpr (INST) {
+        uint2 stack[WD_STACK];
+        WideRay r = wide_ray(v3(0, 0, 0), v3(0, 0, 0));
+        DeepWalk w;
+        uint32_t s = 0;
+        const BatchJob *J = jobs;
+        deep_begin(J->S, w, 0.0f);
+        wf_walk_queue(
+            &W.ctl[2], count,
+            [&](uint32_t k) {
+                s = W.rq[k];
+                J = &jobs[W.job[s]];
+                r = wide_ray(v3f(W.ro[s]), v3f(W.rd[s]));
+                deep_begin(J->S, w, 1e30f);
+            },
+            [&](int with) {
+                return deep_step<false>(J->S, r, w, stack, RT_EPS, with, err, [&](V3 &o, V3 &d) { o = v3f(W.ro[s]); d = v3f(W.rd[s]); });
+            },
+            [&]() {
+                const bool in = w.inst >= 0;
+                answer(s, w.best, w.tie ? WF_TIE : in ? -1 : w.id, w.inst,
+                       in ? w.id - (int)__ldg(&J->S.mesh_info[__float_as_uint(ld4(J->S.inst + 8 * (size_t)w.inst + 6).w)]).y : -1);
+            });
     } else {
         uint2 stack[WD_STACK];
         WideRay r = wide_ray(v3(0, 0, 0), v3(0, 0, 0));
@@ -360,8 +387,9 @@ __global__ void __launch_bounds__(SHADE_BLOCK, SMINB) wf_shade_kernel(const Batc
             const BatchJob &J = jobs[W.job[s]];
             float4 hh = W.hit[s];
             if (__float_as_int(hh.y) == WF_TIE) {
-                hh.x = 1e30f;
-                hh.y = __int_as_float(walk_binary<false>(J.S, v3f(W.ro[s]), v3f(W.rd[s]), RT_EPS, hh.x, err));
+                int id, inst, tri;
+                find_binary(J.S, v3f(W.ro[s]), v3f(W.rd[s]), RT_EPS, hh.x, id, inst, tri, err);
+                hh = make_float4(hh.x, __int_as_float(id), __int_as_float(inst), __int_as_float(tri));
             }
             const float4 ro = W.ro[s], rd = W.rd[s], th = W.thr[s], ra = W.rad[s];
             PathState ps;
@@ -419,14 +447,14 @@ __global__ void __launch_bounds__(SHADE_BLOCK, SMINB) wf_shade_kernel(const Batc
 // the any-hit test of every queued shadow ray; clears the ray queue and counts the pass for the
 // next one
 template <int BLOCK, int MINB, bool INST>
-__global__ void __launch_bounds__(BLOCK, MINB) wf_shadow_kernel(const BatchJob *__restrict__ jobs,
+__global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_shadow_kernel(const BatchJob *__restrict__ jobs,
                                                                 const __grid_constant__ WfState W, uint32_t *err) {
     const uint32_t count = *reinterpret_cast<volatile uint32_t *>(&W.ctl[1]);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         W.ctl[0] = 0;
         W.ctl[4]++;
     }
-    if (INST || wf_any_binary(jobs, (uint32_t)W.run[1])) {
+    if (wf_any_binary(jobs, (uint32_t)W.run[1])) {
         wf_each(&W.ctl[3], count, [&](uint32_t k) {
             const float4 o = W.sq_o[k], d = W.sq_d[k];
             const uint32_t e = __float_as_uint(o.w);
@@ -440,6 +468,28 @@ __global__ void __launch_bounds__(BLOCK, MINB) wf_shadow_kernel(const BatchJob *
             }
             W.vis[e] = hit ? 0 : 1;
         });
+    } else if constexpr (INST) {
+        uint2 stack[WD_STACK];
+        WideRay r = wide_ray(v3(0, 0, 0), v3(0, 0, 0));
+        DeepWalk w;
+        uint32_t e = 0, at = 0;
+        const BatchJob *J = jobs;
+        deep_begin(J->S, w, 0.0f);
+        wf_walk_queue(
+            &W.ctl[3], count,
+            [&](uint32_t k) {
+                const float4 o = W.sq_o[k], d = W.sq_d[k];
+                at = k;
+                e = __float_as_uint(o.w);
+                J = &jobs[W.job[e >> 1]];
+                r = wide_ray(v3f(o), v3f(d));
+                deep_begin(J->S, w, d.w);
+            },
+            [&](int with) {
+                return deep_step<true>(J->S, r, w, stack, RT_EPS, with, err,
+                                       [&](V3 &o, V3 &d) { o = v3f(W.sq_o[at]); d = v3f(W.sq_d[at]); });
+            },
+            [&]() { W.vis[e] = w.id >= 0 ? 0 : 1; });
     } else {
         uint2 stack[WD_STACK];
         WideRay r = wide_ray(v3(0, 0, 0), v3(0, 0, 0));

@@ -9,8 +9,7 @@
 // take numbers in order and wait for theirs to be posted, so a tree's levels follow one another
 // without a launch or the host between them (the wait is bounded, and a group whose number is never
 // posted leaves when every node posted has been made). Bound by the chain of node reads a level (an
-// opened child's record, 7 times) times the levels: 71 us for 4k triangles, 88 for 20k, 148 for 200k
-// and 812 for 2M.
+// opened child's record, 7 times) times the levels: 4M soup triangles 1.0 ms, 200k triangles 55 us.
 #include "pt_device.cuh"
 #include <algorithm>
 
@@ -25,11 +24,13 @@ enum { CT_HEAD = 0, CT_MADE = 2, CT_STOP = 3, CT_ALLOC = 4 };   // words of the 
 
 struct Collapse {
     const Node *bin;
-    uint32_t nn;
+    uint32_t root, nn;
     const uint32_t *aux;
     uint32_t naux;
+    uint32_t entries;                            // the tree's leaf entries (of aux's naux)
     const float4 *tris;
     uint32_t nprims, ntris;
+    float widen;                                 // every box is widened by this share of the root box's largest coordinate
     float4 *nodes;
     uint32_t ncap;
     float4 *leaves;
@@ -89,6 +90,10 @@ __device__ __forceinline__ uint32_t scale_field(float lo, float hi) {
 
 __global__ void __launch_bounds__(WD_THREADS) collapse_kernel(const __grid_constant__ Collapse C) {
     const uint32_t all = 0xffffffffu, lane = threadIdx.x & 31u, s = lane & 7u;
+    // (the root box's largest coordinate: its widening, none where it is no number a grid holds)
+    const float4 rl = __ldg(reinterpret_cast<const float4 *>(&C.bin[C.root])), rh = __ldg(reinterpret_cast<const float4 *>(&C.bin[C.root]) + 1);
+    float pad = C.widen * fmaxf(fmaxf(fmaxf(fabsf(rl.x), fabsf(rl.y)), fabsf(rl.z)), fmaxf(fmaxf(fabsf(rh.x), fabsf(rh.y)), fabsf(rh.z)));
+    if (!(pad < 1e18f)) pad = 0.0f;
     uint32_t idx = 0, spins = 0, made = 0;       // made: the nodes this warp made, not yet counted in CT_MADE
     bool claimed = false;
     for (;;) {
@@ -102,7 +107,7 @@ __global__ void __launch_bounds__(WD_THREADS) collapse_kernel(const __grid_const
             claimed = true;
         }
         uint32_t item = 0;
-        if (s == 0u && idx < C.ncap) item = idx ? ld_now(&C.items[idx]) : 1u;
+        if (s == 0u && idx < C.ncap) item = idx ? ld_now(&C.items[idx]) : C.root + 1u;
         item = __shfl_sync(all, item, 0, 8);
         const bool ready = item != 0u;
         if (!__any_sync(all, ready)) {
@@ -267,7 +272,7 @@ __global__ void __launch_bounds__(WD_THREADS) collapse_kernel(const __grid_const
                              (unsigned long long)(total & 0xffffu) | (unsigned long long)(total >> 16) << 32);
         base = __shfl_sync(all, base, 0);
         const uint32_t child0 = 1u + (uint32_t)base + (before & 0xffffu), leaf0 = (uint32_t)(base >> 32) + (before >> 16);
-        const bool fits = child0 + __popc(inner) <= C.ncap && leaf0 + __popc(leaf) <= C.naux;
+        const bool fits = child0 + __popc(inner) <= C.ncap && leaf0 + __popc(leaf) <= C.entries;
         if (ready && !fits) {                    // (more nodes than a tree of this size has)
             atomicOr(C.err, ST_BAD_TREE);
             C.ctr[CT_STOP] = 1u;
@@ -279,11 +284,13 @@ __global__ void __launch_bounds__(WD_THREADS) collapse_kernel(const __grid_const
             float p[3];
 #pragma unroll
             for (int a = 0; a < 3; a++) {
-                field[a] = scale_field(lo[a], hi[a]);
+                const float l0 = __fsub_rd(lo[a], pad), h0 = __fadd_ru(hi[a], pad);
+                field[a] = scale_field(l0, h0);
                 const float step = __uint_as_float(field[a] << 23);
-                p[a] = __fsub_rd(lo[a], step);
+                p[a] = __fsub_rd(l0, step);
                 const double per = (double)__uint_as_float((254u - field[a]) << 23);   // 1 / step
-                const double l = ((double)c.lo[a] - (double)p[a]) * per - 0x1p-6, h = ((double)c.hi[a] - (double)p[a]) * per + 0x1p-6;
+                const double l = ((double)c.lo[a] - pad - (double)p[a]) * per - 0x1p-6;
+                const double h = ((double)c.hi[a] + pad - (double)p[a]) * per + 0x1p-6;
                 out[32 + 8 * a + slot] = have ? (uint8_t)fmin(fmax(floor(l), 0.0), 255.0) : (uint8_t)255;
                 out[56 + 8 * a + slot] = have ? (uint8_t)fmin(fmax(ceil(h), 0.0), 255.0) : (uint8_t)0;
             }
@@ -521,23 +528,26 @@ WideScene wide_view(void *buf, uint32_t naux, bool single) {
     return W;
 }
 
-cudaError_t wide_build(const Node *d_bin, uint32_t nn, const uint32_t *d_aux, uint32_t naux, uint32_t nprims,
-                       const float *d_tris, uint32_t ntris, void *buf, bool single, uint32_t *d_status, int num_sms,
-                       cudaStream_t st) {
-    if (!nn || !naux) return cudaErrorInvalidValue;
-    const WideScene W = wide_view(buf, naux, single);
+cudaError_t wide_build_part(const Node *d_bin, uint32_t root, uint32_t nn, const uint32_t *d_aux, uint32_t naux,
+                            uint32_t entries, uint32_t nprims, const float *d_tris, uint32_t ntris, float widen, void *buf,
+                            bool single, uint32_t *d_status, int num_sms, cudaStream_t st) {
+    if (!nn || !entries) return cudaErrorInvalidValue;
+    const WideScene W = wide_view(buf, entries, single);
     Collapse C{};
     C.bin = d_bin;
+    C.root = root;
     C.nn = nn;
     C.aux = d_aux;
     C.naux = naux;
+    C.entries = entries;
+    C.widen = widen;
     C.tris = reinterpret_cast<const float4 *>(d_tris);
     C.nprims = nprims;
     C.ntris = ntris;
     C.nodes = const_cast<float4 *>(W.nodes);
     C.ncap = W.nnodes;
     C.leaves = const_cast<float4 *>(W.leaves);
-    char *items = static_cast<char *>(buf) + up256((size_t)C.ncap * 80) + up256((size_t)naux * 48);
+    char *items = static_cast<char *>(buf) + up256((size_t)C.ncap * 80) + up256((size_t)entries * 48);
     const size_t item_bytes = up256((size_t)C.ncap * 4);
     C.items = reinterpret_cast<uint32_t *>(items);
     C.ctr = reinterpret_cast<uint32_t *>(items + item_bytes);
@@ -546,9 +556,15 @@ cudaError_t wide_build(const Node *d_bin, uint32_t nn, const uint32_t *d_aux, ui
     if (!e) e = cudaMemsetAsync(buf, 0, 80, st);
     if (e) return e;
     // 16 nodes a block at once; no more blocks than are resident together (they wait for one another's nodes)
-    const uint32_t blocks = std::min<uint32_t>((uint32_t)num_sms * 4u, std::max<uint32_t>(naux / 64u, 1u));
+    const uint32_t blocks = std::min<uint32_t>((uint32_t)num_sms * 4u, std::max<uint32_t>(entries / 64u, 1u));
     collapse_kernel<<<blocks, WD_THREADS, 0, st>>>(C);
     return cudaGetLastError();
+}
+
+cudaError_t wide_build(const Node *d_bin, uint32_t nn, const uint32_t *d_aux, uint32_t naux, uint32_t nprims,
+                       const float *d_tris, uint32_t ntris, float widen, void *buf, bool single, uint32_t *d_status, int num_sms,
+                       cudaStream_t st) {
+    return wide_build_part(d_bin, 0, nn, d_aux, naux, naux, nprims, d_tris, ntris, widen, buf, single, d_status, num_sms, st);
 }
 
 cudaError_t wide_intersect(const WideScene &W, const TraceTables &tt, const float *d_orig, const float *d_dir, uint64_t nrays,
