@@ -921,8 +921,8 @@ def run_serve(a):
     # rate, each job alone on the one-kernel path)
     line["plain_best_mrays_s"] = line["plain_mrays_s"]
     line["plain_megakernel_mrays_s"] = r_mid["plain_megakernel"]["mrays_s"]
-    line["denominators"] = ("plain_mrays_s: each job alone through lrc_trace as shipped (jobs of 2^20 paths and "
-                            "more on the wavefront engine); served_vs_plain_megakernel: at the middle rate, each "
+    line["denominators"] = ("plain_mrays_s: each job alone through lrc_trace as shipped (large jobs, from 98304 paths "
+                            "side by side, on the wavefront engine); served_vs_plain_megakernel: at the middle rate, each "
                             "job alone on the one-kernel path (LRC_TRACE_MEGAKERNEL)")
     for s_ in scenes:
         s_.close()

@@ -247,13 +247,23 @@ int make_walk(lrc_scene *s) {
 // A large image runs as a one-job batch on the wavefront engine: its kernels keep their own registers
 // (the one-kernel path sits at its cap with every bounce's code in one loop), and its image is the
 // call's to the bit (a batch task traces a pixel's samples as the one-kernel path's lanes do and the
-// resolve pass adds them in that path's order). The line (LRC_TRACE_WAVEFRONT_PATHS): a pass of the
-// wavefront waits for its longest walk whatever its size, which the one-kernel path does not; scenes of 4k
-// / 20k / 200k triangles at 256 x 256 pixels, 1 spp: the one-kernel path 0.83 / 1.13 / 1.36 ms, the
-// wavefront 1.08 / 1.46 / 1.67; at 360 x 360 1.45 / 1.77 / 2.26 and 1.23 / 1.65 / 1.90.
+// resolve pass adds them in that path's order). The line: a pass of the wavefront waits for its longest
+// walk whatever its size, which the one-kernel path does not, and a deeper image has more passes with few
+// paths left. One-kernel path and wavefront at 1 spp, depth 8, scenes of 4k / 20k / 200k triangles: 256 x
+// 256 pixels 0.83 / 1.13 / 1.36 and 1.08 / 1.46 / 1.67 ms, 360 x 360 1.45 / 1.77 / 2.26 and 1.23 / 1.65 /
+// 1.90. Depth 12, 20k / 1M triangles: 320 x 320 1.85 / 2.57 and 2.17 / 3.13, 400 x 400 2.44 / 3.25 and
+// 2.32 / 3.40, 512 x 512 3.54 / 4.78 and 2.63 / 3.97. With instances (8000 triangles each), whose walks are
+// longer: depth 4, 320 x 320 2.60 and 2.41; depth 12, 400 x 400 4.88 and 5.66, 512 x 512 6.83 and 6.34.
+// What counts is the tasks, which run side by side (exact mode has one a pixel, fast mode up to 16); from
+// 2^20 paths on the wavefront whatever their number.
 bool wavefront_call(const lrc_scene *s, const lrc_trace_params *p, int32_t rows, uint32_t spp) {
-    const uint64_t paths = (uint64_t)p->width * (uint64_t)rows * spp;
-    return !s->nvol && rows > 0 && spp > 0 && paths >= LRC_TRACE_WAVEFRONT_PATHS;
+    if (s->nvol || rows <= 0 || spp == 0) return false;
+    const uint64_t pixels = (uint64_t)p->width * (uint64_t)rows, most = 1u << 20;
+    const int64_t depth = p->max_depth;
+    const uint64_t deeper = s->tlas_n ? 12288u * (uint64_t)std::max<int64_t>(depth - 4, 0)
+                                      : 24576u * (uint64_t)std::max<int64_t>(depth - 8, 0);
+    const uint64_t tasks = pixels * (p->exact ? 1u : std::min<uint32_t>(spp, 16u));
+    return pixels * spp >= most || tasks >= std::min<uint64_t>(LRC_TRACE_WAVEFRONT_PATHS + deeper, most);
 }
 
 int trace_wavefront(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows, uint32_t spp0, uint32_t spp,

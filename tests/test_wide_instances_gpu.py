@@ -119,3 +119,24 @@ def test_first_use_in_a_capture_and_on_another_stream(own):
     finally:
         own.check(own.L.lrc_set_stream(own.h, None))
     s.close()
+
+
+@pytest.mark.parametrize("world", ["box", "field"])
+@pytest.mark.parametrize("exact", [0, 1])
+@pytest.mark.parametrize("w,h,spp,depth", [(384, 256, 1, 4), (383, 256, 1, 4), (96, 64, 16, 8), (96, 96, 16, 8), (96, 64, 40, 8),
+                                           (512, 384, 1, 12), (512, 383, 1, 12), (256, 256, 16, 3)])
+def test_images_at_the_wavefronts_line(own, world, exact, w, h, spp, depth):
+    """lrc_trace on both sides of where it takes the wavefront engine: the one-kernel path's image."""
+    if world == "field":
+        sc, s = scene(own, "few", 1)
+    else:
+        sc = W.box_scene(5, 1000, w, h)
+        mask, tab = np.zeros(4096, np.uint16), np.zeros(2112, np.float32)
+        L.lib().lrc_default_blue_noise(mask.ctypes.data)
+        L.lib().lrc_default_bsdf_tables(tab.ctypes.data)
+        s = R.world_scene(own, sc, 1, 30, mask, tab)
+    p = L.native.trace_params(R.camera12(sc), w, h, depth, 1, 1, exact, 3)
+    want, rays = s.trace(p, spp, flags=L.native.LRC_TRACE_MEGAKERNEL)
+    got, r = s.trace(p, spp)
+    assert np.array_equal(got, want) and r == rays
+    s.close()
