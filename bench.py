@@ -894,7 +894,10 @@ def run_serve(a):
                                "kernel); bytes per ray = box tests x 32 + triangle tests x 48 from the counting "
                                "build of the kernel on the same run"}
     value = served_rays / served_span / 1e6
-    cpu_v, cores, _, _, text = serve_cpu_sample(dicts, 15.0)
+    cpu = None
+    if not a.no_cpu:
+        cpu_v, cores, _, _, text = serve_cpu_sample(dicts, 15.0)
+        cpu = {"value": cpu_v, "unit": "Mrays/s", "cores": cores, "kind": "reference", "sample": text}
     line = {"metric": METRIC_SERVE, "value": value, "unit": "Mrays/s", "n_gpus": 1, "steps": a.steps,
             "warmup": a.warmup, "ms_per_step": 1e3 * served_span / a.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
@@ -903,7 +906,7 @@ def run_serve(a):
             "gpu_launches_counted": "the served streams' trace kernels: per wave the wavefront's clear and resolve "
                                     "and 4 kernels a pass (advance, closest hit, shade, shadow), passes read from "
                                     "the device; admission copies, refits and the denoiser not counted",
-            "cpu_baseline": {"value": cpu_v, "unit": "Mrays/s", "cores": cores, "kind": "reference", "sample": text},
+            "cpu_baseline": cpu,
             "plain_mrays_s": sum(r["plain"]["mrays_s"] * r["plain"]["span_s"] for k, r in results.items()
                                  if k != "sub_capacity") / sum(r["plain"]["span_s"] for k, r in results.items()
                                                                if k != "sub_capacity"),
@@ -1602,10 +1605,20 @@ def run_realtime(a):
                       "gpu_launches": REALTIME_LAUNCHES * a.steps, "cpu_baseline": cpu}), flush=True)
 
 
+# the workloads whose reference arm times the reference's CPU engine, and their metrics
+REFERENCE_ARMS = {"serve": METRIC_SERVE, "batch": METRIC_BATCH, "caustics": METRIC_CAUSTICS, "builder": METRIC}
+
+
 def main():
     a = parse()
+    from oracle import oracle as O
+    if a.workload != "denoise":                      # (its CPU leg is the numpy restatement)
+        a.no_cpu = a.no_cpu or not O.have_reference()
     if a.impl == "reference":
-        if a.workload == "serve":
+        if a.workload in REFERENCE_ARMS and not O.have_reference():
+            print(json.dumps({"impl": "reference", "metric": REFERENCE_ARMS[a.workload], "unavailable":
+                              "the reference's sources are absent here and its CPU engine is not built"}), flush=True)
+        elif a.workload == "serve":
             run_reference_serve(a)
         elif a.workload == "batch":
             run_reference_batch(a)

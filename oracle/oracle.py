@@ -24,12 +24,27 @@ _i64p = np.ctypeslib.ndpointer(np.int64, flags="C_CONTIGUOUS")
 _u16p = np.ctypeslib.ndpointer(np.uint16, flags="C_CONTIGUOUS")
 
 
+class ReferenceAbsent(RuntimeError):
+    """The reference's CPU engine is asked for where neither its sources nor a built _ref/ are."""
+
+
+def reference_sources():
+    """The reference's checkout, or None where there is none."""
+    ref = os.environ.get("LR_REFERENCE", "/root/reference")
+    return ref if os.path.isfile(os.path.join(ref, "engine", "rt", "tracer.c")) else None
+
+
+def have_reference():
+    """Whether the reference's CPU engine is built (_ref/), or could be (build)."""
+    return os.path.exists(os.path.join(HERE, "_ref", "libref_f.so")) or reference_sources() is not None
+
+
 def build():
     """Builds liboracle.so and, where the reference sources are present, _ref/*.so."""
     import subprocess
-    make = ["make", "-s", "-C", HERE, "all"]
-    ref = os.environ.get("LR_REFERENCE", "/root/reference")   # the reference's checkout, where present
-    if os.path.isfile(os.path.join(ref, "engine", "rt", "tracer.c")):
+    ref = reference_sources()
+    make = ["make", "-s", "-C", HERE, "all" if have_reference() else "oracle"]
+    if ref:
         make.append(f"REF={ref}")
     subprocess.run(make, check=True)
 
@@ -39,6 +54,8 @@ def _load(name):
         return _libs[name]
     path = os.path.join(HERE, name)
     if not os.path.exists(path):
+        if name.startswith("_ref") and not have_reference():
+            raise ReferenceAbsent(f"{path}: the reference's sources are absent and it is not built")
         raise RuntimeError(f"oracle library {path} is not built (make -C oracle)")
     lib = C.CDLL(path)
     _libs[name] = lib
