@@ -75,10 +75,6 @@ int scene_build_on(lrc_scene *s, int builder, int key_bits, void **scratch, size
     return LRC_OK;
 }
 
-static bool capturing(cudaStream_t st) {
-    cudaStreamCaptureStatus now = cudaStreamCaptureStatusNone;
-    return cudaStreamIsCapturing(st, &now) != cudaSuccess || now != cudaStreamCaptureStatusNone;
-}
 // Wide nodes are made on a first use, on the stream of that use. The scene's later uses may be on other
 // streams (lrc_set_stream), which the caller has no reason to order after it: each waits for the event.
 static int wide_noted(lrc_scene *s, cudaStream_t st) {
@@ -88,14 +84,13 @@ static int wide_noted(lrc_scene *s, cudaStream_t st) {
     return e ? cuda_status(s->ctx, e, "the wide nodes' event") : LRC_OK;
 }
 static int wide_ordered(lrc_scene *s, cudaStream_t st) {
-    if (s->wide_done) return LRC_OK;
-    const bool in_graph = capturing(st);
-    if (!in_graph && cudaEventQuery(s->wide_made) == cudaSuccess) {
+    if (s->wide_done || capturing(st)) return LRC_OK;   // (no wide nodes are walked in a capture)
+    if (cudaEventQuery(s->wide_made) == cudaSuccess) {
         s->wide_done = true;
         return LRC_OK;
     }
-    if (!in_graph) cudaGetLastError();               // (not ready)
-    cudaError_t e = cudaStreamWaitEvent(st, s->wide_made, in_graph ? cudaEventWaitExternal : 0);
+    cudaGetLastError();                              // (not ready)
+    cudaError_t e = cudaStreamWaitEvent(st, s->wide_made, 0);
     return e ? cuda_status(s->ctx, e, "the wide nodes' event") : LRC_OK;
 }
 
@@ -154,7 +149,7 @@ int instances_wide(lrc_scene *s, cudaStream_t st) {
 int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc) {
     if (!no_alloc) {                                 // (no_alloc: a batch's capture, in its own order)
         int rc = wide_ordered(s, st);
-        if (rc || capturing(st)) return rc;          // (what is made by now is walked, else the binary nodes)
+        if (rc || capturing(st)) return rc;
     }
     if (s->pwide_ok || !s->built_n || !s->most_leaf || s->most_leaf > kMostLeaf) return LRC_OK;
     lrc_ctx *c = s->ctx;
@@ -177,13 +172,14 @@ int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc) {
 }
 
 // The queries' wide nodes, from the walk's tree (a tree with larger leaves than a node has slots, no memory,
-// a first query inside a capture: the binary walk). Made by the first query after a build: a scene that
+// a query inside a capture: the binary walk). Made by the first query after a build: a scene that
 // is built each frame and only path traced would pay for nodes it never walks (scene builds of 200k / 4M
 // triangles 0.25 / 1.5 ms, with them 0.37 / 3.0).
 static int query_wide(lrc_scene *s) {
     lrc_ctx *c = s->ctx;
     int rc = wide_ordered(s, c->st);
-    if (rc || s->wide_ok || !s->walk_ok || !s->most_leaf || s->most_leaf > kMostLeaf || capturing(c->st)) return rc;
+    if (rc || s->wide_ok || !s->walk_ok || !s->most_leaf || s->most_leaf > kMostLeaf || capturing(c->st))
+        return rc;
     const bool single = !s->tree_nnodes;
     const uint32_t nn = single ? 2 * s->built_n - 1 : s->tree_nnodes, na = single ? s->built_n : s->tree_naux;
     if (s->wide_cap < lrc::wide_bytes(na, single)) return LRC_OK;
@@ -685,6 +681,7 @@ int lrc_scene_intersect(lrc_scene *s, const float *orig, const float *dir, uint6
     DeviceGuard g(c->device);
     lrc::TraceTables tt = tables(s);
     if (int rc = s->nprims ? scene_wide(s, c->st, false) : query_wide(s)) return rc;
+    const bool wide = s->wide_ok && !capturing(c->st);
     // LRC_SORT_RAYS: the reordering's scratch (large batches); without it the rays go in their order
     void *sort_scratch = nullptr;
     if ((flags & LRC_SORT_RAYS) && lrc::intersect_scratch_bytes(nrays)) {
@@ -694,7 +691,7 @@ int lrc_scene_intersect(lrc_scene *s, const float *orig, const float *dir, uint6
     // a world with primitives walks shape ids (primitives, then triangles); a mesh, triangles alone
     auto run = [&](const float *o, const float *d, int32_t *p, float *tt_out) {
         if (s->nprims) return lrc::pt_intersect(pt_scene(s), o, d, nrays, tmin, tmax, p, nullptr, tt_out, c->d_status, c->st);
-        if (s->wide_ok && !sort_scratch)
+        if (wide && !sort_scratch)
             return lrc::wide_intersect(wide_tables(s), tt, o, d, nrays, tmin, tmax, p, tt_out, c->d_status, c->st);
         return lrc::intersect_device(tt, o, d, nrays, tmin, tmax, p, tt_out, c->d_status, c->st, c->num_sms, sort_scratch,
                                      c->scratch_cap);
@@ -764,8 +761,9 @@ int lrc_scene_occluded(lrc_scene *s, const float *orig, const float *dir, const 
     DeviceGuard g(c->device);
     lrc::TraceTables tt = tables(s);
     if (int rc = query_wide(s)) return rc;
+    const bool wide = s->wide_ok && !capturing(c->st);
     if (flags & LRC_DEVICE) {
-        cudaError_t e = s->wide_ok ? lrc::wide_occluded(wide_tables(s), tt, orig, dir, tmax, nrays, tmin, out, c->d_status, c->st)
+        cudaError_t e = wide ? lrc::wide_occluded(wide_tables(s), tt, orig, dir, tmax, nrays, tmin, out, c->d_status, c->st)
                                    : lrc::occluded_device(tt, orig, dir, tmax, nrays, tmin, out, c->d_status, c->st);
         return cuda_status(c, e, "lrc_scene_occluded");
     }
@@ -779,7 +777,7 @@ int lrc_scene_occluded(lrc_scene *s, const float *orig, const float *dir, const 
     e = cudaMemcpyAsync(d_o, orig, nrays * 12, cudaMemcpyHostToDevice, c->st);
     if (!e) e = cudaMemcpyAsync(d_d, dir, nrays * 12, cudaMemcpyHostToDevice, c->st);
     if (!e) e = cudaMemcpyAsync(d_tm, tmax, nrays * 4, cudaMemcpyHostToDevice, c->st);
-    if (!e) e = s->wide_ok ? lrc::wide_occluded(wide_tables(s), tt, d_o, d_d, d_tm, nrays, tmin, d_out, c->d_status, c->st)
+    if (!e) e = wide ? lrc::wide_occluded(wide_tables(s), tt, d_o, d_d, d_tm, nrays, tmin, d_out, c->d_status, c->st)
                            : lrc::occluded_device(tt, d_o, d_d, d_tm, nrays, tmin, d_out, c->d_status, c->st);
     if (!e) e = cudaMemcpyAsync(out, d_out, nrays, cudaMemcpyDeviceToHost, c->st);
     if (e) return cuda_status(c, e, "lrc_scene_occluded");

@@ -131,6 +131,12 @@ inline int cuda_status(lrc_ctx *c, cudaError_t e, const char *what) {
     return fail(c, LRC_E_CUDA, what, e);
 }
 
+// whether a caller's graph is being captured on the stream
+inline bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus now = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &now) != cudaSuccess || now != cudaStreamCaptureStatusNone;
+}
+
 struct DeviceGuard {
     int prev = -1;
     explicit DeviceGuard(int d) {
@@ -187,7 +193,10 @@ inline lrc::PtScene pt_scene(const lrc_scene *s) {
     S.root = 0;
     S.nnodes = s->tree_nnodes ? s->tree_nnodes : (s->built_n ? 2 * s->built_n - 1 : 0);
     S.naux = s->tree_nnodes ? s->tree_naux : s->built_n;
-    if (s->pwide_ok) S.wide = lrc::wide_view(s->d_pwide, S.naux, !s->tree_nnodes);
+    // (a graph may be replayed after a build, which leaves the wide nodes as they were: in a caller's
+    // capture the binary nodes are walked, which a build makes again in place)
+    const bool wide = !capturing(s->ctx->st);
+    if (s->pwide_ok && wide) S.wide = lrc::wide_view(s->d_pwide, S.naux, !s->tree_nnodes);
     S.prims = reinterpret_cast<const float4 *>(s->d_prims);
     S.nprims = s->nprims;
     S.tris = reinterpret_cast<const float4 *>(s->d_tris);
@@ -214,7 +223,7 @@ inline lrc::PtScene pt_scene(const lrc_scene *s) {
         S.mnaux = s->nmtris;
         S.mesh_info = s->d_mesh_info;
         S.nmeshes = (uint32_t)s->mesh_counts.size();
-        if (s->twide_ok && s->mwide_ok) {
+        if (s->twide_ok && s->mwide_ok && wide) {
             S.tlas_wide = lrc::wide_view(s->d_twide, s->ninst, true);
             S.mesh_wide = static_cast<const lrc::WideScene *>(s->d_mwide);
         }

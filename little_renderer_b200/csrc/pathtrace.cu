@@ -24,7 +24,7 @@ namespace lrc {
 namespace pt {
 
 // Every lane on its own way, through the binary nodes: scenes with media (their shadow rays are traced in
-// place, path_shade) and calls of more paths than PT_WARP_PATHS (below).
+// place, path_shade), scenes without wide nodes and calls of more paths than PT_WARP_PATHS (below).
 // exact mode: one thread per pixel of rows [y0, y0 + rows), samples [0, spp) in order from the
 // CPU's per-pixel stream (trace_image, tracer.c:337-353)
 template <bool MEDIA, bool GUIDED>
@@ -392,7 +392,7 @@ cudaError_t pt_trace(const PtScene &S, const PtParams &P, float *d_accum, unsign
     float4 *acc = reinterpret_cast<float4 *>(d_accum);
     const uint64_t paths = P.exact ? (uint64_t)P.W * P.rows : (uint64_t)P.W * P.rows * P.group;
     const int k = P.moments ? 1 : 0, x = P.exact ? 1 : 0;
-    if (S.nvol || paths > pt::PT_WARP_PATHS) {
+    if (S.nvol || paths > pt::PT_WARP_PATHS || !S.wide.nodes) {
         // (kernels compiled with and without the media's tracking and the denoiser's moments: each
         // holds registers that a scene or an image without them would pay for)
         using Fn = void (*)(PtScene, PtParams, float4 *, unsigned long long *, uint32_t *);
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(128) grad_kernel(const __grid_constant__ PtSce
 cudaError_t pt_gradients(const PtScene &S, const PtParams &P, GradTile *d_tiles, uint32_t ntiles, const float4 *d_guide,
                          unsigned long long *d_rays, uint32_t *d_status, cudaStream_t st) {
     if (!ntiles) return cudaSuccess;
-    const bool warp = !S.nvol && ntiles <= pt::PT_WARP_PATHS;   // (pt_trace's line)
+    const bool warp = !S.nvol && ntiles <= pt::PT_WARP_PATHS && S.wide.nodes;   // (pt_trace's line)
     uint32_t spread = 1;
     while (warp && spread < pt::SPREAD_MOST && (uint64_t)ntiles * spread * 2 <= pt::SPREAD_LANES) spread *= 2;
     (S.nvol ? pt::grad_kernel<true, false> : warp ? pt::grad_kernel<false, true> : pt::grad_kernel<false, false>)

@@ -1,0 +1,152 @@
+"""What else may happen to a scene between the making of its wide nodes and a walk over them - builds and
+moves in a caller's graph or a batch's, queries in one, other streams, boxes and rays that are no
+numbers, trees deeper than a stack - against the binary walk (LRC_SORT_RAYS, the one-kernel path) or
+a scene made anew."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import little_renderer_b200 as L
+from little_renderer_b200 import render as R, workloads as W
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+DEVICE = L.native.LRC_DEVICE
+
+
+@pytest.fixture(scope="module")
+def own():
+    return L.Context(0)
+
+
+def dev(a):
+    t = torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    torch.cuda.synchronize()
+    return t
+
+
+def soup(n, seed):
+    return L.pack_tris(W.corners_to_quv(W.soup(n, seed)))
+
+
+def hits(own, tris, o, d):
+    """The closest hits of a scene made anew."""
+    s = L.native.Scene(own)
+    s.set_triangles(tris)
+    s.build(1, 30)
+    out = s.intersect(o, d)
+    s.close()
+    return out
+
+
+def captured(own, fn):
+    """fn's calls as a graph of a caller's."""
+    side = torch.cuda.Stream()
+    own.set_stream(side.cuda_stream)
+    g = torch.cuda.CUDAGraph()
+    try:
+        with torch.cuda.graph(g, stream=side):
+            fn()
+    finally:
+        own.set_stream(None)
+    return g
+
+
+def replay(own, g):
+    own.sync()
+    g.replay()
+    torch.cuda.synchronize()
+
+
+def field(own, few=True, wild=None):
+    """An instanced field: the scene, its dict and its records. few: meshes of some 25 triangles. wild: one
+    triangle of each mesh has a coordinate of that value, the instances' boxes as they were."""
+    sc = W.instanced_field(seed=3, n_instances=200, n_meshes=4, tri_range=(20, 30) if few else (200, 900),
+                           width=72, height=40, sky_w=64, sky_h=32, spp=1, max_depth=6)
+    records = W.instance_records(sc)
+    if wild is not None:
+        sc["meshes"] = [m.copy() for m in sc["meshes"]]
+        for i, m in enumerate(sc["meshes"]):
+            m[1 + i % 3, 0, i % 3] = wild
+    s = L.native.Scene(own)
+    g = sc["ground"]
+    s.set_prims(W.make_quad(g["q"], g["u"], g["v"], g["material"]))
+    s.set_light(-1)
+    s.set_materials(W.material_records(sc["materials"]))
+    s.build(1, 30)
+    s.set_meshes([L.pack_tris(W.corners_to_quv(t), np.full(t.shape[0], m, np.int32))
+                  for t, m in zip(sc["meshes"], sc["mesh_mats"])])
+    s.set_instances(records)
+    s.build_instances(1, 30)
+    s.set_sky(sc["sky"])
+    return s, sc, records
+
+
+def wavefront(own, s, p, spp, **run):
+    """The image by the wavefront engine (with a stepped run's flags: and its statistics)."""
+    img = torch.zeros(p.height, p.width, 4, device="cuda")
+    torch.cuda.synchronize()
+    q = L.native.Batch(own)
+    q.set_wavefront(1024)
+    q.add(s, p, spp, img.data_ptr())
+    q.run(**run)
+    own.sync()
+    stats = q.step_stats()
+    q.close()
+    return (img.cpu().numpy(), stats) if run else img.cpu().numpy()
+
+
+def one_kernel(s, p, spp):
+    return s.trace(p, spp, flags=L.native.LRC_TRACE_MEGAKERNEL)[0]
+
+
+@pytest.mark.parametrize("m", [1000, 40_000])            # 8 lanes a ray, one
+def test_captured_queries_see_the_next_build(own, m):
+    n = 5000
+    o, d = W.rays_at_cube(m, 2)
+    s = L.native.Scene(own)
+    s.set_triangles(soup(n, 5))
+    s.build(1, 30)
+    s.intersect(o, d)                                    # (the wide nodes are there when the graph is captured)
+    ro, rd, far = dev(o), dev(d), torch.full((m,), 3.0, device="cuda")
+    prim, t = torch.zeros(m, dtype=torch.int32, device="cuda"), torch.zeros(m, device="cuda")
+    blocked = torch.zeros(m, dtype=torch.uint8, device="cuda")
+
+    def queries():
+        s.intersect_device(ro.data_ptr(), rd.data_ptr(), m, prim.data_ptr(), t.data_ptr())
+        own.check(own.L.lrc_scene_occluded(s.h, *[C.c_void_p(x.data_ptr()) for x in (ro, rd, far)], m, 0.0,
+                                           C.c_void_p(blocked.data_ptr()), DEVICE))
+
+    g = captured(own, queries)
+    for seed in (6, 7):
+        s.set_triangles(soup(n, seed))
+        s.build(1, 30)
+        replay(own, g)
+        want = hits(own, soup(n, seed), o, d)
+        assert np.array_equal(prim.cpu().numpy(), want[0]) and np.array_equal(t.cpu().numpy(), want[1])
+        assert np.array_equal(blocked.cpu().numpy().astype(bool), want[0] >= 0)
+    s.close()
+
+
+def test_captured_small_images_see_the_next_build(own):
+    a, b = W.box_scene(5, 3000, 72, 40), W.box_scene(6, 3000, 72, 40)
+    s = R.world_scene(own, a, 1)
+    p = L.native.trace_params(R.camera12(a), 72, 40, 8, 1, 1, 0, 3)
+    first = s.trace(p, 2)[0]
+    img, planes = torch.zeros(40, 72, 4, device="cuda"), torch.zeros(4, 40, 72, 4, device="cuda")
+    torch.cuda.synchronize()
+
+    def images():
+        s.trace_device(p, 2, img.data_ptr())
+        s.guide_device(p, planes.data_ptr())
+
+    g = captured(own, images)
+    s.set_triangles(L.pack_tris(W.corners_to_quv(b["corners"]), a["tri_mats"]))
+    s.build(1, 30)
+    img.zero_()
+    replay(own, g)
+    got = img.cpu().numpy()
+    assert np.array_equal(got, s.trace(p, 2)[0]) and not np.array_equal(got, first)
+    assert np.array_equal(planes.cpu().numpy(), s.guide(p))
+    s.close()
