@@ -28,7 +28,10 @@ int scene_build_on(lrc_scene *s, int builder, int key_bits, void **scratch, size
     DeviceGuard g(c->device);
     // the shapes: primitives, then triangles (their ids as the reference's, scene.h:101-106)
     const uint32_t n = s->ntris + s->nprims;
-    if (!no_alloc) s->built_n = 0;
+    if (!no_alloc) {
+        s->built_n = 0;
+        s->replayed = s->replayed || capturing(st);
+    }
     s->tree_nnodes = s->tree_naux = 0;
     s->walk_ok = false;
     s->wide_ok = false;
@@ -100,7 +103,7 @@ int instances_wide(lrc_scene *s, cudaStream_t st) {
     lrc_ctx *c = s->ctx;
     if (!s->meshes_built || !s->ninst || s->tlas_n != s->ninst) return LRC_OK;
     int rc = wide_ordered(s, st);
-    if (rc || (s->twide_ok && s->mwide_ok) || capturing(st)) return rc;
+    if (rc || (s->twide_ok && s->mwide_ok) || s->inst_replayed || capturing(st)) return rc;
     const size_t nm = s->mesh_counts.size();
     cudaError_t e = cudaSuccess;
     if (!s->mwide_ok) {
@@ -151,7 +154,7 @@ int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc) {
         int rc = wide_ordered(s, st);
         if (rc || capturing(st)) return rc;
     }
-    if (s->pwide_ok || !s->built_n || !s->most_leaf || s->most_leaf > kMostLeaf) return LRC_OK;
+    if (s->pwide_ok || s->replayed || !s->built_n || !s->most_leaf || s->most_leaf > kMostLeaf) return LRC_OK;
     lrc_ctx *c = s->ctx;
     const bool single = !s->tree_nnodes;
     const uint32_t nn = single ? 2 * s->built_n - 1 : s->tree_nnodes, na = single ? s->built_n : s->tree_naux;
@@ -172,13 +175,13 @@ int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc) {
 }
 
 // The queries' wide nodes, from the walk's tree (a tree with larger leaves than a node has slots, no memory,
-// a query inside a capture: the binary walk). Made by the first query after a build: a scene that
+// a query inside a capture, a scene that a graph builds: the binary walk). Made by the first query after a build: a scene that
 // is built each frame and only path traced would pay for nodes it never walks (scene builds of 200k / 4M
 // triangles 0.25 / 1.5 ms, with them 0.37 / 3.0).
 static int query_wide(lrc_scene *s) {
     lrc_ctx *c = s->ctx;
     int rc = wide_ordered(s, c->st);
-    if (rc || s->wide_ok || !s->walk_ok || !s->most_leaf || s->most_leaf > kMostLeaf || capturing(c->st))
+    if (rc || s->wide_ok || !s->walk_ok || s->replayed || !s->most_leaf || s->most_leaf > kMostLeaf || capturing(c->st))
         return rc;
     const bool single = !s->tree_nnodes;
     const uint32_t nn = single ? 2 * s->built_n - 1 : s->tree_nnodes, na = single ? s->built_n : s->tree_naux;
@@ -514,6 +517,7 @@ int lrc_scene_set_triangles(lrc_scene *s, const uint32_t *tris, uint32_t n, unsi
     if (n) e = cudaMemcpyAsync(s->d_tris, tris, (size_t)n * 48,
                                (flags & LRC_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->st);
     if (e) return cuda_status(c, e, "triangles");
+    s->replayed = s->replayed || capturing(c->st);
     s->ntris = n;
     s->built_n = 0;
     s->tree_nnodes = s->tree_naux = 0;
@@ -608,6 +612,7 @@ int lrc_scene_set_tree(lrc_scene *s, const uint32_t *nodes, uint32_t nnodes, con
     if (!e) e = cudaMemcpyAsync(s->d_nodes, nodes, (size_t)nnodes * 32, k, c->st);
     if (!e) e = cudaMemcpyAsync(s->d_aux, aux, (size_t)naux * 4, k, c->st);
     if (e) return cuda_status(c, e, "lrc_scene_set_tree");
+    s->replayed = s->replayed || capturing(c->st);
     s->built_n = naux;
     s->tree_nnodes = nnodes;
     s->tree_naux = naux;
@@ -794,6 +799,7 @@ int lrc_scene_set_prims(lrc_scene *s, const float *prims, uint32_t n, unsigned f
         e = cudaMemcpyAsync(s->d_prims, prims, (size_t)n * 96, (flags & LRC_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                             c->st);
     if (e) return cuda_status(c, e, "primitives");
+    s->replayed = s->replayed || capturing(c->st);
     s->nprims = n;
     s->built_n = 0;
     s->tree_nnodes = s->tree_naux = 0;
@@ -899,6 +905,7 @@ int lrc_scene_set_meshes(lrc_scene *s, const uint32_t *tris, const uint32_t *tri
         e = cudaMemcpyAsync(s->d_mtris, tris, total * 48, (flags & LRC_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                             c->st);
     if (e) return cuda_status(c, e, "meshes");
+    s->inst_replayed = s->inst_replayed || capturing(c->st);
     return (flags & LRC_DEVICE) ? LRC_OK : check_status(c);
 }
 
@@ -912,6 +919,7 @@ int lrc_scene_set_instances(lrc_scene *s, const float *records, uint32_t n, unsi
         e = cudaMemcpyAsync(s->d_inst, records, (size_t)n * 128,
                             (flags & LRC_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->st);
     if (e) return cuda_status(c, e, "instances");
+    s->inst_replayed = s->inst_replayed || capturing(c->st);
     s->ninst = n;
     s->tlas_n = 0;
     s->twide_ok = false;
@@ -959,6 +967,7 @@ int lrc_scene_build_instances(lrc_scene *s, int mesh_builder, int key_bits) {
     }
     s->tlas_n = 0;
     s->twide_ok = false;
+    s->inst_replayed = s->inst_replayed || capturing(c->st);
     const uint32_t n = s->ninst;
     if (!n) return LRC_OK;
     if (s->tlas_cap < n) {
@@ -988,6 +997,7 @@ int lrc_scene_move_instances(lrc_scene *s, const float *records, uint32_t n, int
     if (!s->tlas_n || n != s->ninst) return fail(c, LRC_E_INVALID, "moves the built instances only (same count)");
     DeviceGuard g(c->device);
     s->twide_ok = false;
+    s->inst_replayed = s->inst_replayed || capturing(c->st);
     cudaError_t e = cudaMemcpyAsync(s->d_inst, records, (size_t)n * 128,
                                     (flags & LRC_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->st);
     if (e) return cuda_status(c, e, "instances");

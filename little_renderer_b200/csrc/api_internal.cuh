@@ -55,6 +55,9 @@ struct lrc_scene {
     size_t twide_cap = 0;
     bool twide_ok = false;
     uint32_t most_leaf = 1;       // the largest leaf of the tree (0: not known)
+    // A change of the world (of the instances) that a caller's graph has captured happens again with each
+    // replay, unseen here: nothing made from the trees on the host's word is walked from then on.
+    bool replayed = false, inst_replayed = false;
     float *d_boxes = nullptr;
     size_t boxes_cap = 0;
     uint32_t *d_small = nullptr;  // 6 bound keys, 6 bounds, 6 lo/ext

@@ -156,7 +156,8 @@ lrc::PtScene view_of(const lrc_batch::Job &J, bool building) {
         S.nnodes = n ? 2 * n - 1 : 0;
         S.naux = n;
         // (its wide nodes are made behind the build, in the buffer an earlier run sized)
-        S.wide = n && J.s->pwide_cap >= lrc::wide_bytes(n, true) ? lrc::wide_view(J.s->d_pwide, n, true) : lrc::WideScene{};
+        S.wide = n && !J.s->replayed && J.s->pwide_cap >= lrc::wide_bytes(n, true) ? lrc::wide_view(J.s->d_pwide, n, true)
+                                                                                   : lrc::WideScene{};
     }
     return S;
 }
@@ -521,7 +522,7 @@ void note_built(lrc_batch *b) {   // (what captured builds' host side records)
     for (const lrc_batch::Job *J : builds_of(b)) {
         J->s->built_n = J->s->ntris + J->s->nprims;
         J->s->most_leaf = 1;
-        J->s->pwide_ok = J->s->built_n && J->s->pwide_cap >= lrc::wide_bytes(J->s->built_n, true);
+        J->s->pwide_ok = J->s->built_n && !J->s->replayed && J->s->pwide_cap >= lrc::wide_bytes(J->s->built_n, true);
     }
 }
 

@@ -150,3 +150,46 @@ def test_captured_small_images_see_the_next_build(own):
     assert np.array_equal(got, s.trace(p, 2)[0]) and not np.array_equal(got, first)
     assert np.array_equal(planes.cpu().numpy(), s.guide(p))
     s.close()
+
+
+def test_captured_builds_are_seen_by_the_next_query(own):
+    n, m = 5000, 40_000
+    o, d = W.rays_at_cube(m, 2)
+    s = L.native.Scene(own)
+    tris = dev(soup(n, 5).view(np.int32))
+
+    def build():
+        s.set_triangles(None, tris.data_ptr(), n)
+        s.build(1, 30)
+
+    build()
+    s.intersect(o, d)
+    g = captured(own, build)
+    for seed in (6, 7):
+        tris.copy_(dev(soup(n, seed).view(np.int32)))
+        torch.cuda.synchronize()
+        replay(own, g)
+        got, want = s.intersect(o, d), hits(own, soup(n, seed), o, d)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    s.close()
+
+
+@pytest.mark.parametrize("mode", [0, 1])                 # refitted, rebuilt
+def test_captured_moves_are_seen_by_the_next_image(own, mode):
+    s, sc, records = field(own)
+    p = L.native.trace_params(R.camera12(sc), 72, 40, 6, 1, 1, 0, 3)
+    wavefront(own, s, p, 3)
+    r = dev(records)
+
+    def move():
+        own.check(own.L.lrc_scene_move_instances(s.h, C.c_void_p(r.data_ptr()), records.shape[0], mode, DEVICE))
+
+    move()
+    g = captured(own, move)
+    for _ in range(2):
+        sc["xf"][:, 0, 3] += np.float32(1.5)
+        r.copy_(dev(W.instance_records(sc)))
+        torch.cuda.synchronize()
+        replay(own, g)
+        assert np.array_equal(wavefront(own, s, p, 3), one_kernel(s, p, 3))
+    s.close()
