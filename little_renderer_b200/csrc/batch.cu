@@ -521,6 +521,8 @@ int tune_wavefront(lrc_batch *b, unsigned long long n, int32_t *variant, int32_t
 void note_built(lrc_batch *b) {   // (what captured builds' host side records)
     for (const lrc_batch::Job *J : builds_of(b)) {
         J->s->built_n = J->s->ntris + J->s->nprims;
+        J->s->tree_nnodes = J->s->tree_naux = 0;     // (a tree given or built meanwhile, and its copy, are gone)
+        J->s->walk_ok = J->s->wide_ok = false;
         J->s->most_leaf = 1;
         J->s->pwide_ok = J->s->built_n && !J->s->replayed && J->s->pwide_cap >= lrc::wide_bytes(J->s->built_n, true);
     }

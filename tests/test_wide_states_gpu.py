@@ -193,3 +193,48 @@ def test_captured_moves_are_seen_by_the_next_image(own, mode):
         replay(own, g)
         assert np.array_equal(wavefront(own, s, p, 3), one_kernel(s, p, 3))
     s.close()
+
+
+@pytest.mark.parametrize("engine", [0, 1])
+def test_replayed_builds_are_recorded(own, engine):
+    """A batch's replayed build after a tree of another kind: given with larger leaves, or built by PLOC."""
+    sc = W.box_scene(5, 3000, 72, 40)
+    s = L.native.Scene(own)                              # (triangles alone: queries walk a copy of the tree)
+    s.set_triangles(L.pack_tris(W.corners_to_quv(sc["corners"]), sc["tri_mats"]))
+    s.set_materials(W.material_records(sc["materials"]))
+    s.set_light(-1)
+    s.build(0, 30)
+    o, d = W.rays_at_cube(40_000, 4, centre=(278, 278, 278), scale=555.0)
+    want = s.intersect(o, d)
+    p = L.native.trace_params(R.camera12(sc), 72, 40, 8, 1, 1, 0, 3)
+    image = s.trace(p, 2)[0]
+    n = sc["corners"].shape[0]
+    pairs = np.zeros((2 * n, 8), np.uint32), np.arange(n, dtype=np.uint32)
+    box = pairs[0].view(np.float32)                      # (a list of leaves of 3 under one box)
+    leaves = [(i, min(3, n - i)) for i in range(0, n, 3)]
+    for k, (i, c) in enumerate(leaves[:-1]):
+        for at in (2 * k, 2 * k + 1):
+            box[at, 0:3], box[at, 4:7] = -1e4, 1e4
+        pairs[0][2 * k][[3, 7]] = 2 * k + 1, 2 * k + 2
+        pairs[0][2 * k + 1][[3, 7]] = i, 0x80000000 | c
+    last = 2 * (len(leaves) - 1)
+    box[last, 0:3], box[last, 4:7] = -1e4, 1e4
+    pairs[0][last][[3, 7]] = leaves[-1][0], 0x80000000 | leaves[-1][1]
+    img = torch.zeros(40, 72, 4, device="cuda")
+    torch.cuda.synchronize()
+    q = L.native.Batch(own)
+    q.set_engine(engine)
+    q.add(s, p, 2, img.data_ptr(), builder=0)
+    run = lambda: q.run(build=True, graph=True, zero=True)
+    for other in (lambda: s.build(1, 30), lambda: s.set_tree(pairs[0][: last + 1], pairs[1])):
+        for _ in range(3):
+            run()
+        other()
+        run()
+        own.sync()
+        assert q.info()["graph_used"] == 1
+        got = s.intersect(o, d)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+        assert np.array_equal(s.trace(p, 2)[0], image) and np.array_equal(img.cpu().numpy(), image)
+    s.close()
+    q.close()
