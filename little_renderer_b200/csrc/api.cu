@@ -108,7 +108,8 @@ int instances_wide(lrc_scene *s, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     if (!s->mwide_ok) {
         std::vector<lrc::WideScene> views(nm);
-        size_t off = al(nm * sizeof(lrc::WideScene)), nodes = 0;
+        const size_t table = al(nm * sizeof(lrc::WideScene) + 4);   // (the views, then the meshes' common mark)
+        size_t off = table, nodes = 0;
         for (uint32_t n : s->mesh_counts) {
             off += n ? lrc::wide_bytes(n, true) : 0;
             nodes += n ? 2 * (size_t)n - 1 : 0;
@@ -118,20 +119,22 @@ int instances_wide(lrc_scene *s, cudaStream_t st) {
             return LRC_OK;
         }
         char *b = static_cast<char *>(s->d_mwide);
-        off = al(nm * sizeof(lrc::WideScene));
+        uint32_t *wild = reinterpret_cast<uint32_t *>(b + nm * sizeof(lrc::WideScene));
+        e = cudaMemsetAsync(wild, 0, 4, st);
+        off = table;
         uint32_t node0 = 0;
         for (size_t m = 0; m < nm && !e; m++) {
             const uint32_t n = s->mesh_counts[m];
             if (!n) continue;
             views[m] = lrc::wide_view(b + off, n, true);
             e = lrc::wide_build_part(s->d_mnodes, node0, (uint32_t)nodes, s->d_maux, s->nmtris, n, 0,
-                                     reinterpret_cast<const float *>(s->d_mtris), s->nmtris, lrc::WD_WIDEN, b + off, true, c->d_status,
-                                     c->num_sms, st);
+                                     reinterpret_cast<const float *>(s->d_mtris), s->nmtris, lrc::WD_WIDEN, b + off, true, wild,
+                                     c->d_status, c->num_sms, st);
             off += lrc::wide_bytes(n, true);
             node0 += 2 * n - 1;
         }
         // (pageable memory: read before the call returns)
-        if (!e) e = cudaMemcpyAsync(b, views.data(), nm * sizeof(lrc::WideScene), cudaMemcpyHostToDevice, st);
+        if (!e && nm) e = cudaMemcpyAsync(b, views.data(), nm * sizeof(lrc::WideScene), cudaMemcpyHostToDevice, st);
         if (e) return cuda_status(c, e, "the meshes' wide nodes");
         s->mwide_ok = true;
         rc = wide_noted(s, st);

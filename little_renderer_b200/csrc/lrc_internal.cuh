@@ -158,10 +158,11 @@ cudaError_t wide_build(const Node *d_bin, uint32_t nn, const uint32_t *d_aux, ui
                        const float *d_tris, uint32_t ntris, float widen, void *buf, bool single, uint32_t *d_status, int num_sms,
                        cudaStream_t st);
 // the same of one tree among several in d_bin and d_aux: its root, its leaf entries' number (entries of the
-// view in buf); nn and naux bound the arrays
+// view in buf); nn and naux bound the arrays. d_wild: a word set when a box is none the nodes can hold (null:
+// the root's last word, wide_walked)
 cudaError_t wide_build_part(const Node *d_bin, uint32_t root, uint32_t nn, const uint32_t *d_aux, uint32_t naux,
                             uint32_t entries, uint32_t nprims, const float *d_tris, uint32_t ntris, float widen, void *buf,
-                            bool single, uint32_t *d_status, int num_sms, cudaStream_t st);
+                            bool single, uint32_t *d_wild, uint32_t *d_status, int num_sms, cudaStream_t st);
 // queries of a scene of triangles alone; tt: the binary tree the wide one was made from
 cudaError_t wide_intersect(const WideScene &W, const TraceTables &tt, const float *d_orig, const float *d_dir, uint64_t nrays,
                            float tmin, float tmax, int32_t *d_prim, float *d_t, uint32_t *d_status, cudaStream_t st);
@@ -242,7 +243,8 @@ struct PtScene {
     uint32_t mnnodes, mnaux;
     const uint4 *mesh_info;
     uint32_t nmeshes;
-    // both levels' wide nodes (none: null): the top level's (leaf entries: instances), each mesh's
+    // both levels' wide nodes (none: null): the top level's (leaf entries: instances), each mesh's (behind
+    // them a word that is not 0 where some mesh's cannot be walked)
     WideScene tlas_wide;
     const WideScene *mesh_wide;
     // the sky: radiance + pixel probability (w x h), each row's distribution, the rows'

@@ -390,7 +390,9 @@ struct DeepWalk {
     bool tie;
 };
 __device__ __forceinline__ bool deep_wide(const PtScene &S) {
-    return (!S.nnodes || world_wide(S)) && (!S.ninst || (S.tlas_wide.nodes && wide_walked(S.tlas_wide)));
+    return (!S.nnodes || world_wide(S)) &&
+           (!S.ninst || (S.tlas_wide.nodes && wide_walked(S.tlas_wide) &&
+                         __ldg(reinterpret_cast<const uint32_t *>(S.mesh_wide + S.nmeshes)) == 0u));
 }
 __device__ __forceinline__ void deep_begin(const PtScene &S, DeepWalk &w, float tmax) {
     w.level = S.nnodes ? 0 : 1;

@@ -33,6 +33,7 @@ struct Collapse {
     float widen;                                 // every box is widened by this share of the root box's largest coordinate
     float4 *nodes;
     uint32_t ncap;
+    uint32_t *wild;                              // set when a box is none the grid can hold
     float4 *leaves;
     uint32_t *items;
     uint32_t *ctr;
@@ -207,11 +208,12 @@ __global__ void __launch_bounds__(WD_THREADS) collapse_kernel(const __grid_const
             }
         }
         // boxes the grid cannot hold (a NaN, an infinity, coordinates beyond 1e18): the tree is not
-        // walked (the root's last word says so; the callers walk the binary one)
+        // walked (C.wild: the root's last word, or the mark a scene's meshes share, says so; the callers
+        // walk the binary one)
         bool plain = true;
 #pragma unroll
         for (int a = 0; a < 3; a++) plain = plain && (!have || (fabsf(c.lo[a]) <= 1e18f && fabsf(c.hi[a]) <= 1e18f));
-        if (!plain) atomicOr(reinterpret_cast<uint32_t *>(C.nodes) + 7, 1u);
+        if (!plain) atomicOr(C.wild, 1u);
         // a slot for each child: of the pairs left the one that lies best (its middle farthest to the
         // slot's corner), again and again
         float e[3];
@@ -530,7 +532,7 @@ WideScene wide_view(void *buf, uint32_t naux, bool single) {
 
 cudaError_t wide_build_part(const Node *d_bin, uint32_t root, uint32_t nn, const uint32_t *d_aux, uint32_t naux,
                             uint32_t entries, uint32_t nprims, const float *d_tris, uint32_t ntris, float widen, void *buf,
-                            bool single, uint32_t *d_status, int num_sms, cudaStream_t st) {
+                            bool single, uint32_t *d_wild, uint32_t *d_status, int num_sms, cudaStream_t st) {
     if (!nn || !entries) return cudaErrorInvalidValue;
     const WideScene W = wide_view(buf, entries, single);
     Collapse C{};
@@ -546,6 +548,7 @@ cudaError_t wide_build_part(const Node *d_bin, uint32_t root, uint32_t nn, const
     C.ntris = ntris;
     C.nodes = const_cast<float4 *>(W.nodes);
     C.ncap = W.nnodes;
+    C.wild = d_wild ? d_wild : static_cast<uint32_t *>(buf) + 7;
     C.leaves = const_cast<float4 *>(W.leaves);
     char *items = static_cast<char *>(buf) + up256((size_t)C.ncap * 80) + up256((size_t)entries * 48);
     const size_t item_bytes = up256((size_t)C.ncap * 4);
@@ -564,7 +567,8 @@ cudaError_t wide_build_part(const Node *d_bin, uint32_t root, uint32_t nn, const
 cudaError_t wide_build(const Node *d_bin, uint32_t nn, const uint32_t *d_aux, uint32_t naux, uint32_t nprims,
                        const float *d_tris, uint32_t ntris, float widen, void *buf, bool single, uint32_t *d_status, int num_sms,
                        cudaStream_t st) {
-    return wide_build_part(d_bin, 0, nn, d_aux, naux, naux, nprims, d_tris, ntris, widen, buf, single, d_status, num_sms, st);
+    return wide_build_part(d_bin, 0, nn, d_aux, naux, naux, nprims, d_tris, ntris, widen, buf, single, nullptr, d_status, num_sms,
+                           st);
 }
 
 cudaError_t wide_intersect(const WideScene &W, const TraceTables &tt, const float *d_orig, const float *d_dir, uint64_t nrays,

@@ -238,3 +238,13 @@ def test_replayed_builds_are_recorded(own, engine):
         assert np.array_equal(s.trace(p, 2)[0], image) and np.array_equal(img.cpu().numpy(), image)
     s.close()
     q.close()
+
+
+@pytest.mark.parametrize("few", [True, False])
+@pytest.mark.parametrize("wild", [np.nan, np.inf, 1e19])
+@pytest.mark.parametrize("exact", [0, 1])
+def test_meshes_that_no_grid_holds(own, exact, wild, few):
+    s, sc, _ = field(own, few, wild)
+    p = L.native.trace_params(R.camera12(sc), 72, 40, 6, 1, 1, exact, 3)
+    assert np.array_equal(wavefront(own, s, p, 5), one_kernel(s, p, 5))
+    s.close()
