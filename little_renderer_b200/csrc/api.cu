@@ -276,6 +276,11 @@ int trace_wavefront(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t
         rc = lrc_batch_create(c, &c->single);
         if (rc) return rc;
     }
+    // (all large images of the context share the batch's table, run block and state: one queued on another
+    // stream, which lrc_set_stream orders after nothing, would write them under a run)
+    cudaError_t e = c->single_ran ? cudaStreamWaitEvent(c->st, c->single_ran, 0)
+                                  : cudaEventCreateWithFlags(&c->single_ran, cudaEventDisableTiming);
+    if (e) return cuda_status(c, e, "the wavefront's event");
     // The paths in flight: all of them up to 2^22, in three sizes (a size's graph is captured when it is
     // first used, and two are kept): a pass costs most in its longest walks, so there should be few.
     // 640 x 640 pixels at 8 spp of 20k triangles: 2^20 12.4 ms, 2^21 11.9, 2^22 11.2. Up to 2^21 paths the
@@ -293,7 +298,8 @@ int trace_wavefront(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t
         if (!rc) rc = lrc_batch_run(c->single, 0);
         if (rc != LRC_RETRY || slots <= (1u << 20)) break;   // (no memory for so many: fewer)
     }
-    return rc;
+    e = cudaEventRecord(c->single_ran, c->st);
+    return rc || !e ? rc : cuda_status(c, e, "the wavefront's event");
 }
 
 }  // namespace lrcapi
@@ -333,6 +339,10 @@ void lrc_close(lrc_ctx *c) {
     if (!c) return;
     DeviceGuard g(c->device);
     cudaStreamSynchronize(c->st);
+    if (c->single_ran) {
+        cudaEventSynchronize(c->single_ran);
+        cudaEventDestroy(c->single_ran);
+    }
     if (c->single) lrc_batch_destroy(c->single);
     if (c->scratch) cudaFree(c->scratch);
     if (c->stage) cudaFree(c->stage);

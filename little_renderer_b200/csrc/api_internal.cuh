@@ -23,6 +23,7 @@ struct lrc_ctx {
     void *dn = nullptr;           // the denoiser's scratch (packed image ping-pong and guide)
     size_t dn_cap = 0;
     lrc_batch *single = nullptr;  // lrc_trace's one-job batch on the wavefront engine (large images)
+    cudaEvent_t single_ran = nullptr;   // after its last run, which the next one on another stream waits for
 };
 
 struct lrc_scene {

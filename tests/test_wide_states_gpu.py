@@ -248,3 +248,29 @@ def test_meshes_that_no_grid_holds(own, exact, wild, few):
     p = L.native.trace_params(R.camera12(sc), 72, 40, 6, 1, 1, exact, 3)
     assert np.array_equal(wavefront(own, s, p, 5), one_kernel(s, p, 5))
     s.close()
+
+
+def test_images_on_two_streams_at_once(own):
+    """Large images (one batch of the context's traces them) queued on two streams, nothing between them."""
+    jobs = []
+    for seed, (w, h) in enumerate([(512, 512), (640, 400), (1100, 1000), (512, 512)]):
+        sc = W.box_scene(5 + seed, 4000, w, h)
+        s = R.world_scene(own, sc, 1)
+        p = L.native.trace_params(R.camera12(sc), w, h, 8, 1, 1, 0, 3)
+        jobs.append((s, p, one_kernel(s, p, 1), torch.zeros(h, w, 4, device="cuda")))
+    streams = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    try:
+        for _ in range(3):
+            for k, (s, p, _, img) in enumerate(jobs):
+                own.set_stream(streams[k % 2].cuda_stream)
+                with torch.cuda.stream(streams[k % 2]):
+                    img.zero_()
+                s.trace_device(p, 1, img.data_ptr())
+            torch.cuda.synchronize()
+            for _, _, want, img in jobs:
+                assert np.array_equal(img.cpu().numpy(), want)
+    finally:
+        own.set_stream(None)
+    for s, *_ in jobs:
+        s.close()
