@@ -325,7 +325,8 @@ typedef struct {
  * A call of at least LRC_TRACE_WAVEFRONT_PATHS paths side by side (width x rows, in fast mode times
  * spp up to 16; more for depths above 8, or above 4 with instances), or of 2^20 paths, on a scene
  * without media runs as a one-job batch on the wavefront engine (the batch's image is this call's to
- * the bit); smaller ones, scenes with media and calls with LRC_TRACE_MEGAKERNEL run the one-kernel path. */
+ * the bit); smaller ones, scenes with media, calls captured into a graph and calls with
+ * LRC_TRACE_MEGAKERNEL run the one-kernel path. */
 int lrc_trace(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows, uint32_t spp0, uint32_t spp,
               float *accum, uint64_t *rays, unsigned flags);
 #define LRC_TRACE_GUIDED 64u  /* flag: accum is the denoiser's 4 planes (below); each sample's luminance

@@ -257,9 +257,10 @@ int make_walk(lrc_scene *s) {
 // 2.32 / 3.40, 512 x 512 3.54 / 4.78 and 2.63 / 3.97. With instances (8000 triangles each), whose walks are
 // longer: depth 4, 320 x 320 2.60 and 2.41; depth 12, 400 x 400 4.88 and 5.66, 512 x 512 6.83 and 6.34.
 // What counts is the tasks, which run side by side (exact mode has one a pixel, fast mode up to 16); from
-// 2^20 paths on the wavefront whatever their number.
+// 2^20 paths on the wavefront whatever their number. Within a caller's capture the one-kernel path, whose
+// launches can be captured (the wavefront's run is a graph of its own).
 bool wavefront_call(const lrc_scene *s, const lrc_trace_params *p, int32_t rows, uint32_t spp) {
-    if (s->nvol || rows <= 0 || spp == 0) return false;
+    if (s->nvol || rows <= 0 || spp == 0 || capturing(s->ctx->st)) return false;
     const uint64_t pixels = (uint64_t)p->width * (uint64_t)rows, most = 1u << 20;
     const int64_t depth = p->max_depth;
     const uint64_t deeper = s->tlas_n ? 12288u * (uint64_t)std::max<int64_t>(depth - 4, 0)

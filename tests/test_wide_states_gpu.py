@@ -274,3 +274,22 @@ def test_images_on_two_streams_at_once(own):
         own.set_stream(None)
     for s, *_ in jobs:
         s.close()
+
+
+@pytest.mark.parametrize("w,h", [(64, 64), (200, 160), (512, 512)])   # each kind of route, captured on the one-kernel path
+def test_images_in_a_callers_graph(own, w, h):
+    sc = W.box_scene(5, 1000, w, h)
+    s = R.world_scene(own, sc, 1)
+    p = L.native.trace_params(R.camera12(sc), w, h, 8, 1, 1, 0, 3)
+    planes = s.trace_frame(None, p, 0, 1, None, 0, 8)
+    img, new = torch.zeros(h, w, 4, device="cuda"), torch.zeros(4, h, w, 4, device="cuda")
+    torch.cuda.synchronize()
+
+    def images():
+        s.trace_device(p, 1, img.data_ptr())
+        s.trace_frame_device(None, p, 0, 1, 0, new.data_ptr(), 0, 8)
+
+    g = captured(own, images)
+    replay(own, g)
+    assert np.array_equal(img.cpu().numpy(), one_kernel(s, p, 1)) and np.array_equal(new.cpu().numpy(), planes)
+    s.close()
