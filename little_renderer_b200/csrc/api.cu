@@ -1207,11 +1207,14 @@ int lrc_trace(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows,
         P.moments = reinterpret_cast<float4 *>(d_acc) + N;
         P.guide = reinterpret_cast<const float4 *>(d_acc) + 3 * N;
     }
+    int wf = LRC_RETRY;                                  // (no memory for the wavefront's state: the one-kernel path)
     if (!e && !(flags & LRC_TRACE_MEGAKERNEL) && wavefront_call(s, p, rows, spp)) {
         c->timer.begin(LRC_TS_SHADE, c->st);
-        int rc = trace_wavefront(s, p, y0, rows, spp0, spp, d_acc, guided);
+        wf = trace_wavefront(s, p, y0, rows, spp0, spp, d_acc, guided);
         c->timer.end(c->st);
-        if (rc) return rc;
+        if (wf && wf != LRC_RETRY) return wf;
+    }
+    if (!wf) {
         if (!(flags & LRC_DEVICE)) {
             e = cudaMemcpyAsync(accum, d_acc, bytes, cudaMemcpyDeviceToHost, c->st);
             if (e) return cuda_status(c, e, "lrc_trace");

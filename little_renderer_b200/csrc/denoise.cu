@@ -860,12 +860,13 @@ int lrc_trace_frame(lrc_scene *s, const lrc_trace_params *old_p, const lrc_trace
     } else if (!e) {
         e = cudaMemsetAsync(d_new, 0, N * 32, c->st);   // (the first frame: no history)
     }
+    rc = LRC_RETRY;                                      // (no memory for the wavefront's state: the one-kernel path)
     if (!e && wavefront_call(s, new_p, H, spp))
         rc = trace_wavefront(s, new_p, 0, H, spp0, spp, reinterpret_cast<float *>(d_new), true);
-    else if (!e)
+    if (!e && rc == LRC_RETRY)
         e = lrc::pt_trace(pt_scene(s), P, reinterpret_cast<float *>(d_new), s->d_rays, c->d_status, c->st);
     c->timer.end(c->st);
-    if (rc) return rc;
+    if (rc && rc != LRC_RETRY) return rc;
     if (!e && !(flags & LRC_DEVICE)) e = cudaMemcpyAsync(new_planes, d_new, N * 64, cudaMemcpyDeviceToHost, c->st);
     if (e) return cuda_status(c, e, "lrc_trace_frame");
     return (flags & LRC_DEVICE) ? LRC_OK : check_status(c);

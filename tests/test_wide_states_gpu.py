@@ -293,3 +293,34 @@ def test_images_in_a_callers_graph(own, w, h):
     replay(own, g)
     assert np.array_equal(img.cpu().numpy(), one_kernel(s, p, 1)) and np.array_equal(new.cpu().numpy(), planes)
     s.close()
+
+
+def test_images_without_memory_for_the_wavefront():
+    own = L.Context(0)                                   # (a context whose engine has no memory yet)
+    w = h = 512
+    sc = W.box_scene(5, 1000, w, h)
+    s = R.world_scene(own, sc, 1)
+    p = L.native.trace_params(R.camera12(sc), w, h, 8, 1, 1, 0, 3)
+    want = one_kernel(s, p, 1)
+    planes = s.guide(p)
+    img, new = torch.zeros(h, w, 4, device="cuda"), torch.zeros(4, h, w, 4, device="cuda")
+    s.trace_frame_device(None, p, 0, 1, 0, new.data_ptr(), 0, 8)
+    frame = new.cpu().numpy()
+    other = L.Context(0)
+    s2 = R.world_scene(other, sc, 1)
+    s2.guide(p)
+    torch.cuda.synchronize()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (24 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        s2.trace_device(p, 1, img.data_ptr())
+        new.zero_()
+        torch.cuda.synchronize()
+        s2.trace_frame_device(None, p, 0, 1, 0, new.data_ptr(), 0, 8)
+        other.sync()
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    assert np.array_equal(img.cpu().numpy(), want) and np.array_equal(new.cpu().numpy(), frame)
+    assert np.array_equal(frame[2:], planes[2:])
+    for x in (s, s2, own, other):
+        x.close()
