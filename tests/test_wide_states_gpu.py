@@ -78,7 +78,7 @@ def field(own, few=True, wild=None):
     s.set_meshes([L.pack_tris(W.corners_to_quv(t), np.full(t.shape[0], m, np.int32))
                   for t, m in zip(sc["meshes"], sc["mesh_mats"])])
     s.set_instances(records)
-    s.build_instances(1, 30)
+    s.build_instances(0, 30)
     s.set_sky(sc["sky"])
     return s, sc, records
 
@@ -130,7 +130,8 @@ def test_captured_queries_see_the_next_build(own, m):
 
 
 def test_captured_small_images_see_the_next_build(own):
-    a, b = W.box_scene(5, 3000, 72, 40), W.box_scene(6, 3000, 72, 40)
+    a = W.box_scene(5, 3000, 72, 40)
+    other = (a["corners"] * np.float32([0.9, 1, 1])).astype(np.float32)
     s = R.world_scene(own, a, 1)
     p = L.native.trace_params(R.camera12(a), 72, 40, 8, 1, 1, 0, 3)
     first = s.trace(p, 2)[0]
@@ -142,7 +143,7 @@ def test_captured_small_images_see_the_next_build(own):
         s.guide_device(p, planes.data_ptr())
 
     g = captured(own, images)
-    s.set_triangles(L.pack_tris(W.corners_to_quv(b["corners"]), a["tri_mats"]))
+    s.set_triangles(L.pack_tris(W.corners_to_quv(other), a["tri_mats"]))
     s.build(1, 30)
     img.zero_()
     replay(own, g)
@@ -304,7 +305,9 @@ def test_images_without_memory_for_the_wavefront():
     want = one_kernel(s, p, 1)
     planes = s.guide(p)
     img, new = torch.zeros(h, w, 4, device="cuda"), torch.zeros(4, h, w, 4, device="cuda")
+    torch.cuda.synchronize()
     s.trace_frame_device(None, p, 0, 1, 0, new.data_ptr(), 0, 8)
+    own.sync()
     frame = new.cpu().numpy()
     other = L.Context(0)
     s2 = R.world_scene(other, sc, 1)
