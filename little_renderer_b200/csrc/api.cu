@@ -1170,10 +1170,6 @@ int lrc_trace(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows,
         int rc = lrc_scene_set_tables(s, nullptr, nullptr);
         if (rc) return rc;
     }
-    {
-        int rc = scene_wide(s, c->st, false);
-        if (rc) return rc;
-    }
     cudaError_t e = cudaSuccess;
     if (!s->d_rays) e = cudaMalloc(&s->d_rays, 256);
     if (!e) e = cudaMemsetAsync(s->d_rays, 0, 8, c->st);
@@ -1221,6 +1217,10 @@ int lrc_trace(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows,
         }
         if (rays) return lrc_batch_rays(c->single, rays, nullptr);   // (waits)
         return (flags & LRC_DEVICE) ? LRC_OK : check_status(c);
+    }
+    if (!e && lrc::pt_walks_wide(P, s->nvol != 0)) {
+        int rc = scene_wide(s, c->st, false);
+        if (rc) return rc;
     }
     c->timer.begin(LRC_TS_SHADE, c->st);
     if (!e) e = lrc::pt_trace(pt_scene(s), P, d_acc, s->d_rays, c->d_status, c->st);

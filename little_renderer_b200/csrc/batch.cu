@@ -142,8 +142,9 @@ void swap_graphs(lrc_batch *b) {
 }
 
 // the path tracer's view of a job's scene once the run's builds are done (a build makes the tree
-// over all its shapes)
-lrc::PtScene view_of(const lrc_batch::Job &J, bool building) {
+// over all its shapes); wide: with the wide nodes (the wavefront's kernels walk them, the
+// megakernel the binary ones)
+lrc::PtScene view_of(const lrc_batch::Job &J, bool building, bool wide) {
     lrc::PtScene S = pt_scene(J.s);
     if (J.view.inst) {
         S.inst = reinterpret_cast<const float4 *>(J.view.inst);
@@ -159,6 +160,7 @@ lrc::PtScene view_of(const lrc_batch::Job &J, bool building) {
         S.wide = n && !J.s->replayed && J.s->pwide_cap >= lrc::wide_bytes(n, true) ? lrc::wide_view(J.s->d_pwide, n, true)
                                                                                    : lrc::WideScene{};
     }
+    if (!wide) S.wide = lrc::WideScene{};
     return S;
 }
 
@@ -171,7 +173,7 @@ std::vector<unsigned char> signature(const lrc_batch *b, unsigned flags) {
     };
     put(&flags, sizeof flags);
     for (const lrc_batch::Job &J : b->jobs) {
-        lrc::PtScene S = view_of(J, (flags & LRC_BATCH_BUILD) != 0);
+        lrc::PtScene S = view_of(J, (flags & LRC_BATCH_BUILD) != 0, b->engine == 1);
         put(&S, sizeof S);
         const void *bufs[4] = {J.s->d_boxes, J.s->d_small, J.s->d_nodes, J.s->d_aux};
         put(bufs, sizeof bufs);
@@ -219,7 +221,7 @@ int build_job(lrc_batch *b, const lrc_batch::Job *J, cudaStream_t st, bool captu
     const int first = J->builder == 2 ? 0 : J->builder;
     int rc = scene_build_on(J->s, first, J->key_bits, &b->scratch, &b->scratch_cap, st, nullptr, capturing);
     if (!rc && J->builder == 2) rc = scene_build_on(J->s, 1, J->key_bits, &b->scratch, &b->scratch_cap, st, nullptr, capturing);
-    if (!rc) rc = scene_wide(J->s, st, capturing);
+    if (!rc && b->engine == 1) rc = scene_wide(J->s, st, capturing);
     return rc;
 }
 
@@ -232,9 +234,9 @@ int prepare(lrc_batch *b, bool building) {
     lrc_ctx *c = b->ctx;
     const size_t nj = b->jobs.size();
     for (const lrc_batch::Job &J : b->jobs) {
-        if (building && J.builder >= 0) continue;
+        if (b->engine != 1 || (building && J.builder >= 0)) continue;
         int rc = scene_wide(J.s, c->st, false);
-        if (!rc && b->engine == 1) rc = instances_wide(J.s, c->st);
+        if (!rc) rc = instances_wide(J.s, c->st);
         if (rc) return rc;
     }
     b->order.resize(nj);
@@ -251,7 +253,7 @@ int prepare(lrc_batch *b, bool building) {
     for (size_t q = 0; q < nj; q++) {
         const lrc_batch::Job &J = b->jobs[b->order[q]];
         lrc::BatchJob &T = b->table[q];
-        T.S = view_of(J, building);
+        T.S = view_of(J, building, b->engine == 1);
         T.P = params_of(J);
         T.task0 = task;
         T.pix0 = pix;
@@ -524,7 +526,7 @@ void note_built(lrc_batch *b) {   // (what captured builds' host side records)
         J->s->tree_nnodes = J->s->tree_naux = 0;     // (a tree given or built meanwhile, and its copy, are gone)
         J->s->walk_ok = J->s->wide_ok = false;
         J->s->most_leaf = 1;
-        J->s->pwide_ok = J->s->built_n && !J->s->replayed && J->s->pwide_cap >= lrc::wide_bytes(J->s->built_n, true);
+        J->s->pwide_ok = b->engine == 1 && J->s->built_n && !J->s->replayed && J->s->pwide_cap >= lrc::wide_bytes(J->s->built_n, true);
     }
 }
 

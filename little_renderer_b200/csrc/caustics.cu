@@ -322,12 +322,8 @@ int lt_check(lrc_scene *s, const lrc_trace_params *p, uint64_t photons, bool *sk
     if (!s->d_mats || !s->nmats) return fail(c, LRC_E_INVALID, "the scene has no materials (lrc_scene_set_materials)");
     if (s->light >= (int32_t)s->nprims) return fail(c, LRC_E_INVALID, "the light is not one of the primitives");
     *skip = photons == 0 || s->light < 0 || !s->specular;
-    if (*skip) return LRC_OK;
-    if (!s->tables) {
-        int rc = lrc_scene_set_tables(s, nullptr, nullptr);
-        if (rc) return rc;
-    }
-    return scene_wide(s, c->st, false);
+    if (!*skip && !s->tables) return lrc_scene_set_tables(s, nullptr, nullptr);
+    return LRC_OK;
 }
 
 int lt_run(lrc_scene *s, const lrc_trace_params *p, uint64_t photons, uint64_t seed, unsigned long long *d_sums,

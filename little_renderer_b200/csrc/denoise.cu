@@ -635,7 +635,7 @@ int scene_traceable(lrc_scene *s) {
         int rc = lrc_scene_set_tables(s, nullptr, nullptr);
         if (rc) return rc;
     }
-    return scene_wide(s, c->st, false);
+    return LRC_OK;
 }
 
 lrc::PtParams trace_params_of(const lrc_trace_params *p) {
@@ -763,9 +763,10 @@ int lrc_reproject_gradients(lrc_scene *s, const lrc_trace_params *old_p, const l
         return fail(c, LRC_E_INVALID, "temporal gradients trace a sample again: the old image in fast mode (exact = 0)");
     DeviceGuard g(c->device);
     int rc = scene_traceable(s);
-    if (rc) return rc;
     const size_t N = (size_t)W * H;
     const uint32_t ntiles = grad_tiles(W, H);
+    if (!rc && lrc::pt_gradients_walk_wide(ntiles, s->nvol != 0)) rc = scene_wide(s, c->st, false);
+    if (rc) return rc;
     const float4 *d_old = reinterpret_cast<const float4 *>(old_planes);
     float4 *d_new = reinterpret_cast<float4 *>(new_planes);
     float4 *d_tout = reinterpret_cast<float4 *>(tiles_out);
@@ -822,6 +823,7 @@ int lrc_trace_frame(lrc_scene *s, const lrc_trace_params *old_p, const lrc_trace
         return fail(c, LRC_E_INVALID, "temporal gradients trace a sample again: the old image in fast mode (exact = 0)");
     DeviceGuard g(c->device);
     int rc = scene_traceable(s);
+    if (!rc) rc = scene_wide(s, c->st, false);           // (the guide walks them)
     if (rc) return rc;
     const size_t N = (size_t)W * H;
     const uint32_t ntiles = grad_tiles(W, H);

@@ -296,6 +296,9 @@ struct GradTile {
 cudaError_t pt_gradients(const PtScene &S, const PtParams &P, GradTile *d_tiles, uint32_t ntiles, const float4 *d_guide,
                          unsigned long long *d_rays, uint32_t *d_status, cudaStream_t st);
 cudaError_t pt_prim_boxes(const float *d_prims, uint32_t n, float *d_boxes, cudaStream_t st);
+// whether pt_trace's (pt_gradients') kernel for these walks the world's wide nodes, if the scene has them
+bool pt_walks_wide(const PtParams &P, bool media);
+bool pt_gradients_walk_wide(uint32_t ntiles, bool media);
 cudaError_t pt_trace(const PtScene &S, const PtParams &P, float *d_accum, unsigned long long *d_rays, uint32_t *d_status,
                      cudaStream_t st);
 cudaError_t pt_intersect(const PtScene &S, const float *d_orig, const float *d_dir, uint64_t n, float tmin, float tmax,

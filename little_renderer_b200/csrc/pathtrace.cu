@@ -386,13 +386,18 @@ cudaError_t pt_prim_boxes(const float *d_prims, uint32_t n, float *d_boxes, cuda
     return cudaGetLastError();
 }
 
+static uint64_t pt_paths(const PtParams &P) { return (uint64_t)P.W * P.rows * (P.exact ? 1 : P.group); }
+
+bool pt_walks_wide(const PtParams &P, bool media) { return !media && pt_paths(P) <= pt::PT_WARP_PATHS; }
+bool pt_gradients_walk_wide(uint32_t ntiles, bool media) { return !media && ntiles <= pt::PT_WARP_PATHS; }
+
 cudaError_t pt_trace(const PtScene &S, const PtParams &P, float *d_accum, unsigned long long *d_rays, uint32_t *d_status,
                      cudaStream_t st) {
     if (P.rows <= 0 || P.spp <= 0 || P.W <= 0) return cudaSuccess;
     float4 *acc = reinterpret_cast<float4 *>(d_accum);
-    const uint64_t paths = P.exact ? (uint64_t)P.W * P.rows : (uint64_t)P.W * P.rows * P.group;
+    const uint64_t paths = pt_paths(P);
     const int k = P.moments ? 1 : 0, x = P.exact ? 1 : 0;
-    if (S.nvol || paths > pt::PT_WARP_PATHS || !S.wide.nodes) {
+    if (!pt_walks_wide(P, S.nvol != 0) || !S.wide.nodes) {
         // (kernels compiled with and without the media's tracking and the denoiser's moments: each
         // holds registers that a scene or an image without them would pay for)
         using Fn = void (*)(PtScene, PtParams, float4 *, unsigned long long *, uint32_t *);
@@ -474,7 +479,7 @@ __global__ void __launch_bounds__(128) grad_kernel(const __grid_constant__ PtSce
 cudaError_t pt_gradients(const PtScene &S, const PtParams &P, GradTile *d_tiles, uint32_t ntiles, const float4 *d_guide,
                          unsigned long long *d_rays, uint32_t *d_status, cudaStream_t st) {
     if (!ntiles) return cudaSuccess;
-    const bool warp = !S.nvol && ntiles <= pt::PT_WARP_PATHS && S.wide.nodes;   // (pt_trace's line)
+    const bool warp = pt_gradients_walk_wide(ntiles, S.nvol != 0) && S.wide.nodes;
     uint32_t spread = 1;
     while (warp && spread < pt::SPREAD_MOST && (uint64_t)ntiles * spread * 2 <= pt::SPREAD_LANES) spread *= 2;
     (S.nvol ? pt::grad_kernel<true, false> : warp ? pt::grad_kernel<false, true> : pt::grad_kernel<false, false>)

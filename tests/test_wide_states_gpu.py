@@ -327,3 +327,25 @@ def test_images_without_memory_for_the_wavefront():
     assert np.array_equal(frame[2:], planes[2:])
     for x in (s, s2, own, other):
         x.close()
+
+
+def test_no_wide_nodes_where_none_are_walked(own):
+    """Images between the warps' line and the wavefront's, the megakernel engine, caustics: they walk the
+    binary nodes, and no memory goes to others."""
+    n = 1_000_000
+    sc = W.box_scene(5, n, 200, 160)
+    s = R.world_scene(own, sc, 1)
+    p = L.native.trace_params(R.camera12(sc), 200, 160, 8, 1, 1, 0, 3)
+    img = torch.zeros(160, 200, 4, device="cuda")
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    s.trace_device(p, 1, img.data_ptr())
+    q = L.native.Batch(own)
+    q.set_engine(0)
+    q.add(s, p, 1, img.data_ptr(), builder=1)
+    q.run(build=False)
+    s.caustics(p, 1000, 3)
+    own.sync()
+    assert free - torch.cuda.mem_get_info()[0] < 48 * n  # (the wide nodes of a million shapes: 94 MB)
+    q.close()
+    s.close()
