@@ -324,6 +324,7 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_in
                 J = &jobs[W.job[s]];
                 r = wide_ray(v3f(W.ro[s]), v3f(W.rd[s]));
                 deep_begin(J->S, w, 1e30f);
+                if (!wide_plain(r.o, r.d)) deep_odd(w);
             },
             [&](int with) {
                 return deep_step<false>(J->S, r, w, stack, RT_EPS, with, err, [&](V3 &o, V3 &d) { o = v3f(W.ro[s]); d = v3f(W.rd[s]); });
@@ -350,6 +351,7 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_in
                 r = wide_ray(v3f(W.ro[s]), v3f(W.rd[s]));
                 wide_begin(w, 1e30f);
                 if (!J->S.nnodes) w.ng.y = 0u;       // (an empty world: over after one step)
+                else if (!wide_plain(r.o, r.d)) wide_odd(w);
             },
             [&](int with) { return wide_step<false, COUNT>(wide, r, w, stack, RT_EPS, with, err, WorldLeaf{J->S}, cnt); },
             [&]() { answer(s, w.best, w.tie ? WF_TIE : w.hit, -1, -1); });

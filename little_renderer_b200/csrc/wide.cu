@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(WD_THREADS) collapse_kernel(const __grid_const
     // (the root box's largest coordinate: its widening, none where it is no number a grid holds)
     const float4 rl = __ldg(reinterpret_cast<const float4 *>(&C.bin[C.root])), rh = __ldg(reinterpret_cast<const float4 *>(&C.bin[C.root]) + 1);
     float pad = C.widen * fmaxf(fmaxf(fmaxf(fabsf(rl.x), fabsf(rl.y)), fabsf(rl.z)), fmaxf(fmaxf(fabsf(rh.x), fabsf(rh.y)), fabsf(rh.z)));
-    if (!(pad < 1e18f)) pad = 0.0f;
+    if (!(pad < WD_FAR)) pad = 0.0f;
     uint32_t idx = 0, spins = 0, made = 0;       // made: the nodes this warp made, not yet counted in CT_MADE
     bool claimed = false;
     for (;;) {
@@ -207,12 +207,12 @@ __global__ void __launch_bounds__(WD_THREADS) collapse_kernel(const __grid_const
                 hi[a] = fmaxf(hi[a], __shfl_xor_sync(all, hi[a], o, 8));
             }
         }
-        // boxes the grid cannot hold (a NaN, an infinity, coordinates beyond 1e18): the tree is not
+        // boxes of a NaN or an infinity, which the grid cannot hold, or beyond WD_FAR (wide_plain): the tree is not
         // walked (C.wild: the root's last word, or the mark a scene's meshes share, says so; the callers
         // walk the binary one)
         bool plain = true;
 #pragma unroll
-        for (int a = 0; a < 3; a++) plain = plain && (!have || (fabsf(c.lo[a]) <= 1e18f && fabsf(c.hi[a]) <= 1e18f));
+        for (int a = 0; a < 3; a++) plain = plain && (!have || (fabsf(c.lo[a]) <= WD_FAR && fabsf(c.hi[a]) <= WD_FAR));
         if (!plain) atomicOr(C.wild, 1u);
         // a slot for each child: of the pairs left the one that lies best (its middle farthest to the
         // slot's corner), again and again
@@ -402,6 +402,7 @@ __device__ __forceinline__ void query_done(const Query &Q, uint64_t i, int32_t h
 template <bool ANY>
 __global__ void __launch_bounds__(WD_THREADS, 8) wide_query_kernel(const __grid_constant__ Query Q) {
     constexpr int32_t TIE = (int32_t)0x80000000;
+    constexpr uint8_t ASK = 2;
     __shared__ uint32_t s_next, s_tie;
     const uint32_t all = 0xffffffffu, lane = threadIdx.x & 31u;
     const uint64_t first = (uint64_t)blockIdx.x * Q.chunk;
@@ -433,6 +434,7 @@ __global__ void __launch_bounds__(WD_THREADS, 8) wide_query_kernel(const __grid_
                     i = first + k;
                     r = query_ray(Q, i);
                     wide_begin(w, ANY ? Q.tmaxs[i] : Q.tmax);
+                    if (!wide_plain(r.o, r.d)) wide_odd(w);
                 }
             }
             m = __ballot_sync(all, at);
@@ -440,21 +442,20 @@ __global__ void __launch_bounds__(WD_THREADS, 8) wide_query_kernel(const __grid_
         over = !m;
         if (at && wide_step<ANY, false>(Q.W, r, w, stack, Q.tmin, __popc(m), Q.err, TriLeaf{})) {
             at = false;
-            if (ANY || !w.tie) {
+            if (!w.tie) {
                 query_done<ANY>(Q, i, w.hit, w.best, false);
             } else {
-                Q.prim[i] = TIE;
+                if (ANY) Q.blocked[i] = ASK;
+                else Q.prim[i] = TIE;
                 s_tie = 1;
             }
         }
     }
     // (the binary walk's code and registers stay out of the loop above)
-    if (!ANY) {
-        __syncthreads();
-        if (s_tie)
-            for (uint32_t k = threadIdx.x; k < n; k += WD_THREADS)
-                if (Q.prim[first + k] == TIE) query_binary<false>(Q, first + k);
-    }
+    __syncthreads();
+    if (s_tie)
+        for (uint32_t k = threadIdx.x; k < n; k += WD_THREADS)
+            if (ANY ? Q.blocked[first + k] == ASK : Q.prim[first + k] == TIE) query_binary<ANY>(Q, first + k);
 }
 
 template <bool ANY>
@@ -462,11 +463,11 @@ __global__ void __launch_bounds__(WD_THREADS, 8) wide_query8_kernel(const __grid
     const uint64_t i = ((uint64_t)blockIdx.x * WD_THREADS + threadIdx.x) >> 3;
     if (i >= Q.n) return;
     const bool one = (threadIdx.x & 7u) == 0u;
-    if (!wide_walked(Q.W)) {
+    const WideRay r = query_ray(Q, i);
+    if (!wide_walked(Q.W) || !wide_plain(r.o, r.d)) {
         if (one) query_binary<ANY>(Q, i);
         return;
     }
-    const WideRay r = query_ray(Q, i);
     float best = ANY ? Q.tmaxs[i] : Q.tmax;
     bool tie;
     const int32_t hit = wide_walk8<ANY>(Q.W, r, Q.tmin, best, tie, Q.err, TriLeaf{});
@@ -481,6 +482,7 @@ __global__ void __launch_bounds__(WD_THREADS) wide_count_kernel(const __grid_con
         const WideRay r = query_ray(Q, i);
         WideWalk w;
         wide_begin(w, Q.tmax);
+        if (!wide_plain(r.o, r.d)) wide_odd(w);
         wide_run<false, true>(Q.W, r, w, Q.tmin, Q.err, TriLeaf{}, cnt);
     }
     unsigned long long a = cnt[0], b = cnt[1];

@@ -17,7 +17,8 @@
 // The same closest hits as the binary walk of the tree the nodes were made from: every shape whose
 // boxes the ray meets there is tested here, by the same operations, and where two shapes are hit at
 // the same t - the one case in which the order of the tests decides - `tie` says so and the caller
-// asks the binary walk.
+// asks the binary walk. Rays that a shape could be hit by at a t that is no number (the binary walk then
+// takes whatever it meets next) go to the binary walk at once (wide_plain).
 #pragma once
 #include "lrc_internal.cuh"
 
@@ -162,7 +163,7 @@ struct WideWalk {
     int sp;
     int32_t hit;                             // the closest shape's id so far (-1: none)
     float best;                              // its t (at first the ray's end)
-    bool tie;                                // another shape was hit at t = best
+    bool tie;                                // another shape was hit at t = best (or wide_odd): ask the binary walk
 };
 __device__ __forceinline__ void wide_begin(WideWalk &w, float tmax) {
     w.ng = make_uint2(0u, 0x80000000u);      // (the root: its relative index comes out 0 of no inner slots)
@@ -170,6 +171,20 @@ __device__ __forceinline__ void wide_begin(WideWalk &w, float tmax) {
     w.hit = -1;
     w.best = tmax;
     w.tie = false;
+}
+
+// Whether the shape tests of a ray give numbers: with o, d and the shapes (collapse_kernel's bound) within 1e9
+// and d not (nearly) zero, the products of hit_sphere_t ((6 |d| |c - o|)^2) and wide_tri (24 |q|^3) stay
+// finite and no zero is divided by zero.
+constexpr float WD_FAR = 1e9f;
+__device__ __forceinline__ bool wide_plain(V3 o, V3 d) {
+    const float dd = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
+    return fabsf(o.x) + fabsf(o.y) + fabsf(o.z) <= WD_FAR && dd <= WD_FAR && dd >= 1e-18f;   // (not so for a NaN)
+}
+// a walk that ends with its first step, the binary one to be asked
+__device__ __forceinline__ void wide_odd(WideWalk &w) {
+    w.ng.y = 0u;
+    w.tie = true;
 }
 
 // with: how many lanes of the warp take this step together (they are to be reconverged before each step:

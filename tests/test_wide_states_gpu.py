@@ -349,3 +349,77 @@ def test_no_wide_nodes_where_none_are_walked(own):
     assert free - torch.cuda.mem_get_info()[0] < 48 * n  # (the wide nodes of a million shapes: 94 MB)
     q.close()
     s.close()
+
+
+def odd_rays(m, seed):
+    """Rays whose components are no numbers, infinite, all zero, very long or short, or far away: a 16th each."""
+    o, d = W.rays_at_cube(m, seed)
+    part = [slice(i * m // 16, (i + 1) * m // 16) for i in range(9)]
+    o[part[0], seed % 3] = np.nan
+    d[part[1], 1] = np.nan
+    o[part[2], 0] = np.inf
+    d[part[3], 2] = -np.inf
+    d[part[4]] = 0.0
+    d[part[5]] *= np.float32(1e30)
+    d[part[6]] *= np.float32(1e19)
+    d[part[7]] *= np.float32(1e-15)
+    o[part[8]] *= np.float32(1e6)
+    return o, d
+
+
+def binary(own, s, o, d, tmin, tmax):
+    m = o.shape[0]
+    prim, t = np.zeros(m, np.int32), np.zeros(m, np.float32)
+    own.check(own.L.lrc_scene_intersect(s.h, o.ctypes.data, d.ctypes.data, m, tmin, tmax, prim.ctypes.data, t.ctypes.data, 2))
+    return prim, t
+
+
+@pytest.mark.parametrize("tmin,tmax", [(0.0, 1e30), (0.0, np.inf), (0.0, np.nan), (-5.0, 2.5), (-4.0, -0.5), (2.0, 1.0),
+                                       (np.nan, 1e30)])
+def test_odd_rays(own, tmin, tmax):
+    s = L.native.Scene(own)
+    s.set_triangles(soup(5000, 3))
+    s.build(1, 30)
+    m = 1 << 18
+    o, d = odd_rays(m, 4)
+    want = binary(own, s, o, d, tmin, tmax)
+    for idx in (slice(0, m), slice(0, m, 32)):           # one lane a ray, 8
+        got = s.intersect(o[idx], d[idx], tmin, tmax)
+        for g, w in zip(got, want):
+            assert np.array_equal(g.view(np.uint32), w[idx].view(np.uint32))
+        far = np.full(m, tmax, np.float32)[idx]
+        blocked = s.occluded(o[idx], d[idx], far, tmin)
+        s.set_walk(0)
+        assert np.array_equal(blocked, s.occluded(o[idx], d[idx], far, tmin))
+        s.set_walk(1)
+    s.close()
+
+
+@pytest.mark.parametrize("tmin,tmax", [(0.0, 1e30), (0.0, np.inf), (0.0, np.nan), (-900.0, 900.0), (-900.0, -0.5)])
+def test_odd_rays_in_a_world_with_primitives(own, tmin, tmax):
+    """Spheres and quads, some twice, beside triangles: the wide nodes against the tree given as device arrays."""
+    rng = np.random.default_rng(4)
+    prims = np.zeros((40, 24), np.float32)
+    prims[:, 0:3], prims[:, 3] = rng.random((40, 3)) * 555, 40.0
+    for i in range(0, 40, 4):
+        prims[i] = W.make_quad(rng.random(3) * 555, rng.random(3) * 200, -rng.random(3) * 200, 0)
+    prims[20:] = prims[:20]
+    scenes = []
+    for _ in range(2):
+        s = L.native.Scene(own)
+        s.set_triangles(L.pack_tris(W.corners_to_quv(W.soup(500, 3) * np.float32(555))))
+        s.set_prims(prims)
+        s.build(1, 30)
+        scenes.append(s)
+    n = 540
+    nodes, aux = np.zeros((2 * n - 1, 8), np.uint32), np.zeros(n, np.uint32)
+    own.check(own.L.lrc_scene_tree(scenes[0].h, nodes.ctypes.data, aux.ctypes.data, 0))
+    dn, da = dev(nodes.view(np.int32)), dev(aux.view(np.int32))
+    own.check(own.L.lrc_scene_set_tree(scenes[1].h, C.c_void_p(dn.data_ptr()), 2 * n - 1, C.c_void_p(da.data_ptr()), n, DEVICE))
+    o, d = odd_rays(40_000, 4)
+    o = (o * np.float32(555)).astype(np.float32)
+    got, want = (s.intersect(o, d, tmin, tmax) for s in scenes)
+    for g, w in zip(got, want):
+        assert np.array_equal(g.view(np.uint32), w.view(np.uint32))
+    for s in scenes:
+        s.close()
