@@ -113,15 +113,16 @@ __device__ __forceinline__ float slab(const RayBox &r, float4 lo, float4 hi, flo
 // end the walk (an any-hit found). Entries of a leaf in order; a hit at the same t as the best is
 // not taken (t >= tmax rejects), as the CPU's walk does. Returns true if a leaf ended it.
 // COUNT: cnt[0] += the boxes tested (32-byte node records read), cnt[1] += the leaf entries tested
-// (a kernel compiled with it measures the walk's algorithmic bytes; the others never carry it)
-template <bool COUNT = false, typename Leaf>
+// (a kernel compiled with it measures the walk's algorithmic bytes; the others never carry it).
+// STACK: pending nodes a ray may have
+template <bool COUNT = false, int STACK = PT_STACK, typename Leaf>
 __device__ bool bvh_walk(const float4 *nodes, uint32_t root, uint32_t nnodes, const uint32_t *aux, uint32_t naux, V3 o,
                          V3 d, float tmin, float &best, uint32_t *err, Leaf &&leaf, uint32_t *cnt = nullptr) {
     RayBox rb = ray_box(o, d);
     float4 r0 = ld4(&nodes[2 * (size_t)root]), r1 = ld4(&nodes[2 * (size_t)root + 1]);
     if constexpr (COUNT) cnt[0] += 1;
     if (!(slab(rb, r0, r1, tmin, best) <= best)) return false;
-    uint2 stack[PT_STACK];
+    uint2 stack[STACK];
     int sp = 0;
     uint32_t a = __float_as_uint(r0.w), b = __float_as_uint(r1.w);
     while (true) {
@@ -141,8 +142,8 @@ __device__ bool bvh_walk(const float4 *nodes, uint32_t root, uint32_t nnodes, co
             bool c0 = t0 <= best, c1 = t1 <= best;
             if (c0 && c1) {
                 bool first0 = t0 <= t1;
-                if (sp < PT_STACK) stack[sp++] = first0 ? make_uint2(__float_as_uint(h0.w), __float_as_uint(h1.w))
-                                                        : make_uint2(__float_as_uint(l0.w), __float_as_uint(l1.w));
+                if (sp < STACK) stack[sp++] = first0 ? make_uint2(__float_as_uint(h0.w), __float_as_uint(h1.w))
+                                                     : make_uint2(__float_as_uint(l0.w), __float_as_uint(l1.w));
                 else { atomicOr(err, ST_STACK_OVERFLOW); return false; }
                 a = first0 ? __float_as_uint(l0.w) : __float_as_uint(h0.w);
                 b = first0 ? __float_as_uint(l1.w) : __float_as_uint(h1.w);
@@ -425,7 +426,7 @@ __device__ __forceinline__ bool deep_step(const PtScene &S, WideRay &r, DeepWalk
         const uint32_t slot = (bit - 24u) ^ r.up;
         const uint32_t ni = w.ng.x + __popc(w.ng.y & 0xffu & ((1u << slot) - 1u));
         if (w.ng.y & WD_INNER) {
-            if (w.sp >= WD_STACK) { atomicOr(err, ST_STACK_OVERFLOW); return true; }
+            if (w.sp >= WD_STACK) return wide_full(w.tie);
             stack[w.sp++] = w.ng;
         }
         if (ni >= w.at.nnodes) { atomicOr(err, ST_BAD_TREE); return true; }
@@ -453,7 +454,7 @@ __device__ __forceinline__ bool deep_step(const PtScene &S, WideRay &r, DeepWalk
             if (mesh >= S.nmeshes) continue;         // (shapes: not in these scenes)
             const WideScene m = S.mesh_wide[mesh];
             if (!m.nodes) continue;                  // (a mesh of no triangles)
-            if (w.sp + 2 > WD_STACK) { atomicOr(err, ST_STACK_OVERFLOW); return true; }
+            if (w.sp + 2 > WD_STACK) return wide_full(w.tie);
             if (w.ng.y & WD_INNER) stack[w.sp++] = w.ng;
             if (tg.y & 0xffu) stack[w.sp++] = make_uint2(tg.x, tg.y & 0xffffu);
             V3 o, d;

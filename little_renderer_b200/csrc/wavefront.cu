@@ -491,7 +491,10 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_sh
                 return deep_step<true>(J->S, r, w, stack, RT_EPS, with, err,
                                        [&](V3 &o, V3 &d) { o = v3f(W.sq_o[at]); d = v3f(W.sq_d[at]); });
             },
-            [&]() { W.vis[e] = w.id >= 0 ? 0 : 1; });
+            [&]() {
+                if (w.tie) atomicOr(err, ST_STACK_OVERFLOW);
+                W.vis[e] = w.id >= 0 ? 0 : 1;
+            });
     } else {
         uint2 stack[WD_STACK];
         WideRay r = wide_ray(v3(0, 0, 0), v3(0, 0, 0));
@@ -512,7 +515,10 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_sh
                 if (!J->S.nnodes) w.ng.y = 0u;
             },
             [&](int with) { return wide_step<true, false>(wide, r, w, stack, RT_EPS, with, err, WorldLeaf{J->S}); },
-            [&]() { W.vis[e] = w.hit >= 0 ? 0 : 1; });
+            [&]() {
+                if (w.tie) atomicOr(err, ST_STACK_OVERFLOW);
+                W.vis[e] = w.hit >= 0 ? 0 : 1;
+            });
     }
 }
 

@@ -364,13 +364,15 @@ __device__ __forceinline__ V3 query_v3(const float *p, uint64_t i) { return v3(p
 __device__ __forceinline__ WideRay query_ray(const Query &Q, uint64_t i) { return wide_ray(query_v3(Q.orig, i), query_v3(Q.dir, i)); }
 
 // ray i through the binary tree: where two triangles are hit at the same t (the binary walk's order
-// decides), and where the tree is not walked wide
+// decides), and where the tree is not walked wide. Its stack is as deep as traverse.cu's, that the queries
+// of any tree are answered as they are there (LBVH trees over 63-bit keys reach 93 levels).
+constexpr int QUERY_STACK = 96;
 template <bool ANY>
 __device__ __noinline__ void query_binary(const Query &Q, uint64_t i) {
     float best = ANY ? Q.tmaxs[i] : Q.tmax;
     int32_t hit = -1;
     const V3 o = query_v3(Q.orig, i), d = query_v3(Q.dir, i);
-    bvh_walk<false>(reinterpret_cast<const float4 *>(Q.tt.nodes), Q.tt.root, Q.tt.nnodes, Q.tt.aux, Q.tt.naux, o, d, Q.tmin,
+    bvh_walk<false, QUERY_STACK>(reinterpret_cast<const float4 *>(Q.tt.nodes), Q.tt.root, Q.tt.nnodes, Q.tt.aux, Q.tt.naux, o, d, Q.tmin,
                     best, Q.err, [&](uint32_t id) {
         if (id >= Q.tt.ntris) { atomicOr(Q.err, ST_BAD_TREE); return true; }
         float t;
@@ -389,10 +391,10 @@ __device__ __noinline__ void query_binary(const Query &Q, uint64_t i) {
 
 template <bool ANY>
 __device__ __forceinline__ void query_done(const Query &Q, uint64_t i, int32_t hit, float best, bool tie) {
-    if (ANY) {
+    if (tie) {
+        query_binary<ANY>(Q, i);
+    } else if (ANY) {
         Q.blocked[i] = hit >= 0 ? 1 : 0;
-    } else if (tie) {
-        query_binary<false>(Q, i);
     } else {
         Q.prim[i] = hit;
         Q.t[i] = hit >= 0 ? best : -1.0f;

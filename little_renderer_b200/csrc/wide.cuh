@@ -163,7 +163,7 @@ struct WideWalk {
     int sp;
     int32_t hit;                             // the closest shape's id so far (-1: none)
     float best;                              // its t (at first the ray's end)
-    bool tie;                                // another shape was hit at t = best (or wide_odd): ask the binary walk
+    bool tie;                                // another shape was hit at t = best (or wide_odd, wide_full): ask the binary walk
 };
 __device__ __forceinline__ void wide_begin(WideWalk &w, float tmax) {
     w.ng = make_uint2(0u, 0x80000000u);      // (the root: its relative index comes out 0 of no inner slots)
@@ -187,6 +187,13 @@ __device__ __forceinline__ void wide_odd(WideWalk &w) {
     w.tie = true;
 }
 
+// A walk whose stack is full ends: the binary walk, whose pending nodes are others, is asked. (The
+// wavefront's shadow rays, where nothing asks it, report it.)
+__device__ __forceinline__ bool wide_full(bool &tie) {
+    tie = true;
+    return true;
+}
+
 // with: how many lanes of the warp take this step together (they are to be reconverged before each step:
 // wide_run, or the refilling loops' ballots; left to themselves the lanes of a warp part at their first
 // triangle and stay apart).
@@ -205,7 +212,7 @@ __device__ __forceinline__ bool wide_step(const WideScene &S, const WideRay &r, 
         const uint32_t slot = (bit - 24u) ^ r.up;
         const uint32_t ni = w.ng.x + __popc(w.ng.y & 0xffu & ((1u << slot) - 1u));
         if (w.ng.y & WD_INNER) {
-            if (w.sp >= WD_STACK) { atomicOr(err, ST_STACK_OVERFLOW); return true; }
+            if (w.sp >= WD_STACK) return wide_full(w.tie);
             stack[w.sp++] = w.ng;
         }
         if (ni >= S.nnodes) { atomicOr(err, ST_BAD_TREE); return true; }
@@ -336,7 +343,7 @@ __device__ __forceinline__ int32_t wide_walk8(const WideScene &S, const WideRay 
         const uint32_t slot = (bit - 24u) ^ r.up;
         ni = ng.x + __popc(ng.y & 0xffu & ((1u << slot) - 1u));
         if (ng.y & WD_INNER) {
-            if (sp >= WD_STACK) { atomicOr(err, ST_STACK_OVERFLOW); return -1; }
+            if (sp >= WD_STACK) { tie = true; return -1; }   // (wide_full)
             stack[sp++] = ng;
         }
     }

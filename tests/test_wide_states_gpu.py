@@ -423,3 +423,35 @@ def test_odd_rays_in_a_world_with_primitives(own, tmin, tmax):
         assert np.array_equal(g.view(np.uint32), w.view(np.uint32))
     for s in scenes:
         s.close()
+
+
+@pytest.mark.parametrize("ties", [1, 2])
+def test_trees_as_deep_as_the_queries_stack(own, ties):
+    """80 levels, each one's leaf behind all that lies below it; the nearest triangle twice (the binary
+    walk decides between the two)."""
+    depth = 80
+    n = depth + ties
+    quv = np.tile(np.float32([-1, -1, 0, 4, 0, 0, 0, 4, 0]), (n, 1))
+    quv[:, 2] = 100.0 - np.minimum(np.arange(n), depth)
+    corners = np.stack([quv[:, 0:3], quv[:, 0:3] + quv[:, 3:6], quv[:, 0:3] + quv[:, 6:9]])
+    lo, hi = corners.min(0) - np.float32(1e-3), corners.max(0) + np.float32(1e-3)
+    nodes = np.zeros((2 * n - 1, 8), np.uint32)
+    f = nodes.view(np.float32)
+    for i in range(n):                                   # node 2 i: over the triangles from i on; 2 i + 1: leaf i
+        f[2 * i, 0:3], f[2 * i, 4:7] = lo[i:].min(0), hi[i:].max(0)
+        if i < n - 1:
+            nodes[2 * i][[3, 7]] = 2 * i + 1, 2 * i + 2
+            f[2 * i + 1, 0:3], f[2 * i + 1, 4:7] = lo[i], hi[i]
+        nodes[min(2 * i + 1, 2 * n - 2)][[3, 7]] = i, 0x80000001
+    s = L.native.Scene(own)
+    s.set_triangles(L.pack_tris(quv))
+    s.set_tree(nodes, np.arange(n, dtype=np.uint32))
+    m = 1 << 18
+    o, d = np.zeros((m, 3), np.float32), np.tile(np.float32([0, 0, 1]), (m, 1))
+    want = binary(own, s, o, d, 0.0, 1e30)
+    assert want[1][0] == 100.0 - depth
+    for k in (100, 40_000):
+        got = s.intersect(o[:k], d[:k])
+        assert np.array_equal(got[0], want[0][:k]) and np.array_equal(got[1], want[1][:k])
+        assert s.occluded(o[:k], d[:k], np.full(k, 200, np.float32)).all()
+    s.close()
