@@ -189,19 +189,6 @@ __global__ void __launch_bounds__(PREP_W *PREP_H) prep_kernel(const float4 *__re
 // the B3 spline's weights 1/16, 1/4, 3/8, 1/4, 1/16
 __device__ __forceinline__ float b3(int i) { return i == 2 ? 0.375f : (i == 1 || i == 3 ? 0.25f : 0.0625f); }
 
-// 2^x and the square root of the special function unit (2 ulp and 1 ulp of a float: their results go
-// into weights whose sums are kept as halves)
-__device__ __forceinline__ float ex2(float x) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ float sqrt_sfu(float x) {
-    float r;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
 // One a-trous pass: a 5 x 5 B3 spline with holes `step` apart, each tap jittered within its hole
 // (but the centre), weighted by luminance (against the noise of the noisier of the two), normal
 // (cos^128) and distance (against how fast it changes here); the variance filtered with the
@@ -209,9 +196,10 @@ __device__ __forceinline__ float sqrt_sfu(float x) {
 //
 // Bound by instructions (84 % of the issue slots, the taps hit L1 / L2), so a tap is kept short: the
 // centre (the only tap that can fall on the pixel itself: a jitter is at most half a hole) is no
-// longer told apart at run time, a surface's taps read the distance and the kind as one sign test,
-// the luminance's and the distance's exponentials are one 2^x, and JIT = false (step 1) has no
-// random numbers.
+// longer told apart at run time, a surface's taps read the distance and the kind as one sign test, and
+// JIT = false (step 1) has no random numbers. (The square root stays the rounded one, the
+// luminance's and the distance's exponentials two: an approximate root and one 2^x of their sum are
+// shorter and less exact.)
 template <bool JIT>
 __global__ void __launch_bounds__(256) atrous_kernel(const float4 *__restrict__ px, int W, int H, int step, int last,
                                                      float sigma_l, float sigma_z, const uint2 *__restrict__ src,
@@ -254,7 +242,6 @@ __global__ void __launch_bounds__(256) atrous_kernel(const float4 *__restrict__ 
     const float zb = 1e-3f * gp.z + 1e-6f;
     gx *= sigma_z;
     gy *= sigma_z;
-    constexpr float L2E = 1.4426950408889634f;       // (exp(x) = 2^(x log2 e))
     uint32_t seed = JIT ? hash32((k * 0x9e3779b9u) ^ ((uint32_t)step * 0x85ebca6bu)) : 0u;
     const int jit = step / 2;
     const uint32_t jn = (uint32_t)(2 * jit + 1);
@@ -285,19 +272,19 @@ __global__ void __launch_bounds__(256) atrous_kernel(const float4 *__restrict__ 
             const float4 gq = gd[q];
             const float4 s = get_iv(src[q]);
             if (s.w < 0.0f) continue;
-            float ex = __fdividef(fabsf(lp - luma(s.x, s.y, s.z)), sigma_l * sqrt_sfu(fmaxf(v, s.w)) + 1e-6f);
             float w = b3(i) * bj;
+            w *= __expf(__fdividef(-fabsf(lp - luma(s.x, s.y, s.z)), sigma_l * sqrtf(fmaxf(v, s.w)) + 1e-6f));
             if (surface) {
                 if (!(gq.w >= 0.0f)) continue;       // (not a surface)
                 float wn = fmaxf(gp.n.x * gq.x + gp.n.y * gq.y + gp.n.z * gq.z, 0.0f);
 #pragma unroll
                 for (int e = 0; e < 7; e++) wn *= wn;   // cos^128
                 w *= wn;
-                ex += __fdividef(fabsf(gp.z - gq.w), gx * fabsf((float)ox) + gy * fabsf((float)oy) + zb);
+                w *= __expf(__fdividef(-fabsf(gp.z - gq.w), gx * fabsf((float)ox) + gy * fabsf((float)oy) + zb));
             } else if (gq.w >= 0.0f || gq.w < -1e37f) {
                 continue;                            // (not a medium)
             }
-            add_tap(w * ex2(-L2E * ex), s);
+            add_tap(w, s);
         }
     };
     row(0, b3(0));
