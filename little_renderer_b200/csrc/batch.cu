@@ -68,12 +68,16 @@ struct lrc_batch {
     cudaGraphExec_t exec = nullptr;
     unsigned graph_flags = 0;
     std::vector<unsigned char> graph_sig;
-    // the wavefront's graph captured before the current one, kept: runs that alternate between two
-    // keys (a server's waves with and without instanced jobs) replay both, capturing neither again
-    cudaGraph_t alt_graph = nullptr;
-    cudaGraphExec_t alt_exec = nullptr;
-    unsigned alt_flags = 0;
-    std::vector<unsigned char> alt_sig;
+    // the wavefront's graphs captured before the current one, the last used first, up to kGraphs with it:
+    // runs that take turns between keys (a server's waves with and without instanced jobs, lrc_trace's
+    // four wavefront sizes, each with and without instances) replay them, capturing none again
+    struct Graph {
+        cudaGraph_t graph;
+        cudaGraphExec_t exec;
+        unsigned flags;
+        std::vector<unsigned char> sig;
+    };
+    std::vector<Graph> kept;
     int graph_used = 0;
     cudaEvent_t ev_launch = nullptr;      // recorded right before a run's trace is launched (the server's wave timing)
     lrc::BatchJob *h_table = nullptr;     // pinned staging of the job table's upload (and the run block after it)
@@ -114,7 +118,7 @@ lrc::PtParams params_of(const lrc_batch::Job &J) {
     return P;
 }
 
-// the current graph dropped (the kept one stays)
+// the current graph dropped (the kept ones stay)
 void drop_graph(lrc_batch *b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
@@ -123,22 +127,45 @@ void drop_graph(lrc_batch *b) {
     b->graph_sig.clear();
 }
 
-// both graphs dropped (their buffers may move)
-void destroy_graph(lrc_batch *b) {
-    drop_graph(b);
-    if (b->alt_exec) cudaGraphExecDestroy(b->alt_exec);
-    if (b->alt_graph) cudaGraphDestroy(b->alt_graph);
-    b->alt_exec = nullptr;
-    b->alt_graph = nullptr;
-    b->alt_sig.clear();
+constexpr size_t kGraphs = 8;
+
+// the kept graph i dropped
+void drop_kept(lrc_batch *b, size_t i) {
+    cudaGraphExecDestroy(b->kept[i].exec);
+    cudaGraphDestroy(b->kept[i].graph);
+    b->kept.erase(b->kept.begin() + (ptrdiff_t)i);
 }
 
-// the current graph and the kept one trade places
-void swap_graphs(lrc_batch *b) {
-    std::swap(b->graph, b->alt_graph);
-    std::swap(b->exec, b->alt_exec);
-    std::swap(b->graph_flags, b->alt_flags);
-    b->graph_sig.swap(b->alt_sig);
+// all graphs dropped (their buffers may move)
+void destroy_graph(lrc_batch *b) {
+    drop_graph(b);
+    while (!b->kept.empty()) drop_kept(b, b->kept.size() - 1);
+}
+
+// the current graph among the kept ones (the one unused for longest dropped where there are too many)
+void keep_graph(lrc_batch *b) {
+    if (!b->exec) return;
+    b->kept.insert(b->kept.begin(), {b->graph, b->exec, b->graph_flags, std::move(b->graph_sig)});
+    b->graph = nullptr;
+    b->exec = nullptr;
+    b->graph_sig.clear();
+    if (b->kept.size() >= kGraphs) drop_kept(b, b->kept.size() - 1);
+}
+
+// a kept graph of that key made the current one; false if there is none
+bool use_kept(lrc_batch *b, unsigned flags, const std::vector<unsigned char> &key) {
+    for (size_t i = 0; i < b->kept.size(); i++) {
+        if (b->kept[i].flags != flags || b->kept[i].sig != key) continue;
+        lrc_batch::Graph g = std::move(b->kept[i]);
+        b->kept.erase(b->kept.begin() + (ptrdiff_t)i);
+        keep_graph(b);
+        b->graph = g.graph;
+        b->exec = g.exec;
+        b->graph_flags = g.flags;
+        b->graph_sig = std::move(g.sig);
+        return true;
+    }
+    return false;
 }
 
 // the path tracer's view of a job's scene once the run's builds are done (a build makes the tree
@@ -690,12 +717,9 @@ int lrc_batch_run(lrc_batch *b, unsigned flags) {
         if (rc) return rc;
         const std::vector<unsigned char> key = graph_key(b, flags);
         bool reuse = b->exec && b->graph_flags == flags && key == b->graph_sig;
-        if (!reuse && b->alt_exec && b->alt_flags == flags && key == b->alt_sig) {
-            swap_graphs(b);
-            reuse = true;
-        }
+        if (!reuse) reuse = use_kept(b, flags, key);
         if (!reuse) {
-            swap_graphs(b);                             // (the current graph kept, the one kept before it dropped)
+            keep_graph(b);
             rc = capture(b, flags, key);
             if (rc) return rc;
         }

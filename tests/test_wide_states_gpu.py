@@ -455,3 +455,25 @@ def test_trees_as_deep_as_the_queries_stack(own, ties):
         assert np.array_equal(got[0], want[0][:k]) and np.array_equal(got[1], want[1][:k])
         assert s.occluded(o[:k], d[:k], np.full(k, 200, np.float32)).all()
     s.close()
+
+
+def test_sizes_in_turn_replay_their_graphs(own):
+    sc = W.box_scene(5, 1000, 72, 40)
+    s = R.world_scene(own, sc, 1)
+    p = L.native.trace_params(R.camera12(sc), 72, 40, 8, 1, 1, 0, 3)
+    want = one_kernel(s, p, 1)
+    img = torch.zeros(40, 72, 4, device="cuda")
+    torch.cuda.synchronize()
+    q = L.native.Batch(own)
+    q.set_wavefront(1 << 14)                             # (the largest first: its buffer holds the others)
+    q.add(s, p, 1, img.data_ptr())
+    for k in range(3):
+        for slots in (1 << 14, 1 << 12, 1 << 13, 1 << 11):
+            for variant in (9, 11):
+                q.set_wavefront(slots, variant)
+                q.run(zero=True)
+                own.sync()
+                assert np.array_equal(img.cpu().numpy(), want)
+                assert k == 0 or q.info()["graph_used"] == 1
+    q.close()
+    s.close()
