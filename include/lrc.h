@@ -465,7 +465,8 @@ int lrc_batch_rays(lrc_batch *b, uint64_t *per_job, uint64_t *total);
 int lrc_batch_passes(lrc_batch *b, uint32_t *passes, uint64_t *kernels);
 /* The last LRC_BATCH_STEPPED run of the wavefront (each optional): its closest-hit kernel's device
  * time (CUDA events around each launch) and the rays it traced; with LRC_BATCH_COUNT its walks' box
- * tests (32-byte node records read; an 80-byte wide node counts 2.5) and triangle tests (48-byte triangles read), counted by a
+ * tests (32-byte node records read; an 80-byte wide node counts 2.5) and leaf entries tested (triangles,
+ * primitives, instances; 48 bytes each), counted by a
  * counting build of that kernel (for the launch shapes of 128 threads, registers capped for 4 or 8
  * blocks an SM, the default's among them; with other shapes the counts are 0; it tests what the
  * plain one does: the same hits, the images the same to the bit); and the kernels the run

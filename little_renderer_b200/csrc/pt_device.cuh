@@ -415,10 +415,10 @@ __device__ __forceinline__ void deep_odd(DeepWalk &w) {
     w.ng.y = 0u;
     w.tie = true;
 }
-// world(o, d): the ray as it was given
-template <bool ANY, typename World>
+// world(o, d): the ray as it was given. COUNT as wide_step's.
+template <bool ANY, bool COUNT, typename World>
 __device__ __forceinline__ bool deep_step(const PtScene &S, WideRay &r, DeepWalk &w, uint2 *stack, float tmin, int with,
-                                          uint32_t *err, World &&world) {
+                                          uint32_t *err, World &&world, uint32_t *cnt = nullptr) {
     uint2 tg = make_uint2(0u, 0u);
     if (w.ng.y & WD_INNER) {
         const uint32_t bit = 31 - __clz(w.ng.y);
@@ -430,6 +430,7 @@ __device__ __forceinline__ bool deep_step(const PtScene &S, WideRay &r, DeepWalk
             stack[w.sp++] = w.ng;
         }
         if (ni >= w.at.nnodes) { atomicOr(err, ST_BAD_TREE); return true; }
+        if constexpr (COUNT) cnt[0]++;
         wide_node(w.at.nodes, ni, r, tmin, w.best, w.ng, tg);
     } else {
         tg = w.ng;
@@ -444,6 +445,7 @@ __device__ __forceinline__ bool deep_step(const PtScene &S, WideRay &r, DeepWalk
         tg.y &= ~(1u << slot);
         const uint32_t e = tg.x + __popc((tg.y >> 8) & ((1u << slot) - 1u));
         if (e >= w.at.nleaves) { atomicOr(err, ST_BAD_TREE); return true; }
+        if constexpr (COUNT) cnt[1]++;
         const float4 *lp = w.at.leaves + 3 * (size_t)e;
         const float4 q = __ldg(lp);
         const uint32_t id = __float_as_uint(q.w);

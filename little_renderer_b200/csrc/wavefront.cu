@@ -299,14 +299,14 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_in
     auto answer = [&](uint32_t s, float t, int id, int inst, int tri) {
         W.hit[s] = make_float4(t, __int_as_float(id), __int_as_float(inst), __int_as_float(tri));
     };
-    if ((INST && COUNT) || wf_any_binary(jobs, (uint32_t)W.run[1])) {
+    if (wf_any_binary(jobs, (uint32_t)W.run[1])) {
         wf_each(&W.ctl[2], count, [&](uint32_t k) {
             const uint32_t s = W.rq[k];
             const BatchJob &J = jobs[W.job[s]];
             const V3 o = v3f(W.ro[s]), d = v3f(W.rd[s]);
             float t = 1e30f;
             int id = -1, inst = -1, tri = -1;
-            if constexpr (INST) scene_find<true, COUNT>(J.S, o, d, RT_EPS, 1e30f, t, id, inst, tri, err, cnt);
+            if constexpr (INST || COUNT) scene_find<INST, COUNT>(J.S, o, d, RT_EPS, 1e30f, t, id, inst, tri, err, cnt);
             else if (J.S.nnodes) id = walk_binary<false>(J.S, o, d, RT_EPS, t, err);
             answer(s, t, id, inst, tri);
         });
@@ -327,13 +327,15 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_in
                 if (!wide_plain(r.o, r.d)) deep_odd(w);
             },
             [&](int with) {
-                return deep_step<false>(J->S, r, w, stack, RT_EPS, with, err, [&](V3 &o, V3 &d) { o = v3f(W.ro[s]); d = v3f(W.rd[s]); });
+                return deep_step<false, COUNT>(J->S, r, w, stack, RT_EPS, with, err,
+                                               [&](V3 &o, V3 &d) { o = v3f(W.ro[s]); d = v3f(W.rd[s]); }, cnt);
             },
             [&]() {
                 const bool in = w.inst >= 0;
                 answer(s, w.best, w.tie ? WF_TIE : in ? -1 : w.id, w.inst,
                        in ? w.id - (int)__ldg(&J->S.mesh_info[__float_as_uint(ld4(J->S.inst + 8 * (size_t)w.inst + 6).w)]).y : -1);
             });
+        if constexpr (COUNT) cnt[0] = (5 * cnt[0] + 1) / 2;   // (an 80-byte node: 2.5 records of 32 bytes)
     } else {
         uint2 stack[WD_STACK];
         WideRay r = wide_ray(v3(0, 0, 0), v3(0, 0, 0));
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_in
             },
             [&](int with) { return wide_step<false, COUNT>(wide, r, w, stack, RT_EPS, with, err, WorldLeaf{J->S}, cnt); },
             [&]() { answer(s, w.best, w.tie ? WF_TIE : w.hit, -1, -1); });
-        if constexpr (COUNT) cnt[0] = (5 * cnt[0] + 1) / 2;   // (an 80-byte node: 2.5 records of 32 bytes)
+        if constexpr (COUNT) cnt[0] = (5 * cnt[0] + 1) / 2;
     }
     if constexpr (COUNT) {
         unsigned long long a = cnt[0], b = cnt[1];
@@ -488,7 +490,7 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_sh
                 deep_begin(J->S, w, d.w);
             },
             [&](int with) {
-                return deep_step<true>(J->S, r, w, stack, RT_EPS, with, err,
+                return deep_step<true, false>(J->S, r, w, stack, RT_EPS, with, err,
                                        [&](V3 &o, V3 &d) { o = v3f(W.sq_o[at]); d = v3f(W.sq_d[at]); });
             },
             [&]() {

@@ -477,3 +477,32 @@ def test_sizes_in_turn_replay_their_graphs(own):
                 assert k == 0 or q.info()["graph_used"] == 1
     q.close()
     s.close()
+
+
+def test_the_counting_kernel_counts_the_walk_that_is_walked(own):
+    """Its images are the plain one's; with instances it counts the wide walk (fewer and larger nodes than
+    the binary walk of the same field, which a mesh without a grid has it take), and the binary walk's
+    tests where that is walked."""
+    counts = []
+    for wild in (None, np.nan):
+        s, sc, _ = field(own, False, wild)
+        p = L.native.trace_params(R.camera12(sc), 72, 40, 6, 1, 1, 0, 3)
+        img, stats = wavefront(own, s, p, 5, stepped=True, count=True)
+        plain, _ = wavefront(own, s, p, 5, stepped=True)
+        assert np.array_equal(img, plain)
+        counts.append(stats["box_tests"] / stats["intersect_rays"])
+        s.close()
+    assert 0 < counts[0] < 0.9 * counts[1]
+    sc = W.box_scene(5, 1000, 72, 40)
+    p = L.native.trace_params(R.camera12(sc), 72, 40, 6, 1, 1, 0, 3)
+    n = sc["corners"].shape[0] + 1
+    for given in (False, True):
+        s = R.world_scene(own, sc, 1)
+        if given:                                        # (device arrays: walked as they are)
+            nodes, aux = np.zeros((2 * n - 1, 8), np.uint32), np.zeros(n, np.uint32)
+            own.check(own.L.lrc_scene_tree(s.h, nodes.ctypes.data, aux.ctypes.data, 0))
+            dn, da = dev(nodes.view(np.int32)), dev(aux.view(np.int32))
+            own.check(own.L.lrc_scene_set_tree(s.h, C.c_void_p(dn.data_ptr()), 2 * n - 1, C.c_void_p(da.data_ptr()), n, DEVICE))
+        img, stats = wavefront(own, s, p, 5, stepped=True, count=True)
+        assert np.array_equal(img, one_kernel(s, p, 5)) and stats["box_tests"] > 0 and stats["tri_tests"] > 0
+        s.close()
