@@ -184,7 +184,9 @@ template <bool ANY>
 static __device__ __noinline__ int32_t walk_binary(const PtScene &S, V3 o, V3 d, float tmin, float &best, uint32_t *err) {
     return walk<ANY>(S, S.nodes, S.root, S.nnodes, S.aux, S.naux, o, d, tmin, best, err);
 }
-// a leaf entry's shape: a primitive's record, or the entry's own triangle; t in (tmin, tmax]
+// a leaf entry's shape: a primitive's record, or the entry's own triangle; t in (tmin, tmax]. PATH: a path's
+// ray (tmax is finite and above 0, and one addition the float after it)
+template <bool PATH>
 struct WorldLeaf {
     const PtScene &S;
     __device__ __forceinline__ bool operator()(uint32_t id, float4 q, const float4 *lp, const WideRay &r, float tmin, float tmax,
@@ -195,9 +197,9 @@ struct WorldLeaf {
         // (the float after tmax, their ends being open; after infinity and for no number: no number, which
         // ends nothing, as in hit_sphere_t itself)
         const uint32_t b = __float_as_uint(tmax);
-        const float end = __uint_as_float(tmax > 0.0f ? b + 1u : tmax < 0.0f ? b - 1u : tmax == 0.0f ? 1u : b);
+        const float end = __uint_as_float(PATH || tmax > 0.0f ? b + 1u : tmax < 0.0f ? b - 1u : tmax == 0.0f ? 1u : b);
         return (ld4(pr + 1).w == 0.0f ? hit_sphere_t(v3(c.x, c.y, c.z), c.w, r.o, r.d, tmin, end, t)
-                                      : hit_quad_t(pr, r.o, r.d, tmin, end, t)) && !(t > tmax);
+                                      : hit_quad_t(pr, r.o, r.d, tmin, end, t)) && t <= tmax;
     }
 };
 __device__ __forceinline__ bool world_wide(const PtScene &S) { return S.wide.nodes && wide_walked(S.wide); }
@@ -218,7 +220,7 @@ __device__ __forceinline__ int32_t warp_walk(const PtScene &S, bool on, V3 o, V3
         while (true) {
             const uint32_t m = __ballot_sync(0xffffffffu, going);
             if (!m) break;
-            if (going && wide_step<ANY, false>(S.wide, r, w, stack, tmin, __popc(m), err, WorldLeaf{S})) going = false;
+            if (going && wide_step<ANY, false>(S.wide, r, w, stack, tmin, __popc(m), err, WorldLeaf<false>{S})) going = false;
         }
         binary = on && w.tie;
         hit = w.hit;
@@ -383,7 +385,7 @@ __device__ bool walk_instances(const PtScene &S, V3 o, V3 d, float tmin, float &
 // stack, and the ray goes on in the mesh's space until the stack is back where it was. The same hits as
 // scene_find's: an instance's hit counts only before the world's, and where two triangles of instances
 // are hit at the same t, or the ray is not wide_plain in a mesh's space, tie says so (scene_find then
-// decides).
+// decides, as it does for a ray that is not wide_plain itself: the caller's to see).
 // A field of instances of some 2000 triangles each, 640 x 640 pixels, through the binary nodes of both levels
 // 32 rays at a time and through this with the lanes refilled: 5.12 -> 4.17 ms at 1 spp, 20.1 -> 16.5 at 8.
 struct DeepWalk {
@@ -409,12 +411,6 @@ __device__ __forceinline__ void deep_begin(const PtScene &S, DeepWalk &w, float 
     w.best = tmax;
     w.tie = false;
 }
-// a walk that ends with its first step, scene_find to be asked (wide_odd)
-__device__ __forceinline__ void deep_odd(DeepWalk &w) {
-    w.level = 1;
-    w.ng.y = 0u;
-    w.tie = true;
-}
 // world(o, d): the ray as it was given. COUNT as wide_step's.
 template <bool ANY, bool COUNT, typename World>
 __device__ __forceinline__ bool deep_step(const PtScene &S, WideRay &r, DeepWalk &w, uint2 *stack, float tmin, int with,
@@ -426,7 +422,7 @@ __device__ __forceinline__ bool deep_step(const PtScene &S, WideRay &r, DeepWalk
         const uint32_t slot = (bit - 24u) ^ r.up;
         const uint32_t ni = w.ng.x + __popc(w.ng.y & 0xffu & ((1u << slot) - 1u));
         if (w.ng.y & WD_INNER) {
-            if (w.sp >= WD_STACK) return wide_full(w.tie);
+            if (w.sp >= WD_STACK) return wide_full<!ANY>(w.tie, err);
             stack[w.sp++] = w.ng;
         }
         if (ni >= w.at.nnodes) { atomicOr(err, ST_BAD_TREE); return true; }
@@ -456,7 +452,7 @@ __device__ __forceinline__ bool deep_step(const PtScene &S, WideRay &r, DeepWalk
             if (mesh >= S.nmeshes) continue;         // (shapes: not in these scenes)
             const WideScene m = S.mesh_wide[mesh];
             if (!m.nodes) continue;                  // (a mesh of no triangles)
-            if (w.sp + 2 > WD_STACK) return wide_full(w.tie);
+            if (w.sp + 2 > WD_STACK) return wide_full<!ANY>(w.tie, err);
             if (w.ng.y & WD_INNER) stack[w.sp++] = w.ng;
             if (tg.y & 0xffu) stack[w.sp++] = make_uint2(tg.x, tg.y & 0xffffu);
             V3 o, d;
@@ -472,7 +468,7 @@ __device__ __forceinline__ bool deep_step(const PtScene &S, WideRay &r, DeepWalk
             break;
         }
         float t;
-        if (w.level == 0 ? !WorldLeaf{S}(id, q, lp, r, tmin, w.best, t)
+        if (w.level == 0 ? !WorldLeaf<true>{S}(id, q, lp, r, tmin, w.best, t)
                          : !wide_tri(q, __ldg(lp + 1), __ldg(lp + 2), r.o, r.d, tmin, w.best, t)) continue;
         const int32_t inst = w.level == 2 ? w.cur : -1;
         if (t < w.best) {

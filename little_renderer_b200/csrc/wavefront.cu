@@ -269,7 +269,8 @@ __device__ __forceinline__ bool wf_any_binary(const BatchJob *__restrict__ jobs,
     return __syncthreads_or(b);
 }
 // a closest hit left to the shading kernel, which asks the binary walk: another shape was hit at its t
-// (the walk's call in the closest-hit kernel's loop would cost that loop's registers)
+// (the walk's call in the closest-hit kernel's loop would cost that loop's registers; so would the look at
+// whether the ray is wide_plain, which the shading kernel takes itself: in the loops it took 25 % of an image)
 constexpr int WF_TIE = (int)0x80000000;
 
 // the closest hit of every queued ray; sets the loop's condition (another pass while rays are queued)
@@ -324,7 +325,6 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_in
                 J = &jobs[W.job[s]];
                 r = wide_ray(v3f(W.ro[s]), v3f(W.rd[s]));
                 deep_begin(J->S, w, 1e30f);
-                if (!wide_plain(r.o, r.d)) deep_odd(w);
             },
             [&](int with) {
                 return deep_step<false, COUNT>(J->S, r, w, stack, RT_EPS, with, err,
@@ -353,9 +353,8 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_in
                 r = wide_ray(v3f(W.ro[s]), v3f(W.rd[s]));
                 wide_begin(w, 1e30f);
                 if (!J->S.nnodes) w.ng.y = 0u;       // (an empty world: over after one step)
-                else if (!wide_plain(r.o, r.d)) wide_odd(w);
             },
-            [&](int with) { return wide_step<false, COUNT>(wide, r, w, stack, RT_EPS, with, err, WorldLeaf{J->S}, cnt); },
+            [&](int with) { return wide_step<false, COUNT>(wide, r, w, stack, RT_EPS, with, err, WorldLeaf<true>{J->S}, cnt); },
             [&]() { answer(s, w.best, w.tie ? WF_TIE : w.hit, -1, -1); });
         if constexpr (COUNT) cnt[0] = (5 * cnt[0] + 1) / 2;
     }
@@ -390,7 +389,7 @@ __global__ void __launch_bounds__(SHADE_BLOCK, SMINB) wf_shade_kernel(const Batc
             s = W.rq[k];
             const BatchJob &J = jobs[W.job[s]];
             float4 hh = W.hit[s];
-            if (__float_as_int(hh.y) == WF_TIE) {
+            if (__float_as_int(hh.y) == WF_TIE || !wide_plain(v3f(W.ro[s]), v3f(W.rd[s]))) {
                 int id, inst, tri;
                 find_binary(J.S, v3f(W.ro[s]), v3f(W.rd[s]), RT_EPS, hh.x, id, inst, tri, err);
                 hh = make_float4(hh.x, __int_as_float(id), __int_as_float(inst), __int_as_float(tri));
@@ -493,10 +492,7 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_sh
                 return deep_step<true, false>(J->S, r, w, stack, RT_EPS, with, err,
                                        [&](V3 &o, V3 &d) { o = v3f(W.sq_o[at]); d = v3f(W.sq_d[at]); });
             },
-            [&]() {
-                if (w.tie) atomicOr(err, ST_STACK_OVERFLOW);
-                W.vis[e] = w.id >= 0 ? 0 : 1;
-            });
+            [&]() { W.vis[e] = w.id >= 0 ? 0 : 1; });
     } else {
         uint2 stack[WD_STACK];
         WideRay r = wide_ray(v3(0, 0, 0), v3(0, 0, 0));
@@ -516,11 +512,8 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_sh
                 wide_begin(w, d.w);
                 if (!J->S.nnodes) w.ng.y = 0u;
             },
-            [&](int with) { return wide_step<true, false>(wide, r, w, stack, RT_EPS, with, err, WorldLeaf{J->S}); },
-            [&]() {
-                if (w.tie) atomicOr(err, ST_STACK_OVERFLOW);
-                W.vis[e] = w.hit >= 0 ? 0 : 1;
-            });
+            [&](int with) { return wide_step<true, false, false>(wide, r, w, stack, RT_EPS, with, err, WorldLeaf<true>{J->S}); },
+            [&]() { W.vis[e] = w.hit >= 0 ? 0 : 1; });
     }
 }
 

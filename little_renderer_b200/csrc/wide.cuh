@@ -187,10 +187,12 @@ __device__ __forceinline__ void wide_odd(WideWalk &w) {
     w.tie = true;
 }
 
-// A walk whose stack is full ends: the binary walk, whose pending nodes are others, is asked. (The
-// wavefront's shadow rays, where nothing asks it, report it.)
-__device__ __forceinline__ bool wide_full(bool &tie) {
-    tie = true;
+// A walk whose stack is full ends: the binary walk, whose pending nodes are others, is asked. (ASK =
+// false, the wavefront's shadow rays, where nothing asks it: it is reported.)
+template <bool ASK>
+__device__ __forceinline__ bool wide_full(bool &tie, uint32_t *err) {
+    if (ASK) tie = true;
+    else atomicOr(err, ST_STACK_OVERFLOW);
     return true;
 }
 
@@ -202,7 +204,7 @@ __device__ __forceinline__ bool wide_full(bool &tie) {
 // would be tested by fewer than a quarter of the lanes at it keep them for later (triangles tested with a
 // few lanes are what a divergent walk loses most by; an any-hit walk is better off testing them).
 // COUNT: cnt[0] += nodes (80 bytes each), cnt[1] += leaf entries. True: the walk is over.
-template <bool ANY, bool COUNT, typename Shape>
+template <bool ANY, bool COUNT, bool ASK = true, typename Shape>
 __device__ __forceinline__ bool wide_step(const WideScene &S, const WideRay &r, WideWalk &w, uint2 *stack, float tmin, int with,
                                           uint32_t *err, Shape &&shape, uint32_t *cnt = nullptr) {
     uint2 tg;
@@ -212,7 +214,7 @@ __device__ __forceinline__ bool wide_step(const WideScene &S, const WideRay &r, 
         const uint32_t slot = (bit - 24u) ^ r.up;
         const uint32_t ni = w.ng.x + __popc(w.ng.y & 0xffu & ((1u << slot) - 1u));
         if (w.ng.y & WD_INNER) {
-            if (w.sp >= WD_STACK) return wide_full(w.tie);
+            if (w.sp >= WD_STACK) return wide_full<ASK>(w.tie, err);
             stack[w.sp++] = w.ng;
         }
         if (ni >= S.nnodes) { atomicOr(err, ST_BAD_TREE); return true; }

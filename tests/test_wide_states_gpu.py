@@ -387,11 +387,15 @@ def test_odd_rays(own, tmin, tmax):
         got = s.intersect(o[idx], d[idx], tmin, tmax)
         for g, w in zip(got, want):
             assert np.array_equal(g.view(np.uint32), w[idx].view(np.uint32))
-        far = np.full(m, tmax, np.float32)[idx]
-        blocked = s.occluded(o[idx], d[idx], far, tmin)
-        s.set_walk(0)
-        assert np.array_equal(blocked, s.occluded(o[idx], d[idx], far, tmin))
-        s.set_walk(1)
+    far = np.full(m, tmax, np.float32)
+    arrays = [dev(x) for x in (o, d, far)]
+    out = torch.zeros(m, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    replay(own, captured(own, lambda: own.check(own.L.lrc_scene_occluded(      # (in a capture: the binary walk)
+        s.h, *[C.c_void_p(x.data_ptr()) for x in arrays], m, tmin, C.c_void_p(out.data_ptr()), DEVICE))))
+    blocked = out.cpu().numpy()
+    for idx in (slice(0, m), slice(0, m, 32)):
+        assert np.array_equal(s.occluded(o[idx], d[idx], far[idx], tmin), blocked[idx])
     s.close()
 
 
