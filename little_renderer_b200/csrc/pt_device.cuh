@@ -422,7 +422,7 @@ __device__ __forceinline__ bool deep_step(const PtScene &S, WideRay &r, DeepWalk
         const uint32_t slot = (bit - 24u) ^ r.up;
         const uint32_t ni = w.ng.x + __popc(w.ng.y & 0xffu & ((1u << slot) - 1u));
         if (w.ng.y & WD_INNER) {
-            if (w.sp >= WD_STACK) return wide_full<!ANY>(w.tie, err);
+            if (w.sp >= WD_STACK) return wide_full<false>(w.tie, err);
             stack[w.sp++] = w.ng;
         }
         if (ni >= w.at.nnodes) { atomicOr(err, ST_BAD_TREE); return true; }
@@ -452,7 +452,7 @@ __device__ __forceinline__ bool deep_step(const PtScene &S, WideRay &r, DeepWalk
             if (mesh >= S.nmeshes) continue;         // (shapes: not in these scenes)
             const WideScene m = S.mesh_wide[mesh];
             if (!m.nodes) continue;                  // (a mesh of no triangles)
-            if (w.sp + 2 > WD_STACK) return wide_full<!ANY>(w.tie, err);
+            if (w.sp + 2 > WD_STACK) return wide_full<false>(w.tie, err);
             if (w.ng.y & WD_INNER) stack[w.sp++] = w.ng;
             if (tg.y & 0xffu) stack[w.sp++] = make_uint2(tg.x, tg.y & 0xffffu);
             V3 o, d;

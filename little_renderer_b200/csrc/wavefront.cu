@@ -269,8 +269,8 @@ __device__ __forceinline__ bool wf_any_binary(const BatchJob *__restrict__ jobs,
     return __syncthreads_or(b);
 }
 // a closest hit left to the shading kernel, which asks the binary walk: another shape was hit at its t
-// (the walk's call in the closest-hit kernel's loop would cost that loop's registers; so would the look at
-// whether the ray is wide_plain, which the shading kernel takes itself: in the loops it took 25 % of an image)
+// (the walk's call in the closest-hit kernel's loop would cost that loop's registers), or none was and the ray
+// is not wide_plain (asked when the walk is over: its shapes' t are no numbers and the walk takes none)
 constexpr int WF_TIE = (int)0x80000000;
 
 // the closest hit of every queued ray; sets the loop's condition (another pass while rays are queued)
@@ -332,6 +332,7 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_in
             },
             [&]() {
                 const bool in = w.inst >= 0;
+                if (w.id < 0 && !wide_plain(v3f(W.ro[s]), v3f(W.rd[s]))) w.tie = true;
                 answer(s, w.best, w.tie ? WF_TIE : in ? -1 : w.id, w.inst,
                        in ? w.id - (int)__ldg(&J->S.mesh_info[__float_as_uint(ld4(J->S.inst + 8 * (size_t)w.inst + 6).w)]).y : -1);
             });
@@ -354,8 +355,11 @@ __global__ void __launch_bounds__(BLOCK, wf_min_blocks(BLOCK, MINB, INST)) wf_in
                 wide_begin(w, 1e30f);
                 if (!J->S.nnodes) w.ng.y = 0u;       // (an empty world: over after one step)
             },
-            [&](int with) { return wide_step<false, COUNT>(wide, r, w, stack, RT_EPS, with, err, WorldLeaf<true>{J->S}, cnt); },
-            [&]() { answer(s, w.best, w.tie ? WF_TIE : w.hit, -1, -1); });
+            [&](int with) { return wide_step<false, COUNT, false>(wide, r, w, stack, RT_EPS, with, err, WorldLeaf<true>{J->S}, cnt); },
+            [&]() {
+                if (w.hit < 0 && J->S.nnodes && !wide_plain(r.o, r.d)) w.tie = true;
+                answer(s, w.best, w.tie ? WF_TIE : w.hit, -1, -1);
+            });
         if constexpr (COUNT) cnt[0] = (5 * cnt[0] + 1) / 2;
     }
     if constexpr (COUNT) {
@@ -389,7 +393,7 @@ __global__ void __launch_bounds__(SHADE_BLOCK, SMINB) wf_shade_kernel(const Batc
             s = W.rq[k];
             const BatchJob &J = jobs[W.job[s]];
             float4 hh = W.hit[s];
-            if (__float_as_int(hh.y) == WF_TIE || !wide_plain(v3f(W.ro[s]), v3f(W.rd[s]))) {
+            if (__float_as_int(hh.y) == WF_TIE) {
                 int id, inst, tri;
                 find_binary(J.S, v3f(W.ro[s]), v3f(W.rd[s]), RT_EPS, hh.x, id, inst, tri, err);
                 hh = make_float4(hh.x, __int_as_float(id), __int_as_float(inst), __int_as_float(tri));

@@ -18,14 +18,14 @@
 // boxes the ray meets there is tested here, by the same operations, and where two shapes are hit at
 // the same t - the one case in which the order of the tests decides - `tie` says so and the caller
 // asks the binary walk. Rays that a shape could be hit by at a t that is no number (the binary walk then
-// takes whatever it meets next) go to the binary walk at once (wide_plain).
+// takes whatever it meets next) go to the binary walk (wide_plain): at once, or when the wide walk found none.
 #pragma once
 #include "lrc_internal.cuh"
 
 namespace lrc {
 namespace pt {
 
-constexpr int WD_STACK = 64;                 // pending groups of children a ray (one a level; triangles put off)
+constexpr int WD_STACK = 96;                 // pending groups of children a ray (one a level; triangles put off)
 constexpr int WD_PUT_OFF_BELOW = 48;         // (triangles are put off only while the stack has room for every level)
 constexpr uint32_t WD_INNER = 0xff000000u;   // a group's hit inner children, the nearest at the top bit
 
@@ -187,8 +187,9 @@ __device__ __forceinline__ void wide_odd(WideWalk &w) {
     w.tie = true;
 }
 
-// A walk whose stack is full ends: the binary walk, whose pending nodes are others, is asked. (ASK =
-// false, the wavefront's shadow rays, where nothing asks it: it is reported.)
+// A walk whose stack is full ends: the binary walk, whose pending nodes are others, is asked. ASK = false (the
+// wavefront's kernels): it is reported, as the path tracer's binary walk reports its 64 (a group waits for a
+// node of which that walk holds one or more back, so that it would be full first).
 template <bool ASK>
 __device__ __forceinline__ bool wide_full(bool &tie, uint32_t *err) {
     if (ASK) tie = true;
