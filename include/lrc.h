@@ -164,7 +164,7 @@ int lrc_scene_set_tree(lrc_scene *s, const uint32_t *nodes, uint32_t nnodes, con
  * collapsed into 8-wide nodes with their children's boxes quantised to bytes (80 bytes a node; made by
  * the first query; a given tree whose leaves hold more than 8 shapes, or that names a node twice, stays
  * binary, and so does a query that is captured into a graph, and a scene once one of its changes
- * was captured: replays change it unseen): the same hits as the
+ * was captured: replays change it unseen): the hits of the
  * tree as built, two shapes hit at the same t among them (the binary walk decides those).
  * The modes differ in what lrc_scene_trace_stats counts: 1 the binary walk of that copy, 2 the wide
  * one. mode 0: the tree as built. lrc_scene_tree always gives the tree as built (the reference's). The

@@ -362,6 +362,16 @@ struct TriLeaf {
 
 __device__ __forceinline__ V3 query_v3(const float *p, uint64_t i) { return v3(p[3 * i], p[3 * i + 1], p[3 * i + 2]); }
 __device__ __forceinline__ WideRay query_ray(const Query &Q, uint64_t i) { return wide_ray(query_v3(Q.orig, i), query_v3(Q.dir, i)); }
+// Whether the wide walk tests all that the binary walk meets: both find a box within 4 (|o| + m) 2^-24 in all (m: the
+// tree's largest coordinate; the binary slab test rounds once, the wide one three times), and the wide boxes are
+// WD_WIDEN_TIGHT = 2^-16 of m larger, so for origins within 60 m. (Rays from farther off take the binary walk,
+// whose rounding loses hits there too: the same ones.)
+__device__ __forceinline__ bool query_plain(const Query &Q, const WideRay &r) {
+    const float4 *root = reinterpret_cast<const float4 *>(Q.tt.nodes + Q.tt.root);
+    const float4 l = __ldg(root), h = __ldg(root + 1);
+    const float m = fmaxf(fmaxf(fmaxf(fabsf(l.x), fabsf(l.y)), fmaxf(fabsf(l.z), fabsf(h.x))), fmaxf(fabsf(h.y), fabsf(h.z)));
+    return wide_plain(r.o, r.d) && fmaxf(fmaxf(fabsf(r.o.x), fabsf(r.o.y)), fabsf(r.o.z)) <= 60.0f * m;
+}
 
 // ray i through the binary tree: where two triangles are hit at the same t (the binary walk's order
 // decides), and where the tree is not walked wide. Its stack is as deep as traverse.cu's, that the queries
@@ -436,7 +446,7 @@ __global__ void __launch_bounds__(WD_THREADS, 8) wide_query_kernel(const __grid_
                     i = first + k;
                     r = query_ray(Q, i);
                     wide_begin(w, ANY ? Q.tmaxs[i] : Q.tmax);
-                    if (!wide_plain(r.o, r.d)) wide_odd(w);
+                    if (!query_plain(Q, r)) wide_odd(w);
                 }
             }
             m = __ballot_sync(all, at);
@@ -466,7 +476,7 @@ __global__ void __launch_bounds__(WD_THREADS, 8) wide_query8_kernel(const __grid
     if (i >= Q.n) return;
     const bool one = (threadIdx.x & 7u) == 0u;
     const WideRay r = query_ray(Q, i);
-    if (!wide_walked(Q.W) || !wide_plain(r.o, r.d)) {
+    if (!wide_walked(Q.W) || !query_plain(Q, r)) {
         if (one) query_binary<ANY>(Q, i);
         return;
     }

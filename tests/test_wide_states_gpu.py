@@ -429,6 +429,33 @@ def test_odd_rays_in_a_world_with_primitives(own, tmin, tmax):
         s.close()
 
 
+@pytest.mark.parametrize("away", [1.0, 100.0, 1000.0, 30_000.0])
+@pytest.mark.parametrize("slivers", [False, True])
+def test_hits_that_the_binary_boxes_round_away(own, slivers, away):
+    """Rays from far beyond the boxes' padding, and triangles whose t is mostly rounding: the wide boxes
+    let more of them through, the answer is the binary walk's, closest hits and any."""
+    n, m = 20_000, 1 << 18
+    quv = W.corners_to_quv(W.soup(n, 3))
+    if slivers:
+        quv[:, 6:9] = quv[:, 3:6] * np.float32(1.0001) + quv[:, 6:9] * np.float32(1e-5)
+    s = L.native.Scene(own)
+    s.set_triangles(L.pack_tris(quv))
+    s.build(1, 30)
+    rng = np.random.default_rng(2)
+    o = rng.normal(size=(m, 3))
+    o = 0.5 + 2.0 * away * o / np.linalg.norm(o, axis=1, keepdims=True)
+    at = rng.integers(0, n, m)
+    d = quv[at, 0:3] + (quv[at, 3:6] + quv[at, 6:9]) * rng.random((m, 1)) * 0.5 - o
+    o, d = o.astype(np.float32), (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+    want = binary(own, s, o, d, 0.0, 1e30)
+    far = np.full(m, 1e30, np.float32)
+    for idx in (slice(0, m), slice(0, m, 32)):
+        got = s.intersect(o[idx], d[idx])
+        assert np.array_equal(got[0], want[0][idx]) and np.array_equal(got[1], want[1][idx])
+        assert np.array_equal(s.occluded(o[idx], d[idx], far[idx]).astype(bool), want[0][idx] >= 0)
+    s.close()
+
+
 @pytest.mark.parametrize("ties", [1, 2])
 def test_trees_as_deep_as_the_queries_stack(own, ties):
     """80 levels, each one's leaf behind all that lies below it; the nearest triangle twice (the binary
