@@ -32,7 +32,8 @@ extern "C" {
 #define LRC_E_NODEVICE (-5)    /* no CUDA device (the caller then path traces on the CPU, gpu.h:32-35) */
 
 #define LRC_DEVICE 1u          /* flag: array arguments are device pointers */
-#define LRC_SORT_RAYS 2u       /* flag (ray queries): reorder a large batch by a coherence key first */
+#define LRC_SORT_RAYS 2u       /* flag (closest hits of a triangle scene): a batch of at least 2^18 rays is
+                                  reordered by a coherence key first and walks the binary tree */
 
 typedef struct lrc_ctx lrc_ctx;
 

@@ -768,7 +768,7 @@ int lrc_scene_trace_stats(lrc_scene *s, const float *orig, const float *dir, uin
     if (!e) e = cudaMemcpyAsync(stats, d_stats, 16, cudaMemcpyDeviceToHost, c->st);
     if (e) return cuda_status(c, e, "lrc_scene_trace_stats");
     const int rc = check_status(c);
-    if (!rc && wide) stats[0] = (stats[0] * 5 + 1) / 2;   // (an 80-byte wide node: 2.5 records of 32 bytes)
+    if (!rc && wide) stats[0] = (stats[0] + 1) / 2;      // (wide_count's halves of records)
     return rc;
 }
 

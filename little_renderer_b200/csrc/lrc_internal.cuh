@@ -169,7 +169,7 @@ cudaError_t wide_intersect(const WideScene &W, const TraceTables &tt, const floa
 cudaError_t wide_occluded(const WideScene &W, const TraceTables &tt, const float *d_orig, const float *d_dir,
                           const float *d_tmax, uint64_t nrays, float tmin, uint8_t *d_out, uint32_t *d_status,
                           cudaStream_t st);
-// totals: [0] wide nodes fetched (80 bytes each), [1] triangle tests
+// totals: [0] box tests in halves of 32-byte records (an 80-byte wide node: 5), [1] triangle tests
 cudaError_t wide_count(const WideScene &W, const TraceTables &tt, const float *d_orig, const float *d_dir, uint64_t nrays,
                        float tmin, float tmax, unsigned long long *d_stats, uint32_t *d_status, cudaStream_t st);
 // the walk's tree of a triangle tree (nn nodes, root at 0, leaves' aux = triangle ids): the same

@@ -486,16 +486,29 @@ __global__ void __launch_bounds__(WD_THREADS, 8) wide_query8_kernel(const __grid
     if (one) query_done<ANY>(Q, i, hit, best, tie);
 }
 
-// the closest-hit walk's nodes and triangle tests: [0] and [1]
+// the closest-hit walk's box tests in halves of 32-byte records (an 80-byte node: 5) and triangle tests: [0] and [1];
+// of the binary walk where that is walked
 __global__ void __launch_bounds__(WD_THREADS) wide_count_kernel(const __grid_constant__ Query Q, unsigned long long *stats) {
     const uint64_t i = (uint64_t)blockIdx.x * WD_THREADS + threadIdx.x;
     uint32_t cnt[2] = {0, 0};
-    if (i < Q.n && wide_walked(Q.W)) {
+    if (i < Q.n) {
         const WideRay r = query_ray(Q, i);
-        WideWalk w;
-        wide_begin(w, Q.tmax);
-        if (!wide_plain(r.o, r.d)) wide_odd(w);
-        wide_run<false, true>(Q.W, r, w, Q.tmin, Q.err, TriLeaf{}, cnt);
+        if (wide_walked(Q.W) && query_plain(Q, r)) {
+            WideWalk w;
+            wide_begin(w, Q.tmax);
+            wide_run<false, true>(Q.W, r, w, Q.tmin, Q.err, TriLeaf{}, cnt);
+            cnt[0] *= 5u;
+        } else {
+            float best = Q.tmax;
+            bvh_walk<true, QUERY_STACK>(reinterpret_cast<const float4 *>(Q.tt.nodes), Q.tt.root, Q.tt.nnodes, Q.tt.aux, Q.tt.naux,
+                                        r.o, r.d, Q.tmin, best, Q.err, [&](uint32_t id) {
+                if (id >= Q.tt.ntris) { atomicOr(Q.err, ST_BAD_TREE); return true; }
+                float t;
+                if (hit_tri_t(Q.tt.tris + 3 * (size_t)id, r.o, r.d, Q.tmin, best, t)) best = t;
+                return false;
+            }, cnt);
+            cnt[0] *= 2u;
+        }
     }
     unsigned long long a = cnt[0], b = cnt[1];
     for (int o = 16; o > 0; o >>= 1) {

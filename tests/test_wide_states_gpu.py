@@ -537,3 +537,19 @@ def test_the_counting_kernel_counts_the_walk_that_is_walked(own):
         img, stats = wavefront(own, s, p, 5, stepped=True, count=True)
         assert np.array_equal(img, one_kernel(s, p, 5)) and stats["box_tests"] > 0 and stats["tri_tests"] > 0
         s.close()
+
+
+@pytest.mark.parametrize("wild", [None, np.nan, np.inf])
+def test_walk_statistics_of_trees_that_no_grid_holds(own, wild):
+    quv = W.corners_to_quv(W.soup(5000, 3))
+    if wild is not None:
+        quv[7, 0] = wild
+    s = L.native.Scene(own)
+    s.set_triangles(L.pack_tris(quv))
+    s.build(0, 30)
+    o, d = W.rays_at_cube(3000, 2)
+    binary = s.trace_stats(o, d)
+    s.set_walk(2)
+    wide = s.trace_stats(o, d)
+    assert wide == binary if wild is not None else 0 < wide[0] < binary[0]
+    s.close()
