@@ -1706,7 +1706,11 @@ def main():
     ctx.sync()
     # traversal statistics (the algorithmic bytes per ray), outside the timed region
     sample = min(a.rays, 1 << 20)
+    # (the walk that the queries take: mode 2 counts the wide one, mode 1 the binary tree it is made from)
+    if a.walk:
+        scene.set_walk(2)
     boxes_tested, tris_tested = scene.trace_stats((sample, d_o.data_ptr(), d_d.data_ptr()))
+    scene.set_walk(a.walk)
 
     if dist:
         dist.barrier()
@@ -1771,7 +1775,7 @@ def main():
     trace_bytes = bytes_per_ray * a.rays
     kb = 8 if a.bits == 63 else 4
     sort_bytes = a.n * (kb + (a.bits + 7) // 8 * 2 * (kb + 4))
-    rl_trace = {"kernel": "closest_kernel", "bound": "hbm", "achieved": trace_bytes / (trace_ms / 1e3) / 1e9,
+    rl_trace = {"kernel": "wide_query_kernel" if a.walk else "closest_kernel", "bound": "hbm", "achieved": trace_bytes / (trace_ms / 1e3) / 1e9,
                 "peak": peak, "unit": "GB/s", "peak_kind": peak_kind, "traffic": None,
                 "algorithmic_bytes_per_launch": trace_bytes, "bytes_per_ray": bytes_per_ray,
                 "ms_per_launch": trace_ms}

@@ -163,15 +163,16 @@ int lrc_scene_set_tree(lrc_scene *s, const uint32_t *nodes, uint32_t nnodes, con
  * copy of the tree whose boxes are the triangles' own bounds widened by 2^-17 of the root box's
  * largest coordinate (at most the 1e-3 of triangle_bounds, scene.c:65-74), inner boxes their unions,
  * collapsed into 8-wide nodes with their children's boxes quantised to bytes (80 bytes a node; made by
- * the first query; a given tree whose leaves hold more than 8 shapes, or that names a node twice, stays
+ * a query once the queries since the build, this one with them, would have gained what the making
+ * takes: many rays at once, else a few calls; a given tree whose leaves hold more than 8 shapes, or that names a node twice, stays
  * binary, and so does a query that is captured into a graph, and a scene once one of its changes
  * was captured: replays change it unseen): the hits of the
  * tree as built, two shapes hit at the same t among them (the binary walk decides those).
  * The modes differ in what lrc_scene_trace_stats counts: 1 the binary walk of that copy, 2 the wide
  * one. mode 0: the tree as built. lrc_scene_tree always gives the tree as built (the reference's). The
  * guide, the wavefront engine and images of at most 24576 paths at once on scenes without media walk
- * that tree's own 8-wide nodes (made by the first of them after a build, about 1 ms at 4M shapes, 120
- * bytes a shape), other images, the megakernel engine and the caustics the tree as built. A triangle
+ * that tree's own 8-wide nodes (made likewise, by the wavefront engine at its first use; 1.6 ms at 4M
+ * shapes, 120 bytes a shape), other images, the megakernel engine and the caustics the tree as built. A triangle
  * scene reserves as much again for the queries' when it is built. */
 int lrc_scene_set_walk(lrc_scene *s, int mode);
 

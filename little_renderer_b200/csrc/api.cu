@@ -7,6 +7,7 @@
 // synchronise; calls with LRC_DEVICE only enqueue (lrc_sync waits and reports).
 #include "api_internal.cuh"
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -34,8 +35,8 @@ int scene_build_on(lrc_scene *s, int builder, int key_bits, void **scratch, size
     }
     s->tree_nnodes = s->tree_naux = 0;
     s->walk_ok = false;
-    s->wide_ok = false;
-    s->pwide_ok = false;
+    s->wide_ok = s->pwide_ok = false;
+    s->query_saved = s->path_saved = 0.0;
     s->most_leaf = 1;
     if (!n) return LRC_OK;
     const size_t need_scratch = lrc::build_scratch_bytes(n, key_bits, builder);
@@ -78,7 +79,7 @@ int scene_build_on(lrc_scene *s, int builder, int key_bits, void **scratch, size
     return LRC_OK;
 }
 
-// Wide nodes are made on a first use, on the stream of that use. The scene's later uses may be on other
+// Wide nodes are made by a use, on the stream of that use. The scene's later uses may be on other
 // streams (lrc_set_stream), which the caller has no reason to order after it: each waits for the event.
 static int wide_noted(lrc_scene *s, cudaStream_t st) {
     cudaError_t e = s->wide_made ? cudaSuccess : cudaEventCreateWithFlags(&s->wide_made, cudaEventDisableTiming);
@@ -152,12 +153,29 @@ int instances_wide(lrc_scene *s, cudaStream_t st) {
     return wide_noted(s, st);
 }
 
-int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc) {
+// Making the nodes of n shapes takes about this long, in us (2000 shapes 60, 200k 150, 1M 460, 4M 1640); a use of the
+// binary nodes that wide ones would have shortened is reckoned up, and the nodes are made when that comes to
+// as much: a tree that is built again after a few queries does not pay for nodes it has no use for, one that
+// stays has them after a few. (First query after a build, binary and with the making in it: 1 ray on 4M triangles
+// 330 and 1740 us, 1024 on 20k 93 and 118, 32768 on 1M 378 and 612; 2M on 1M 8.7 and 4.5 ms. The first 128 x 128
+// image: of 200k 1070 and 920 us, of 4M 2010 and 2800.)
+static double wide_cost(uint32_t n) { return 60.0 + 0.38e-3 * n; }
+// what wide nodes save, us: a query's chain of nodes (about a third of the cost, less with few rays to be the
+// slowest of), and of many rays their instructions; an image's bounces; the guide's rays
+double query_saving(const lrc_scene *s, uint64_t rays) {
+    const double c = wide_cost(s->built_n), per_ray = 0.125e-3 * std::max(std::log2((double)s->built_n + 1.0) - 10.5, 0.4);
+    return c * (0.06 + 0.29 * std::min((double)rays / 1024.0, 1.0)) + per_ray * (double)rays;
+}
+double image_saving(const lrc_scene *s) { return 0.55 * wide_cost(s->built_n) + 200.0; }
+double guide_saving(const lrc_scene *s) { return 0.08 * wide_cost(s->built_n) + 30.0; }
+
+int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc, double saving) {
     if (!no_alloc) {                                 // (no_alloc: a batch's capture, in its own order)
         int rc = wide_ordered(s, st);
         if (rc || capturing(st)) return rc;
     }
     if (s->pwide_ok || s->replayed || !s->built_n || !s->most_leaf || s->most_leaf > kMostLeaf) return LRC_OK;
+    if (!no_alloc && (s->path_saved += saving) < wide_cost(s->built_n)) return LRC_OK;
     lrc_ctx *c = s->ctx;
     const bool single = !s->tree_nnodes;
     const uint32_t nn = single ? 2 * s->built_n - 1 : s->tree_nnodes, na = single ? s->built_n : s->tree_naux;
@@ -178,17 +196,16 @@ int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc) {
 }
 
 // The queries' wide nodes, from the walk's tree (a tree with larger leaves than a node has slots, no memory,
-// a query inside a capture, a scene that a graph builds: the binary walk). Made by the first query after a build: a scene that
-// is built each frame and only path traced would pay for nodes it never walks (scene builds of 200k / 4M
-// triangles 0.25 / 1.5 ms, with them 0.37 / 3.0).
-static int query_wide(lrc_scene *s) {
+// a query inside a capture, a scene that a graph builds: the binary walk). Made by a query, when the queries since the
+// build have come to their cost: not by the build (4M triangles 1.5 ms, with them 3.0).
+static int query_wide(lrc_scene *s, double saving) {
     lrc_ctx *c = s->ctx;
     int rc = wide_ordered(s, c->st);
     if (rc || s->wide_ok || !s->walk_ok || s->replayed || !s->most_leaf || s->most_leaf > kMostLeaf || capturing(c->st))
         return rc;
     const bool single = !s->tree_nnodes;
     const uint32_t nn = single ? 2 * s->built_n - 1 : s->tree_nnodes, na = single ? s->built_n : s->tree_naux;
-    if (s->wide_cap < lrc::wide_bytes(na, single)) return LRC_OK;
+    if (s->wide_cap < lrc::wide_bytes(na, single) || (s->query_saved += saving) < wide_cost(s->built_n)) return LRC_OK;
     c->timer.begin(LRC_TS_HIERARCHY, c->st);
     cudaError_t e = lrc::wide_build(s->d_wnodes, nn, s->d_aux, na, 0, reinterpret_cast<const float *>(s->d_tris), s->ntris,
                                     lrc::WD_WIDEN_TIGHT, s->d_wide, single, c->d_status, c->num_sms, c->st);
@@ -220,6 +237,7 @@ cudaError_t build_tlas_on(lrc_ctx *c, const float *d_inst, uint32_t n, Node *d_n
 int make_walk(lrc_scene *s) {
     s->walk_ok = false;
     s->wide_ok = false;
+    s->query_saved = 0.0;
     if (!s->walk_mode || s->nprims || !s->built_n || !s->ntris) return LRC_OK;
     lrc_ctx *c = s->ctx;
     const size_t nn = s->tree_nnodes ? s->tree_nnodes : 2 * (size_t)s->built_n - 1;
@@ -239,7 +257,7 @@ int make_walk(lrc_scene *s) {
     c->timer.end(c->st);
     if (e) return cuda_status(c, e, "the walk's tree");
     s->walk_ok = true;
-    // (room for the wide nodes that the first query makes; none: the binary walk)
+    // (room for the wide nodes that a query makes; none: the binary walk)
     if (s->most_leaf && s->most_leaf <= kMostLeaf &&
         reserve(&s->d_wide, &s->wide_cap, lrc::wide_bytes((uint32_t)na, !s->tree_nnodes)) != cudaSuccess)
         cudaGetLastError();
@@ -283,7 +301,7 @@ int trace_wavefront(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t
                                   : cudaEventCreateWithFlags(&c->single_ran, cudaEventDisableTiming);
     if (e) return cuda_status(c, e, "the wavefront's event");
     // The paths in flight: all of them up to 2^22, in three sizes (a size's graph is captured when it is
-    // first used, and two are kept): a pass costs most in its longest walks, so there should be few.
+    // first used, and eight are kept): a pass costs most in its longest walks, so there should be few.
     // 640 x 640 pixels at 8 spp of 20k triangles: 2^20 12.4 ms, 2^21 11.9, 2^22 11.2. Up to 2^21 paths the
     // walks run 6 blocks an SM (their registers unspilled: 410k paths 2.65 -> 2.50 ms), with more paths
     // the default's 8 (3.3M paths: 11.55 against 11.19 ms).
@@ -536,8 +554,8 @@ int lrc_scene_set_triangles(lrc_scene *s, const uint32_t *tris, uint32_t n, unsi
     s->built_n = 0;
     s->tree_nnodes = s->tree_naux = 0;
     s->walk_ok = false;
-    s->wide_ok = false;
-    s->pwide_ok = false;
+    s->wide_ok = s->pwide_ok = false;
+    s->query_saved = s->path_saved = 0.0;
     if (!(flags & LRC_DEVICE)) return check_status(c);   // (the host array may be freed on return)
     return LRC_OK;
 }
@@ -607,8 +625,8 @@ int lrc_scene_set_tree(lrc_scene *s, const uint32_t *nodes, uint32_t nnodes, con
     }
     DeviceGuard g(c->device);
     s->walk_ok = false;
-    s->wide_ok = false;
-    s->pwide_ok = false;
+    s->wide_ok = s->pwide_ok = false;
+    s->query_saved = s->path_saved = 0.0;
     s->most_leaf = most;
     const size_t cap = std::max<size_t>(naux, ((size_t)nnodes + 1) / 2);   // (2 cap - 1 nodes, cap aux)
     cudaError_t e = cudaSuccess;
@@ -699,14 +717,17 @@ int lrc_scene_intersect(lrc_scene *s, const float *orig, const float *dir, uint6
     if (!s->built_n) return fail(c, LRC_E_INVALID, "the scene has no built BVH (lrc_scene_build)");
     DeviceGuard g(c->device);
     lrc::TraceTables tt = tables(s);
-    if (int rc = s->nprims ? scene_wide(s, c->st, false) : query_wide(s)) return rc;
-    const bool wide = s->wide_ok && !capturing(c->st);
     // LRC_SORT_RAYS: the reordering's scratch (large batches); without it the rays go in their order
     void *sort_scratch = nullptr;
     if ((flags & LRC_SORT_RAYS) && lrc::intersect_scratch_bytes(nrays)) {
         if (reserve(&c->scratch, &c->scratch_cap, lrc::intersect_scratch_bytes(nrays)) == cudaSuccess) sort_scratch = c->scratch;
         else cudaGetLastError();
     }
+    if (s->nprims || !sort_scratch) {                // (sorted rays walk the binary nodes)
+        const double saving = query_saving(s, nrays);
+        if (int rc = s->nprims ? scene_wide(s, c->st, false, saving) : query_wide(s, saving)) return rc;
+    }
+    const bool wide = s->wide_ok && !capturing(c->st);
     // a world with primitives walks shape ids (primitives, then triangles); a mesh, triangles alone
     auto run = [&](const float *o, const float *d, int32_t *p, float *tt_out) {
         if (s->nprims) return lrc::pt_intersect(pt_scene(s), o, d, nrays, tmin, tmax, p, nullptr, tt_out, c->d_status, c->st);
@@ -747,7 +768,7 @@ int lrc_scene_trace_stats(lrc_scene *s, const float *orig, const float *dir, uin
     DeviceGuard g(c->device);
     lrc::TraceTables tt = tables(s);
     if (s->walk_mode == 2)
-        if (int rc = query_wide(s)) return rc;
+        if (int rc = query_wide(s, kAlways)) return rc;
     const size_t b_ray = al(nrays * 12);
     cudaError_t e = reserve(&c->stage, &c->stage_cap, 2 * b_ray + 256);
     if (e) return cuda_status(c, e, "ray staging");
@@ -779,7 +800,7 @@ int lrc_scene_occluded(lrc_scene *s, const float *orig, const float *dir, const 
     if (!s->built_n) return fail(c, LRC_E_INVALID, "the scene has no built BVH (lrc_scene_build)");
     DeviceGuard g(c->device);
     lrc::TraceTables tt = tables(s);
-    if (int rc = query_wide(s)) return rc;
+    if (int rc = query_wide(s, query_saving(s, nrays))) return rc;
     const bool wide = s->wide_ok && !capturing(c->st);
     if (flags & LRC_DEVICE) {
         cudaError_t e = wide ? lrc::wide_occluded(wide_tables(s), tt, orig, dir, tmax, nrays, tmin, out, c->d_status, c->st)
@@ -818,8 +839,8 @@ int lrc_scene_set_prims(lrc_scene *s, const float *prims, uint32_t n, unsigned f
     s->built_n = 0;
     s->tree_nnodes = s->tree_naux = 0;
     s->walk_ok = false;
-    s->wide_ok = false;
-    s->pwide_ok = false;
+    s->wide_ok = s->pwide_ok = false;
+    s->query_saved = s->path_saved = 0.0;
     return (flags & LRC_DEVICE) ? LRC_OK : check_status(c);
 }
 
@@ -1131,7 +1152,7 @@ int lrc_scene_intersect_ex(lrc_scene *s, const float *orig, const float *dir, ui
     if (!s->built_n && !(s->meshes_built && s->tlas_n)) return fail(c, LRC_E_INVALID, "the scene has nothing built");
     DeviceGuard g(c->device);
     {
-        int rc = scene_wide(s, c->st, false);
+        int rc = scene_wide(s, c->st, false, query_saving(s, nrays));
         if (rc) return rc;
     }
     if (flags & LRC_DEVICE) {
@@ -1219,7 +1240,7 @@ int lrc_trace(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows,
         return (flags & LRC_DEVICE) ? LRC_OK : check_status(c);
     }
     if (!e && lrc::pt_walks_wide(P, s->nvol != 0)) {
-        int rc = scene_wide(s, c->st, false);
+        int rc = scene_wide(s, c->st, false, image_saving(s));
         if (rc) return rc;
     }
     c->timer.begin(LRC_TS_SHADE, c->st);

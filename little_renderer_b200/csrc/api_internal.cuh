@@ -44,7 +44,7 @@ struct lrc_scene {
     void *d_wide = nullptr;       // the ray queries' wide nodes, made from d_wnodes (walk_mode 1, 2)
     size_t wide_cap = 0;
     bool wide_ok = false;
-    cudaEvent_t wide_made = nullptr;   // after the last wide nodes made on a first use (scene_wide, query_wide)
+    cudaEvent_t wide_made = nullptr;   // after the last wide nodes made by a use (scene_wide, query_wide)
     bool wide_done = true;        // it is known to have passed
     void *d_pwide = nullptr;      // the path tracer's wide nodes, made from d_nodes when first traced
     size_t pwide_cap = 0;
@@ -55,6 +55,7 @@ struct lrc_scene {
     void *d_twide = nullptr;      // the top level's
     size_t twide_cap = 0;
     bool twide_ok = false;
+    double query_saved = 0.0, path_saved = 0.0;   // what wide nodes would have saved since the build, us (wide_cost)
     uint32_t most_leaf = 1;       // the largest leaf of the tree (0: not known)
     // A change of the world (of the instances) that a caller's graph has captured happens again with each
     // replay, unseen here: nothing made from the trees on the host's word is walked from then on.
@@ -285,12 +286,16 @@ inline lrc::WideScene wide_tables(const lrc_scene *s) {
 constexpr uint32_t kMostLeaf = 8;
 
 // the path tracer's wide nodes of the scene's world tree, on stream st, unless they are there: every
-// caller that traces paths asks first, so that a tree is collapsed once, by the first call that traces
-// it, and a build that is only queried or refitted does not pay for it. A tree that cannot be (no memory,
-// leaves too large) is walked as it is.
-// no_alloc: within a graph's capture (a buffer too small is then an error).
+// caller whose kernels walk them asks first, so that a tree is collapsed once and a build that is not traced
+// does not pay for it. A tree that cannot be (no memory, leaves too large) is walked as it is.
+// no_alloc: within a graph's capture (a buffer too small is then an error). saving: what this use would gain by them
+// (us); they are made once the uses since the build have come to their cost, kAlways at once.
+constexpr double kAlways = 1e30;
+double query_saving(const lrc_scene *s, uint64_t rays);
+double image_saving(const lrc_scene *s);
+double guide_saving(const lrc_scene *s);
 int instances_wide(lrc_scene *s, cudaStream_t st);
-int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc);
+int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc, double saving = kAlways);
 
 // lrc_trace's way of a large image: whether a call goes the wavefront engine's way, and the call (device
 // image, or planes when guided)

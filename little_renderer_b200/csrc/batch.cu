@@ -552,6 +552,7 @@ void note_built(lrc_batch *b) {   // (what captured builds' host side records)
         J->s->built_n = J->s->ntris + J->s->nprims;
         J->s->tree_nnodes = J->s->tree_naux = 0;     // (a tree given or built meanwhile, and its copy, are gone)
         J->s->walk_ok = J->s->wide_ok = false;
+        J->s->query_saved = J->s->path_saved = 0.0;
         J->s->most_leaf = 1;
         J->s->pwide_ok = b->engine == 1 && J->s->built_n && !J->s->replayed && J->s->pwide_cap >= lrc::wide_bytes(J->s->built_n, true);
     }

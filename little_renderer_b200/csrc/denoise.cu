@@ -682,7 +682,7 @@ int lrc_guide(lrc_scene *s, const lrc_trace_params *p, float *planes, unsigned f
         if (rc) return rc;
     }
     {
-        int rc = scene_wide(s, c->st, false);
+        int rc = scene_wide(s, c->st, false, guide_saving(s));
         if (rc) return rc;
     }
     const size_t N = (size_t)p->width * p->height;
@@ -752,7 +752,7 @@ int lrc_reproject_gradients(lrc_scene *s, const lrc_trace_params *old_p, const l
     int rc = scene_traceable(s);
     const size_t N = (size_t)W * H;
     const uint32_t ntiles = grad_tiles(W, H);
-    if (!rc && lrc::pt_gradients_walk_wide(ntiles, s->nvol != 0)) rc = scene_wide(s, c->st, false);
+    if (!rc && lrc::pt_gradients_walk_wide(ntiles, s->nvol != 0)) rc = scene_wide(s, c->st, false, image_saving(s));
     if (rc) return rc;
     const float4 *d_old = reinterpret_cast<const float4 *>(old_planes);
     float4 *d_new = reinterpret_cast<float4 *>(new_planes);
@@ -810,7 +810,6 @@ int lrc_trace_frame(lrc_scene *s, const lrc_trace_params *old_p, const lrc_trace
         return fail(c, LRC_E_INVALID, "temporal gradients trace a sample again: the old image in fast mode (exact = 0)");
     DeviceGuard g(c->device);
     int rc = scene_traceable(s);
-    if (!rc) rc = scene_wide(s, c->st, false);           // (the guide walks them)
     if (rc) return rc;
     const size_t N = (size_t)W * H;
     const uint32_t ntiles = grad_tiles(W, H);
@@ -838,6 +837,10 @@ int lrc_trace_frame(lrc_scene *s, const lrc_trace_params *old_p, const lrc_trace
     P.guide = d_new + 3 * N;
     lrc::GradTile *d_tiles = static_cast<lrc::GradTile *>(c->dn);
     const bool edit = (flags & LRC_REPROJECT_EDIT) != 0;
+    // (the guide walks wide nodes, and the trace: the wavefront's, or a small image's)
+    const bool walked = lrc::pt_walks_wide(P, s->nvol != 0) || (grads && lrc::pt_gradients_walk_wide(ntiles, s->nvol != 0));
+    rc = scene_wide(s, c->st, false, wavefront_call(s, new_p, H, spp) ? kAlways : guide_saving(s) + (walked ? image_saving(s) : 0.0));
+    if (rc) return rc;
     c->timer.begin(LRC_TS_SHADE, c->st);
     e = lrc::dn_guide(pt_scene(s), P, d_new, c->d_status, c->st);
     if (!e && grads) e = grad_chain(s, old_p, new_p, spp0, d_old, d_new, d_tiles, edit, c->st);

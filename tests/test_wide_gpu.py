@@ -27,6 +27,12 @@ def tables():
     return mask, tab
 
 
+def made(s):
+    """The queries' wide nodes made now (counting their walk makes them, else a few queries do)."""
+    s.set_walk(2)
+    s.trace_stats(np.zeros((1, 3), np.float32), np.ones((1, 3), np.float32))
+
+
 def triangles(kind, n, seed):
     rng = np.random.default_rng(seed)
     if kind == "soup":
@@ -72,6 +78,7 @@ def test_queries_are_the_binary_walks(own, kind, n, builder):
     s = L.native.Scene(own)
     s.set_triangles(L.pack_tris(triangles(kind, n, 3)))
     s.build(builder, 30)
+    made(s)
     m = 1 << 18                                      # (LRC_SORT_RAYS: the binary walk, from this many rays)
     o, d = rays(kind, m, 4)
     prim, t = np.zeros(m, np.int32), np.zeros(m, np.float32)
@@ -174,6 +181,7 @@ def test_given_trees_with_larger_leaves(own, leaf):
 
     make(np.arange(n))
     s.set_tree(np.array(nodes), np.array(aux, np.uint32))
+    made(s)
     got = s.intersect(o, d)
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
     s.close()

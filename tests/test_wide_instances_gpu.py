@@ -104,7 +104,8 @@ def test_first_use_in_a_capture_and_on_another_stream(own):
             s.build(1, 30)
             own.sync()
             if used:
-                query(other)
+                for _ in range(4):                   # (a few queries make the wide nodes)
+                    query(other)
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, stream=side):
                 query(side)

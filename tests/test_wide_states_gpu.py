@@ -30,6 +30,12 @@ def soup(n, seed):
     return L.pack_tris(W.corners_to_quv(W.soup(n, seed)))
 
 
+def made(s):
+    """The queries' wide nodes made now (counting their walk makes them, else a few queries do)."""
+    s.set_walk(2)
+    s.trace_stats(np.zeros((1, 3), np.float32), np.ones((1, 3), np.float32))
+
+
 def hits(own, tris, o, d):
     """The closest hits of a scene made anew."""
     s = L.native.Scene(own)
@@ -108,7 +114,7 @@ def test_captured_queries_see_the_next_build(own, m):
     s = L.native.Scene(own)
     s.set_triangles(soup(n, 5))
     s.build(1, 30)
-    s.intersect(o, d)                                    # (the wide nodes are there when the graph is captured)
+    made(s)                                              # (the wide nodes are there when the graph is captured)
     ro, rd, far = dev(o), dev(d), torch.full((m,), 3.0, device="cuda")
     prim, t = torch.zeros(m, dtype=torch.int32, device="cuda"), torch.zeros(m, device="cuda")
     blocked = torch.zeros(m, dtype=torch.uint8, device="cuda")
@@ -164,7 +170,7 @@ def test_captured_builds_are_seen_by_the_next_query(own):
         s.build(1, 30)
 
     build()
-    s.intersect(o, d)
+    made(s)
     g = captured(own, build)
     for seed in (6, 7):
         tris.copy_(dev(soup(n, seed).view(np.int32)))
@@ -380,6 +386,7 @@ def test_odd_rays(own, tmin, tmax):
     s = L.native.Scene(own)
     s.set_triangles(soup(5000, 3))
     s.build(1, 30)
+    made(s)
     m = 1 << 18
     o, d = odd_rays(m, 4)
     want = binary(own, s, o, d, tmin, tmax)
@@ -422,7 +429,8 @@ def test_odd_rays_in_a_world_with_primitives(own, tmin, tmax):
     own.check(own.L.lrc_scene_set_tree(scenes[1].h, C.c_void_p(dn.data_ptr()), 2 * n - 1, C.c_void_p(da.data_ptr()), n, DEVICE))
     o, d = odd_rays(40_000, 4)
     o = (o * np.float32(555)).astype(np.float32)
-    got, want = (s.intersect(o, d, tmin, tmax) for s in scenes)
+    for _ in range(4):                                   # (a few queries make the wide nodes)
+        got, want = (s.intersect(o, d, tmin, tmax) for s in scenes)
     for g, w in zip(got, want):
         assert np.array_equal(g.view(np.uint32), w.view(np.uint32))
     for s in scenes:
@@ -441,6 +449,7 @@ def test_hits_that_the_binary_boxes_round_away(own, slivers, away):
     s = L.native.Scene(own)
     s.set_triangles(L.pack_tris(quv))
     s.build(1, 30)
+    made(s)
     rng = np.random.default_rng(2)
     o = rng.normal(size=(m, 3))
     o = 0.5 + 2.0 * away * o / np.linalg.norm(o, axis=1, keepdims=True)
@@ -477,6 +486,7 @@ def test_trees_as_deep_as_the_queries_stack(own, ties):
     s = L.native.Scene(own)
     s.set_triangles(L.pack_tris(quv))
     s.set_tree(nodes, np.arange(n, dtype=np.uint32))
+    made(s)
     m = 1 << 18
     o, d = np.zeros((m, 3), np.float32), np.tile(np.float32([0, 0, 1]), (m, 1))
     want = binary(own, s, o, d, 0.0, 1e30)
@@ -552,4 +562,30 @@ def test_walk_statistics_of_trees_that_no_grid_holds(own, wild):
     s.set_walk(2)
     wide = s.trace_stats(o, d)
     assert wide == binary if wild is not None else 0 < wide[0] < binary[0]
+    s.close()
+
+
+def test_nodes_are_made_when_the_queries_are_worth_them(own):
+    """A few rays after a build walk the binary nodes (no wide ones are made, 94 MB of a million shapes), as more
+    calls come, or many rays, the wide ones: the same answers."""
+    n = 1_000_000
+    o, d = W.rays_at_cube(1 << 20, 2)
+    s = L.native.Scene(own)
+    s.set_triangles(soup(n, 3))
+    s.set_prims(W.make_quad([0, 0, 0.5], [1, 0, 0], [0, 1, 0], 0))
+    s.build(1, 30)
+    want = s.intersect(o, d)                             # (makes them)
+    s.close()
+    s = L.native.Scene(own)
+    s.set_triangles(soup(n, 3))
+    s.set_prims(W.make_quad([0, 0, 0.5], [1, 0, 0], [0, 1, 0], 0))
+    s.build(1, 30)
+    s.intersect(o[:1], d[:1])
+    free = torch.cuda.mem_get_info()[0]
+    taken = []
+    for k in range(30):
+        got = s.intersect(o[:1000], d[:1000])
+        assert np.array_equal(got[0], want[0][:1000]) and np.array_equal(got[1], want[1][:1000])
+        taken.append(free - torch.cuda.mem_get_info()[0] > 48 * n)
+    assert not taken[0] and taken[-1]
     s.close()
