@@ -305,8 +305,10 @@ __global__ void __launch_bounds__(OS_THREADS, OS_MINB) onesweep_kernel(const K *
 // A tree over at most SS_ITEMS items (a frame's top level) spends its time in launches and in passes of
 // one tile each, so the codes and every pass run in one launch: 1024 threads, the keys and items in
 // registers between passes and in shared memory across one (the onesweep pass's ranking, without
-// its histograms and its look-back). The line is the block's capacity; a whole build of 4988 items,
-// 30-bit keys, with the block-wise climb below: 93 -> 61 us.
+// its histograms and its look-back). The line is the block's capacity (8192 items, 63-bit keys: 107 us in
+// all, 8193 by the passes 160); a whole build of 4988 items, 30-bit keys, with the block-wise climb below:
+// 93 -> 59 us. A thread's items are ranked one after another, so short lists have fewer a thread, 2, 5 or 8 (2048
+// items 50.6 us, one more, with 5 a thread, 60.0; 5120 63.6, one more, with 8, 71.8).
 constexpr int SS_THREADS = 1024, SS_WARPS = SS_THREADS / 32, SS_PER = 8;
 constexpr int SS_ITEMS = SS_THREADS * SS_PER;
 template <typename K>
@@ -528,12 +530,13 @@ __global__ void __launch_bounds__(256) lbvh_kernel(const K *__restrict__ codes, 
 // The climb is a chain of exchanges, a level after a level, each a trip through memory. A short list
 // is one such chain long whatever its length, so there a block first joins what meets among its own 512
 // leaves, with the exchange, the boxes and the codes in shared memory; what is left over - a subtree
-// whose sibling reaches out of the block - goes on through memory, from where it was left. A long
-// list has the blocks to cover the trips, and the barrier costs it more than they do: LB_SHARED_TO is
-// the line (whole builds, 30-bit keys, through memory against in blocks: 65k items 118 and 116 us, 202k
-// 137 and 139, 871k 226 and 231, 4M 684 and 702).
+// whose sibling reaches out of the block - goes on through memory, from where it was left. A longer
+// list has the blocks to cover the trips, and the barrier costs it more than they do: lb_shared_to is
+// the line (whole builds of a soup's and a surface's boxes, through memory against in blocks, us. 30-bit keys: 1000
+// items 42.7 / 46.8 and 36.7 / 44.7, 4988 60.0 / 67.9 and 59.9 / 63.2, 8193 93.3 / 101.0 and 95.9 / 101.5, 16384 100.2 /
+// 110.1 and 104.4 / 113.0; 63-bit: 1000 50.0 / 55.3 and 47.0 / 55.6, 4988 81.8 / 87.9 and 89.0 / 89.5).
 constexpr int LB_THREADS = 512;
-constexpr uint32_t LB_SHARED_TO = 1u << 16;
+template <typename K> constexpr uint32_t lb_shared_to() { return sizeof(K) == 4 ? 5120u : 2048u; }
 
 template <typename K>
 __global__ void __launch_bounds__(LB_THREADS) lbvh_block_kernel(const K *__restrict__ codes, const uint32_t *__restrict__ items,
@@ -1263,7 +1266,7 @@ static cudaError_t build_typed(const lrc_build_params &p, const float *d_boxes, 
     if (!ploc) {
         uint32_t *other = reinterpret_cast<uint32_t *>(scratch + L.other);
         if (n > 1) cudaMemsetAsync(other, 0xff, (size_t)(n - 1) * 4, st);
-        if (n <= LB_SHARED_TO)
+        if (n <= lb_shared_to<K>())
             lbvh_block_kernel<K><<<(n + LB_THREADS - 1) / LB_THREADS, LB_THREADS, 0, st>>>(kin, vin, boxes, n, p.node0, p.ref0, p.ref_add, d_nodes, d_aux, other, d_status);
         else
             lbvh_kernel<K><<<blocks, 256, 0, st>>>(kin, vin, boxes, n, p.node0, p.ref0, p.ref_add, d_nodes, d_aux, other, d_status);
