@@ -124,9 +124,9 @@ def parse():
 # DRAM bytes read + written by one launch of the builder line's closest-hit kernel at the default
 # configuration (4M soup triangles, 16M rays, PLOC 30-bit, the walk's tree) and that launch's
 # duration under the profiler: one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum,
-# gpu__time_duration.sum) of the 4th closest_kernel launch in
+# gpu__time_duration.sum) of the 4th wide_query_kernel launch in
 # `python bench.py --workload builder --steps 1 --warmup 3 --no-cpu --e2e-steps 1`
-BUILDER_CLOSEST_DRAM = {"bytes_per_launch": 216.0e9, "ms_per_launch": 127.97}
+BUILDER_CLOSEST_DRAM = {"bytes_per_launch": 22.06e9, "ms_per_launch": 53.96}
 
 
 def config(a, world):
@@ -509,7 +509,7 @@ SERVE_JOBS_PER_STEP = 5      # a serve step: 5 jobs of each rate's stream
 # launch's duration under the profiler: one ncu capture (dram__bytes_read.sum +
 # dram__bytes_write.sum, gpu__time_duration.sum) of launches 81-83 of wf_intersect_kernel in
 # `python bench.py --steps 2 --warmup 3 --rates 200` (the timed stepped run's full-queue passes)
-SERVE_ISECT_DRAM = {"bytes_per_launch": 474.4e6, "ms_per_launch": 3.74}
+SERVE_ISECT_DRAM = {"bytes_per_launch": 460.0e6, "ms_per_launch": 2.53}
 
 
 def serve_jobs(n, rate, seed, nscenes, inst_ids):
@@ -1782,7 +1782,7 @@ def main():
     if (a.n, a.rays, a.builder, a.bits, a.scale, a.walk) == (4 << 20, 16 << 20, "ploc", 30, 1.0, 1):
         dram_gbs = BUILDER_CLOSEST_DRAM["bytes_per_launch"] / (BUILDER_CLOSEST_DRAM["ms_per_launch"] / 1e3) / 1e9
         rl_trace.update({"traffic": BUILDER_CLOSEST_DRAM["bytes_per_launch"],
-                         "traffic_from": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the 4th closest_kernel "
+                         "traffic_from": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the 4th wide_query_kernel "
                                          "launch of `python bench.py --workload builder --steps 1 --warmup 3 --no-cpu "
                                          "--e2e-steps 1`", "dram_gbs": dram_gbs, "frac_dram": dram_gbs / peak})
     rl_trace["frac"] = rl_trace["achieved"] / peak
