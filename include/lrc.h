@@ -327,8 +327,8 @@ typedef struct {
  * height x 4 floats: the sum of the samples' linear RGB and their count, as gpu_view_trace_read
  * gives them, view_gpu.h:118-124). exact = 1 needs spp0 = 0 (the streams start at each pixel's
  * first sample). rays (optional, host): the closest-hit and shadow rays traced.
- * A call of at least LRC_TRACE_WAVEFRONT_PATHS paths side by side (width x rows, in fast mode times
- * spp up to 16; more for depths above 8, or above 4 with instances), or of 2^20 paths, on a scene
+ * A call of at least LRC_TRACE_WAVEFRONT_PATHS paths side by side (width x rows, in fast mode times the
+ * largest power of two up to spp and 16; more for deep images and for several samples), or of 2^20 paths, on a scene
  * without media runs as a one-job batch on the wavefront engine (the batch's image is this call's to
  * the bit); smaller ones, scenes with media, calls captured into a graph and calls with
  * LRC_TRACE_MEGAKERNEL run the one-kernel path. */

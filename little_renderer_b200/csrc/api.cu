@@ -267,24 +267,28 @@ int make_walk(lrc_scene *s) {
 // A large image runs as a one-job batch on the wavefront engine: its kernels keep their own registers
 // (the one-kernel path sits at its cap with every bounce's code in one loop), and its image is the
 // call's to the bit (a batch task traces a pixel's samples as the one-kernel path's lanes do and the
-// resolve pass adds them in that path's order). The line: a pass of the wavefront waits for its longest
-// walk whatever its size, which the one-kernel path does not, and a deeper image has more passes with few
-// paths left. One-kernel path and wavefront at 1 spp, depth 8, scenes of 4k / 20k / 200k triangles: 256 x
-// 256 pixels 0.83 / 1.13 / 1.36 and 1.08 / 1.46 / 1.67 ms, 360 x 360 1.45 / 1.77 / 2.26 and 1.23 / 1.65 /
-// 1.90. Depth 12, 20k / 1M triangles: 320 x 320 1.85 / 2.57 and 2.17 / 3.13, 400 x 400 2.44 / 3.25 and
-// 2.32 / 3.40, 512 x 512 3.54 / 4.78 and 2.63 / 3.97. With instances (8000 triangles each), whose walks are
-// longer: depth 4, 320 x 320 2.60 and 2.41; depth 12, 400 x 400 4.88 and 5.66, 512 x 512 6.83 and 6.34.
-// What counts is the tasks, which run side by side (exact mode has one a pixel, fast mode up to 16); from
-// 2^20 paths on the wavefront whatever their number. Within a caller's capture the one-kernel path, whose
-// launches can be captured (the wavefront's run is a graph of its own).
+// resolve pass adds them in that path's order). What counts is the tasks, which run side by side: a pixel's, in exact
+// mode, or the lanes that share its samples (a power of two up to 16). A pass of the wavefront waits for its longest
+// walk whatever its size, which the one-kernel path does not, and a deeper image has more passes with few paths
+// left; several lanes a pixel make the one-kernel path's warps walk alike. One-kernel path over wavefront, 4k and
+// 200k triangles: one lane a pixel, 98k tasks at depth 4 / 8 / 12: 1.08, 1.05 / 1.01, 0.98 / 0.87, 0.88; 147k at depth
+// 12 1.13, 1.01. 4 or 16 lanes, 98k tasks: 0.90 to 1.08 / 0.87 to 1.02 / 0.72 to 0.87, 147k 1.03 to 1.21 / 1.01 to 1.29 / 0.88 to
+// 1.16, 196k at depth 12 1.02 to 1.32. With instances (2000 to 20000 triangles each): 98k at depth 4 1.04 to 1.16, 147k at
+// depth 8 1.10 to 1.19, 196k at depth 12 1.12 to 1.25. From 2^20 paths on the wavefront whatever the tasks. Within a
+// caller's capture the one-kernel path, whose launches can be captured (the wavefront's run is a graph of its own).
+static uint64_t side_by_side(const lrc_trace_params *p, int32_t rows, uint32_t spp) {
+    uint32_t lanes = 1;
+    while (!p->exact && lanes * 2 <= spp && lanes < 16) lanes *= 2;
+    return (uint64_t)p->width * (uint64_t)rows * lanes;
+}
 bool wavefront_call(const lrc_scene *s, const lrc_trace_params *p, int32_t rows, uint32_t spp) {
     if (s->nvol || rows <= 0 || spp == 0 || capturing(s->ctx->st)) return false;
-    const uint64_t pixels = (uint64_t)p->width * (uint64_t)rows, most = 1u << 20;
-    const int64_t depth = p->max_depth;
-    const uint64_t deeper = s->tlas_n ? 12288u * (uint64_t)std::max<int64_t>(depth - 4, 0)
-                                      : 24576u * (uint64_t)std::max<int64_t>(depth - 8, 0);
-    const uint64_t tasks = pixels * (p->exact ? 1u : std::min<uint32_t>(spp, 16u));
-    return pixels * spp >= most || tasks >= std::min<uint64_t>(LRC_TRACE_WAVEFRONT_PATHS + deeper, most);
+    const uint64_t paths = (uint64_t)p->width * (uint64_t)rows * spp, tasks = side_by_side(p, rows, spp), most = 1u << 20;
+    const uint64_t above4 = (uint64_t)std::max<int64_t>((int64_t)p->max_depth - 4, 0),
+                   above7 = (uint64_t)std::max<int64_t>((int64_t)p->max_depth - 7, 0);
+    const uint64_t more = s->tlas_n ? 12288u * above4
+                          : tasks > (uint64_t)p->width * (uint64_t)rows ? 24576u + 9216u * above4 : 9830u * above7;
+    return paths >= most || tasks >= std::min<uint64_t>(LRC_TRACE_WAVEFRONT_PATHS + more, most);
 }
 
 int trace_wavefront(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows, uint32_t spp0, uint32_t spp,
@@ -305,7 +309,7 @@ int trace_wavefront(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t
     // 640 x 640 pixels at 8 spp of 20k triangles: 2^20 12.4 ms, 2^21 11.9, 2^22 11.2. Up to 2^21 paths the
     // walks run 6 blocks an SM (their registers unspilled: 410k paths 2.65 -> 2.50 ms), with more paths
     // the default's 8 (3.3M paths: 11.55 against 11.19 ms).
-    const uint64_t tasks = (uint64_t)p->width * (uint64_t)rows * (p->exact ? 1u : std::min<uint32_t>(spp, 16u));
+    const uint64_t tasks = side_by_side(p, rows, spp);
     uint32_t slots = 1u << 18;
     while (slots < tasks && slots < (1u << 22)) slots <<= 2;
     const int32_t shape = tasks <= (1u << 21) ? lrc::LRC_WAVEFRONT_SMALL_VARIANT : LRC_WAVEFRONT_DEFAULT_VARIANT;
