@@ -436,7 +436,7 @@ typedef struct lrc_batch lrc_batch;
 #define LRC_BATCH_BUILD 4u    /* build each job's scene first (its builder and key bits; once per scene) */
 #define LRC_BATCH_GRAPH 8u    /* run as one CUDA graph: captured after the first such run (which runs
                                  uncaptured, sizing every buffer), replayed while nothing it names changed
-                                 (the wavefront keeps up to 7 graphs before too, and goes back to them when
+                                 (the wavefront keeps up to 9 graphs before too, and goes back to them when
                                  runs take turns: jobs with instances and without, other sizes) */
 #define LRC_BATCH_ZERO 16u    /* clear each job's band of its image first */
 #define LRC_BATCH_STEPPED 32u /* wavefront: launch each pass's kernels from the host, no graph (slower;

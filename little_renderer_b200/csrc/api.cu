@@ -285,9 +285,9 @@ bool wavefront_call(const lrc_scene *s, const lrc_trace_params *p, int32_t rows,
     if (s->nvol || rows <= 0 || spp == 0 || capturing(s->ctx->st)) return false;
     const uint64_t paths = (uint64_t)p->width * (uint64_t)rows * spp, tasks = side_by_side(p, rows, spp), most = 1u << 20;
     const uint64_t above4 = (uint64_t)std::max<int64_t>((int64_t)p->max_depth - 4, 0),
-                   above7 = (uint64_t)std::max<int64_t>((int64_t)p->max_depth - 7, 0);
+                   above8 = (uint64_t)std::max<int64_t>((int64_t)p->max_depth - 8, 0);
     const uint64_t more = s->tlas_n ? 12288u * above4
-                          : tasks > (uint64_t)p->width * (uint64_t)rows ? 24576u + 9216u * above4 : 9830u * above7;
+                          : tasks > (uint64_t)p->width * (uint64_t)rows ? 24576u + 9216u * above4 : 5000u * above4 + 2300u * above8;
     return paths >= most || tasks >= std::min<uint64_t>(LRC_TRACE_WAVEFRONT_PATHS + more, most);
 }
 
@@ -304,14 +304,14 @@ int trace_wavefront(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t
     cudaError_t e = c->single_ran ? cudaStreamWaitEvent(c->st, c->single_ran, 0)
                                   : cudaEventCreateWithFlags(&c->single_ran, cudaEventDisableTiming);
     if (e) return cuda_status(c, e, "the wavefront's event");
-    // The paths in flight: all of them up to 2^22, in three sizes (a size's graph is captured when it is
-    // first used, and eight are kept): a pass costs most in its longest walks, so there should be few.
-    // 640 x 640 pixels at 8 spp of 20k triangles: 2^20 12.4 ms, 2^21 11.9, 2^22 11.2. Up to 2^21 paths the
-    // walks run 6 blocks an SM (their registers unspilled: 410k paths 2.65 -> 2.50 ms), with more paths
-    // the default's 8 (3.3M paths: 11.55 against 11.19 ms).
+    // The paths in flight: all of them up to 2^22, in powers of two from 2^18 (a size's graph is captured when it is
+    // first used, and ten are kept): a pass costs most in its longest walks, so there should be few, and goes
+    // through all slots, so there should be no more than are used. 640 x 640 pixels at 8 spp of 20k triangles: 2^20 12.4
+    // ms, 2^21 11.9, 2^22 11.2. Up to 2^21 paths the walks run 6 blocks an SM (their registers unspilled: 410k paths
+    // 2.65 -> 2.50 ms), with more paths the default's 8 (3.3M paths: 11.55 against 11.19 ms).
     const uint64_t tasks = side_by_side(p, rows, spp);
     uint32_t slots = 1u << 18;
-    while (slots < tasks && slots < (1u << 22)) slots <<= 2;
+    while (slots < tasks && slots < (1u << 22)) slots <<= 1;
     const int32_t shape = tasks <= (1u << 21) ? lrc::LRC_WAVEFRONT_SMALL_VARIANT : LRC_WAVEFRONT_DEFAULT_VARIANT;
     for (;; slots = 1u << 20) {
         rc = lrc_batch_set_wavefront(c->single, slots, shape);

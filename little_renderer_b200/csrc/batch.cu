@@ -70,7 +70,7 @@ struct lrc_batch {
     std::vector<unsigned char> graph_sig;
     // the wavefront's graphs captured before the current one, the last used first, up to kGraphs with it:
     // runs that take turns between keys (a server's waves with and without instanced jobs, lrc_trace's
-    // four wavefront sizes, each with and without instances) replay them, capturing none again
+    // five wavefront sizes, each with and without instances) replay them, capturing none again
     struct Graph {
         cudaGraph_t graph;
         cudaGraphExec_t exec;
@@ -127,7 +127,7 @@ void drop_graph(lrc_batch *b) {
     b->graph_sig.clear();
 }
 
-constexpr size_t kGraphs = 8;
+constexpr size_t kGraphs = 10;
 
 // the kept graph i dropped
 void drop_kept(lrc_batch *b, size_t i) {

@@ -125,7 +125,7 @@ def test_first_use_in_a_capture_and_on_another_stream(own):
 @pytest.mark.parametrize("world", ["box", "field"])
 @pytest.mark.parametrize("exact", [0, 1])
 @pytest.mark.parametrize("w,h,spp,depth", [(384, 256, 1, 4), (383, 256, 1, 4), (96, 96, 16, 8), (95, 96, 16, 8), (104, 96, 16, 8),
-                                           (103, 96, 16, 8), (104, 96, 40, 8), (512, 288, 1, 12), (512, 287, 1, 12),
+                                           (103, 96, 16, 8), (104, 96, 40, 8), (512, 289, 1, 12), (512, 288, 1, 12),
                                            (512, 384, 1, 12), (512, 383, 1, 12), (320, 256, 3, 8), (256, 256, 16, 3)])
 def test_images_at_the_wavefronts_line(own, world, exact, w, h, spp, depth):
     """lrc_trace on both sides of where it takes the wavefront engine: the one-kernel path's image."""
