@@ -161,12 +161,15 @@ int instances_wide(lrc_scene *s, cudaStream_t st) {
 // image: of 200k 1070 and 920 us, of 4M 2010 and 2800.)
 static double wide_cost(uint32_t n) { return 60.0 + 0.38e-3 * n; }
 // what wide nodes save, us: a query's chain of nodes (about a third of the cost, less with few rays to be the
-// slowest of), and of many rays their instructions; an image's bounces; the guide's rays
+// slowest of), and of many rays their instructions; an image's bounces (128 x 128 pixels of 4k triangles 70, 32 x 32
+// 250); the guide's rays
 double query_saving(const lrc_scene *s, uint64_t rays) {
     const double c = wide_cost(s->built_n), per_ray = 0.125e-3 * std::max(std::log2((double)s->built_n + 1.0) - 10.5, 0.4);
     return c * (0.06 + 0.29 * std::min((double)rays / 1024.0, 1.0)) + per_ray * (double)rays;
 }
-double image_saving(const lrc_scene *s) { return 0.55 * wide_cost(s->built_n) + 200.0; }
+double image_saving(const lrc_scene *s, uint64_t paths) {
+    return (0.55 * wide_cost(s->built_n) + 200.0) * std::min(4096.0 / (double)std::max<uint64_t>(paths, 1), 1.0);
+}
 double guide_saving(const lrc_scene *s) { return 0.08 * wide_cost(s->built_n) + 30.0; }
 
 int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc, double saving) {
@@ -1244,7 +1247,7 @@ int lrc_trace(lrc_scene *s, const lrc_trace_params *p, int32_t y0, int32_t rows,
         return (flags & LRC_DEVICE) ? LRC_OK : check_status(c);
     }
     if (!e && lrc::pt_walks_wide(P, s->nvol != 0)) {
-        int rc = scene_wide(s, c->st, false, image_saving(s));
+        int rc = scene_wide(s, c->st, false, image_saving(s, lrc::pt_paths(P)));
         if (rc) return rc;
     }
     c->timer.begin(LRC_TS_SHADE, c->st);

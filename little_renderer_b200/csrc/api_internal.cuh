@@ -292,7 +292,7 @@ constexpr uint32_t kMostLeaf = 8;
 // (us); they are made once the uses since the build have come to their cost, kAlways at once.
 constexpr double kAlways = 1e30;
 double query_saving(const lrc_scene *s, uint64_t rays);
-double image_saving(const lrc_scene *s);
+double image_saving(const lrc_scene *s, uint64_t paths);
 double guide_saving(const lrc_scene *s);
 int instances_wide(lrc_scene *s, cudaStream_t st);
 int scene_wide(lrc_scene *s, cudaStream_t st, bool no_alloc, double saving = kAlways);

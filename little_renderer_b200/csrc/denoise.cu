@@ -752,7 +752,7 @@ int lrc_reproject_gradients(lrc_scene *s, const lrc_trace_params *old_p, const l
     int rc = scene_traceable(s);
     const size_t N = (size_t)W * H;
     const uint32_t ntiles = grad_tiles(W, H);
-    if (!rc && lrc::pt_gradients_walk_wide(ntiles, s->nvol != 0)) rc = scene_wide(s, c->st, false, image_saving(s));
+    if (!rc && lrc::pt_gradients_walk_wide(ntiles, s->nvol != 0)) rc = scene_wide(s, c->st, false, image_saving(s, ntiles));
     if (rc) return rc;
     const float4 *d_old = reinterpret_cast<const float4 *>(old_planes);
     float4 *d_new = reinterpret_cast<float4 *>(new_planes);
@@ -839,7 +839,7 @@ int lrc_trace_frame(lrc_scene *s, const lrc_trace_params *old_p, const lrc_trace
     const bool edit = (flags & LRC_REPROJECT_EDIT) != 0;
     // (the guide walks wide nodes, and the trace: the wavefront's, or a small image's)
     const bool walked = lrc::pt_walks_wide(P, s->nvol != 0) || (grads && lrc::pt_gradients_walk_wide(ntiles, s->nvol != 0));
-    rc = scene_wide(s, c->st, false, wavefront_call(s, new_p, H, spp) ? kAlways : guide_saving(s) + (walked ? image_saving(s) : 0.0));
+    rc = scene_wide(s, c->st, false, wavefront_call(s, new_p, H, spp) ? kAlways : guide_saving(s) + (walked ? image_saving(s, std::min<uint64_t>(lrc::pt_paths(P), ntiles)) : 0.0));
     if (rc) return rc;
     c->timer.begin(LRC_TS_SHADE, c->st);
     e = lrc::dn_guide(pt_scene(s), P, d_new, c->d_status, c->st);

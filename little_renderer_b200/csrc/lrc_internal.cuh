@@ -297,6 +297,7 @@ cudaError_t pt_gradients(const PtScene &S, const PtParams &P, GradTile *d_tiles,
                          unsigned long long *d_rays, uint32_t *d_status, cudaStream_t st);
 cudaError_t pt_prim_boxes(const float *d_prims, uint32_t n, float *d_boxes, cudaStream_t st);
 // whether pt_trace's (pt_gradients') kernel for these walks the world's wide nodes, if the scene has them
+uint64_t pt_paths(const PtParams &P);         // the paths (lanes) of pt_trace's launch
 bool pt_walks_wide(const PtParams &P, bool media);
 bool pt_gradients_walk_wide(uint32_t ntiles, bool media);
 cudaError_t pt_trace(const PtScene &S, const PtParams &P, float *d_accum, unsigned long long *d_rays, uint32_t *d_status,

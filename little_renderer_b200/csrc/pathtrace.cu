@@ -386,7 +386,7 @@ cudaError_t pt_prim_boxes(const float *d_prims, uint32_t n, float *d_boxes, cuda
     return cudaGetLastError();
 }
 
-static uint64_t pt_paths(const PtParams &P) { return (uint64_t)P.W * P.rows * (P.exact ? 1 : P.group); }
+uint64_t pt_paths(const PtParams &P) { return (uint64_t)P.W * P.rows * (P.exact ? 1 : P.group); }
 
 bool pt_walks_wide(const PtParams &P, bool media) { return !media && pt_paths(P) <= pt::PT_WARP_PATHS; }
 bool pt_gradients_walk_wide(uint32_t ntiles, bool media) { return !media && ntiles <= pt::PT_WARP_PATHS; }
